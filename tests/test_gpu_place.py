@@ -160,3 +160,66 @@ def test_feather_blend_and_keep(dev, present, oo, on):
     assert np.array_equal(zs.download(), e3[S:].ravel())
     assert np.array_equal(ys.download(), e3[:S, S:, :].ravel())
     assert np.array_equal(xs.download(), e3[:S, :S, S:].ravel())
+
+
+@pytest.mark.parametrize("S,B,oo,on", [(21, 5, (0, 0, 0), (21, 21, 21)), (24, 8, (3, 0, 9), (21, 24, 15)), (9, 9, (0, 2, 1), (9, 7, 8)), (1040, 2, (1, 0, 0), (2, 3, 1040))])
+def test_feather_parts_at_ragged_sizes(dev, S, B, oo, on):
+    """the blend's parts where rows are unaligned, where the shell is the whole window, and where a row has more groups than a block has threads;
+    the kept slabs of a window whose rows are not whole words"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf, Feather
+    L = ufsm_b200.lib()
+    if S > 1000:                                      # one thin box of a long row: planes beyond the ones it reads are not needed
+        E, planes = S + B, oo[0] + on[0]
+        g = synth.rng(331)
+        e = g.integers(0, 256, planes * E * E, dtype=np.uint8)
+        ed, xd = DevBuf(data=e), DevBuf(data=g.integers(0, 256, planes * S * B, dtype=np.uint8))
+        od = DevBuf(on[0] * S * S).fill(0xEE)
+        f = Feather()
+        f.S, f.B, f.e, f.osh, f.out = S, B, ed.ptr, S, od.ptr
+        f.nb[1] = xd.ptr
+        for k in range(3):
+            f.oo[k], f.on[k] = oo[k], on[k]
+        assert L.umx_feather_blend(C.byref(f)) == 0
+        ufsm_b200.check()
+        got = od.download().reshape(on[0], S, S)[:, 2:3, :]          # the row y = 2 is past the y shell; z = 2 past the z shell
+        want = e.reshape(planes, E, E)[2, 2, B:S]
+        assert np.array_equal(got[1, 0, B:], want)
+        return
+    E, osh = S + B, S + 3
+    g = synth.rng(332)
+    e = g.integers(0, 256, E ** 3, dtype=np.uint8)
+    nb = [None] + [g.integers(0, 256, B * E * E if d & 4 else S * B * E if d & 2 else S * S * B, dtype=np.uint8) for d in range(1, 8)]
+    want = orc.feather_blend(e, nb, S, B, oo, on, osh, np.full(osh ** 3, 0xEE, np.uint8))
+    ed, od, bufs = DevBuf(data=e), DevBuf(osh ** 3).fill(0xEE), [DevBuf(data=v) if v is not None else None for v in nb]
+    f = Feather()
+    f.S, f.B, f.e, f.osh, f.out = S, B, ed.ptr, osh, od.ptr
+    for d in range(1, 8):
+        f.nb[d] = bufs[d].ptr
+    for k in range(3):
+        f.oo[k], f.on[k] = oo[k], on[k]
+    assert L.umx_feather_blend(C.byref(f)) == 0
+    zs, ys, xs = DevBuf(B * E * E).fill(0), DevBuf(S * B * E).fill(0), DevBuf(S * S * B).fill(0)
+    L.umx_feather_keep(ed.ptr, S, B, zs.ptr, ys.ptr, xs.ptr)
+    ufsm_b200.check()
+    assert np.array_equal(od.download(), want)
+    e3 = e.reshape(E, E, E)
+    assert np.array_equal(zs.download(), e3[S:].ravel()) and np.array_equal(ys.download(), e3[:S, S:].ravel()) and np.array_equal(xs.download(), e3[:S, :S, S:].ravel())
+
+
+@pytest.mark.parametrize("W,nz,bits", [(33, 3, 8), (45, 50, 4), (7, 2, 8)])
+def test_pred_input_ragged_planes(dev, W, nz, bits):
+    """planes that are not a whole number of warps' runs, rows shorter than a warp, more planes than groups of planes"""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    L = ufsm_b200.lib()
+    g = synth.rng(341)
+    ct, dyo, dxo = synth.ct_u8(342, (nz + 1) * W * W), (g.standard_normal(nz + 1) * 3 - 8).astype(np.float32), (g.standard_normal(nz + 1) * 3 - 7).astype(np.float32)
+    vals = orc.pred_input(ct, W, np.float32(110), np.float32(1 / 40), dyo, dxo, -1, 1, nz, 2)
+    want = orc.pm_to_mx(vals, 0, 1, 4, nz * W * W, bits)
+    bufs = [DevBuf(data=v) for v in (ct, dyo, dxo)]
+    yd = DevBuf(want.size).fill(0xEE)
+    L.lp_pred_input_mx(bufs[0].ptr, W, 110.0, 1 / 40, bufs[1].ptr, bufs[2].ptr, -1, 1, nz, yd.ptr, 2, bits)
+    ufsm_b200.check()
+    assert np.array_equal(yd.download(), want)

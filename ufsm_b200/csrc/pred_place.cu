@@ -5,8 +5,8 @@
 
    Geometry (place_isect of the reference): window voxel (z, y, x) sits at shard coordinate (oz + z, oy + y, ox + x); it is written when
    it is interior (z in [hz, D - hz), y and x in [halo, W - halo)) and inside the shard's extent ([0, ez) x [0, ey) x [0, ex)).  The box of
-   such voxels is worked out on the host and a thread takes four consecutive x of one box row, so a warp reads and writes runs of 128
-   voxels of a row. */
+   such voxels is worked out on the host and a thread takes eight consecutive x of one box row, so a warp reads and writes runs of 256
+   voxels of a row or of neighbouring rows. */
 #include "mx_common.cuh"
 
 namespace {
@@ -19,41 +19,70 @@ PlaceBox place_box_of(int D, int W, int hz, int halo, int oz, int oy, int ox, in
     b.nz = z1 > b.z0 ? z1 - b.z0 : 0; b.ny = y1 > b.y0 ? y1 - b.y0 : 0; b.nx = x1 > b.x0 ? x1 - b.x0 : 0;
     return b;
 }
-__device__ __forceinline__ unsigned prob255(float l) { return (unsigned)(__fdividef(255.f, 1.f + __expf(-l)) + 0.5f) & 0xffu; }
+/* trunc(255 / (1 + exp(-l)) + 0.5), a NaN as 0; the truncation as an addition of 2^23 rounded down, which keeps the conversion unit free for the
+   two approximations */
+__device__ __forceinline__ unsigned prob255(float l) { return __float_as_uint(__fadd_rd(fmaxf(__fdividef(255.f, 1.f + __expf(-l)) + 0.5f, 0.f), 8388608.f)) & 0xffu; }
 template <typename LT> __device__ __forceinline__ float logit_at(const LT *lg, size_t k);
 template <> __device__ __forceinline__ float logit_at<float>(const float *lg, size_t k) { return __ldg(lg + k); }
 template <> __device__ __forceinline__ float logit_at<__half>(const __half *lg, size_t k) { return __half2float(__ldg(lg + k)); }
 
-/* MASK 0: material where ct[k] >= iso; 1: where bit k of `bits` is set.  zoff: the window is held from its plane zoff on (a half of a split window) */
+/* MASK 0: material where ct[k] >= iso; 1: where bit k of `bits` is set.  zoff: the window is held from its plane zoff on (a half of a split window).
+   A block takes R = 256 / nq whole rows of the box at a time (nq groups of eight x a row), so a thread works out its place once and needs
+   one 32-bit division a trip; eight voxels go with one load of their logits, one of their mask bits and one store where these are aligned.
+   Bound by latency and issue: 160^3 of a 192^3 window 12.4 us with 64-bit index divisions every four voxels, 7.6 us in this form. */
 template <typename LT, int MASK>
 __global__ void __launch_bounds__(256) pred_place_k(const LT *__restrict__ lg, const uint8_t *__restrict__ ct, const uint32_t *__restrict__ bits, PlaceBox B, int W, int zoff,
                                                     int oz, int oy, int ox, int shard, uint8_t *__restrict__ dsh, int iso) {
-    const int nq = (B.nx + 3) >> 2;                         /* groups of four x a row */
-    const size_t total = (size_t)B.nz * B.ny * nq;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int q = (int)(i % nq), y = B.y0 + (int)((i / nq) % B.ny), z = B.z0 + (int)(i / ((size_t)nq * B.ny));
-        const int xa = B.x0 + 4 * q, n = min(4, B.x0 + B.nx - xa);
-        const size_t k = ((size_t)(z - zoff) * W + y) * W + xa;
-        uint8_t *o = dsh + ((size_t)(oz + z) * shard + (oy + y)) * shard + (ox + xa);
-        unsigned v[4];
+    pdl_trigger(); pdl_wait();
+    const int nq = (B.nx + 7) >> 3, R = nq < 256 ? 256 / nq : 1, tr = (int)threadIdx.x / nq;
+    const unsigned rows = (unsigned)B.nz * (unsigned)B.ny;
+    if (R > 1 && tr >= R) return;
+    for (unsigned row = blockIdx.x * (unsigned)R + (R > 1 ? tr : 0); row < rows; row += gridDim.x * (unsigned)R) {
+        const int zz = (int)(row / (unsigned)B.ny), y = B.y0 + (int)(row - (unsigned)zz * (unsigned)B.ny), z = B.z0 + zz;
+        const size_t kr = ((size_t)(z - zoff) * W + y) * W;
+        uint8_t *orow = dsh + ((size_t)(oz + z) * shard + (oy + y)) * shard + ox;
+        for (int q = R > 1 ? (int)threadIdx.x - tr * nq : (int)threadIdx.x; q < nq; q += 256) {
+            const int xa = B.x0 + 8 * q, n = min(8, B.x0 + B.nx - xa);
+            const size_t k = kr + xa;
+            uint8_t *o = orow + xa;
+            float l[8]; unsigned on = 0u;
+            if (n == 8 && !((size_t)(lg + k) & 15)) {
+                if (sizeof(LT) == 2) {
+                    const uint4 r = __ldg((const uint4 *)(lg + k)); const __half2 *h = (const __half2 *)&r;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            v[j] = 0u;
-            if (j < n) {
-                const bool on = MASK ? (__ldg(bits + ((k + j) >> 5)) >> ((k + j) & 31)) & 1u : (int)__ldg(ct + k + j) >= iso;
-                if (on) v[j] = prob255(logit_at<LT>(lg, k + j));
+                    for (int j = 0; j < 4; j++) { const float2 f = __half22float2(h[j]); l[2 * j] = f.x; l[2 * j + 1] = f.y; }
+                } else {
+                    const float4 r = __ldg((const float4 *)(lg + k)), t = __ldg((const float4 *)(lg + k) + 1);
+                    l[0] = r.x; l[1] = r.y; l[2] = r.z; l[3] = r.w; l[4] = t.x; l[5] = t.y; l[6] = t.z; l[7] = t.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j++) l[j] = j < n ? logit_at<LT>(lg, k + j) : 0.f;
             }
+            if (MASK) {
+                const unsigned sh = (unsigned)(k & 31);
+                on = __ldg(bits + (k >> 5)) >> sh;
+                if (sh + n > 32) on |= __ldg(bits + (k >> 5) + 1) << (32 - sh);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j++) if (j < n && (int)__ldg(ct + k + j) >= iso) on |= 1u << j;
+            }
+            unsigned v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) { const unsigned t = prob255(l[j]); v[j] = (on >> j) & 1u ? t : 0u; }
+            if (n == 8 && !((size_t)o & 7)) *(uint2 *)o = make_uint2(v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24), v[4] | (v[5] << 8) | (v[6] << 16) | (v[7] << 24));
+            else for (int j = 0; j < n; j++) o[j] = (uint8_t)v[j];
         }
-        if (n == 4 && !((size_t)o & 3)) *(uint32_t *)o = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
-        else for (int j = 0; j < n; j++) o[j] = (uint8_t)v[j];
     }
 }
 __global__ void __launch_bounds__(256) pred_out_k(const void *lg, int h16, const uint8_t *__restrict__ ct, size_t n, uint8_t *__restrict__ out) {
+    pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = __ldg(ct + i) ? (uint8_t)prob255(h16 ? logit_at<__half>((const __half *)lg, i) : logit_at<float>((const float *)lg, i)) : (uint8_t)0;
 }
 /* one 32-voxel word a thread: two 16-byte loads where the bytes are there and aligned, byte compares four at a time */
 __global__ void __launch_bounds__(256) ctmask_k(const uint8_t *__restrict__ ct, size_t n, uint32_t *__restrict__ bits, int t) {
+    pdl_trigger(); pdl_wait();
     const size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x, i0 = w * 32;
     if (i0 >= n) return;
     uint32_t m = 0;
@@ -78,44 +107,106 @@ __global__ void __launch_bounds__(256) ctmask_k(const uint8_t *__restrict__ ct, 
    A neighbour's spill is its z slab [B][E][E] when it lies a window back in z, else its y slab [S][B][E] when back in y, else its x slab
    [S][S][B] (fe_val).  fp32 products and sums in the reference's order, without contraction. */
 struct FeatherArgs { int S, B, E, osh; int oo[3], on[3]; const uint8_t *e; const uint8_t *nb[8]; const float *u; uint8_t *out; };
-__device__ __forceinline__ float fe_val(const FeatherArgs &f, int d, int z, int y, int x) {
-    if (!d) return (float)__ldg(f.e + ((size_t)z * f.E + y) * f.E + x);
+/* the row (z, y) of window d's spill, addressed with this window's x: byte x of the row is its value at (z, y, x) */
+__device__ __forceinline__ const uint8_t *fe_row(const FeatherArgs &f, int d, int z, int y) {
+    if (!d) return f.e + ((size_t)z * f.E + y) * f.E;
     const uint8_t *p = f.nb[d];
-    const int uz = z + ((d & 4) ? f.S : 0), uy = y + ((d & 2) ? f.S : 0), ux = x + ((d & 1) ? f.S : 0);
-    if (uz >= f.S) return (float)__ldg(p + ((size_t)(uz - f.S) * f.E + uy) * f.E + ux);
-    if (uy >= f.S) return (float)__ldg(p + ((size_t)uz * f.B + (uy - f.S)) * f.E + ux);
-    return (float)__ldg(p + ((size_t)uz * f.S + uy) * f.B + (ux - f.S));
+    const int uy = y + ((d & 2) ? f.S : 0), ux = (d & 1) ? f.S : 0;
+    if (d & 4) return p + ((size_t)z * f.E + uy) * f.E + ux;
+    if (d & 2) return p + ((size_t)z * f.B + y) * f.E + ux;
+    return p + ((size_t)z * f.S + y) * f.B;
 }
-__global__ void __launch_bounds__(256) feather_k(const FeatherArgs f) {
-    const size_t total = (size_t)f.on[0] * f.on[1] * f.on[2];
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int lx = (int)(i % f.on[2]), ly = (int)((i / f.on[2]) % f.on[1]), lz = (int)(i / ((size_t)f.on[2] * f.on[1]));
-        const int z = f.oo[0] + lz, y = f.oo[1] + ly, x = f.oo[2] + lx, B = f.B;
-        unsigned v;
-        if (z >= B && y >= B && x >= B) v = __ldg(f.e + ((size_t)z * f.E + y) * f.E + x);
-        else {
-            float s = 0.f, w = 0.f;
-            for (int d = 0; d < 8; d++) {
-                if (d && !f.nb[d]) continue;
-                const int dz = d >> 2 & 1, dy = d >> 1 & 1, dx = d & 1;
-                if ((dz && z >= B) || (dy && y >= B) || (dx && x >= B)) continue;
-                const float wi = __fmul_rn(__fmul_rn(z < B ? __ldg(f.u + dz * B + z) : 1.f, y < B ? __ldg(f.u + dy * B + y) : 1.f), x < B ? __ldg(f.u + dx * B + x) : 1.f);
-                s = __fadd_rn(s, __fmul_rn(wi, fe_val(f, d, z, y, x)));
-                w = __fadd_rn(w, wi);
-            }
-            v = w > 0.f ? (unsigned)fminf(255.f, __fadd_rn(__fdiv_rn(s, w), 0.5f)) : 0u;
+/* four bytes of a row from x on (n of them real) */
+__device__ __forceinline__ unsigned fe_four(const uint8_t *r, int x, int n) {
+    const uint8_t *p = r + x;
+    if (n == 4 && !((size_t)p & 3)) return __ldg((const uint32_t *)p);
+    unsigned v = 0u;
+    for (int j = 0; j < n; j++) v |= (unsigned)__ldg(p + j) << (8 * j);
+    return v;
+}
+/* The output box in up to eight parts by which axes lie in the lower shell (bit 0 x, 1 y, 2 z), so that the windows that reach a voxel are the
+   part's subsets and every warp runs the sum its part needs and no more.  Blocks [first, next first) of the grid work on a part. */
+struct FeatherPart { int z0, y0, x0, nz, ny, nx; unsigned first; };
+struct FeatherParts { FeatherPart p[8]; };
+/* byte j of v as a float (2^23 + byte, minus 2^23: no conversion unit) */
+__device__ __forceinline__ float byte_f(unsigned v, int j) { return __fsub_rn(__uint_as_float(__byte_perm(v, 0x4b000000u, 0x7440u | j)), 8388608.f); }
+/* the four bytes of part M at (z, y, x .. x + n): the weighted mean over the windows d within M that are present, in ascending d */
+template <int M> __device__ __forceinline__ unsigned fe_mean(const FeatherArgs &f, int z, int y, int x, int n) {
+    const unsigned own = fe_four(fe_row(f, 0, z, y), x, n);
+    if (M == 0) return own;
+    const int B = f.B;
+    unsigned b[8]; bool have[8];
+#pragma unroll
+    for (int d = 0; d < 8; d++) {
+        have[d] = d == 0; b[d] = own;
+        if (d && (d & ~M) == 0) { have[d] = f.nb[d] != nullptr; if (have[d]) b[d] = fe_four(fe_row(f, d, z, y), x, n); }
+    }
+    float wz[2] = {1.f, 1.f}, wy[2] = {1.f, 1.f};
+#pragma unroll
+    for (int k = 0; k < 2; k++) { if (M & 4) wz[k] = __ldg(f.u + k * B + z); if (M & 2) wy[k] = __ldg(f.u + k * B + y); }
+    unsigned v = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        float wx[2] = {1.f, 1.f};
+        if ((M & 1) && j < n) { wx[0] = __ldg(f.u + x + j); wx[1] = __ldg(f.u + B + x + j); }
+        float s = 0.f, w = 0.f;
+#pragma unroll
+        for (int d = 0; d < 8; d++) {
+            if ((d & ~M) || !have[d]) continue;
+            const float wi = __fmul_rn(__fmul_rn(wz[d >> 2], wy[(d >> 1) & 1]), wx[d & 1]);
+            s = __fadd_rn(s, __fmul_rn(wi, byte_f(b[d], j)));
+            w = __fadd_rn(w, wi);
         }
-        f.out[((size_t)lz * f.osh + ly) * f.osh + lx] = (uint8_t)v;
+        v |= (w > 0.f ? (unsigned)fminf(255.f, __fadd_rn(__fdiv_rn(s, w), 0.5f)) : 0u) << (8 * j);
+    }
+    return v;
+}
+template <int M> __device__ __forceinline__ void fe_part(const FeatherArgs &f, const FeatherPart &pt, unsigned nblk) {
+    const int nq = (pt.nx + 3) >> 2, R = nq < 256 ? 256 / nq : 1, tr = (int)threadIdx.x / nq;
+    const unsigned rows = (unsigned)pt.nz * (unsigned)pt.ny;
+    if (R > 1 && tr >= R) return;
+    for (unsigned row = (blockIdx.x - pt.first) * (unsigned)R + (R > 1 ? tr : 0); row < rows; row += nblk * (unsigned)R) {
+        const int rz = (int)(row / (unsigned)pt.ny), z = pt.z0 + rz, y = pt.y0 + (int)(row - (unsigned)rz * (unsigned)pt.ny);
+        for (int q = R > 1 ? (int)threadIdx.x - tr * nq : (int)threadIdx.x; q < nq; q += 256) {
+            const int x = pt.x0 + 4 * q, n = min(4, pt.nx - 4 * q);
+            uint8_t *o = f.out + ((size_t)(z - f.oo[0]) * f.osh + (y - f.oo[1])) * f.osh + (x - f.oo[2]);
+            const unsigned v = fe_mean<M>(f, z, y, x, n);
+            if (n == 4 && !((size_t)o & 3)) *(uint32_t *)o = v;
+            else for (int j = 0; j < n; j++) o[j] = (uint8_t)(v >> (8 * j));
+        }
     }
 }
-/* a window's upper slabs, kept for the windows after it (feather_keep, src/predict.c:362-376) */
-__global__ void __launch_bounds__(256) feather_keep_k(const uint8_t *__restrict__ e, int S, int B, uint8_t *__restrict__ zs, uint8_t *__restrict__ ys, uint8_t *__restrict__ xs) {
-    const int E = S + B;
-    const size_t nz = (size_t)B * E * E, ny = (size_t)S * B * E, nx = (size_t)S * S * B;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nz + ny + nx; i += (size_t)gridDim.x * blockDim.x) {
-        if (i < nz) zs[i] = e[(size_t)S * E * E + i];
-        else if (i < nz + ny) { const size_t k = i - nz; const int x = (int)(k % E), y = (int)((k / E) % B), z = (int)(k / ((size_t)E * B)); ys[k] = e[((size_t)z * E + S + y) * E + x]; }
-        else { const size_t k = i - nz - ny; const int x = (int)(k % B), y = (int)((k / B) % S), z = (int)(k / ((size_t)B * S)); xs[k] = e[((size_t)z * E + y) * E + S + x]; }
+/* A thread takes four x of a row of its part (a block R = 256 / nq whole rows of nq such groups); their bytes come as one word a window where rows
+   are aligned, all loads ahead of the sums.  Bound by instruction issue in the shell: 144^3 with seven neighbours 24.5 us at one thread and
+   three 64-bit divisions a voxel with the eight windows tested for each, 9.7 us in this form. */
+__global__ void __launch_bounds__(256) feather_k(const FeatherArgs f, const FeatherParts parts) {
+    pdl_trigger(); pdl_wait();
+    int pi = 0;
+#pragma unroll
+    for (int k = 1; k < 8; k++) if (blockIdx.x >= parts.p[k].first) pi = k;
+    const FeatherPart pt = parts.p[pi];
+    const unsigned nblk = (pi < 7 ? parts.p[pi + 1].first : gridDim.x) - pt.first;
+    switch (7 - pi) {                                         /* the shell first: its blocks take longest */
+    case 0: fe_part<0>(f, pt, nblk); break;
+    case 1: fe_part<1>(f, pt, nblk); break;
+    case 2: fe_part<2>(f, pt, nblk); break;
+    case 3: fe_part<3>(f, pt, nblk); break;
+    case 4: fe_part<4>(f, pt, nblk); break;
+    case 5: fe_part<5>(f, pt, nblk); break;
+    case 6: fe_part<6>(f, pt, nblk); break;
+    default: fe_part<7>(f, pt, nblk); break;
+    }
+}
+/* a window's upper slabs, kept for the windows after it (feather_keep, src/predict.c:362-376): one T (byte or four-byte word) a thread, indices of type I */
+template <typename T, typename I>
+__global__ void __launch_bounds__(256) feather_keep_k(const T *__restrict__ e, I S, I B, I SX, I BX, T *__restrict__ zs, T *__restrict__ ys, T *__restrict__ xs) {
+    pdl_trigger(); pdl_wait();
+    /* S, B, E in voxels; SX, BX, EX along x in units of T */
+    const I E = S + B, EX = SX + BX, nz = B * E * EX, ny = S * B * EX, nx = S * S * BX;
+    for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < nz + ny + nx; i += (I)gridDim.x * blockDim.x) {
+        if (i < nz) zs[i] = __ldg(e + S * E * EX + i);
+        else if (i < nz + ny) { const I k = i - nz, r = k / EX, x = k - r * EX, z = r / B, y = r - z * B; ys[k] = __ldg(e + (z * E + S + y) * EX + x); }
+        else { const I k = i - nz - ny, r = k / BX, x = k - r * BX, z = r / S, y = r - z * S; xs[k] = __ldg(e + (z * E + y) * EX + SX + x); }
     }
 }
 
@@ -126,8 +217,9 @@ unsigned grid_of(size_t n) { const size_t g = (n + 255) / 256; return (unsigned)
 template <int MASK>
 void place(const char *fn, const void *lg, const uint8_t *ct, const uint32_t *bits, PlaceBox B, int W, int zoff, int oz, int oy, int ox, int shard, uint8_t *dsh) {
     if (!umx_ready(fn)) return;
-    const size_t n = (size_t)B.nz * B.ny * ((B.nx + 3) >> 2);
+    const size_t n = (size_t)B.nz * B.ny * ((B.nx + 7) >> 3);
     if (!n) return;
+    if ((size_t)B.nz * B.ny >= (size_t)1 << 31) { fprintf(stderr, "%s: 2^31 rows or more\n", fn); abort(); }
     const int d = cur_dev(), iso = g_iso[d] < 1 ? 1 : g_iso[d];
     if (g_logits_h16[d]) umx_launch(pred_place_k<__half, MASK>, dim3(grid_of(n)), dim3(256), 0, (const __half *)lg, ct, bits, B, W, zoff, oz, oy, ox, shard, dsh, iso);
     else umx_launch(pred_place_k<float, MASK>, dim3(grid_of(n)), dim3(256), 0, (const float *)lg, ct, bits, B, W, zoff, oz, oy, ox, shard, dsh, iso);
@@ -160,7 +252,7 @@ extern "C" void nn_pred_place(const float *lg, const uint8_t *ct, int W, int hal
 extern "C" void nn_pred_ctmask_t(const uint8_t *ct, size_t n, uint32_t *bits, int t) {
     if (!umx_ready("nn_pred_ctmask") || !n) return;
     const size_t words = (n + 31) / 32;
-    ctmask_k<<<(unsigned)((words + 255) / 256), 256>>>(ct, n, bits, t < 1 ? 1 : t > 255 ? 256 : t);
+    umx_launch(ctmask_k, dim3((unsigned)((words + 255) / 256)), dim3(256), 0, ct, n, bits, t < 1 ? 1 : t > 255 ? 256 : t);
     g_umx_launches++;
     UMX_CK("nn_pred_ctmask");
 }
@@ -207,15 +299,34 @@ extern "C" int umx_feather_blend(const umx_feather_t *h) {
     for (int d = 1; d < 8; d++) f.nb[d] = h->nb[d];
     const size_t n = (size_t)f.on[0] * f.on[1] * f.on[2];
     if (!n) return 0;
-    feather_k<<<grid_of(n), 256>>>(f);
+    if ((size_t)f.on[0] * f.on[1] >= (size_t)1 << 31) { umx_latch_msg("umx_feather_blend: 2^31 rows or more"); return -1; }
+    FeatherParts parts; memset(&parts, 0, sizeof parts);
+    int lo[3]; unsigned blocks = 0;
+    for (int d = 0; d < 3; d++) lo[d] = f.oo[d] < h->B ? (h->B < f.oo[d] + f.on[d] ? h->B - f.oo[d] : f.on[d]) : 0;      /* voxels of the box below B, per axis */
+    for (int k = 0; k < 8; k++) {
+        FeatherPart &pt = parts.p[k];
+        const int m = 7 - k, bit[3] = {m >> 2 & 1, m >> 1 & 1, m & 1};
+        int o[3], n[3];
+        for (int d = 0; d < 3; d++) { o[d] = bit[d] ? f.oo[d] : f.oo[d] + lo[d]; n[d] = bit[d] ? lo[d] : f.on[d] - lo[d]; }
+        pt = {o[0], o[1], o[2], n[0], n[1], n[2], blocks};
+        const size_t rows = (size_t)n[0] * n[1];
+        if (!rows || !n[2]) continue;                          /* an empty part gets no block */
+        const size_t nq = ((size_t)n[2] + 3) >> 2, per = nq < 256 ? 256 / nq : 1, g = (rows + per - 1) / per;
+        blocks += (unsigned)(g < 148 * 32 ? g : 148 * 32);
+    }
+    umx_launch(feather_k, dim3(blocks), dim3(256), 0, f, parts);
     g_umx_launches++;
     UMX_CK("umx_feather_blend");
     return 0;
 }
 extern "C" void umx_feather_keep(const uint8_t *e, int S, int B, uint8_t *zslab, uint8_t *yslab, uint8_t *xslab) {
     if (!umx_ready("umx_feather_keep") || S < 1 || B < 1) return;
-    const int E = S + B;
-    feather_keep_k<<<grid_of((size_t)B * E * E + (size_t)S * B * E + (size_t)S * S * B), 256>>>(e, S, B, zslab, yslab, xslab);
+    const size_t E = (size_t)S + B, n = B * E * E + (size_t)S * B * E + (size_t)S * S * B;
+    /* words where every row starts on one; 32-bit indices while the window has fewer than 2^32 bytes */
+    const bool words = !((S | B) & 3) && !(((size_t)e | (size_t)zslab | (size_t)yslab | (size_t)xslab) & 3);
+    if (E * E * E >= (size_t)1 << 32) umx_launch(feather_keep_k<uint8_t, size_t>, dim3(grid_of(n)), dim3(256), 0, e, S, B, S, B, zslab, yslab, xslab);
+    else if (words) umx_launch(feather_keep_k<uint32_t, unsigned>, dim3(grid_of(n / 4)), dim3(256), 0, (const uint32_t *)e, S, B, S / 4, B / 4, (uint32_t *)zslab, (uint32_t *)yslab, (uint32_t *)xslab);
+    else umx_launch(feather_keep_k<uint8_t, unsigned>, dim3(grid_of(n)), dim3(256), 0, e, S, B, S, B, zslab, yslab, xslab);
     g_umx_launches++;
     UMX_CK("umx_feather_keep");
 }
