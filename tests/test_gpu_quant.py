@@ -137,3 +137,21 @@ def test_gn_sums_mx_non_finite(dev):
     ufsm_b200.check()
     got = _slots(sd.download())
     assert np.isnan(got[0]) and np.isnan(got[1]) and np.isfinite(got[2]) and np.isfinite(got[3])
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N,Cn,S", [(1, 32, 2), (2, 96, 254), (1, 64, 258), (1, 32, 131)])
+def test_h16_pairs_of_voxels(dev, bits, N, Cn, S):
+    """whole blocks of fp16: two voxels a thread (even S) or one (odd S), rows of every magnitude beside each other (a pair with one row outside the
+    range of the packed path), subnormals, infinities and NaN, both layouts; and back"""
+    r = synth.rng(77)
+    mag = np.exp2(r.integers(-26, 17, (N, 1, S)).astype(np.float64))
+    with np.errstate(over="ignore"):
+        x = (r.standard_normal((N, Cn, S)) * mag).astype(np.float16)
+    if S > 100:
+        x[0, 3, 5], x[0, 4, 6], x[0, 5, 9] = np.nan, np.inf, -np.inf
+    x = np.ascontiguousarray(x).ravel()
+    want = orc.pm_to_mx(x, 2, N, Cn, S, bits, 32)
+    assert np.array_equal(G.quantise_pm(x, 2, N, Cn, S, bits, wide32=True), want)
+    assert np.array_equal(G.from_split(G.quantise_pm(x, 2, N, Cn, S, bits, wide32=True, layout=1), N, Cn, S, bits), want)
+    assert np.array_equal(G.dequantise(want, bits, N, Cn, S), orc.mx_to_pm(want, bits, N, Cn, S), equal_nan=True)

@@ -23,6 +23,9 @@ void umx_prof_close(int id);
    likes to let its own successor be scheduled.  What is gained is the launch latency (and, in the conv kernels, the prologue: barrier
    set-up, TMEM allocation, weight loads) of some 80 dependent launches per forward.  UMX_PDL=0 in the environment turns it off. ---- */
 int umx_pdl(void);
+/* > 0 while the next launches must wait for everything before them in the stream (a conv whose weight images were prepared just ahead of it
+   reads them before its pdl_wait) */
+extern thread_local int umx_plain_launch;
 #ifdef __CUDACC__
 #include <string.h>
 template <typename... KA, typename... A>
@@ -31,7 +34,7 @@ static inline void umx_launch(void (*kern)(KA...), dim3 grid, dim3 block, size_t
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = 0;
     cudaLaunchAttribute at[1]; memset(at, 0, sizeof at);
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
-    if (umx_pdl()) { cfg.attrs = at; cfg.numAttrs = 1; }
+    if (umx_pdl() && !umx_plain_launch) { cfg.attrs = at; cfg.numAttrs = 1; }
     cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
 }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -48,6 +51,18 @@ __device__ __forceinline__ int mx_exp(float amax, float inv_qmax) {
     return max(1, min(253, eb)) - 127;
 }
 __device__ __forceinline__ float exp2i(int e) { return __uint_as_float((unsigned)(127 + e) << 23); }
+/* the same as scale byte and factor: sb = e + 127 (0xFF for inf / NaN) and m = 2^-e (-inf there, which is what exp2i(-128) gives); amax without a sign */
+struct mx_sb { unsigned sb; float m; };
+__device__ __forceinline__ mx_sb mx_scale_of(float amax, float inv_qmax) {
+    const unsigned u = __float_as_uint(__fmul_rn(amax, inv_qmax));
+    const int eb = max(1, min(253, (int)((u + 0x7fffffu) >> 23)));
+    mx_sb r;
+    r.sb = u >= 0x7f800000u ? 255u : (unsigned)eb;
+    r.m = __uint_as_float((254u - r.sb) << 23);
+    return r;
+}
+/* the largest of three magnitudes, a NaN if one of them is: one instruction on sm_100 */
+__device__ __forceinline__ float absmax3_nan(float a, float b, float c) { float d; asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 /* NaN-propagating amax on the magnitude bits (src/lp_common.cuh:486) */
 __device__ __forceinline__ unsigned amax_u(unsigned a, float v) { return max(a, __float_as_uint(v) & 0x7fffffffu); }
 /* scale byte -> factor; 0xFF -> +inf, 0 -> 2^-127 */
@@ -66,8 +81,12 @@ __device__ __forceinline__ unsigned cvt_e2m1x2(float lo, float hi) {
     asm("{ .reg .b8 t; cvt.rn.satfinite.e2m1x2.f32 t, %1, %2; cvt.u16.u8 %0, t; }" : "=h"(r) : "f"(hi), "f"(lo));
     return (unsigned)r & 0xffu;
 }
+/* eight floats -> eight e2m1 nibbles of a word (v[0] lowest) */
+__device__ __forceinline__ unsigned cvt_e2m1_word(float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7) {
+    return cvt_e2m1x2(v0, v1) | (cvt_e2m1x2(v2, v3) << 8) | (cvt_e2m1x2(v4, v5) << 16) | (cvt_e2m1x2(v6, v7) << 24);
+}
 __device__ __forceinline__ unsigned cvt_e2m1x8(const float *v, float m) {
-    return cvt_e2m1x2(v[0] * m, v[1] * m) | (cvt_e2m1x2(v[2] * m, v[3] * m) << 8) | (cvt_e2m1x2(v[4] * m, v[5] * m) << 16) | (cvt_e2m1x2(v[6] * m, v[7] * m) << 24);
+    return cvt_e2m1_word(v[0] * m, v[1] * m, v[2] * m, v[3] * m, v[4] * m, v[5] * m, v[6] * m, v[7] * m);
 }
 __device__ __forceinline__ float dec_e4m3(unsigned b) {
     const unsigned e = (b >> 3) & 15u, m = b & 7u;
@@ -127,11 +146,12 @@ __device__ __forceinline__ unsigned mx_encode_row32_h8(const __half2 *h, unsigne
 }
 /* a row of 32 floats -> MX codes: q8 receives 32 bytes (BITS 8: w[0..8)) or 16 bytes (BITS 4: w[0..4)); returns the scale byte */
 template <int BITS> __device__ __forceinline__ unsigned mx_encode_row32(const float *v, unsigned *w) {
-    unsigned am = 0u;
+    float am = absmax3_nan(v[0], v[1], v[2]);
 #pragma unroll
-    for (int k = 0; k < 32; k++) am = amax_u(am, v[k]);
-    const int e = mx_exp(__uint_as_float(am), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
-    const float m = exp2i(-e);
+    for (int k = 3; k < 31; k += 2) am = absmax3_nan(am, v[k], v[k + 1]);
+    am = absmax3_nan(am, v[31], v[31]);
+    const mx_sb q = mx_scale_of(am, BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
+    const float m = q.m;
     if (BITS == 4) {
 #pragma unroll
         for (int j = 0; j < 4; j++) w[j] = cvt_e2m1x8(v + 8 * j, m);
@@ -139,5 +159,5 @@ template <int BITS> __device__ __forceinline__ unsigned mx_encode_row32(const fl
 #pragma unroll
         for (int j = 0; j < 8; j++) w[j] = cvt_e4m3x4(v[4 * j] * m, v[4 * j + 1] * m, v[4 * j + 2] * m, v[4 * j + 3] * m);
     }
-    return (unsigned)(e + 127) & 0xffu;
+    return q.sb;
 }

@@ -19,24 +19,20 @@ template <int BITS> __device__ __forceinline__ void qrow_dec(uint2 raw, float fx
 #pragma unroll
     for (int j = 0; j < 4; j++) r[j] = __fmul2_rn(make_float2(t[2 * j], t[2 * j + 1]), f2);
 }
-/* magnitude of the larger of |a|, |b|, a NaN if either is one; the sign of the result carries no meaning */
-__device__ __forceinline__ float absmax_nan(float a, float b) { float d; asm("max.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
 /* this lane's eight values of a row -> its codes; returns the row's scale byte (the same in the four lanes).  All 32 lanes of the warp
    call it together.  Same results as mx_encode_row32: NaN-propagating amax, v * 2^-e, hardware conversion. */
 template <int BITS> __device__ __forceinline__ unsigned qrow_enc(const float2 *r, uint2 &w) {
-    const float a01 = absmax_nan(absmax_nan(r[0].x, r[0].y), absmax_nan(r[1].x, r[1].y)), a23 = absmax_nan(absmax_nan(r[2].x, r[2].y), absmax_nan(r[3].x, r[3].y));
-    unsigned am = __float_as_uint(absmax_nan(a01, a23)) & 0x7fffffffu;
-    am = max(am, __shfl_xor_sync(0xffffffffu, am, 1));
-    am = max(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    const int e = mx_exp(__uint_as_float(am), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
-    const float m = exp2i(-e);
-    const float2 m2 = make_float2(m, m);
+    float am = absmax3_nan(absmax3_nan(r[0].x, r[0].y, r[1].x), absmax3_nan(r[1].y, r[2].x, r[2].y), absmax3_nan(r[3].x, r[3].y, 0.f));
+    am = absmax3_nan(am, __shfl_xor_sync(0xffffffffu, am, 1), 0.f);
+    am = absmax3_nan(am, __shfl_xor_sync(0xffffffffu, am, 2), 0.f);
+    const mx_sb q = mx_scale_of(am, BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
+    const float2 m2 = make_float2(q.m, q.m);
     float2 s[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) s[j] = __fmul2_rn(r[j], m2);
     if (BITS == 8) { w.x = cvt_e4m3x4(s[0].x, s[0].y, s[1].x, s[1].y); w.y = cvt_e4m3x4(s[2].x, s[2].y, s[3].x, s[3].y); }
-    else { w.x = cvt_e2m1x2(s[0].x, s[0].y) | (cvt_e2m1x2(s[1].x, s[1].y) << 8) | (cvt_e2m1x2(s[2].x, s[2].y) << 16) | (cvt_e2m1x2(s[3].x, s[3].y) << 24); w.y = 0u; }
-    return (unsigned)(e + 127) & 0xffu;
+    else { w.x = cvt_e2m1_word(s[0].x, s[0].y, s[1].x, s[1].y, s[2].x, s[2].y, s[3].x, s[3].y); w.y = 0u; }
+    return q.sb;
 }
 template <int BITS> __device__ __forceinline__ void qrow_st(uint8_t *__restrict__ codes, size_t row, int q, uint2 w) {
     if (BITS == 8) ((uint2 *)(codes + row * 32))[q] = w; else ((unsigned *)(codes + row * 16))[q] = w.x;

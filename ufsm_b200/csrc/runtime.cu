@@ -54,7 +54,21 @@ extern "C" void *nn_malloc(size_t bytes) {
     return p;
 }
 extern "C" void nn_free(void *p) { if (p) cudaFree(p); }
-extern "C" void nn_zero(void *p, size_t bytes) { cudaError_t e = cudaMemset(p, 0, bytes); if (e != cudaSuccess) umx_latch("nn_zero", e); }
+/* A kernel of the library's own launch chain (programmatic launch: it is scheduled while its predecessor drains) where memset would break the chain:
+   3.7 us between two kernels, 2 in this form.  Devices the library has no kernels for take memset. */
+__global__ void __launch_bounds__(256) zero_k(uint4 *p, size_t n) {
+    pdl_trigger(); pdl_wait();
+    for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+extern "C" void nn_zero(void *p, size_t bytes) {
+    int d = -1;
+    if (!(((size_t)p | bytes) & 15) && bytes && cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 16 && g_ready[d] > 0) {
+        size_t g = (bytes / 16 + 255) / 256; if (g > 148u * 16u) g = 148u * 16u;
+        umx_launch(zero_k, dim3((unsigned)g), dim3(256), 0, (uint4 *)p, bytes / 16);
+        UMX_CK("nn_zero");
+        return;
+    }
+    cudaError_t e = cudaMemset(p, 0, bytes); if (e != cudaSuccess) umx_latch("nn_zero", e); }
 extern "C" void nn_h2d(void *dst, const void *src, size_t bytes) { cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice); if (e != cudaSuccess) umx_latch("nn_h2d", e); }
 extern "C" void nn_d2h(void *dst, const void *src, size_t bytes) { cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost); if (e != cudaSuccess) umx_latch("nn_d2h", e); }
 extern "C" void nn_sync(void) {
@@ -71,6 +85,7 @@ extern "C" void nn_free_host(void *p) { if (p) cudaFreeHost(p); }
 
 /* ---- copy streams and events for the host entry that overlaps the copies of one patch with the forward of the next.  Streams are
    non-blocking (they do not synchronise with the legacy default stream the kernels run on); the order is made with events. ---- */
+thread_local int umx_plain_launch = 0;
 int umx_pdl(void) { static int v = -1; if (v < 0) { const char *e = getenv("UMX_PDL"); v = !(e && *e == '0'); } return v; }
 extern "C" void *umx_stream_new(void) { cudaStream_t s = nullptr; cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking); if (e != cudaSuccess) { umx_latch("umx_stream_new", e); return nullptr; } return (void *)s; }
 extern "C" void umx_stream_free(void *s) { if (s) cudaStreamDestroy((cudaStream_t)s); }
@@ -93,7 +108,7 @@ extern "C" void umx_copy2d_async(void *dst, size_t dpitch, const void *src, size
 }
 
 /* scratch: per device, per slot, grows on demand, never shrinks */
-enum { WS_SLOTS = 13 };
+enum { WS_SLOTS = 16 };     /* 13 to 15: weight images and bias of a conv that is prepared on every call */
 static void *g_ws[16][WS_SLOTS];
 static size_t g_ws_bytes[16][WS_SLOTS];
 void *umx_ws(int slot, size_t bytes) {
@@ -106,6 +121,12 @@ void *umx_ws(int slot, size_t bytes) {
         g_ws_bytes[d][slot] = nb;
     }
     return g_ws[d][slot];
+}
+/* gives a slot's memory back */
+void umx_ws_free(int slot) {
+    int d = 0; cudaGetDevice(&d); d &= 15;
+    if (g_ws[d][slot]) { cudaDeviceSynchronize(); cudaFree(g_ws[d][slot]); }
+    g_ws[d][slot] = nullptr; g_ws_bytes[d][slot] = 0;
 }
 int *umx_errflag(void) {
     int d = 0; cudaGetDevice(&d); d &= 15;
