@@ -20,14 +20,16 @@ struct GnSlabs { int ns, zs, zo; size_t zhw; };             /* slab-local statis
 template <int XK, int BY, int FORM, bool SL>
 __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ xv, uint8_t *__restrict__ y, int C, int G, size_t S,
                                                       const float *__restrict__ gamma, const float *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd, int y_split,
-                                                      int c_off, int cpg, const GnSlabs sl) {
+                                                      int c_off, int cpg, const GnSlabs sl, int nb_dst, int b0) {
+    pdl_trigger(); pdl_wait();
     const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, T = gridDim.x;
     const int q = threadIdx.x & 3, ph = threadIdx.x >> 2;
     constexpr int RBY = BY == 8 ? 32 : 16;
     const size_t nbk = (size_t)n * nb + blk, v0 = S * blockIdx.x / T, vend = S * (blockIdx.x + 1) / T;
     const uint8_t *xq = (const uint8_t *)xv;
     const uint8_t *xs = XK == 8 ? xq + (size_t)N * nb * S * 32 : xq + (size_t)N * nb * S * 16;
-    uint8_t *ys = y + (size_t)N * nb * S * RBY;
+    const size_t dbk = (size_t)n * nb_dst + b0 + blk;      /* the block of the destination tensor, which has nb_dst a sample */
+    uint8_t *ys = y + (size_t)N * nb_dst * S * RBY;
     bool live[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) live[k] = blk * 32 + q * 8 + k < C;
@@ -41,32 +43,39 @@ __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ x
         nr = n * sl.ns + sb_;
         if (sb_ < sl.ns - 1) { const long long zb = (long long)(sb_ + 1) * sl.zs - sl.zo; if (zb > 0) v1 = min(vend, max(va + 1, (size_t)zb * sl.zhw)); }
     }
+    /* an MX source's rows of one trip; the first trip's are asked for ahead of the coefficients */
+    constexpr bool MXIN = XK == 8 || XK == 4;
+    uint2 raw[4]; unsigned sb[4];
+    auto fetch = [&](size_t vb) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const size_t v = vb + u * 64 + ph;
+            raw[u] = make_uint2(0u, 0u); sb[u] = 127u;
+            if (v < v1) { raw[u] = qrow_ld<(XK == 4 ? 4 : 8)>(xq, nbk * S + v, q); sb[u] = __ldg(xs + nbk * S + v); }
+        }
+    };
+    if (MXIN) fetch(va);
     /* per channel: FORM 0 (mean, rstd, gamma, beta) in (k0, k1, k2, k3); FORM 1 (a, b) in (k0, k1) */
     float2 k0[4], k1[4], k2[4], k3[4];                       /* FORM 0: k0 holds -mean */
+    int grp = (c_off + blk * 32 + q * 8) / cpg, rem = c_off + blk * 32 + q * 8 - grp * cpg;      /* the channel's group, counted along */
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const int c = blk * 32 + q * 8 + k;
         float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
         if (live[k]) {
-            const int cl = c_off + c, ng = nr * G + cl / cpg;      /* cl: the channel's index in the tensor the groups are counted over */
+            const int cl = c_off + blk * 32 + q * 8 + k, ng = nr * G + grp;      /* cl: the channel's index in the tensor the groups are counted over */
             if (FORM == 0) { t0 = -mean[ng]; t1 = rstd[ng]; t2 = gamma[cl]; t3 = beta[cl]; }
             else { t0 = __fmul_rn(rstd[ng], gamma[cl]); t1 = __fmaf_rn(-mean[ng], t0, beta[cl]); }
         }
+        if (++rem == cpg) { rem = 0; grp++; }
         if (k & 1) { k0[k >> 1].y = t0; k1[k >> 1].y = t1; k2[k >> 1].y = t2; k3[k >> 1].y = t3; }
         else { k0[k >> 1].x = t0; k1[k >> 1].x = t1; k2[k >> 1].x = t2; k3[k >> 1].x = t3; }
     }
     for (size_t vb = va; vb < v1; vb += 256) {
         float2 r[4][4];
-        if (XK == 8 || XK == 4) {
-            uint2 raw[4]; unsigned sb[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const size_t v = vb + u * 64 + ph;
-                raw[u] = make_uint2(0u, 0u); sb[u] = 127u;
-                if (v < v1) { raw[u] = qrow_ld<(XK == 4 ? 4 : 8)>(xq, nbk * S + v, q); sb[u] = __ldg(xs + nbk * S + v); }
-            }
+        if (MXIN) {
 #pragma unroll
             for (int u = 0; u < 4; u++) qrow_dec<(XK == 4 ? 4 : 8)>(raw[u], mx_scale(sb[u]), r[u]);
+            if (vb + 256 < v1) fetch(vb + 256);              /* the next trip's rows arrive while this one is worked on */
         } else {
             /* plane-major source: eight lanes of a plane read eight consecutive voxels */
 #pragma unroll
@@ -91,11 +100,11 @@ __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ x
                 r[u][j] = make_float2(live[2 * j] ? silu_hw(t.x) : 0.f, live[2 * j + 1] ? silu_hw(t.y) : 0.f);
             }
             uint2 w;
-            const unsigned sb = qrow_enc<BY>(r[u], w);       /* every lane, also those past the end of the run */
+            const unsigned so = qrow_enc<BY>(r[u], w);       /* every lane, also those past the end of the run */
             if (v < v1) {
-                if (BY == 8 && y_split) *(uint2 *)(y + ((nbk * 2 + (q >> 1)) * S + v) * 16 + (q & 1) * 8) = w;
-                else qrow_st<BY>(y, nbk * S + v, q, w);
-                if (q == 0) ys[nbk * S + v] = (uint8_t)sb;
+                if (BY == 8 && y_split) *(uint2 *)(y + ((dbk * 2 + (q >> 1)) * S + v) * 16 + (q & 1) * 8) = w;
+                else qrow_st<BY>(y, dbk * S + v, q, w);
+                if (q == 0) ys[dbk * S + v] = (uint8_t)so;
             }
         }
     }
@@ -105,12 +114,11 @@ __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ x
 }
 
 template <int XK, int BY>
-void launch_form(int form, dim3 grid, const void *x, uint8_t *y, int C, int G, size_t S, const float *gamma, const float *beta, const float *mean, const float *rstd, int y_split, int c_off, int cpg, GnSlabs sl) {
-    if (sl.ns) {
-        if (form == 0) gn_silu_rows_k<XK, BY, 0, true><<<grid, 256>>>(x, y, C, G, S, gamma, beta, mean, rstd, y_split, c_off, cpg, sl);
-        else gn_silu_rows_k<XK, BY, 1, true><<<grid, 256>>>(x, y, C, G, S, gamma, beta, mean, rstd, y_split, c_off, cpg, sl);
-    } else if (form == 0) gn_silu_rows_k<XK, BY, 0, false><<<grid, 256>>>(x, y, C, G, S, gamma, beta, mean, rstd, y_split, c_off, cpg, sl);
-    else gn_silu_rows_k<XK, BY, 1, false><<<grid, 256>>>(x, y, C, G, S, gamma, beta, mean, rstd, y_split, c_off, cpg, sl);
+void launch_form(int form, dim3 grid, const void *x, uint8_t *y, int C, int G, size_t S, const float *gamma, const float *beta, const float *mean, const float *rstd, int y_split, int c_off, int cpg, GnSlabs sl, int nb_dst, int b0) {
+#define UMX_GSL(F, SLB) umx_launch(gn_silu_rows_k<XK, BY, F, SLB>, grid, dim3(256), 0, x, y, C, G, S, gamma, beta, mean, rstd, y_split, c_off, cpg, sl, nb_dst, b0)
+    if (sl.ns) { if (form == 0) UMX_GSL(0, true); else UMX_GSL(1, true); }
+    else if (form == 0) UMX_GSL(0, false); else UMX_GSL(1, false);
+#undef UMX_GSL
 }
 
 }   // namespace
@@ -120,9 +128,10 @@ void launch_form(int form, dim3 grid, const void *x, uint8_t *y, int C, int G, s
    concat input with one GroupNorm over both parts): its channel 0 is channel c_off of C_all (0, C for a whole tensor); gamma, beta,
    mean, rstd are the larger tensor's.  ns != 0: slab-local statistics, mean and rstd [N][ns][G], plane z = voxel / zhw of the tensor in slab
    (z + zo) / zs clamped to [0, ns) (gnp_t, src/nn_lp.h:15-18; zo may be negative here: a tensor that is a z range of the one the slabs are
-   counted in).  Returns 0, -1 on an unsupported combination (the caller reports it). */
-int umx_gn_silu_apply_seg_slabs(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
-                                void *y, int bits, int layout, int form, int c_off, int C_all, int ns, int zs, int zo, size_t zhw) {
+   counted in).  The result goes to blocks [b0, ...) of a destination tensor of nb_dst blocks (a conv's operand assembled from parts).
+   Returns 0, -1 on an unsupported combination (the caller reports it). */
+int umx_gn_silu_apply_to(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
+                         void *y, int bits, int layout, int form, int c_off, int C_all, int ns, int zs, int zo, size_t zhw, int nb_dst, int b0) {
     if (ns < 0 || (ns && (zs < 1 || !zhw || S % zhw))) return -1;
     const GnSlabs sl = {ns, zs, zo, zhw};
     if (C < 1 || G < 1 || C_all % G || c_off < 0 || c_off + C > C_all || (bits != 8 && bits != 4) || (xdt != UMX_F32 && xdt != UMX_F16 && xdt != UMX_MX8 && xdt != UMX_MX4)) return -1;
@@ -130,16 +139,24 @@ int umx_gn_silu_apply_seg_slabs(const void *x, int xdt, int N, int C, size_t S, 
     const int nb = (C + 31) / 32;
     if (!N || !S) return 0;
     if (N > 65535 || nb > 65535) return -1;
-    /* runs of about 2048 voxels (eight trips a block) */
+    /* runs of about 2048 voxels (eight trips a block), shorter ones, down to one trip of 256, while that leaves a multiprocessor fewer than the
+       three blocks it holds: the pass is a chain of a load, some forty dependent instructions and a store a trip (64 channels x 48^3: 15.3 us in
+       108 blocks, 9 us in 432) */
     size_t T = (S + 2047) / 2048; if (T > 0x7fffffffu) return -1;
+    const size_t rowsets = (size_t)N * nb, fill = (3 * 148 + rowsets - 1) / rowsets, most = (S + 255) / 256;
+    if (T < fill) T = fill < most ? fill : most;
     const dim3 blocks((unsigned)T, (unsigned)nb, (unsigned)N);
     const int ys = bits == 8 && layout == UMX_LAYOUT_SPLIT;
     uint8_t *yb = (uint8_t *)y;
-#define UMX_GSA(XK) do { if (bits == 8) launch_form<XK, 8>(form, blocks, x, yb, C, G, S, gamma, beta, mean, rstd, ys, c_off, cpg, sl); else launch_form<XK, 4>(form, blocks, x, yb, C, G, S, gamma, beta, mean, rstd, ys, c_off, cpg, sl); } while (0)
+#define UMX_GSA(XK) do { if (bits == 8) launch_form<XK, 8>(form, blocks, x, yb, C, G, S, gamma, beta, mean, rstd, ys, c_off, cpg, sl, nb_dst, b0); else launch_form<XK, 4>(form, blocks, x, yb, C, G, S, gamma, beta, mean, rstd, ys, c_off, cpg, sl, nb_dst, b0); } while (0)
     if (xdt == UMX_MX8) UMX_GSA(8); else if (xdt == UMX_MX4) UMX_GSA(4); else if (xdt == UMX_F16) UMX_GSA(2); else UMX_GSA(0);
 #undef UMX_GSA
     g_umx_launches++;
     return 0;
+}
+int umx_gn_silu_apply_seg_slabs(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
+                                void *y, int bits, int layout, int form, int c_off, int C_all, int ns, int zs, int zo, size_t zhw) {
+    return umx_gn_silu_apply_to(x, xdt, N, C, S, G, gamma, beta, mean, rstd, y, bits, layout, form, c_off, C_all, ns, zs, zo, zhw, (C + 31) / 32, 0);
 }
 /* statistics per sample */
 int umx_gn_silu_apply_seg(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
