@@ -524,3 +524,49 @@ def test_probability_bytes_from_the_head(dev, bits, Ci, Co, N, D, H, W):
     assert np.array_equal(pb, od.download())
     p = 1.0 / (1.0 + np.exp(-lg.view(np.float16).astype(np.float64)))
     assert np.abs(pb.astype(np.float64) - 254.0 * p).max() <= 0.5 + 1e-3
+
+
+def test_weights_without_a_key_may_change_between_calls(dev):
+    """lp_conv_fwd_f8 / _f4 / _s2_f8 without split_t.wkey prepare their weights on every call, in scratch that the calls share: other values in the
+    same buffer, other shapes (either conv kernel, ragged channel counts, more K items than a block of the preparation has warps) and the
+    conv of the call before must not show.  Expected: the same conv through a handle of its own."""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf, Shape5, Gnp, Split
+    L = ufsm_b200.lib()
+    wbuf, bbuf = DevBuf(192 * 320 * 27 * 4), DevBuf(192 * 4)
+    outs, wants = [], []
+    cases = [(8, 32, 32, 8, 16, 16), (8, 160, 72, 3, 6, 10), (4, 64, 64, 4, 16, 16), (4, 40, 192, 3, 5, 7), (8, 24, 40, 4, 9, 16), (4, 320, 33, 2, 4, 6), (8, 32, 32, 8, 16, 16)]
+    for i, (bits, ci, co, D, H, W) in enumerate(cases):
+        S = D * H * W
+        x = synth.act_h16(400 + i, ci * S)
+        w, b = synth.kaiming(420 + i, co, ci, 27), synth.bias(440 + i, co, 0.1)
+        wbuf.upload(w)
+        bbuf.upload(b)
+        xd, yd = DevBuf(data=x), DevBuf(co * S * 2).fill(0xEE)
+        fn = L.lp_conv_fwd_f8 if bits == 8 else L.lp_conv_fwd_f4
+        assert fn(xd.ptr, 2, Shape5(1, ci, D, H, W), wbuf.ptr, bbuf.ptr, co, yd.ptr, 2, Gnp(), None, 0, Split()) == 0
+        outs.append(yd)
+        c = G.Conv("conv3", w, b, co, ci, bits)
+        raw, _ = c.fwd(orc.pm_to_mx(x, 2, 1, ci, S, bits, 32), 1, D, H, W, G.OUT_PM16)
+        c.free()
+        wants.append(raw)
+    ufsm_b200.check()
+    for i, (y, want) in enumerate(zip(outs, wants)):
+        assert np.array_equal(y.download(), want), cases[i]
+    # the stride-2 conv: two calls in a row on one weight buffer
+    got, want = [], []
+    for i, (bits, ci, co, D, H, W) in enumerate([(8, 72, 40, 5, 9, 12), (4, 96, 64, 4, 6, 8)]):
+        S, So = D * H * W, ((D + 1) // 2) * ((H + 1) // 2) * ((W + 1) // 2)
+        w, b = synth.kaiming(460 + i, co, ci, 27), synth.bias(470 + i, co, 0.1)
+        wbuf.upload(w)
+        bbuf.upload(b)
+        mx = orc.pm_to_mx(synth.act_h16(480 + i, ci * S), 2, 1, ci, S, bits, 32)
+        xd, yd = DevBuf(data=mx), DevBuf(co * So * 2).fill(0xEE)
+        L.lp_conv_fwd_s2_f8(xd.ptr, 3 if bits == 8 else 4, Shape5(1, ci, D, H, W), wbuf.ptr, bbuf.ptr, co, yd.ptr, 2, Shape5(1, co, (D + 1) // 2, (H + 1) // 2, (W + 1) // 2), Gnp())
+        got.append(yd)
+        c = G.Conv("conv3s2", w, b, co, ci, bits)
+        want.append(c.fwd(mx, 1, D, H, W, G.OUT_PM16)[0])
+        c.free()
+    ufsm_b200.check()
+    for g, wnt in zip(got, want):
+        assert np.array_equal(g.download(), wnt)

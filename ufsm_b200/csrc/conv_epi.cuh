@@ -9,6 +9,7 @@ struct umx_conv {
     uint8_t *wr;                    /* weight image of the z-marching kernel, or NULL */
     uint8_t *wp;                    /* weight image of the one-tap streaming kernel, or NULL */
     uint8_t *wstem;                 /* weight tile of the tap-packed one-channel kernel, or NULL */
+    const float *w_src, *b_src;     /* set in a conv that lives for one call (umx_conv_per_call): its images are made in scratch when a kernel asks for them */
 };
 
 struct EpiArgs {
@@ -95,7 +96,11 @@ __device__ __forceinline__ void epi_chunk(const EpiArgs &a, int n, int z, int oy
     }
 }
 
-/* ---- weight preparation shared by the conv kernels: where GEMM row `row`, tap `tap`, K block `kb`, element k comes from ---- */
+/* geometry of the z-marching kernel's weight image (conv_tcr.cu), one image per column tile of nt channels */
+struct RImageGeo { int nt, ncol, w_bytes, w_codes, gt, goff1, goff2; };
+int umx_conv_r_image(const umx_conv *c, RImageGeo *o);
+
+/* ---- weight preparation of the one-tap convs: where GEMM row `row`, tap `tap`, K block `kb`, element k comes from ---- */
 struct PrepArgs {
     const float *w; uint8_t *wpk; const float *bias; float *bias_p;
     int kind, co, ci, bits, cop, cob_t, nkb, nki, taps, nt, ntiles_n, nst, items_max, ipq, nquad, w_stage_bytes;
@@ -103,12 +108,7 @@ struct PrepArgs {
 __device__ __forceinline__ float prep_src(const PrepArgs &p, int row, int tap, int kb, int k) {
     /* value of GEMM row `row`, tap `tap`, K block `kb`, element k (0 outside the real weights) */
     if (kb >= p.nkb) return 0.f;
-    if (p.kind == UMX_CONV3) { const int ci = kb * 32 + k; return (row < p.co && ci < p.ci) ? p.w[((size_t)row * p.ci + ci) * 27 + tap] : 0.f; }
     if (p.kind == UMX_CONV1) { const int ci = kb * 32 + k; return (row < p.co && ci < p.ci) ? p.w[(size_t)row * p.ci + ci] : 0.f; }
-    if (p.kind == UMX_CONV3S2) {   /* K block = tap * blocks(ci) + block; MX-fp4: the blocks of a tap padded to an even count (zero weights) */
-        const int nb = (p.ci + 31) / 32, nbi = p.bits == 4 ? (nb + 1) / 2 * 2 : nb, t = kb / nbi, ci = (kb % nbi) * 32 + k;
-        return (row < p.co && ci < p.ci) ? p.w[((size_t)row * p.ci + ci) * 27 + t] : 0.f;
-    }
     if (p.kind == UMX_DOWN2) {   /* K block = sub-voxel tap * blocks(ci) + block */
         const int nbi = (p.ci + 31) / 32, t = kb / nbi, ci = (kb % nbi) * 32 + k;
         return (row < p.co && ci < p.ci) ? p.w[((size_t)row * p.ci + ci) * 8 + t] : 0.f;
@@ -117,3 +117,5 @@ __device__ __forceinline__ float prep_src(const PrepArgs &p, int row, int tap, i
     const int abc = row / (32 * p.cob_t), o = row % (32 * p.cob_t), ci = kb * 32 + k;
     return (o < p.co && ci < p.ci) ? p.w[((size_t)ci * p.co + o) * 8 + abc] : 0.f;
 }
+/* the 27-tap convs (conv_prep.cu) */
+void umx_prep_w27(const PrepArgs &p, uint8_t *wr, int nt, int w_bytes, int w_codes, int gt, int goff1, int goff2);

@@ -329,23 +329,21 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
     if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, kTmemCols); }
 }
 
-/* ---- weight preparation: fp32 weights -> the shared-memory image of every (column tile, stage): items x [k half][row][16 B]
+/* ---- weight preparation of the one-tap convs: fp32 weights -> the shared-memory image of every (column tile, stage): items x [k half][row][16 B]
    codes, then the scale bytes in the TMEM scale layout (quad, lane, column, byte).  One thread per (column tile, stage, item, row).
    Quantisation per (row, tap, 32 input channels) as the reference's prep_w8_k / prep_w4_k (src/lp_f8fwd.cu:54-71,
    src/lp_f4fwd.cu:53-66). ---- */
 __global__ void __launch_bounds__(128) prep_w_k(const PrepArgs p) {
     const size_t total = (size_t)p.ntiles_n * p.nst * p.items_max * p.nt;
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i == 0 && p.bias_p) for (int c = 0; c < p.cop; c++) {
-        float b = 0.f;
-        if (p.bias) { if (p.kind == UMX_TCONV2) { const int o = c % (32 * p.cob_t); b = o < p.co ? p.bias[o] : 0.f; } else b = c < p.co ? p.bias[c] : 0.f; }
-        p.bias_p[c] = b;
+    if (i < (size_t)p.cop && p.bias_p) {
+        const int c = (int)i, o = p.kind == UMX_TCONV2 ? c % (32 * p.cob_t) : c;
+        p.bias_p[c] = (p.bias && o < p.co) ? p.bias[o] : 0.f;
     }
     if (i >= total) return;
     const int rl = (int)(i % p.nt), j = (int)((i / p.nt) % p.items_max), st = (int)((i / ((size_t)p.nt * p.items_max)) % p.nst), ntile = (int)(i / ((size_t)p.nt * p.items_max * p.nst));
     const int row = ntile * p.nt + rl;
-    int tap, ki;
-    if (p.taps == 27) { ki = st / 3; tap = (st % 3) * 9 + j; } else { ki = 4 * st + j; tap = 0; }
+    const int tap = 0, ki = 4 * st + j;
     uint8_t *stg = p.wpk + ((size_t)ntile * p.nst + st) * p.w_stage_bytes;
     const bool live = row < p.cop && ki < p.nki;
     unsigned w[8]; unsigned sb[2] = {127u, 127u};
@@ -390,23 +388,22 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 }   // namespace
 
 void umx_conv_ks_tickets_reset(void) { void *p = nullptr; if (cudaGetSymbolAddress(&p, g_ks_tickets) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 8192); }
-int umx_conv_r_fits(const umx_conv *c);
-uint8_t *umx_conv_r_prepare(const umx_conv *c, const float *w_dev);
-int umx_conv_fwd_r(const umx_conv *c, const void *x, const CUtensorMap *m0, void *enc, int N, int D, int H, int W, const EpiArgs &e,
+int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e);
+int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, void *enc, int N, int D, int H, int W, const EpiArgs &e,
                    double *part, const float *gamma, const float *beta, float eps, float *coef);
 extern "C" void umx_in_stats_coef(const void *y, int N, int C, int D, int H, int W, const float *gamma, const float *beta, float eps, double *part, float *coef);
 void umx_in_part(const void *y, int N, int C, int D, int H, int W, double *part);
 uint8_t *umx_conv_p_prepare(const umx_conv *c, const float *w_dev);
 uint8_t *umx_conv_stem_prepare(const umx_conv *c, const float *w_dev);
 int umx_conv_fwd_stem(const umx_conv *c, const void *x, int src8, int N, int D, int H, int W, void *y);
-int umx_conv_fwd_p(const umx_conv *c, const void *x, void *enc, int N, int D, int H, int W, const EpiArgs &e);
+int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *enc, int N, int D, int H, int W, const EpiArgs &e);
 const uint8_t *umx_prob_table(void);
+void umx_mx_codes_to_split(const void *x, size_t blocks, size_t S, void *y);
 
 
-static umx_conv *conv_build(int kind, const float *w_dev, const float *bias_dev, int co, int ci, int bits) {
-    if (!umx_ready("umx_conv_create")) return nullptr;
-    if ((bits != 8 && bits != 4) || kind < 0 || kind > 4 || co < 1 || ci < 1 ) { fprintf(stderr, "umx_conv_create: bad arguments (kind %d, co %d, ci %d, bits %d)\n", kind, co, ci, bits); abort(); }
-    umx_conv *c = (umx_conv *)calloc(1, sizeof *c);
+/* the fields of a conv that follow from its kind and sizes */
+static void conv_geometry(umx_conv *c, int kind, int co, int ci, int bits) {
+    memset(c, 0, sizeof *c);
     c->kind = kind; c->co = co; c->ci = ci; c->bits = bits;
     c->taps = kind == UMX_CONV3 ? 27 : 1;
     const int nbi = ceil_div(ci, 32);
@@ -423,24 +420,67 @@ static umx_conv *conv_build(int kind, const float *w_dev, const float *bias_dev,
     c->nquad = ceil_div(c->items_max, c->ipq);
     c->nst = c->taps == 27 ? 3 * c->nki : ceil_div(c->nki, 4);
     c->w_stage_bytes = c->items_max * c->nt * 32 + c->nquad * 512;
-    const size_t wb = (size_t)c->ntiles_n * c->nst * c->w_stage_bytes;
+}
+static size_t wpk_bytes(const umx_conv *c) { return (size_t)c->ntiles_n * c->nst * c->w_stage_bytes; }
+static PrepArgs prep_args(const umx_conv *c, const float *w_dev, const float *bias_dev) {
+    PrepArgs p; memset(&p, 0, sizeof p);
+    p.w = w_dev; p.wpk = c->wpk; p.bias = bias_dev; p.bias_p = c->bias_p; p.kind = c->kind; p.co = c->co; p.ci = c->ci; p.bits = c->bits; p.cop = c->cop; p.cob_t = c->cob_t;
+    p.nkb = c->nkb; p.nki = c->nki; p.taps = c->taps; p.nt = c->nt; p.ntiles_n = c->ntiles_n; p.nst = c->nst; p.items_max = c->items_max; p.ipq = c->ipq; p.nquad = c->nquad; p.w_stage_bytes = c->w_stage_bytes;
+    return p;
+}
+static umx_conv *conv_build(int kind, const float *w_dev, const float *bias_dev, int co, int ci, int bits) {
+    if (!umx_ready("umx_conv_create")) return nullptr;
+    if ((bits != 8 && bits != 4) || kind < 0 || kind > 4 || co < 1 || ci < 1 ) { fprintf(stderr, "umx_conv_create: bad arguments (kind %d, co %d, ci %d, bits %d)\n", kind, co, ci, bits); abort(); }
+    umx_conv *c = (umx_conv *)malloc(sizeof *c);
+    conv_geometry(c, kind, co, ci, bits);
+    const size_t wb = wpk_bytes(c);
     c->wpk = (uint8_t *)nn_malloc(wb); c->bias_p = (float *)nn_malloc((size_t)c->cop * 4);
     if (!c->wpk || !c->bias_p) { umx_conv_free(c); return nullptr; }
     cudaMemset(c->wpk, 127, wb);   /* unused scale slots read as 1 */
-    PrepArgs p; memset(&p, 0, sizeof p);
-    p.w = w_dev; p.wpk = c->wpk; p.bias = bias_dev; p.bias_p = c->bias_p; p.kind = kind; p.co = co; p.ci = ci; p.bits = bits; p.cop = c->cop; p.cob_t = c->cob_t;
-    p.nkb = c->nkb; p.nki = c->nki; p.taps = c->taps; p.nt = c->nt; p.ntiles_n = c->ntiles_n; p.nst = c->nst; p.items_max = c->items_max; p.ipq = c->ipq; p.nquad = c->nquad; p.w_stage_bytes = c->w_stage_bytes;
-    const size_t total = (size_t)c->ntiles_n * c->nst * c->items_max * c->nt;
-    prep_w_k<<<(unsigned)((total + 127) / 128), 128>>>(p);
-    g_umx_launches++;
-    c->wr = umx_conv_r_prepare(c, w_dev);
-    c->wp = umx_conv_p_prepare(c, w_dev);
-    c->wstem = umx_conv_stem_prepare(c, w_dev);
+    const PrepArgs p = prep_args(c, w_dev, bias_dev);
+    if (kind == UMX_CONV3 || kind == UMX_CONV3S2) {
+        RImageGeo g; memset(&g, 0, sizeof g);
+        if (kind == UMX_CONV3 && umx_conv_r_image(c, &g)) {
+            c->wr = (uint8_t *)nn_malloc((size_t)g.w_bytes * g.ncol);
+            if (!c->wr) { umx_conv_free(c); return nullptr; }
+            cudaMemset(c->wr, 127, (size_t)g.w_bytes * g.ncol);
+        }
+        umx_prep_w27(p, c->wr, g.nt, g.w_bytes, g.w_codes, g.gt, g.goff1, g.goff2);
+        c->wstem = umx_conv_stem_prepare(c, w_dev);
+    } else {
+        const size_t total = (size_t)c->ntiles_n * c->nst * c->items_max * c->nt;
+        prep_w_k<<<(unsigned)((total + 127) / 128), 128>>>(p);
+        g_umx_launches++;
+        c->wp = umx_conv_p_prepare(c, w_dev);
+    }
     UMX_CK("umx_conv_create");
     /* the conv kernels read the prepared weights and the bias before their griddepcontrol.wait (they are layer constants that may load while
        the previous kernel still runs), so the preparation kernels must have finished before a conv can be launched behind them */
     cudaStreamSynchronize(0);
     return c;
+}
+/* A conv for one call on weights that may change before the next one: c is the caller's, its images live in scratch and are made by the first
+   kernel that asks for them (image_for_call), in stream order; nothing is allocated, copied or waited for once the scratch has its size.  The
+   caller keeps other users of that scratch out (lp_entry.cu's lock) and leaves no pointer to c behind. */
+void umx_conv_per_call(umx_conv *c, int kind, const float *w_dev, const float *bias_dev, int co, int ci, int bits) {
+    conv_geometry(c, kind, co, ci, bits);
+    c->w_src = w_dev; c->b_src = bias_dev;
+}
+/* which 0: the general kernel's image, 1: the z-marching kernel's; true when it is there.  The launch that follows one made here must not start
+   early: umx_plain_launch is raised until the caller's launch is out. */
+static bool image_for_call(umx_conv *c, int which) {
+    if (which ? c->wr != nullptr : c->wpk != nullptr) return true;
+    if (!c->w_src) return false;
+    c->bias_p = (float *)umx_ws(15, (size_t)c->cop * 4);
+    RImageGeo g; memset(&g, 0, sizeof g);
+    if (which) { if (!umx_conv_r_image(c, &g)) return false; c->wr = (uint8_t *)umx_ws(14, (size_t)g.w_bytes * g.ncol); }
+    else c->wpk = (uint8_t *)umx_ws(13, wpk_bytes(c));
+    if (!c->bias_p || (which ? !c->wr : !c->wpk)) return false;
+    PrepArgs p = prep_args(c, c->w_src, c->b_src);
+    if (which) p.wpk = nullptr;
+    umx_prep_w27(p, which ? c->wr : nullptr, g.nt, g.w_bytes, g.w_codes, g.gt, g.goff1, g.goff2);
+    umx_plain_launch = 1;
+    return true;
 }
 extern "C" umx_conv *umx_conv_create_dev(int kind, const float *w_dev, const float *bias_dev, int co, int ci, int bits) { return conv_build(kind, w_dev, bias_dev, co, ci, bits); }
 extern "C" umx_conv *umx_conv_create(int kind, const float *w, const float *bias, int co, int ci, int bits) {
@@ -531,8 +571,7 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     const size_t S = (size_t)D * H * W;
     const int rb = c->bits == 8 ? 32 : 16;
     a.x_sc = (const uint8_t *)x + (size_t)N * nbx * Sx * rb;
-    a.wpk = c->wpk;
-    a.e.N = N; a.e.D = D; a.e.H = H; a.e.W = W; a.e.cop = c->cop; a.e.bias = c->bias_p;
+    a.e.N = N; a.e.D = D; a.e.H = H; a.e.W = W; a.e.cop = c->cop;
     a.e.out_mode = out_mode; a.e.out_bits = out_bits; a.e.tconv = c->kind == UMX_TCONV2; a.e.co_real = c->co; a.e.cob_t = c->cob_t;
     a.e.nb_dst = nb_dst ? nb_dst : c->cob_t; a.e.b0 = nb_dst ? b0 : 0;
     a.e.y = y; a.e.y_split = (flags & UMX_Y_SPLIT) != 0; a.err = umx_errflag();
@@ -543,8 +582,8 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     if (c->bits == 8 && !(flags & UMX_X_SPLIT)) {   /* reference layout: re-lay the codes into scratch first */
         void *ws = umx_ws(1, umx_mx_bytes32(8, N, nbx * 32, Sx));
         if (!ws) return -1;
-        umx_mx_relayout(x, 8, N, nbx * 32, Sx, ws, UMX_LAYOUT_SPLIT);
-        x = ws; a.x_sc = (const uint8_t *)x + (size_t)N * nbx * Sx * 32;
+        umx_mx_codes_to_split(x, (size_t)N * nbx, Sx, ws);         /* the scale plane stays where it is */
+        x = ws;
     }
     CUtensorMap m0; memset(&m0, 0, sizeof m0);
     if (s2) {
@@ -567,11 +606,13 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     static int force_v1 = -1;
     if (force_v1 < 0) { const char *ev = getenv("UMX_CONV_V1"); force_v1 = ev && *ev && *ev != '0'; }
     /* InstanceNorm statistics are a separate pass over the stored output (umx_in_part below) */
-    if (!force_v1 && c->wr) {   /* resident weights: the persistent z-marching kernel, when the geometry allows */
+    if (!force_v1 && (c->wr || (c->w_src && c->kind == UMX_CONV3 && umx_conv_r_takes(c, a.x_sc, N, D, H, W, a.e) && image_for_call((umx_conv *)c, 1)))) {   /* resident weights: the persistent z-marching kernel, when the geometry allows */
         const int pid = umx_prof_open(flops);
-        int rc = (nrm && (flags & UMX_STATS_EPILOGUE)) ? umx_conv_fwd_r(c, x, &m0, (void *)enc, N, D, H, W, a.e, part, nrm->gamma, nrm->beta, nrm->eps, nrm->coef) : 1;
+        a.e.bias = c->bias_p;
+        int rc = (nrm && (flags & UMX_STATS_EPILOGUE)) ? umx_conv_fwd_r(c, a.x_sc, &m0, (void *)enc, N, D, H, W, a.e, part, nrm->gamma, nrm->beta, nrm->eps, nrm->coef) : 1;
         const bool fused = rc == 0;
-        if (rc > 0) rc = umx_conv_fwd_r(c, x, &m0, (void *)enc, N, D, H, W, a.e, nullptr, nullptr, nullptr, 0.f, nullptr);
+        if (rc > 0) rc = umx_conv_fwd_r(c, a.x_sc, &m0, (void *)enc, N, D, H, W, a.e, nullptr, nullptr, nullptr, 0.f, nullptr);
+        umx_plain_launch = 0;
         if (rc <= 0) {
             umx_prof_close(pid);
             g_umx_launches++; g_last_kernel = 1;
@@ -581,9 +622,10 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
             return rc;
         }
     }
+    a.e.bias = c->bias_p;
     if (!force_v1 && c->wp) {   /* one tap, resident weights: the streaming kernel */
         const int pid = umx_prof_open(flops);
-        const int rc = umx_conv_fwd_p(c, x, (void *)enc, N, D, H, W, a.e);
+        const int rc = umx_conv_fwd_p(c, x, a.x_sc, (void *)enc, N, D, H, W, a.e);
         if (rc <= 0) {
             umx_prof_close(pid);
             g_umx_launches++; g_last_kernel = 2;
@@ -602,13 +644,15 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         if (rc == 0) umx_h16_to_prob_u8(t, ny, (uint8_t *)y);
         return rc;
     }
+    if (!image_for_call((umx_conv *)c, 0)) return -1;
+    a.wpk = c->wpk; a.e.bias = c->bias_p;
     const size_t smem = 1024 + (size_t)a.ring * a.stage_bytes;
     static size_t smem_set[16];
     int dev = 0; cudaGetDevice(&dev); dev &= 15;
     if (smem_set[dev] < smem) {
         cudaError_t e = cudaFuncSetAttribute(conv_mx_k<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_mx_k<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024));
-        if (e != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", e); return -1; }
+        if (e != cudaSuccess) { umx_plain_launch = 0; umx_latch("umx_conv_fwd: shared memory attribute", e); return -1; }
         smem_set[dev] = 227 * 1024;
     }
     /* K split for the layers with fewer tiles than multiprocessors (the deep levels); chosen from one sample's geometry so that a sample's
@@ -629,7 +673,7 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         if (!no_split && ks >= 2 && tiles_all <= 8192) {
             const size_t bytes = (size_t)tiles_all * (size_t)ks * (size_t)(c->nt >> 5) * 4096 * 4;
             void *ws = umx_ws(5, bytes);
-            if (!ws) return -1;
+            if (!ws) { umx_plain_launch = 0; return -1; }
             a.ks_tickets = tickets_of[d0];
             a.ksplit = (int)ks; a.ks_part = (float *)ws;
         }
@@ -637,6 +681,7 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     const dim3 grid(a.tiles_x * a.tiles_y, D, N * a.ntiles_n * a.ksplit);
     const int pid = umx_prof_open(flops);
     if (c->bits == 8) umx_launch(conv_mx_k<8>, grid, dim3(kThreads), smem, m0, a); else umx_launch(conv_mx_k<4>, grid, dim3(kThreads), smem, m0, a);
+    umx_plain_launch = 0;
     umx_prof_close(pid);
     g_umx_launches++; g_last_kernel = 0;
     UMX_CK("umx_conv_fwd");

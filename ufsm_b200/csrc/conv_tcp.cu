@@ -310,7 +310,7 @@ uint8_t *umx_conv_p_prepare(const umx_conv *c, const float *w_dev) {
 }
 /* x: MX tensor (fp8 in the split layout).  Returns 1 when this kernel does not apply (the caller takes the general kernel), 0 after a
    launch, -1 on error. */
-int umx_conv_fwd_p(const umx_conv *c, const void *x, void *enc_v, int N, int D, int H, int W, const EpiArgs &e) {
+int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *enc_v, int N, int D, int H, int W, const EpiArgs &e) {
     typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     PGeo g; ConvPArgs a; memset(&a, 0, sizeof a);
@@ -337,7 +337,6 @@ int umx_conv_fwd_p(const umx_conv *c, const void *x, void *enc_v, int N, int D, 
         const cuuint64_t gd[2] = {(cuuint64_t)S * 2, (cuuint64_t)planes}, gs[1] = {(cuuint64_t)S * 16};
         const cuuint32_t box[2] = {256, 2}, es[2] = {1, 1};
         if (((encode_fn)enc_v)(&m0, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void *)x, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
-        uint8_t *x_sc = (uint8_t *)x + (size_t)N * c->nkb * S * (c->bits == 8 ? 32 : 16);
         const cuuint64_t gd2[2] = {(cuuint64_t)S, (cuuint64_t)N * c->nkb}, gs2[1] = {(cuuint64_t)S};
         const cuuint32_t box2[2] = {128, (cuuint32_t)a.sw_rows};
         if (((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)x_sc, gd2, gs2, box2, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;

@@ -567,45 +567,6 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, (uint32_t)a.tmem_cols); }
 }
 
-/* Weight image of the z-marching kernel: codes [input item][dy dx][k half][dz * nt + channel][16 B], then the B scale bytes in the TMEM
-   scale layout per (input item, tap quad, first dz of the MMA, 128-row group): byte (lane, column, id) = row 128 g + 32 column + lane counted
-   from that dz's first row, tap 4 q + id (fp8) or tap 2 q + id / 2, block id % 2 (fp4).  A block-scaled MMA wants its scale address on a
-   4-column boundary of TMEM (a one-column offset faults with "misaligned address"), hence one re-based image per starting dz.
-   Quantisation per (row, tap, 32 input channels) as the reference's prep_w8_k / prep_w4_k (src/lp_f8fwd.cu:54-71, src/lp_f4fwd.cu:53-66).
-   One thread per (item, dy dx, dz, channel). */
-__global__ void __launch_bounds__(128) prep_wr_k(const float *__restrict__ w, uint8_t *__restrict__ wr_all, int co, int ci, int bits, int nt, int nkb, int nki, int nquad, int gt, int goff1, int goff2, int w_codes, int w_bytes) {
-    const int total = nki * 9 * 3 * nt, i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    uint8_t *wr = wr_all + (size_t)blockIdx.y * w_bytes;      /* one image per column tile */
-    const int cl = i % nt, c = blockIdx.y * nt + cl, dz = (i / nt) % 3, j = (i / (3 * nt)) % 9, ki = i / (27 * nt);
-    const int tap = dz * 9 + j, R3 = 3 * nt, row = dz * nt + cl;
-    unsigned wd[8], sb[2] = {127u, 127u};
-    float v[32];
-    if (bits == 8) {
-#pragma unroll
-        for (int k = 0; k < 32; k++) { const int cc = ki * 32 + k; v[k] = (c < co && cc < ci) ? w[((size_t)c * ci + cc) * 27 + tap] : 0.f; }
-        sb[0] = mx_encode_row32<8>(v, wd);
-    } else {
-        unsigned w4[4];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-#pragma unroll
-            for (int k = 0; k < 32; k++) { const int cc = (2 * ki + h) * 32 + k; v[k] = (c < co && cc < ci && 2 * ki + h < nkb) ? w[((size_t)c * ci + cc) * 27 + tap] : 0.f; }
-            sb[h] = mx_encode_row32<4>(v, w4);
-#pragma unroll
-            for (int t = 0; t < 4; t++) wd[4 * h + t] = w4[t];
-        }
-    }
-    uint8_t *base = wr + (size_t)(ki * 9 + j) * 2 * R3 * 16;
-    *(uint4 *)(base + (size_t)row * 16) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-    *(uint4 *)(base + (size_t)(R3 + row) * 16) = make_uint4(wd[4], wd[5], wd[6], wd[7]);
-    for (int d = 0; d <= dz; d++) {
-        const int rr = row - d * nt, g = rr >> 7, col = (rr & 127) >> 5, l = rr & 31, gb = d == 0 ? 0 : d == 1 ? goff1 : goff2;
-        if (bits == 8) wr[w_codes + ((ki * nquad + (j >> 2)) * gt + gb + g) * 512 + l * 16 + col * 4 + (j & 3)] = (uint8_t)sb[0];
-        else { uint8_t *p = wr + w_codes + ((ki * nquad + (j >> 1)) * gt + gb + g) * 512 + l * 16 + col * 4 + (j & 1) * 2; p[0] = (uint8_t)sb[0]; p[1] = (uint8_t)sb[1]; }
-    }
-}
-
 }   // namespace
 
 /* after a bounded wait gave up, blocks may have left without drawing their ticket: the counters start from zero again */
@@ -664,30 +625,22 @@ static int r_geometry(const umx_conv *c, RGeo *g) {
    slot windows and several-planes-a-block regime that otherwise only volumes with thousands of tile planes reach */
 static int g_r_block_cap = 0;
 extern "C" void umx_conv_r_block_cap(int cap) { g_r_block_cap = cap > 0 ? cap : 0; }
-int umx_conv_r_fits(const umx_conv *c) { RGeo g; return r_geometry(c, &g); }
-/* builds the weight image from device fp32 weights [co][ci][27]; called once when the conv is created */
-uint8_t *umx_conv_r_prepare(const umx_conv *c, const float *w_dev) {
+/* Weight image of the z-marching kernel (made by umx_prep_w27): codes [input item][dy dx][k half][dz * nt + channel][16 B], then the B scale
+   bytes in the TMEM scale layout per (input item, tap quad, first dz of the MMA, 128-row group): byte (lane, column, id) = row 128 g + 32
+   column + lane counted from that dz's first row, tap 4 q + id (fp8) or tap 2 q + id / 2, block id % 2 (fp4).  A block-scaled MMA wants its
+   scale address on a 4-column boundary of TMEM (a one-column offset faults with "misaligned address"), hence one re-based image per
+   starting dz.  0 when the kernel cannot run this conv. */
+int umx_conv_r_image(const umx_conv *c, RImageGeo *o) {
     RGeo g;
-    if (!r_geometry(c, &g)) return nullptr;
-    uint8_t *wr = (uint8_t *)nn_malloc((size_t)g.w_bytes * g.ncol);
-    if (!wr) return nullptr;
-    cudaMemset(wr, 127, (size_t)g.w_bytes * g.ncol);
-    const int total = c->nki * 27 * g.nt;
-    prep_wr_k<<<dim3((total + 127) / 128, g.ncol), 128>>>(w_dev, wr, c->co, c->ci, c->bits, g.nt, c->nkb, c->nki, c->nquad, g.gt, g.goff1, g.goff2, g.w_codes, g.w_bytes);
-    g_umx_launches++;
-    return wr;
+    if (!r_geometry(c, &g)) return 0;
+    o->nt = g.nt; o->ncol = g.ncol; o->w_bytes = g.w_bytes; o->w_codes = g.w_codes; o->gt = g.gt; o->goff1 = g.goff1; o->goff2 = g.goff2;
+    return 1;
 }
-/* x: MX tensor (fp8 in the split layout); m0: tensor map over its codes; enc: the driver's tensor-map encoder (for the scale plane).
-   Returns 1 when this kernel does not apply to the geometry (the caller then takes the general kernel), 0 after a launch, -1 on error. */
-/* coef != NULL (only with the blocked fp16 output): InstanceNorm coefficients are produced by the same launch; part then holds N x (blocks per
-   column tile, at most 512) x cop x 2 doubles of scratch */
-int umx_conv_fwd_r(const umx_conv *c, const void *x, const CUtensorMap *m0, void *enc_v, int N, int D, int H, int W, const EpiArgs &e,
-                   double *part, const float *gamma, const float *beta, float eps, float *coef) {
-    typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    ConvRArgs a; memset(&a, 0, sizeof a);
+/* the launch of this geometry, everything but the operands; 0 when the kernel does not apply */
+static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e, int want_coef, const double *part, ConvRArgs &a, int *grid) {
+    memset(&a, 0, sizeof a);
     RGeo g;
-    if (!r_geometry(c, &g) || !c->wr || (W & 15)) return 1;      /* the scale window needs rows that are multiples of 16 bytes */
+    if (!r_geometry(c, &g) || (W & 15) || ((size_t)x_sc & 15)) return 0;      /* the scale window needs rows that are multiples of 16 bytes */
     a.w_codes = g.w_codes; a.w_bytes = g.w_bytes; a.gt = g.gt; a.goff1 = g.goff1 * 4; a.goff2 = g.goff2 * 4;   /* TMEM column offsets of the dz >= 1, 2 images */
     a.tmem_cols = g.tmem_cols; a.nslot = g.nslot; a.sfa_base = g.sfa_base; a.sfa_cols = g.sfa_cols; a.sfb_base = g.sfb_base;
     a.N = N; a.D = D; a.H = H; a.W = W; a.nkb = c->nkb; a.nki = c->nki; a.bits = c->bits; a.nt = g.nt; a.ncol = g.ncol;
@@ -695,8 +648,8 @@ int umx_conv_fwd_r(const umx_conv *c, const void *x, const CUtensorMap *m0, void
     a.units = (long long)N * a.tiles * D;
     a.nquad = c->nquad;
     a.fast_h16 = e.out_mode == UMX_OUT_H16B && !e.tconv;
-    if (coef && (!a.fast_h16 || !part || g.ncol > 64)) return 1;
-    a.part = part; a.coef = coef; a.gamma = gamma; a.beta = beta; a.eps = eps; a.cop = c->cop;
+    if (want_coef && (!a.fast_h16 || !part || g.ncol > 64)) return 0;
+    a.cop = c->cop;
     /* the codes and the scale window are TMA destinations (128-byte aligned) */
     a.offSW = 5888; a.offSFA = a.offSW + (c->bits == 8 ? 640 : 1152);
     a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
@@ -707,17 +660,35 @@ int umx_conv_fwd_r(const umx_conv *c, const void *x, const CUtensorMap *m0, void
     const int two = g.tmem_cols == 256 && a.off_ring + 4 * a.stage_bytes <= 113 * 1024;
     const int room = (two ? 113 : 227) * 1024 - a.off_ring;
     a.ring = room / a.stage_bytes; if (a.ring > 12) a.ring = 12;
-    if (a.ring < 3) return 1;
+    if (a.ring < 3) return 0;
     long long slots = (long long)sms * (two ? 2 : 1) / g.ncol;      /* blocks per column tile */
-    if (slots < 1) return 1;
+    if (slots < 1) return 0;
     if (g_r_block_cap && slots > g_r_block_cap) slots = g_r_block_cap;
     /* A block pays two halo planes per run: with fewer than eight planes a block (counted for one sample, so that the choice of kernel does not
        depend on the batch) the general kernel is faster.  Volumes with fewer planes than blocks are left here: nothing to gain either way. */
-    { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 1; }
+    { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 0; }
     a.gcol = (int)(a.units < slots ? a.units : slots); if (a.gcol > 512) a.gcol = 512;
-    const int grid = a.gcol * g.ncol;
+    *grid = a.gcol * g.ncol;
+    return 1;
+}
+/* would umx_conv_fwd_r take this conv (its weight image aside)? */
+int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e) {
+    ConvRArgs a; int grid;
+    return r_plan(c, x_sc, N, D, H, W, e, 0, nullptr, a, &grid);
+}
+/* x_sc: the MX tensor's scale plane; m0: tensor map over its codes (fp8 in the split layout); enc: the driver's tensor-map encoder (for the scale plane).
+   Returns 1 when this kernel does not apply to the geometry (the caller then takes the general kernel), 0 after a launch, -1 on error. */
+/* coef != NULL (only with the blocked fp16 output): InstanceNorm coefficients are produced by the same launch; part then holds N x (blocks per
+   column tile, at most 512) x cop x 2 doubles of scratch */
+int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, void *enc_v, int N, int D, int H, int W, const EpiArgs &e,
+                   double *part, const float *gamma, const float *beta, float eps, float *coef) {
+    typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    ConvRArgs a; int grid;
+    if (!c->wr || !r_plan(c, x_sc, N, D, H, W, e, coef != nullptr, part, a, &grid)) return 1;
+    a.part = part; a.coef = coef; a.gamma = gamma; a.beta = beta; a.eps = eps;
+    int dev = 0; cudaGetDevice(&dev);
     const size_t S = (size_t)D * H * W;
-    uint8_t *x_sc = (uint8_t *)x + (size_t)N * c->nkb * S * (c->bits == 8 ? 32 : 16);   /* the scale plane follows the codes in either layout */
     CUtensorMap ms; memset(&ms, 0, sizeof ms);
     {
         const cuuint64_t gd[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N * c->nkb};
@@ -739,7 +710,7 @@ int umx_conv_fwd_r(const umx_conv *c, const void *x, const CUtensorMap *m0, void
         }
         attr_set[dev & 15] = 1;
     }
-    const int variant = (coef ? 4 : 0) | (c->bits == 8 ? 0 : 2) | (g.nt == 32 ? 0 : 1);
+    const int variant = (coef ? 4 : 0) | (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
     switch (variant) {
     case 0: umx_launch(conv_mxr_k<8, 1, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
     case 1: umx_launch(conv_mxr_k<8, 2, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;

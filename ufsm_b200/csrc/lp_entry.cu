@@ -5,17 +5,26 @@
    sums of the stored output), zi0 / Di, zw0 / zw1, yD / yzo (z range, z window, slab output), accum; sr / osr / o_pad stop with
    "not built". */
 #include "mx_common.cuh"
+#include "conv_epi.cuh"
+#include <mutex>
 #include <stdlib.h>
 #include <string.h>
 
+void umx_conv_per_call(umx_conv *c, int kind, const float *w_dev, const float *bias_dev, int co, int ci, int bits);
+void umx_ws_free(int slot);
+/* One call at a time puts its work on the stream: the scratch tensors and, for weights without a key, the images made for the call belong to it
+   until its last launch is out; the next call's launches follow in stream order. */
+static std::recursive_mutex g_lp_mu;
 struct memo_t { unsigned wkey; const float *w, *b; int cout, cin, bits, dev; umx_conv *c; };
 static memo_t g_memo[256];
 static int g_nmemo = 0;
 
 extern "C" void lp_wmemo_clear(void) {
+    std::lock_guard<std::recursive_mutex> lock(g_lp_mu);
     cudaDeviceSynchronize();
     for (int i = 0; i < g_nmemo; i++) umx_conv_free(g_memo[i].c);
     g_nmemo = 0;
+    for (int slot = 13; slot < 16; slot++) umx_ws_free(slot);     /* the images of calls without a key */
 }
 int umx_gn_silu_apply(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
                       void *y, int bits, int layout, int form);
@@ -30,6 +39,10 @@ static void slab_check(const char *fn, const gnp_t &gp, shape5 xs) {
         fprintf(stderr, "%s: slab-local GroupNorm with ns %d, zs %d, zo %d, zhw %d on planes of %d voxels\n", fn, gp.ns, gp.zs, gp.zo, gp.zhw, xs.h * xs.w); abort();
     }
 }
+int umx_gn_silu_apply_to(const void *x, int xdt, int N, int C, size_t S, int G, const float *gamma, const float *beta, const float *mean, const float *rstd,
+                         void *y, int bits, int layout, int form, int c_off, int C_all, int ns, int zs, int zo, size_t zhw, int nb_dst, int b0);
+void umx_up2_to(const char *fn, const void *x, int xdt, shape5 xs, void *y, int ydt, gnp_t gp, int nb_dst, int b0, int split);
+void umx_mx_blocks_put(const void *src, int bits, int N, int nb_src, size_t S, void *dst, int nb_dst, int b0, int to_split);
 static const void *gn_input(const char *fn, const void *x, int xbf, shape5 xs, gnp_t gp, int bits) {
     slab_check(fn, gp, xs);
     const size_t S = (size_t)xs.d * xs.h * xs.w;
@@ -42,6 +55,7 @@ static const void *gn_input(const char *fn, const void *x, int xbf, shape5 xs, g
 }
 int umx_gn_sums_pm32(const float *x, int N, int C, int G, size_t S, double *sums, size_t v0, size_t v1);
 __global__ void f32_to_h16_k(const float *__restrict__ x, __half *__restrict__ y, size_t n) {
+    pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) y[i] = __float2half_rn(x[i]);
 }
 static void not_built(const char *fn, const char *what) { fprintf(stderr, "%s: %s is not built in this library\n", fn, what); abort(); }
@@ -55,19 +69,12 @@ int umx_gn_silu_apply_seg(const void *x, int xdt, int N, int C, size_t S, int G,
 extern "C" void umx_pm_to_mx32_cat(const void *x, const void *x2, int c2, int dt, int N, int C, size_t S, void *y, int bits, int layout);
 static inline int up32(int c) { return (c + 31) / 32 * 32; }
 
-/* blocks [0, nb_src) of every sample of an MX tensor (reference layout) to blocks [b0, b0 + nb_src) of one with nb_dst blocks, or back */
-static void mx_blocks_copy(uint8_t *dst, int nb_dst, int b0, const uint8_t *src, int nb_src, int N, size_t S, int bits, bool gather) {
+/* blocks [b0, b0 + nb) of every sample of an MX tensor of nb_all blocks (reference layout) as a tensor of their own */
+static void mx_blocks_take(const uint8_t *all, int nb_all, int b0, uint8_t *dst, int nb, int N, size_t S, int bits) {
     const size_t rb = bits == 8 ? 32 : 16;
     for (int n = 0; n < N; n++) {
-        uint8_t *dc = dst + ((size_t)n * nb_dst + b0) * S * rb, *ds = dst + (size_t)N * nb_dst * S * rb + ((size_t)n * nb_dst + b0) * S;
-        const uint8_t *sc = src + (size_t)n * nb_src * S * rb, *ss = src + (size_t)N * nb_src * S * rb + (size_t)n * nb_src * S;
-        if (gather) {          /* dst is the small tensor */
-            cudaMemcpyAsync((uint8_t *)sc, dc, (size_t)nb_src * S * rb, cudaMemcpyDeviceToDevice, 0);
-            cudaMemcpyAsync((uint8_t *)ss, ds, (size_t)nb_src * S, cudaMemcpyDeviceToDevice, 0);
-        } else {
-            cudaMemcpyAsync(dc, sc, (size_t)nb_src * S * rb, cudaMemcpyDeviceToDevice, 0);
-            cudaMemcpyAsync(ds, ss, (size_t)nb_src * S, cudaMemcpyDeviceToDevice, 0);
-        }
+        cudaMemcpyAsync(dst + (size_t)n * nb * S * rb, all + ((size_t)n * nb_all + b0) * S * rb, (size_t)nb * S * rb, cudaMemcpyDeviceToDevice, 0);
+        cudaMemcpyAsync(dst + ((size_t)N * rb + n) * nb * S, all + (size_t)N * nb_all * S * rb + ((size_t)n * nb_all + b0) * S, (size_t)nb * S, cudaMemcpyDeviceToDevice, 0);
     }
 }
 /* weights [co][ci][taps] and bias of the logical conv -> those of the conv on padded segments: input channel ci sits at ci (ci < cx) or
@@ -119,11 +126,13 @@ static void *slab_of(int slot, const void *x, int bf, int N, int C, int D, size_
 }
 /* y (fp16 plane-major, n elements) += t */
 __global__ void __launch_bounds__(256) h16_add_k(__half *__restrict__ y, const __half *__restrict__ t, size_t n) {
+    pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) y[i] = __float2half_rn(__fadd_rn(__half2float(y[i]), __half2float(t[i])));
 }
 
 static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs, const float *w, const float *b, int cout, void *y, int ybf, gnp_t gp, double *osum, int Go, split_t sp) {
     if (!umx_ready(fn)) return 0;
+    std::lock_guard<std::recursive_mutex> lock(g_lp_mu);
     if (sp.sr || sp.osr) not_built(fn, "stochastic rounding (split_t.sr / osr)");
     /* o_pad places the second output tensor's rows inside the reference's padded GEMM (src/nn_lp.h:32): here each output tensor has its own
        blocks whatever it says; the values the reference uses are accepted */
@@ -140,7 +149,7 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         split_t s2 = sp; s2.accum = 0;
         conv_fwd(fn, bits, x, xbf, xs, w, b, cout, t, ybf, gp, nullptr, 0, s2);
         size_t g = (ny + 255) / 256; if (g > 148u * 16u) g = 148u * 16u;
-        if (ny) h16_add_k<<<(unsigned)g, 256>>>((__half *)y, t, ny);
+        if (ny) umx_launch(h16_add_k, dim3((unsigned)g), dim3(256), 0, (__half *)y, t, ny);
         UMX_CK(fn);
         return 0;
     }
@@ -253,7 +262,7 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         umx_pm_to_mx32_cat(x, sp.x2, Cx, UMX_F16, xs.n, Ci, S, ws, bits, UMX_LAYOUT_SPLIT);
         xq = ws; xflags = UMX_X_SPLIT;
     } else {
-        /* segment by segment into an MX tensor of the conv's format (reference layout).  MX segments keep their own 32-channel blocks,
+        /* segment by segment into their blocks of an MX tensor of the conv's format, in the layout the conv reads.  MX segments keep their own 32-channel blocks,
            the x part padded to whole blocks (the reference's "per-tensor 32-channel segments", src/lp_f8fwd.cuh:617-623) */
         if (!x_mx && (Cx & 31)) not_built(fn, "a GroupNorm transform of plane-major concat inputs split inside a 32-channel block");
         const int CxP = up32(Cx), nbA = CxP / 32, nbB = up32(C2) / 32, nbT = nbA + nbB;
@@ -266,39 +275,37 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
             const gnp_t q = s2g ? (seg ? sp.gp2 : gp) : gp;
             const int c_off = s2g ? 0 : (seg ? Cx : 0), C_all = s2g ? C : Ci;
             const bool up = !seg && sp.up;
-            const uint8_t *blocks = nullptr;
             if (up) {
                 if (q.G && !s2g) not_built(fn, "split_t.up with one GroupNorm over both input parts");
-                uint8_t *t = (uint8_t *)umx_ws(3, umx_mx_bytes32(bits, xs.n, C, S));
-                if (!t) return 0;
                 const shape5 cs = {xs.n, C, xs.d / 2, xs.h / 2, xs.w / 2};
-                lp_up2_fwd_mx(src, xbf, cs, t, mxin, q);        /* silu(gn(coarse)) blended, quantised to the conv's rows */
-                blocks = t;
-            } else if (q.G) {
-                uint8_t *t = (uint8_t *)umx_ws(3 + seg, umx_mx_bytes32(bits, xs.n, C, S));
+                if (C > 16) { umx_up2_to(fn, src, xbf, cs, T, mxin, q, nbT, b0, 1); continue; }      /* silu(gn(coarse)) blended, quantised to the conv's rows */
+                uint8_t *t = (uint8_t *)umx_ws(4, umx_mx_bytes32(bits, xs.n, C, S));
                 if (!t) return 0;
+                lp_up2_fwd_mx(src, xbf, cs, t, mxin, q);
+                umx_mx_blocks_put(t, bits, xs.n, nbs, S, T, nbT, b0, 1);
+            } else if (q.G) {
                 slab_check(fn, q, xs);
-                if (umx_gn_silu_apply_seg_slabs(src, xbf, xs.n, C, S, q.G, q.gamma, q.beta, q.mean, q.rstd, t, bits, UMX_LAYOUT_REF, 1, c_off, C_all, q.ns, q.zs, q.zo, (size_t)q.zhw) != 0) {
+                if (umx_gn_silu_apply_to(src, xbf, xs.n, C, S, q.G, q.gamma, q.beta, q.mean, q.rstd, T, bits, UMX_LAYOUT_SPLIT, 1, c_off, C_all, q.ns, q.zs, q.zo, (size_t)q.zhw, nbT, b0) != 0) {
                     fprintf(stderr, "%s: the GroupNorm + SiLU input transform of a storage-%d segment of %d channels (%d groups over %d) is not built in this library\n", fn, xbf, C, q.G, C_all); abort();
                 }
-                blocks = t;
             } else if (x_mx) {
                 if (xbf != mxin) { fprintf(stderr, "%s: an MX-fp%d input segment of an MX-fp%d conv without a transform\n", fn, xb_bits, bits); abort(); }
-                blocks = (const uint8_t *)src;
+                const void *blocks = src;
                 if (C <= 16) {                                 /* rows of 8 / 16 channels: the same codes and scale in a 32-wide row */
-                    uint8_t *t = (uint8_t *)umx_ws(3 + seg, umx_mx_bytes32(bits, xs.n, C, S));
+                    void *t = umx_ws(3 + seg, umx_mx_bytes32(bits, xs.n, C, S));
                     if (!t) return 0;
                     umx_mx_rewidth(src, bits, xs.n, C, S, t, 1);
                     blocks = t;
                 }
+                umx_mx_blocks_put(blocks, bits, xs.n, nbs, S, T, nbT, b0, 1);
             } else {
-                uint8_t *t = (uint8_t *)umx_ws(3 + seg, umx_mx_bytes32(bits, xs.n, C, S));
+                void *t = umx_ws(3 + seg, umx_mx_bytes32(bits, xs.n, C, S));
                 if (!t) return 0;
                 umx_pm_to_mx32(src, UMX_F16, xs.n, C, S, t, bits, UMX_LAYOUT_REF);
-                blocks = t;
+                umx_mx_blocks_put(t, bits, xs.n, nbs, S, T, nbT, b0, 1);
             }
-            mx_blocks_copy(T, nbT, b0, blocks, nbs, xs.n, S, bits, false);
         }
+        xflags = UMX_X_SPLIT;
         xq = T;
     }
 
@@ -306,23 +313,25 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
     const bool pad_in = sp.x2 && cin != Ci, mx_split_out = sp.y2 && out_mode == UMX_OUT_MXRAW, pad_out = mx_split_out && (Ox & 31);
     const int OxP = pad_out ? up32(Ox) : Ox, cout_c = pad_out ? OxP + O2 : cout;
     int dev = 0; cudaGetDevice(&dev);
-    umx_conv *c = nullptr; bool temp = true;
-    if (sp.wkey) {
+    umx_conv *c = nullptr, per_call;
+    const bool keyed = sp.wkey != 0;
+    if (keyed) {
         for (int i = 0; i < g_nmemo; i++) { memo_t &m = g_memo[i]; if (m.wkey == sp.wkey && m.w == w && m.b == b && m.cout == cout_c && m.cin == cin && m.bits == bits && m.dev == dev) { c = m.c; break; } }
-        temp = false;
     }
     if (!c) {
         const float *wc = w, *bc = b;
         if (pad_in || pad_out) {
             const size_t nw = (size_t)cout_c * cin * 27;
-            float *wp = (float *)umx_ws(5, (nw + cout_c) * sizeof(float));     /* slot 5 is also the general kernel's K-split scratch: the weights are prepared (and the stream drained) before a launch asks for it */
+            float *wp = (float *)umx_ws(5, (nw + cout_c) * sizeof(float));     /* slot 5 is also the general kernel's K-split scratch: the preparation reads it ahead of that kernel in the stream */
             if (!wp) return 0;
             w_expand_k<<<(unsigned)((nw + 255) / 256), 256>>>(w, b, wp, wp + nw, cout, Ci, 27, pad_in ? Cx : Ci, pad_in ? up32(Cx) : Ci, cin, Ox, OxP, cout_c);
             wc = wp; bc = wp + nw;
         }
-        c = umx_conv_create_dev(UMX_CONV3, wc, bc, cout_c, cin, bits);
-        if (!c) return 0;
-        if (sp.wkey && g_nmemo < 256) { memo_t m = {sp.wkey, w, b, cout_c, cin, bits, dev, c}; g_memo[g_nmemo++] = m; } else temp = true;
+        if (keyed && g_nmemo < 256) {
+            c = umx_conv_create_dev(UMX_CONV3, wc, bc, cout_c, cin, bits);
+            if (!c) return 0;
+            memo_t m = {sp.wkey, w, b, cout_c, cin, bits, dev, c}; g_memo[g_nmemo++] = m;
+        } else { c = &per_call; umx_conv_per_call(c, UMX_CONV3, wc, bc, cout_c, cin, bits); }
     }
     if (osum && !sp.stored_stats) {
         /* statistics of acc + bias before any rounding (the reference's epilogue sums its fp32 values, src/lp_common.cuh:1465-1598): the conv
@@ -334,7 +343,7 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         if (sp.zlo < 0 || sp.zhi < 0 || sp.zlo + sp.zhi > xs.d) { fprintf(stderr, "%s: zlo %d + zhi %d of %d planes\n", fn, sp.zlo, sp.zhi, xs.d); abort(); }
         if (umx_gn_sums_pm32(P, xs.n, cout, Go, S, osum, v0, v1) != 0) { fprintf(stderr, "%s: output statistics of %d channels in %d groups\n", fn, cout, Go); abort(); }
         if (out_mode == UMX_OUT_MXRAW) { if (out_bits == 8) lp_f32_to_mx8(P, xs.n, cout, S, y); else lp_f32_to_mx4(P, xs.n, cout, S, y); }
-        else { const size_t ny = (size_t)xs.n * cout * S; size_t g = (ny + 255) / 256; if (g > 148u * 16u) g = 148u * 16u; f32_to_h16_k<<<(unsigned)g, 256>>>(P, (__half *)y, ny); }
+        else { const size_t ny = (size_t)xs.n * cout * S; size_t g = (ny + 255) / 256; if (g > 148u * 16u) g = 148u * 16u; umx_launch(f32_to_h16_k, dim3((unsigned)g), dim3(256), 0, P, (__half *)y, ny); }
     } else if (narrow_out) {
         void *t = umx_ws(4, umx_mx_bytes32(out_bits, xs.n, cout, S));
         if (!t) return 0;
@@ -358,10 +367,10 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         for (int part = 0; part < 2; part++) {
             const int Cp = part ? O2 : Ox, nbp = part ? nb2 : nb1, b0 = part ? nb1 : 0;
             uint8_t *dst = (uint8_t *)(part ? sp.y2 : y);
-            if (Cp > 16) { mx_blocks_copy(t, nb1 + nb2, b0, dst, nbp, xs.n, S, out_bits, true); continue; }
+            if (Cp > 16) { mx_blocks_take(t, nb1 + nb2, b0, dst, nbp, xs.n, S, out_bits); continue; }
             uint8_t *one = (uint8_t *)umx_ws(7, umx_mx_bytes32(out_bits, xs.n, Cp, S));      /* a part of 16 channels or fewer is stored in rows of 8 / 16 */
             if (!one) return 0;
-            mx_blocks_copy(t, nb1 + nb2, b0, one, 1, xs.n, S, out_bits, true);
+            mx_blocks_take(t, nb1 + nb2, b0, one, 1, xs.n, S, out_bits);
             umx_mx_rewidth(one, out_bits, xs.n, Cp, S, dst, 0);
         }
         if (osum) {                                            /* Ox ends on a block: the scratch tensor is the cout-channel output */
@@ -376,7 +385,6 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         if (sp.zlo < 0 || sp.zhi < 0 || sp.zlo + sp.zhi > xs.d) { fprintf(stderr, "%s: zlo %d + zhi %d of %d planes\n", fn, sp.zlo, sp.zhi, xs.d); abort(); }
         if (lp_gn_sums_mx(y, ybf, xs.n, cout, Go, S, osum, v0, v1) != 0) { fprintf(stderr, "%s: output statistics of %d channels in %d groups\n", fn, cout, Go); abort(); }
     }
-    if (temp) { cudaDeviceSynchronize(); umx_conv_free(c); }
     UMX_CK(fn);
     return 0;
 }
@@ -390,6 +398,7 @@ extern "C" int lp_conv_fwd_f4(const void *x, int xbf, shape5 xs, const float *w,
 extern "C" int lp_conv_fwd_s2_f8(const void *x, int xbf, shape5 xs, const float *w, const float *b, int cout, void *y, int ybf, shape5 ys, gnp_t gp) {
     const char *fn = "lp_conv_fwd_s2_f8";
     if (!umx_ready(fn)) return 0;
+    std::lock_guard<std::recursive_mutex> lock(g_lp_mu);
     const bool x_mx = xbf == UMX_MX8 || xbf == UMX_MX4;
     if (xbf != UMX_F16 && !x_mx) { fprintf(stderr, "%s: input storage %d (this entry takes fp16 plane-major, MX-fp8 or MX-fp4)\n", fn, xbf); abort(); }
     if (ys.n != xs.n || ys.c != cout || ys.d != (xs.d + 1) / 2 || ys.h != (xs.h + 1) / 2 || ys.w != (xs.w + 1) / 2) {
@@ -425,11 +434,9 @@ extern "C" int lp_conv_fwd_s2_f8(const void *x, int xbf, shape5 xs, const float 
     const bool narrow = out_mode == UMX_OUT_MXRAW && cout <= 16;
     void *yq = y;
     if (narrow) { yq = umx_ws(4, umx_mx_bytes32(out_bits, xs.n, cout, So)); if (!yq) return 0; }
-    umx_conv *c = umx_conv_create_dev(UMX_CONV3S2, w, b, cout, xs.c, bits);
-    if (!c) return 0;
-    umx_conv_fwd(c, xq, xs.n, xs.d, xs.h, xs.w, yq, out_mode, out_bits, 0, 0, nullptr, xflags);
+    umx_conv per_call;
+    umx_conv_per_call(&per_call, UMX_CONV3S2, w, b, cout, xs.c, bits);
+    umx_conv_fwd(&per_call, xq, xs.n, xs.d, xs.h, xs.w, yq, out_mode, out_bits, 0, 0, nullptr, xflags);
     if (narrow) umx_mx_rewidth(yq, out_bits, xs.n, cout, So, y, 0);
-    cudaDeviceSynchronize();
-    umx_conv_free(c);
     return bits == 4 ? 3 : 0;
 }
