@@ -20,7 +20,7 @@
    stage, the nine shifted scale sets from the scale plane into that layout in shared memory, and the MMA thread copies them to
    TMEM with tcgen05.cp before issuing the stage's MMAs.  Out-of-range voxels get scale 1 (their codes are zero).
 
-   Roles (192 threads): warp 0 lane 0 = TMA producer; warp 1 = TMEM allocation, lane 0 = MMA issue; warps 2-5 = scale gather,
+   Roles (224 threads): warp 0 lane 0 = TMA producer; warp 1 = TMEM allocation, lane 0 = MMA issue; warp 6 lane 0 = scale copies; warps 2-5 = scale gather,
    then the epilogue (tcgen05.ld of 32 channels per voxel = one MX block per thread: bias, fp16 store or MX requantisation;
    InstanceNorm partial sums are taken by a separate pass over the stored output).  Every wait is bounded; a wait that gives up records (code, block, stage) in a device
    flag, raises a block-wide abort flag and the block tears down normally. */
@@ -31,9 +31,9 @@
 
 namespace {
 
-constexpr int kThreads = 192;
+constexpr int kThreads = 224;
 constexpr int kTmemCols = 256;
-constexpr int kSfBase = 128;        /* TMEM columns: [0, 128) accumulators, then two scale buffers of 40 (A 20 | B 20) */
+constexpr int kSfBase = 128;        /* TMEM columns: [0, 128) accumulators, then up to three scale buffers of 40 (A 20 | B 20) */
 constexpr long long kWaitLimit = 4000000000ll;   /* clock cycles (about two seconds) */
 
 struct ConvArgs {
@@ -49,17 +49,14 @@ struct ConvArgs {
     int items_max, ipq, nquad;      /* K items per stage, items per scale quad (4 fp8 / 2 fp4), quads per stage */
     const uint8_t *x_sc;
     const uint8_t *wpk;
-    /* K split: ksplit blocks share one output tile, each takes a contiguous range of the stages and leaves its fp32 accumulators in
-       ks_part [tile][split][32-column chunk][column quad][row][4] (a warp's 32 rows of one quad are 512 contiguous bytes); the block that draws the tile's last ticket adds the parts in split order and
-       runs the epilogue (no block waits for another; the order of the additions is fixed) */
-    int ksplit; float *ks_part; unsigned *ks_tickets;
+    /* K split: the ksplit blocks of an output tile are a cluster; each takes a contiguous range of the stages and keeps its fp32 accumulators in shared
+       memory, where the blocks add them up chunk by chunk in split order */
+    int ksplit;
     /* 3^3 stride-2 pad-1 conv: K item = (tap, input block), each item's A tile is its own strided TMA load from the input grid Di x Hi x Wi */
     int s2, nbi, nit, Di, Hi, Wi;       /* stride-2 conv: blocks of the input tensor, K items per tap, input grid */
     EpiArgs e;
     int *err;
 };
-
-__device__ unsigned g_ks_tickets[8192];      /* one per output tile of a split launch; the last block of a tile resets it */
 
 
 __device__ __forceinline__ void raise(const ConvArgs &a, volatile int *abort_flag, int code, int stage) {
@@ -69,16 +66,16 @@ __device__ __forceinline__ void raise(const ConvArgs &a, volatile int *abort_fla
 }
 
 template <int BITS>
-__global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CUtensorMap map0, const ConvArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__ CUtensorMap map0, const ConvArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     /* control block, then the stage ring at the next 1024-byte boundary */
-    uint64_t *bars = (uint64_t *)smem_raw;                       /* [0, ring) tma full, [ring, 2 ring) scale full, [2 ring, 3 ring) empty, 3 ring: accumulator full */
-    uint32_t *tmem_slot = (uint32_t *)(smem_raw + 256);
-    volatile int *abort_flag = (volatile int *)(smem_raw + 260);
+    uint64_t *bars = (uint64_t *)smem_raw;                       /* ring each: tma full, scales in shared memory, scales in TMEM, empty; then accumulator full */
+    uint32_t *tmem_slot = (uint32_t *)(smem_raw + 512);
+    volatile int *abort_flag = (volatile int *)(smem_raw + 516);
     uint8_t *stages = smem_raw + 1024;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int R = a.ring;
-    const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_acc = bar_tma + 24 * R, bar_red = bar_acc + 8;
+    const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_cp = bar_tma + 16 * R, bar_empty = bar_tma + 24 * R, bar_acc = bar_tma + 32 * R;
 
     const int txy = blockIdx.x, tx = txy % a.tiles_x, ty = txy / a.tiles_x;
     const int z = blockIdx.y;
@@ -94,8 +91,8 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
     }
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 128); mbar_init(bar_empty + 8 * i, 1); }
-        mbar_init(bar_acc, 1); mbar_init(bar_red, 128); mbar_init(bar_red + 8, 1);
+        for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 4); mbar_init(bar_cp + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
+        mbar_init(bar_acc, 1);
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
@@ -105,29 +102,53 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_wait();                                  /* from here on the block touches activations */
     const uint32_t tmem = *tmem_slot;
+    const int nbuf = R < 3 ? R : 3;               /* TMEM scale buffers in use */
+    /* with a ring of two the stage that waits for the scale thread is the stage the MMAs need next: the MMA thread copies for itself (128 -> 128 on
+       32^3, two blocks a multiprocessor: 19.1 us, 20.6 with the scale thread between) */
+    const bool own_copies = R < 3;
 
     /* a stage is live unless it is a 3^3 stage whose input plane lies outside the volume (it would add zeros) */
     auto stage_live = [&](int st) -> bool { if (a.taps != 27) return true; const int zi = z + st % 3 - 1; return zi >= 0 && zi < a.D; };
     auto stage_items = [&](int st) -> int { return a.taps == 27 ? 9 : min(4, a.nki - 4 * st); };
 
+    /* a stage's A and B scales from shared memory to TMEM buffer buf (one thread) */
+    auto copy_scales = [&](int st, uint32_t so, int buf) {
+        const uint32_t sf_hi = desc_hi(128), sb0 = smem_u32(stages), sfa_lo = desc_lo(sb0 + a.offSFA, 0) + so, sfb_lo = desc_lo(sb0 + a.offSFB, 0) + so;
+        const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
+        const int nq = a.taps == 27 ? a.nquad : (stage_items(st) + a.ipq - 1) / a.ipq;
+        for (int q = 0; q < nq; q++) {
+            utccp_32x128b(sfa_t + 4 * q, desc_make(sfa_lo + 32u * q, sf_hi));
+            utccp_32x128b(sfb_t + 4 * q, desc_make(sfb_lo + 32u * q, sf_hi));
+        }
+    };
+
     if (warp == 0) {
         /* ---------------- TMA producer ---------------- */
         if (lane == 0) {
             tma_prefetch_desc(&map0);
-            int it = 0;
             const uint8_t *wbase = a.wpk + (size_t)ntile * a.nst * a.w_stage_bytes;
+            auto put_weights = [&](int st, int s) {
+                const uint32_t bar = bar_tma + 8 * s;
+                const int abytes = a.taps == 27 ? 5760 : stage_items(st) * 4096;
+                mbar_expect_tx(bar, (uint32_t)(abytes + a.w_stage_bytes));
+                bulk_g2s(smem_u32(stages + (size_t)s * a.stage_bytes + a.offW), wbase + (size_t)st * a.w_stage_bytes, (uint32_t)a.w_stage_bytes, bar);
+            };
+            /* the weights of the first ring's stages are constants of the layer: they load while the previous kernel of the stream is still running */
+            int early = 0;
+            for (int st = st_lo; st < st_hi && early < R; st++) if (stage_live(st)) put_weights(st, early++);
+            pdl_wait();                          /* from here on this thread touches activations */
+            int it = 0;
             for (int st = st_lo; st < st_hi; st++) {
                 if (!stage_live(st)) continue;
                 const int s = it % R, ph = (it / R) & 1;
-                if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 1, st); break; }
                 uint8_t *sb = stages + (size_t)s * a.stage_bytes;
                 const uint32_t bar = bar_tma + 8 * s;
                 const int items = stage_items(st);
-                const int abytes = a.taps == 27 ? 5760 : items * 4096;
-                mbar_expect_tx(bar, (uint32_t)(abytes + a.w_stage_bytes));
-                bulk_g2s(smem_u32(sb + a.offW), wbase + (size_t)st * a.w_stage_bytes, (uint32_t)a.w_stage_bytes, bar);
+                if (it >= early) {
+                    if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 1, st); break; }
+                    put_weights(st, s);
+                }
                 /* two 16-byte-wide planes per K item (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1) */
                 if (a.taps == 27) {
                     const int ki = st / 3, zi = z + st % 3 - 1;
@@ -152,38 +173,54 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
         if (lane == 0) {
             int it = 0, s = 0, ph = 0; bool ok = true;
             const uint32_t sb0 = smem_u32(stages), sstep = (uint32_t)a.stage_bytes >> 4;
-            const uint32_t sf_hi = desc_hi(128), b_hi = desc_hi(128), a_hi = a.taps == 27 ? desc_hi(160) : desc_hi(128);
-            const uint32_t sfa_lo0 = desc_lo(sb0 + a.offSFA, 0), sfb_lo0 = desc_lo(sb0 + a.offSFB, 0);
+            const uint32_t b_hi = desc_hi(128), a_hi = a.taps == 27 ? desc_hi(160) : desc_hi(128);
             const uint32_t a_lo0 = desc_lo(sb0 + a.offA, a.taps == 27 ? 2880 : 2048), b_lo0 = desc_lo(sb0 + a.offW, (uint32_t)a.nt * 16);
             const uint32_t idesc0 = BITS == 8 ? idesc_mxf8(n_cur, 0, 0) : idesc_mxf4(n_cur, 0, 0);
             const uint32_t bstep = (uint32_t)a.nt * 2;
+            int buf = 0;
             for (int st = st_lo; st < st_hi && ok; st++) {
                 if (!stage_live(st)) continue;
-                if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 3, st); ok = false; break; }
-                if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 2, st); ok = false; break; }
-                tc_fence_after();
                 const uint32_t so = (uint32_t)s * sstep;
-                const uint32_t sfa_t = tmem + kSfBase + (it & 1) * 40, sfb_t = sfa_t + 20;
-                if (a.taps == 27) {
-                    constexpr int NQ = BITS == 8 ? 3 : 5;
-#pragma unroll
-                    for (int q = 0; q < NQ; q++) {
-                        utccp_32x128b(sfa_t + 4 * q, desc_make(sfa_lo0 + so + 32u * q, sf_hi));
-                        utccp_32x128b(sfb_t + 4 * q, desc_make(sfb_lo0 + so + 32u * q, sf_hi));
-                    }
-                    issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9);
+                const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
+                if (own_copies) {
+                    if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 3, st); ok = false; break; }
+                    if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 2, st); ok = false; break; }
+                    tc_fence_after();
+                    copy_scales(st, so, buf);
                 } else {
-                    const int items = stage_items(st), nq = (items + a.ipq - 1) / a.ipq;
-                    for (int q = 0; q < nq; q++) {
-                        utccp_32x128b(sfa_t + 4 * q, desc_make(sfa_lo0 + so + 32u * q, sf_hi));
-                        utccp_32x128b(sfb_t + 4 * q, desc_make(sfb_lo0 + so + 32u * q, sf_hi));
-                    }
-                    issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, items);
+                    /* the scale thread passed the stage's load barrier before it copied the scales, so codes and weights have landed too */
+                    if (!mbar_wait(bar_cp + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 3, st); ok = false; break; }
+                    tc_fence_after();
                 }
+                if (a.taps == 27) issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9);
+                else issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, stage_items(st));
                 umma_commit(bar_empty + 8 * s);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
+                if (++buf == nbuf) buf = 0;
             }
             umma_commit(bar_acc);   /* also after a give-up: the epilogue must not wait for its full limit */
+        }
+    } else if (warp == 6) {
+        /* ---------------- scale copies: one thread brings a stage's A and B scales from shared memory to one of nbuf TMEM buffers.  A tcgen05.cp costs
+           the thread that issues it some 40 clocks and the tensor pipe next to nothing, so it is kept out of the MMA thread (a stage of nine N = 128
+           MMAs: 1050 clocks with the six copies in it, 576 of them arithmetic). ---------------- */
+        if (lane == 0 && !own_copies) {
+            const uint32_t sstep = (uint32_t)a.stage_bytes >> 4;
+            int it = 0, s = 0, ph = 0, s3 = 0, ph3 = 0, buf = 0;
+            for (int st = st_lo; st < st_hi; st++) {
+                if (!stage_live(st)) continue;
+                if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 2, st); break; }
+                if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 4, st); break; }
+                if (it >= nbuf) {                /* the MMAs that read this buffer (nbuf stages back; nbuf <= ring, so that barrier is at most one phase ahead) */
+                    if (!mbar_wait(bar_empty + 8 * s3, ph3, abort_flag, kWaitLimit)) { raise(a, abort_flag, 7, st); break; }
+                    if (++s3 == R) { s3 = 0; ph3 ^= 1; }
+                }
+                tc_fence_after();
+                copy_scales(st, (uint32_t)s * sstep, buf);
+                umma_commit(bar_cp + 8 * s);
+                it++; if (++s == R) { s = 0; ph ^= 1; }
+                if (++buf == nbuf) buf = 0;
+            }
         }
     } else {
         /* ---------------- scale gather, then epilogue ---------------- */
@@ -192,120 +229,94 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
         const int oy = y0 + ry, ox = x0 + rx;
         const bool row_ok = oy < a.H && ox < a.W;
         const size_t S = (size_t)a.D * a.H * a.W;
-        int it = 0; bool ok = true;
-        for (int st = st_lo; st < st_hi && ok; st++) {
-            if (!stage_live(st)) continue;
-            const int s = it % R, ph = (it / R) & 1;
-            if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 4, st); ok = false; break; }
-            uint32_t *sfa = (uint32_t *)(stages + (size_t)s * a.stage_bytes + a.offSFA);
-            const int items = stage_items(st);
-            uint32_t wq[5] = {0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu};
+        pdl_wait();
+        /* The scale bytes of a stage come straight from the scale plane, an L2 round trip.  They are asked for a stage ahead of their use, so that the
+           trip of one stage overlaps the packing of the one before: without that the gather was the pipeline's slowest role (a stage of the
+           320 -> 320 conv on 8^3 1650 clocks). */
+        constexpr int NB = 9 * (BITS == 8 ? 1 : 2);
+        unsigned raw[NB];
+        unsigned inm = 0u;                                       /* 3^3: the taps of this row that lie inside the plane */
+        int toff[3];                                             /* and the offsets of its three tap rows */
+        if (a.taps == 27) {
+#pragma unroll
+            for (int j = 0; j < 9; j++) { const int iy = oy + j / 3 - 1, ix = ox + j % 3 - 1; if (iy >= 0 && iy < a.H && ix >= 0 && ix < a.W) inm |= 1u << j; }
+#pragma unroll
+            for (int k = 0; k < 3; k++) toff[k] = (oy + k - 1) * a.W + ox - 1;
+        }
+        auto load_scales = [&](int st) {
             if (a.taps == 27) {
                 const int ki = st / 3, zi = z + st % 3 - 1;
+                const uint8_t *p = a.x_sc + ((size_t)n * a.nkb + (BITS == 8 ? ki : 2 * ki)) * S + (size_t)zi * a.H * a.W;
+                const bool two = BITS == 4 && 2 * ki + 1 < a.nkb;
 #pragma unroll
                 for (int j = 0; j < 9; j++) {
-                    const int iy = oy + j / 3 - 1, ix = ox + j % 3 - 1;
-                    const bool in = iy >= 0 && iy < a.H && ix >= 0 && ix < a.W;
-                    const size_t vox = ((size_t)zi * a.H + iy) * a.W + ix;
-                    if (BITS == 8) {
-                        const unsigned b = in ? a.x_sc[((size_t)n * a.nkb + ki) * S + vox] : 127u;
-                        wq[j >> 2] = (wq[j >> 2] & ~(0xffu << (8 * (j & 3)))) | (b << (8 * (j & 3)));
-                    } else {
-                        const unsigned b0 = in ? a.x_sc[((size_t)n * a.nkb + 2 * ki) * S + vox] : 127u;
-                        const unsigned b1 = (in && 2 * ki + 1 < a.nkb) ? a.x_sc[((size_t)n * a.nkb + 2 * ki + 1) * S + vox] : 127u;
-                        const unsigned h = b0 | (b1 << 8);
-                        wq[j >> 1] = (wq[j >> 1] & ~(0xffffu << (16 * (j & 1)))) | (h << (16 * (j & 1)));
-                    }
+                    const bool in = (inm >> j) & 1u;
+                    raw[j] = in ? __ldg(p + toff[j / 3] + j % 3) : 127u;
+                    if (BITS == 4) raw[9 + j] = in && two ? __ldg(p + S + toff[j / 3] + j % 3) : 127u;
                 }
             } else {
+                const int items = stage_items(st);
                 const size_t vox = ((size_t)z * a.H + oy) * a.W + ox;
-                for (int j = 0; j < items; j++) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    raw[j] = 127u; if (BITS == 4) raw[9 + j] = 127u;
+                    if (j >= items) continue;
                     const int ki = 4 * st + j;
                     if (a.s2) {
                         const int tap = ki / a.nit, blk = ki - tap * a.nit;
                         const int iz = 2 * z + tap / 9 - 1, iy = 2 * oy + (tap / 3) % 3 - 1, ix = 2 * ox + tap % 3 - 1;
                         const bool in = row_ok && iz >= 0 && iz < a.Di && iy >= 0 && iy < a.Hi && ix >= 0 && ix < a.Wi;
                         const size_t Si = (size_t)a.Di * a.Hi * a.Wi, vi = ((size_t)iz * a.Hi + iy) * a.Wi + ix;
-                        if (BITS == 8) {
-                            const unsigned b = in ? a.x_sc[((size_t)n * a.nbi + blk) * Si + vi] : 127u;
-                            wq[j >> 2] = (wq[j >> 2] & ~(0xffu << (8 * (j & 3)))) | (b << (8 * (j & 3)));
-                        } else {
-                            const unsigned b0 = in ? a.x_sc[((size_t)n * a.nbi + 2 * blk) * Si + vi] : 127u;
-                            const unsigned b1 = (in && 2 * blk + 1 < a.nbi) ? a.x_sc[((size_t)n * a.nbi + 2 * blk + 1) * Si + vi] : 127u;
-                            const unsigned h = b0 | (b1 << 8);
-                            wq[j >> 1] = (wq[j >> 1] & ~(0xffffu << (16 * (j & 1)))) | (h << (16 * (j & 1)));
-                        }
-                    } else if (BITS == 8) {
-                        const unsigned b = row_ok ? a.x_sc[((size_t)n * a.nkb + ki) * S + vox] : 127u;
-                        wq[j >> 2] = (wq[j >> 2] & ~(0xffu << (8 * (j & 3)))) | (b << (8 * (j & 3)));
+                        const uint8_t *p = a.x_sc + ((size_t)n * a.nbi + (BITS == 8 ? blk : 2 * blk)) * Si + vi;
+                        if (in) raw[j] = __ldg(p);
+                        if (BITS == 4 && in && 2 * blk + 1 < a.nbi) raw[9 + j] = __ldg(p + Si);
                     } else {
-                        const unsigned b0 = row_ok ? a.x_sc[((size_t)n * a.nkb + 2 * ki) * S + vox] : 127u;
-                        const unsigned b1 = (row_ok && 2 * ki + 1 < a.nkb) ? a.x_sc[((size_t)n * a.nkb + 2 * ki + 1) * S + vox] : 127u;
-                        const unsigned h = b0 | (b1 << 8);
-                        wq[j >> 1] = (wq[j >> 1] & ~(0xffffu << (16 * (j & 1)))) | (h << (16 * (j & 1)));
+                        const uint8_t *p = a.x_sc + ((size_t)n * a.nkb + (BITS == 8 ? ki : 2 * ki)) * S + vox;
+                        if (row_ok) raw[j] = __ldg(p);
+                        if (BITS == 4 && row_ok && 2 * ki + 1 < a.nkb) raw[9 + j] = __ldg(p + S);
                     }
                 }
             }
+        };
+        auto next_live = [&](int st) { while (st < st_hi && !stage_live(st)) st++; return st; };
+        int it = 0;
+        int st = next_live(st_lo);
+        if (st < st_hi) load_scales(st);
+        while (st < st_hi) {
+            const int s = it % R, ph = (it / R) & 1, nst = next_live(st + 1);
+            uint32_t wq[5] = {0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu};
+            const int nj = a.taps == 27 ? 9 : 4;
+#pragma unroll
+            for (int j = 0; j < 9; j++) {
+                if (j >= nj) break;
+                if (BITS == 8) wq[j >> 2] = (wq[j >> 2] & ~(0xffu << (8 * (j & 3)))) | (raw[j] << (8 * (j & 3)));
+                else wq[j >> 1] = (wq[j >> 1] & ~(0xffffu << (16 * (j & 1)))) | ((raw[j] | (raw[9 + j] << 8)) << (16 * (j & 1)));
+            }
+            if (nst < st_hi) load_scales(nst);
+            if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 4, st); break; }
+            uint32_t *sfa = (uint32_t *)(stages + (size_t)s * a.stage_bytes + a.offSFA);
             /* quad q: word (lane, column) = row 32 * column + lane -> this thread's word is at lane * 4 + quarter */
 #pragma unroll
             for (int q = 0; q < 5; q++) if (q < a.nquad) sfa[q * 128 + lane * 4 + q4] = wq[q];
             fence_proxy_async();
-            mbar_arrive(bar_sf + 8 * s);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_sf + 8 * s);        /* one arrival a warp: arrivals on one barrier serialise */
             it++;
+            st = nst;
         }
         /* ---- epilogue ---- */
         if (!mbar_wait(bar_acc, 0, abort_flag, kWaitLimit)) raise(a, abort_flag, 5, 0);
         tc_fence_after();
         const int nchunk = n_cur >> 5;
         if (!*abort_flag && a.ksplit > 1) {
-            const size_t tile_id = ((size_t)bz * a.D + z) * gridDim.x + txy;
-            const size_t tile_f = (size_t)(a.nt >> 5) * 4096;                    /* floats of one part */
-            float *mine = a.ks_part + (tile_id * a.ksplit + sp) * tile_f + (size_t)r * 4;
+            /* this block's part of the sums, [32-column chunk][column quad][row][4], into the now idle stage ring */
+            float4 *mine = (float4 *)stages + r;
             for (int jc = 0; jc < nchunk; jc++) {
                 uint32_t rr[32];
                 tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(jc * 32), rr);
                 tmem_ld_wait();
 #pragma unroll
-                for (int k = 0; k < 8; k++) __stcg((uint4 *)(mine + (size_t)jc * 4096 + k * 512), make_uint4(rr[4 * k], rr[4 * k + 1], rr[4 * k + 2], rr[4 * k + 3]));
-            }
-            __threadfence();
-            volatile unsigned *last_s = (volatile unsigned *)(smem_raw + 264);
-            bool dead = false; uint32_t red_ph = 0;
-            /* the 128 epilogue threads meet on an mbarrier (a bounded wait) */
-            auto esync = [&]() { mbar_arrive(bar_red); if (!mbar_wait(bar_red, red_ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 6, 0); dead = true; } red_ph ^= 1u; };
-            esync();
-            if (r == 0) { const unsigned tk = atomicAdd(&a.ks_tickets[tile_id], 1u); const unsigned l = tk == (unsigned)a.ksplit - 1u; if (l) a.ks_tickets[tile_id] = 0u; *last_s = l; }
-            esync();
-            if (!dead && *last_s) {
-                /* the parts of one 32-column chunk (16 KB per split) come into the now idle stage ring with bulk copies, the next chunk's
-                   while this one goes through the epilogue: summing straight from global memory is a chain of L2 round trips */
-                __threadfence();
-                asm volatile("fence.proxy.async;" ::: "memory");
-                const uint32_t bar_ld = bar_red + 8;
-                const float *tile0 = a.ks_part + tile_id * a.ksplit * tile_f;
-                auto fetch = [&](int jc) {
-                    if (r == 0) {
-                        mbar_expect_tx(bar_ld, (uint32_t)a.ksplit * 16384u);
-                        for (int s2 = 0; s2 < a.ksplit; s2++) bulk_g2s(smem_u32(stages + (size_t)s2 * 16384), tile0 + (size_t)s2 * tile_f + (size_t)jc * 4096, 16384u, bar_ld);
-                    }
-                };
-                fetch(0);
-                for (int jc = 0; jc < nchunk && !dead; jc++) {
-                    if (!mbar_wait(bar_ld, (uint32_t)(jc & 1), abort_flag, kWaitLimit)) { raise(a, abort_flag, 7, jc); break; }
-                    float v[32];
-                    const float *p0 = (const float *)stages + (size_t)r * 4;
-#pragma unroll
-                    for (int k = 0; k < 8; k++) { const float4 t = *(const float4 *)(p0 + k * 512); v[4 * k] = t.x; v[4 * k + 1] = t.y; v[4 * k + 2] = t.z; v[4 * k + 3] = t.w; }
-                    for (int s2 = 1; s2 < a.ksplit; s2++) {
-                        const float *ps = p0 + (size_t)s2 * 4096;
-#pragma unroll
-                        for (int k = 0; k < 8; k++) { const float4 t = *(const float4 *)(ps + k * 512); v[4 * k] += t.x; v[4 * k + 1] += t.y; v[4 * k + 2] += t.z; v[4 * k + 3] += t.w; }
-                    }
-                    esync();                                   /* every thread has read the chunk: the ring may take the next one */
-                    if (dead) break;
-                    if (jc + 1 < nchunk) fetch(jc + 1);
-                    epi_chunk(a.e, n, z, oy, ox, row_ok, (n0 >> 5) + jc, v);
-                }
+                for (int k = 0; k < 8; k++) mine[jc * 1024 + k * 128] = make_float4(__uint_as_float(rr[4 * k]), __uint_as_float(rr[4 * k + 1]), __uint_as_float(rr[4 * k + 2]), __uint_as_float(rr[4 * k + 3]));
             }
         } else if (!*abort_flag) {
             for (int jc = 0; jc < nchunk; jc++) {
@@ -318,6 +329,43 @@ __global__ void __launch_bounds__(kThreads) conv_mx_k(const __grid_constant__ CU
                 epi_chunk(a.e, n, z, oy, ox, row_ok, (n0 >> 5) + jc, v);
             }
         }
+    }
+    if (a.ksplit > 1) {
+        /* K split: the blocks of a tile are a cluster.  Each takes every ksplit-th 32-column chunk, adds the parts of all of them in split order (the order
+           is fixed: results do not depend on scheduling) straight from their shared memory, and runs the chunk's epilogue.  Leaving the parts
+           in global memory for the block that came last cost 5 to 6 us a launch.  Every thread passes both cluster barriers, also after a
+           give-up. */
+        __syncwarp();
+        cluster_sync_all();
+        if (warp >= 2 && warp < 6) {
+            const int q4 = warp & 3, r = q4 * 32 + lane, oy = y0 + (r >> 3), ox = x0 + (r & 7), nchunk = n_cur >> 5;
+            const bool row_ok = oy < a.H && ox < a.W;
+            const uint32_t base = smem_u32(stages) + (uint32_t)r * 16u;
+            for (int jc = sp; jc < nchunk && !*abort_flag; jc += a.ksplit) {
+                const uint32_t cb = base + (uint32_t)jc * 16384u;
+                float4 t[8], nx[8];
+                float v[32];
+                auto fetch = [&](int s2) { const uint32_t ra = cluster_addr(cb, (uint32_t)s2);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) nx[k] = cluster_ld4(ra + (uint32_t)k * 2048u); };
+                fetch(0);
+#pragma unroll
+                for (int k = 0; k < 8; k++) t[k] = nx[k];
+                fetch(1);
+#pragma unroll
+                for (int k = 0; k < 8; k++) { v[4 * k] = t[k].x; v[4 * k + 1] = t[k].y; v[4 * k + 2] = t[k].z; v[4 * k + 3] = t[k].w; }
+                for (int s2 = 1; s2 < a.ksplit; s2++) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++) t[k] = nx[k];
+                    if (s2 + 1 < a.ksplit) fetch(s2 + 1);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) { v[4 * k] += t[k].x; v[4 * k + 1] += t[k].y; v[4 * k + 2] += t[k].z; v[4 * k + 3] += t[k].w; }
+                }
+                epi_chunk(a.e, n, z, oy, ox, row_ok, (n0 >> 5) + jc, v);
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();                                  /* no block leaves while another may still read its part */
     }
     /* ---------------- teardown ---------------- */
     tc_fence_before();
@@ -387,7 +435,6 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 }   // namespace
 
-void umx_conv_ks_tickets_reset(void) { void *p = nullptr; if (cudaGetSymbolAddress(&p, g_ks_tickets) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 8192); }
 int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e);
 int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, void *enc, int N, int D, int H, int W, const EpiArgs &e,
                    double *part, const float *gamma, const float *beta, float eps, float *coef);
@@ -553,15 +600,9 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     auto up128 = [](int v) { return (v + 127) & ~127; };
     a.offW = 0; a.offSFB = c->items_max * c->nt * 32; a.offA = up128(c->w_stage_bytes); a.offSFA = a.offA + up128(abytes);
     a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
-    /* per device, looked up once: the multiprocessor count and the address of the ticket array */
-    static int sms_of[16]; static unsigned *tickets_of[16];
+    static int sms_of[16];                                  /* multiprocessors, looked up once per device */
     int d0 = 0; cudaGetDevice(&d0); d0 &= 15;
-    if (!sms_of[d0]) {
-        int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d0);
-        unsigned *t = nullptr;
-        if (cudaGetSymbolAddress((void **)&t, g_ks_tickets) != cudaSuccess) { umx_latch_msg("umx_conv_fwd: ticket array"); return -1; }
-        tickets_of[d0] = t; sms_of[d0] = v;
-    }
+    if (!sms_of[d0]) { int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d0); sms_of[d0] = v; }
     const int sms = sms_of[d0];
     /* two blocks a multiprocessor (two issuing threads keep the tensor pipe busier than one) for the narrow tiles, and for the wide ones when
        there are more blocks than multiprocessors; a deep ring for one block otherwise */
@@ -667,20 +708,16 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         if (ks > units) ks = units;
         if (ks > c->nst / 6) ks = c->nst / 6;              /* at least six stages a share: shorter shares cost more in the reduction than they save */
         if (ks > 16) ks = 16;
-        /* the parts of a chunk are summed from the stage ring; the bound is that of the shallow ring, whatever ring this launch has, so that
-           the split does not change with the batch */
+        /* at most as many parts as 16 KB pieces fit the shallow ring, whatever ring this launch has, so that the split does not change with the batch
+           (never more than six, a portable cluster) */
         { int rs = 100 * 1024 / a.stage_bytes; if (rs > 8) rs = 8; if (rs < 2) rs = 2; const long long cap = (long long)rs * a.stage_bytes / 16384; if (ks > cap) ks = cap; }
-        if (!no_split && ks >= 2 && tiles_all <= 8192) {
-            const size_t bytes = (size_t)tiles_all * (size_t)ks * (size_t)(c->nt >> 5) * 4096 * 4;
-            void *ws = umx_ws(5, bytes);
-            if (!ws) { umx_plain_launch = 0; return -1; }
-            a.ks_tickets = tickets_of[d0];
-            a.ksplit = (int)ks; a.ks_part = (float *)ws;
-        }
+        if (!no_split && ks >= 2 && ks <= 8 && tiles_all <= 8192) a.ksplit = (int)ks;
     }
     const dim3 grid(a.tiles_x * a.tiles_y, D, N * a.ntiles_n * a.ksplit);
     const int pid = umx_prof_open(flops);
-    if (c->bits == 8) umx_launch(conv_mx_k<8>, grid, dim3(kThreads), smem, m0, a); else umx_launch(conv_mx_k<4>, grid, dim3(kThreads), smem, m0, a);
+    /* the parts need 16 KB a 32-column chunk of the ring */
+    if (a.ksplit > 1) { if (c->bits == 8) umx_launch_cluster(conv_mx_k<8>, grid, dim3(1, 1, (unsigned)a.ksplit), dim3(kThreads), smem, m0, a); else umx_launch_cluster(conv_mx_k<4>, grid, dim3(1, 1, (unsigned)a.ksplit), dim3(kThreads), smem, m0, a); }
+    else if (c->bits == 8) umx_launch(conv_mx_k<8>, grid, dim3(kThreads), smem, m0, a); else umx_launch(conv_mx_k<4>, grid, dim3(kThreads), smem, m0, a);
     umx_plain_launch = 0;
     umx_prof_close(pid);
     g_umx_launches++; g_last_kernel = 0;

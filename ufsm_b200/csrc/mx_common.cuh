@@ -37,6 +37,17 @@ static inline void umx_launch(void (*kern)(KA...), dim3 grid, dim3 block, size_t
     if (umx_pdl() && !umx_plain_launch) { cfg.attrs = at; cfg.numAttrs = 1; }
     cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
 }
+/* the same in clusters of blocks */
+template <typename... KA, typename... A>
+static inline void umx_launch_cluster(void (*kern)(KA...), dim3 grid, dim3 cluster, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = 0;
+    cudaLaunchAttribute at[2]; memset(at, 0, sizeof at);
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = cluster.x; at[0].val.clusterDim.y = cluster.y; at[0].val.clusterDim.z = cluster.z;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = umx_pdl() && !umx_plain_launch ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif

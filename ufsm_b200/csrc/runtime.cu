@@ -30,7 +30,6 @@ int umx_ready(const char *where) {
 }
 static int *g_flag[16];
 void umx_conv_r_tickets_reset(void);
-void umx_conv_ks_tickets_reset(void);
 void umx_stat_tickets_reset(void);
 extern "C" const char *lp_check(void) {
     int d = -1;
@@ -152,7 +151,7 @@ int umx_errflag_read(void) {
         umx_latch_msg(b);
         /* blocks that gave up left without drawing their tickets: zero the ticket counters of the kernels that finalise from the last block,
            so that later launches count from zero again, then clear the flag */
-        umx_conv_r_tickets_reset(); umx_conv_ks_tickets_reset(); umx_stat_tickets_reset();
+        umx_conv_r_tickets_reset(); umx_stat_tickets_reset();
         cudaMemset(f, 0, 256);
     }
     return h[0];
