@@ -570,3 +570,36 @@ def test_weights_without_a_key_may_change_between_calls(dev):
     ufsm_b200.check()
     for g, wnt in zip(got, want):
         assert np.array_equal(g.download(), wnt)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N,Cn,D,H,W", [(1, 32, 4, 8, 8), (2, 64, 5, 7, 9), (1, 96, 2, 2, 2), (1, 320, 8, 8, 8), (3, 32, 10, 10, 10), (1, 64, 16, 16, 16), (2, 32, 12, 20, 16), (1, 128, 17, 16, 16),
+                                        (1, 32, 32, 32, 32), (2, 64, 24, 24, 24), (1, 32, 42, 60, 60), (1, 96, 48, 32, 32), (5, 32, 20, 20, 20)])
+def test_norm_in_one_launch(dev, bits, N, Cn, D, H, W):
+    """statistics, coefficients and apply in one launch: the bytes of the two-launch path at the edges of its forms (one block, a cluster of 8 or 16,
+    blocks that meet through a counter, one or two trips a block, partly filled blocks), with and without the space-to-depth copy, into part
+    of a larger tensor, twice in a row (the counters are cleared); tensors it does not hold return 1 and touch nothing"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    L = dev
+    fn = L.umx_in_norm_apply
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p] + [C.c_int] * 5 + [C.c_float, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int]
+    S, nb = D * H * W, Cn // 32
+    y = (synth.rng(501).standard_normal(N * Cn * S) * np.exp2(synth.rng(502).integers(-3, 4, N * Cn * S))).astype(np.float16)
+    yd, pd, cd = DevBuf(data=y), DevBuf(L.umx_stats_doubles(N, Cn, D, H, W) * 8), DevBuf(N * Cn * 8)
+    rb = 32 * bits // 8 + 1
+    even = not ((D | H | W) & 1)
+    want, want2 = DevBuf(N * 2 * nb * S * rb).fill(0xEE), DevBuf(N * nb * S * rb).fill(0xEE)
+    L.umx_in_stats_coef(yd.ptr, N, Cn, D, H, W, None, None, 1e-5, pd.ptr, cd.ptr)
+    L.umx_in_apply(yd.ptr, cd.ptr, N, Cn, D, H, W, 2, want.ptr, bits, 2 * nb, nb, want2.ptr if even else None, None, 1)
+    for s2d in ([False, True] if even else [False]):
+        for _ in range(2):
+            got, got2 = DevBuf(N * 2 * nb * S * rb).fill(0xEE), DevBuf(N * nb * S * rb).fill(0xEE)
+            rc = fn(yd.ptr, N, Cn, D, H, W, 1e-5, 2, pd.ptr, got.ptr, bits, 2 * nb, nb, got2.ptr if s2d else None, 1)
+            ufsm_b200.check()
+            held = S <= 4096 or (148 // (nb * N)) * 1024 >= S
+            assert rc == (0 if held else 1)
+            assert np.array_equal(got.download(), want.download() if held else np.full(got.nbytes, 0xEE, np.uint8))
+            if s2d and held:
+                assert np.array_equal(got2.download(), want2.download())

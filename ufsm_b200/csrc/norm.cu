@@ -3,6 +3,15 @@
    that when the space-to-depth copy for a down conv is also written).  Semantics: k_in_coef and k_inq of the reference
    (src/nn_xnet.cu:1565-1570, 1577-1620) with 32-channel UE8M0 blocks. */
 #include "mx_common.cuh"
+#include "tc_ptx.cuh"
+#include <string.h>
+
+/* mean and variance of S values to the coefficients (a, b) of an affine map (k_in_coef, src/nn_xnet.cu:1565-1570) */
+__device__ __forceinline__ float2 coef_of(double sum, double sq, double S, float eps, const float *gamma, const float *beta, int c) {
+    const double m = sum / S, v = fmax(sq / S - m * m, 0.0);
+    const float rs = (float)(1.0 / sqrt(v + (double)eps)), ca = __fmul_rn(rs, gamma ? gamma[c] : 1.f);
+    return make_float2(ca, __fmaf_rn(-(float)m, ca, beta ? beta[c] : 0.f));
+}
 
 /* partial sums: part[((n * T + t) * Cop + c) * 2 + {0, 1}], T voxel chunks, Cop = C rounded up to 32.  One block per (c, n); the
    chunk sums are added in a fixed order (strided per thread, then a fixed tree), so the result does not depend on scheduling. */
@@ -15,63 +24,72 @@ __global__ void __launch_bounds__(256) in_coef_k(const double *__restrict__ part
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) { if ((int)threadIdx.x < o) { ss[threadIdx.x] += ss[threadIdx.x + o]; sq[threadIdx.x] += sq[threadIdx.x + o]; } __syncthreads(); }
     if (threadIdx.x == 0) {
-        const double m = ss[0] / S, v = fmax(sq[0] / S - m * m, 0.0);
-        const float rs = (float)(1.0 / sqrt(v + (double)eps)), a = __fmul_rn(rs, gamma ? gamma[c] : 1.f);
-        coef[2 * ((size_t)n * C + c)] = a;
-        coef[2 * ((size_t)n * C + c) + 1] = __fmaf_rn(-(float)m, a, beta ? beta[c] : 0.f);
+        const float2 ab = coef_of(ss[0], sq[0], S, eps, gamma, beta, c);
+        coef[2 * ((size_t)n * C + c)] = ab.x;
+        coef[2 * ((size_t)n * C + c) + 1] = ab.y;
     }
 }
 extern "C" void umx_in_coef(const double *part, int N, int C, int D, int H, int W, const float *gamma, const float *beta, float eps, float *coef);
-/* voxel chunks per (sample, channel) of the partial sums: about 1024 voxels each, at most 512 */
-int umx_stats_chunks(int D, int H, int W) { const size_t S = (size_t)D * H * W; const size_t t = S / 1024; return t < 1 ? 1 : t > 512 ? 512 : (int)t; }
+/* voxel chunks per (sample, channel) of the partial sums: about 1024 voxels each, at most 444 (three blocks on each of 148 multiprocessors), a
+   multiple of 111 where there are that many, so that two or four channel blocks or samples make whole waves too */
+int umx_stats_chunks(int D, int H, int W) { const size_t S = (size_t)D * H * W; const size_t t = S / 1024; return t < 1 ? 1 : t >= 444 ? 444 : t >= 111 ? (int)t / 111 * 111 : (int)t; }
 
+/* fp16 values to fp64 sums and sums of squares: exact to the last bits whatever the order */
+struct StatAcc { double s[8], q[8]; };
+__device__ __forceinline__ void stat_zero(StatAcc &a) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) { a.s[k] = 0.0; a.q[k] = 0.0; }
+}
+__device__ __forceinline__ void stat_add(StatAcc &a, const uint4 &r) {
+    const __half2 *h = (const __half2 *)&r;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 f = __half22float2(h[k]);
+        const double d0 = (double)f.x, d1 = (double)f.y;
+        a.s[2 * k] += d0; a.q[2 * k] = fma(d0, d0, a.q[2 * k]); a.s[2 * k + 1] += d1; a.q[2 * k + 1] = fma(d1, d1, a.q[2 * k + 1]);
+    }
+}
 /* partial sums of chunk t of block blk of sample n of a blocked fp16 tensor: part[((n * T + t) * Cop + c) * 2 + {0, 1}].  A thread owns
-   eight channels (one 16-byte load) of every 64th voxel of the chunk, four loads in flight, so a warp reads 512 contiguous bytes per
+   eight channels (one 16-byte load) of every 64th voxel of the chunk, eight loads in flight, so a warp reads 512 contiguous bytes per
    load; the 64 phases are added in a fixed order.  fp64 throughout: sums of fp16 values and of their squares are then exact to the
    last bits whatever the order.  HBM-bound: reads 2 B per element. */
 /* tickets of the fused finalise: one counter per (sample, block); the block that draws the last ticket finalises and resets it */
 __device__ unsigned g_stat_tickets[8192];
 
 template <bool FINAL>
-__global__ void __launch_bounds__(256) in_part_k(const uint4 *__restrict__ y, size_t S, int T, double *__restrict__ part,
+__global__ void __launch_bounds__(256, 3) in_part_k(const uint4 *__restrict__ y, size_t S, int T, double *__restrict__ part,
                                                  int C, const float *gamma, const float *beta, float eps, float *coef) {
     pdl_trigger(); pdl_wait();
     const int t = blockIdx.x, blk = blockIdx.y, n = blockIdx.z, nb = gridDim.y, Cop = nb * 32;
     const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
-    const size_t v0 = S * t / T, v1 = S * (t + 1) / T;
     const uint4 *p = y + ((size_t)n * nb + blk) * S * 4 + qd;
-    double s[8], q[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) { s[k] = 0.0; q[k] = 0.0; }
-    auto add = [&](const uint4 &r) {
-        const __half2 *h = (const __half2 *)&r;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float2 f = __half22float2(h[k]);
-            const double a = (double)f.x, b = (double)f.y;
-            s[2 * k] += a; q[2 * k] = fma(a, a, q[2 * k]); s[2 * k + 1] += b; q[2 * k + 1] = fma(b, b, q[2 * k + 1]);
-        }
-    };
-    size_t v = v0 + ph;
-    for (; v + 448 < v1; v += 512) {      /* eight loads in flight */
-        const uint4 r0 = __ldg(p + v * 4), r1 = __ldg(p + (v + 64) * 4), r2 = __ldg(p + (v + 128) * 4), r3 = __ldg(p + (v + 192) * 4);
-        const uint4 r4 = __ldg(p + (v + 256) * 4), r5 = __ldg(p + (v + 320) * 4), r6 = __ldg(p + (v + 384) * 4), r7 = __ldg(p + (v + 448) * 4);
+    StatAcc acc;
+    stat_zero(acc);
+    auto add = [&](const uint4 &r) { stat_add(acc, r); };
+    /* all blocks sweep the tensor together, 256 voxels a block and trip, from its end to its start: the conv before left its end in L2, and this pass
+       leaves its start there for the apply (32 channels x 128^3: 35 us, and 37 instead of 41 for the apply; 37 with a contiguous piece a block in ascending order) */
+    const size_t sweep = (size_t)T * 256;
+    size_t k = (S + sweep - 1) / sweep;
+    auto at = [&](size_t trip, int u) { const size_t v = trip * sweep + (size_t)t * 256 + 64 * u + ph; return v < S ? __ldg(p + v * 4) : make_uint4(0u, 0u, 0u, 0u); };      /* rows past the end add zeros */
+    for (; k >= 2; k -= 2) {      /* eight loads in flight */
+        const uint4 r0 = at(k - 1, 0), r1 = at(k - 1, 1), r2 = at(k - 1, 2), r3 = at(k - 1, 3), r4 = at(k - 2, 0), r5 = at(k - 2, 1), r6 = at(k - 2, 2), r7 = at(k - 2, 3);
         add(r0); add(r1); add(r2); add(r3); add(r4); add(r5); add(r6); add(r7);
     }
-    for (; v + 192 < v1; v += 256) {
-        const uint4 r0 = __ldg(p + v * 4), r1 = __ldg(p + (v + 64) * 4), r2 = __ldg(p + (v + 128) * 4), r3 = __ldg(p + (v + 192) * 4);
-        add(r0); add(r1); add(r2); add(r3);
-    }
-    for (; v < v1; v += 64) { const uint4 r0 = __ldg(p + v * 4); add(r0); }
+    if (k) { const uint4 r0 = at(0, 0), r1 = at(0, 1), r2 = at(0, 2), r3 = at(0, 3); add(r0); add(r1); add(r2); add(r3); }
     __shared__ double ss[64][33], sq[64][33];
 #pragma unroll
-    for (int k = 0; k < 8; k++) { ss[ph][qd * 8 + k] = s[k]; sq[ph][qd * 8 + k] = q[k]; }
+    for (int k = 0; k < 8; k++) { ss[ph][qd * 8 + k] = acc.s[k]; sq[ph][qd * 8 + k] = acc.q[k]; }
     __syncthreads();
-    if (threadIdx.x < 64) {
-        const int c = threadIdx.x & 31; double (*src)[33] = threadIdx.x < 32 ? ss : sq;
-        double acc = 0.0;
-        for (int k = 0; k < 64; k++) acc += src[k][c];
-        part[(((size_t)n * T + t) * Cop + blk * 32 + c) * 2 + (threadIdx.x >> 5)] = acc;
+    {
+        /* the 64 phases of 32 channels and two sums: 256 threads add 16 each, then 64 threads the four quarters in order */
+        const int c = threadIdx.x & 31, which = (threadIdx.x >> 5) & 1, g = threadIdx.x >> 6; double (*src)[33] = which ? sq : ss;
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 16; k++) t += src[g * 16 + k][c];
+        __syncthreads();
+        src[g][c] = t;
+        __syncthreads();
+        if (threadIdx.x < 64) part[(((size_t)n * T + blockIdx.x) * Cop + blk * 32 + c) * 2 + which] = ((src[0][c] + src[1][c]) + src[2][c]) + src[3][c];
     }
     if (!FINAL) return;
     /* the last block of this (sample, block) to finish turns the partial sums into coefficients: eight threads a channel add
@@ -88,20 +106,22 @@ __global__ void __launch_bounds__(256) in_part_k(const uint4 *__restrict__ y, si
         double a0 = 0.0, a1 = 0.0;
         const double2 *pb = (const double2 *)part + ((size_t)n * T) * Cop + blk * 32 + c;
         int k = g8;
-        for (; k + 24 < T; k += 32) {      /* four loads in flight; the order of the additions is fixed */
-            const double2 p0 = __ldcg(pb + (size_t)k * Cop), p1 = __ldcg(pb + (size_t)(k + 8) * Cop), p2 = __ldcg(pb + (size_t)(k + 16) * Cop), p3 = __ldcg(pb + (size_t)(k + 24) * Cop);
-            a0 += p0.x; a1 += p0.y; a0 += p1.x; a1 += p1.y; a0 += p2.x; a1 += p2.y; a0 += p3.x; a1 += p3.y;
+        for (; k < T; k += 128) {          /* sixteen loads in flight; the order of the additions is fixed */
+            double2 pv[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) pv[j] = k + 8 * j < T ? __ldcg(pb + (size_t)(k + 8 * j) * Cop) : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int j = 0; j < 16; j++) { a0 += pv[j].x; a1 += pv[j].y; }
         }
-        for (; k < T; k += 8) { const double2 p0 = __ldcg(pb + (size_t)k * Cop); a0 += p0.x; a1 += p0.y; }
+        __syncthreads();
         ss[g8][c] = a0; sq[g8][c] = a1;
         __syncthreads();
         if (g8 == 0 && blk * 32 + c < C) {
             for (int k = 1; k < 8; k++) { a0 += ss[k][c]; a1 += sq[k][c]; }
             const int ch = blk * 32 + c;
-            const double m = a0 / (double)S, v = fmax(a1 / (double)S - m * m, 0.0);
-            const float rs = (float)(1.0 / sqrt(v + (double)eps)), ca = __fmul_rn(rs, gamma ? gamma[ch] : 1.f);
-            coef[2 * ((size_t)n * C + ch)] = ca;
-            coef[2 * ((size_t)n * C + ch) + 1] = __fmaf_rn(-(float)m, ca, beta ? beta[ch] : 0.f);
+            const float2 ab = coef_of(a0, a1, (double)S, eps, gamma, beta, ch);
+            coef[2 * ((size_t)n * C + ch)] = ab.x;
+            coef[2 * ((size_t)n * C + ch) + 1] = ab.y;
         }
     }
 }
@@ -134,6 +154,67 @@ extern "C" void umx_in_coef(const double *part, int N, int C, int D, int H, int 
 
 /* NaN-propagating max of magnitudes in one instruction */
 __device__ __forceinline__ float amax_nan(float a, float v) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(fabsf(v))); return r; }
+
+/* one lane's eight channels of a row (four lanes a row): affine map, LeakyReLU as max(g, slope g), fp16 rounding (o), MX codes (w0, w1) and scale byte.
+   All 32 lanes call it together. */
+template <int BITS, bool COEF, bool FULL>
+__device__ __forceinline__ unsigned apply_row(const uint4 &raw, const float *ca, const float *cb, float slope, const bool *live, uint4 &o, unsigned &w0, unsigned &w1) {
+    const __half2 *hp = (const __half2 *)&raw;
+    __half2 *op = (__half2 *)&o;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 t = __half22float2(hp[k]);
+        float g0 = t.x, g1 = t.y;
+        if (COEF) { g0 = __fmaf_rn(g0, ca[2 * k], cb[2 * k]); g1 = __fmaf_rn(g1, ca[2 * k + 1], cb[2 * k + 1]); }
+        g0 = fmaxf(g0, __fmul_rn(slope, g0)); g1 = fmaxf(g1, __fmul_rn(slope, g1));      /* LeakyReLU for 0 < slope <= 1 (NaN stays NaN) */
+        if (!FULL) { if (!live[2 * k]) g0 = 0.f; if (!live[2 * k + 1]) g1 = 0.f; }
+        op[k] = __floats2half2_rn(g0, g1);
+    }
+    /* amax of the stored fp16 values, NaN-propagating, taken on the halves (exact: the conversion to fp32 is monotonic) */
+    __half2 a2 = __hmax2_nan(__hmax2_nan(__habs2(op[0]), __habs2(op[1])), __hmax2_nan(__habs2(op[2]), __habs2(op[3])));
+    const __half a1 = __hmax_nan(__low2half(a2), __high2half(a2));
+    unsigned am = __float_as_uint(__half2float(a1)) & 0x7fffffffu;
+    am = max(am, __shfl_xor_sync(0xffffffffu, am, 1));
+    am = max(am, __shfl_xor_sync(0xffffffffu, am, 2));
+    const mx_sb mq = mx_scale_of(__uint_as_float(am), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
+    const unsigned sb = mq.sb;
+    w1 = 0u;
+    if (BITS == 8 && sb - 112u <= 29u) {
+        /* 2^-e is a normal fp16: scale the halves (exact, or below 2^-14 where E4M3 rounds to zero either way) and convert pairs */
+        const unsigned mh = (142u - sb) << 10, m2 = mh | (mh << 16);
+        const __half2 mm = *(const __half2 *)&m2;
+        unsigned short c0, c1, c2, c3;
+        const __half2 s0 = __hmul2(op[0], mm), s1 = __hmul2(op[1], mm), s2 = __hmul2(op[2], mm), s3 = __hmul2(op[3], mm);
+        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c0) : "r"(*(const unsigned *)&s0));
+        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c1) : "r"(*(const unsigned *)&s1));
+        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c2) : "r"(*(const unsigned *)&s2));
+        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c3) : "r"(*(const unsigned *)&s3));
+        w0 = (unsigned)c0 | ((unsigned)c1 << 16); w1 = (unsigned)c2 | ((unsigned)c3 << 16);
+    } else {
+        float f[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) { const float2 r = __half22float2(op[k]); f[2 * k] = r.x; f[2 * k + 1] = r.y; }
+        const float m = mq.m;
+        if (BITS == 8) { w0 = cvt_e4m3x4(f[0] * m, f[1] * m, f[2] * m, f[3] * m); w1 = cvt_e4m3x4(f[4] * m, f[5] * m, f[6] * m, f[7] * m); }
+        else w0 = cvt_e2m1x8(f, m);
+    }
+    return sb;
+}
+/* the same codes into the space-to-depth copy: block (tap * nb + blk) at the coarse voxel; wsh >= 0: W and H are powers of two */
+template <int BITS>
+__device__ __forceinline__ void s2d_store(uint8_t *q2, int N, int nb, int n, int blk, int qd, unsigned v, size_t S, int H, int W, int wsh, int hsh, int split, unsigned w0, unsigned w1, unsigned sb) {
+    constexpr int RB = 32 * BITS / 8;
+    unsigned xx, yy, zz;
+    if (wsh >= 0) { xx = v & ((1u << wsh) - 1u); const unsigned t1 = v >> wsh; yy = t1 & ((1u << hsh) - 1u); zz = t1 >> hsh; }      /* W and H powers of two */
+    else { xx = v % (unsigned)W; const unsigned t1 = v / (unsigned)W; yy = t1 % (unsigned)H; zz = t1 / (unsigned)H; }
+    const int tap = ((zz & 1) * 2 + (yy & 1)) * 2 + (xx & 1);
+    const size_t Sc = S / 8, vc = ((size_t)(zz >> 1) * (H >> 1) + (yy >> 1)) * (W >> 1) + (xx >> 1);
+    const size_t ro = (size_t)n * 8 * nb + tap * nb + blk;
+    if (BITS == 8 && split) *(uint2 *)(q2 + ((ro * 2 + (qd >> 1)) * Sc + vc) * 16 + (qd & 1) * 8) = make_uint2(w0, w1);
+    else if (BITS == 8) *(uint2 *)(q2 + (ro * Sc + vc) * 32 + qd * 8) = make_uint2(w0, w1);
+    else *(unsigned *)(q2 + (ro * Sc + vc) * 16 + qd * 4) = w0;
+    if (qd == 0) q2[(size_t)N * 8 * nb * Sc * RB + ro * Sc + vc] = (uint8_t)sb;
+}
 
 /* Four threads per voxel row, eight channels (one 16-byte load) each; a block walks a run of voxels of one (sample, block), so the
    sixteen coefficients a thread needs stay in registers.  The row's amax is combined with two shuffles.  grid = (voxel chunks,
@@ -173,66 +254,20 @@ __global__ void __launch_bounds__(256) in_apply_k(const uint4 *__restrict__ x, c
         /* four rows a thread per trip, their loads issued together */
         uint4 raws[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) { const unsigned v = vb + u * 64 + ph; raws[u] = v < v1 ? __ldg(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }
+        for (int u = 0; u < 4; u++) { const unsigned v = vb + u * 64 + ph; raws[u] = v < v1 ? __ldcs(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* the last use of x */
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const unsigned v = vb + u * 64 + ph; const bool ok = v < v1;      /* all 32 lanes stay for the shuffles */
-            const __half2 *hp = (const __half2 *)&raws[u];
-            uint4 o; __half2 *op = (__half2 *)&o;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float2 t = __half22float2(hp[k]);
-                float g0 = t.x, g1 = t.y;
-                if (COEF) { g0 = __fmaf_rn(g0, ca[2 * k], cb[2 * k]); g1 = __fmaf_rn(g1, ca[2 * k + 1], cb[2 * k + 1]); }
-                g0 = fmaxf(g0, __fmul_rn(slope, g0)); g1 = fmaxf(g1, __fmul_rn(slope, g1));      /* LeakyReLU for 0 < slope <= 1 (NaN stays NaN) */
-                if (!FULL) { if (!live[2 * k]) g0 = 0.f; if (!live[2 * k + 1]) g1 = 0.f; }
-                op[k] = __floats2half2_rn(g0, g1);
-            }
+            uint4 o; unsigned w0, w1;
+            const unsigned sb = apply_row<BITS, COEF, FULL>(raws[u], ca, cb, slope, live, o, w0, w1);
             if (hp_out && ok) hp_out[(size_t)v * 4] = o;
-            /* amax of the stored fp16 values, NaN-propagating, taken on the halves (exact: the conversion to fp32 is monotonic) */
-            __half2 a2 = __hmax2_nan(__hmax2_nan(__habs2(op[0]), __habs2(op[1])), __hmax2_nan(__habs2(op[2]), __habs2(op[3])));
-            const __half a1 = __hmax_nan(__low2half(a2), __high2half(a2));
-            unsigned am = __float_as_uint(__half2float(a1)) & 0x7fffffffu;
-            am = max(am, __shfl_xor_sync(0xffffffffu, am, 1));
-            am = max(am, __shfl_xor_sync(0xffffffffu, am, 2));
-            const int e = mx_exp(__uint_as_float(am), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
-            const unsigned sb = (unsigned)(e + 127) & 0xffu;
-            unsigned w0, w1 = 0u;
-            if (BITS == 8 && e >= -15 && e <= 14) {
-                /* 2^-e is a normal fp16: scale the halves (exact, or below 2^-14 where E4M3 rounds to zero either way) and convert pairs */
-                const unsigned mh = (unsigned)(15 - e) << 10, m2 = mh | (mh << 16);
-                const __half2 mm = *(const __half2 *)&m2;
-                unsigned short c0, c1, c2, c3;
-                const __half2 s0 = __hmul2(op[0], mm), s1 = __hmul2(op[1], mm), s2 = __hmul2(op[2], mm), s3 = __hmul2(op[3], mm);
-                asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c0) : "r"(*(const unsigned *)&s0));
-                asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c1) : "r"(*(const unsigned *)&s1));
-                asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c2) : "r"(*(const unsigned *)&s2));
-                asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c3) : "r"(*(const unsigned *)&s3));
-                w0 = (unsigned)c0 | ((unsigned)c1 << 16); w1 = (unsigned)c2 | ((unsigned)c3 << 16);
-            } else {
-                float f[8];
-#pragma unroll
-                for (int k = 0; k < 4; k++) { const float2 r = __half22float2(op[k]); f[2 * k] = r.x; f[2 * k + 1] = r.y; }
-                const float m = exp2i(-e);
-                if (BITS == 8) { w0 = cvt_e4m3x4(f[0] * m, f[1] * m, f[2] * m, f[3] * m); w1 = cvt_e4m3x4(f[4] * m, f[5] * m, f[6] * m, f[7] * m); }
-                else w0 = cvt_e2m1x8(f, m);
-            }
             if (!ok) continue;
             if (qb) {
                 if (BITS == 8) *(uint2 *)(qb + (size_t)v * qs) = make_uint2(w0, w1); else *(unsigned *)(qb + (size_t)v * qs) = w0;
                 if (qd == 0) qsc[v] = (uint8_t)sb;
             }
             if (S2D) {   /* space-to-depth copy: block (tap * nb + blk) at the coarse voxel */
-                unsigned xx, yy, zz;
-                if (wsh >= 0) { xx = v & ((1u << wsh) - 1u); const unsigned t1 = v >> wsh; yy = t1 & ((1u << hsh) - 1u); zz = t1 >> hsh; }      /* W and H powers of two */
-                else { xx = v % (unsigned)W; const unsigned t1 = v / (unsigned)W; yy = t1 % (unsigned)H; zz = t1 / (unsigned)H; }
-                const int tap = ((zz & 1) * 2 + (yy & 1)) * 2 + (xx & 1);
-                const size_t Sc = S / 8, vc = ((size_t)(zz >> 1) * (H >> 1) + (yy >> 1)) * (W >> 1) + (xx >> 1);
-                const size_t ro = (size_t)n * 8 * nb + tap * nb + blk;
-                if (BITS == 8 && split) *(uint2 *)(q2 + ((ro * 2 + (qd >> 1)) * Sc + vc) * 16 + (qd & 1) * 8) = make_uint2(w0, w1);
-                else if (BITS == 8) *(uint2 *)(q2 + (ro * Sc + vc) * 32 + qd * 8) = make_uint2(w0, w1);
-                else *(unsigned *)(q2 + (ro * Sc + vc) * 16 + qd * 4) = w0;
-                if (qd == 0) q2[(size_t)N * 8 * nb * Sc * RB + ro * Sc + vc] = (uint8_t)sb;
+                s2d_store<BITS>(q2, N, nb, n, blk, qd, v, S, H, W, wsh, hsh, split, w0, w1, sb);
             }
         }
     }
@@ -260,3 +295,189 @@ extern "C" void umx_in_apply(const void *x, const float *coef, int N, int C, int
     g_umx_launches++;
     UMX_CK("umx_in_apply");
 }
+
+/* ---- statistics, coefficients and apply in one launch: what a conv of the U-Net is followed by.  B blocks share a (sample, 32-channel block).
+   A block adds up its share of the voxels, the blocks' sums meet (small tensors: a cluster, through distributed shared memory; others: through
+   global memory and a counter), and the values are transformed where they are, in registers (ROWS rows a thread).  Tensors too large for that
+   take two launches: read again in one launch they were no faster (32 channels x 128^3 87 us against 79).
+   Two launches are each a chain of a load, a reduction and a store behind a device-wide wait, which is what bounds them on the deep levels and on
+   small patches: 8^3 x 320 channels 10 us, 16^3 x 256 14, 32^3 x 128 16, with the space-to-depth copy 26; in one launch 5.5, 7, 9 and 11.
+   Blocks wait for one another through the counter only when the launch has at most one block a multiprocessor: they are all resident once the
+   kernels before them have drained, and no later kernel of the stream starts before all of them have (pdl_trigger).  (Clusters do not give
+   that: of 36 clusters of eight that the occupancy query allows, 32 were scheduled.)  The wait is bounded all the same.  Sums are fp64 in a
+   fixed order: rows of a thread, row phases, blocks. ---- */
+namespace {
+__device__ unsigned g_norm_count[2 * 4096];                  /* per (sample, block): blocks that have left their sums, blocks that have seen them all (the last one clears both) */
+struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl; unsigned vp; double *part; int *err; };      /* vp: voxels of a block's trip, NT / 4 to NT; cl: blocks of a cluster, all B of them, or 1 */
+
+template <int BITS, bool S2D, int ROWS, int NT>
+__global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
+    pdl_trigger();
+    constexpr int RB = 32 * BITS / 8, PH = NT / 4, GR = NT / 64;
+    __shared__ double ss[64][33], sq[64][33];
+    __shared__ double mine[64];
+    __shared__ float2 sc[32];
+    const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, B = gridDim.x, rank = blockIdx.x, CL = a.cl;
+    const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
+    const unsigned S = a.S, vp = a.vp, step = vp * (unsigned)B, K = (S + step - 1) / step, g = (unsigned)(n * nb + blk);
+    const uint4 *xp = a.x + ((size_t)n * nb + blk) * S * 4 + qd;
+    /* row u of this thread in trip k of its block; S where there is none */
+    auto vox = [&](unsigned k, int u) { const unsigned v = k * step + (unsigned)rank * vp + (unsigned)PH * u + (unsigned)ph; return k < K && (unsigned)PH * u < vp && v < S ? v : S; };
+    pdl_wait();
+    uint4 raw[ROWS];
+    {
+        StatAcc acc;
+        stat_zero(acc);
+        auto load4 = [&](uint4 *r, unsigned k) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) { const unsigned v = vox(k, u); r[u] = v < S ? __ldg(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
+        };
+#pragma unroll
+        for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, k);
+#pragma unroll
+        for (int u = 0; u < ROWS; u++) stat_add(acc, raw[u]);
+        if (PH > 64) {                                       /* 128 row phases: two neighbouring ones together */
+#pragma unroll
+            for (int k = 0; k < 8; k++) { acc.s[k] += __shfl_xor_sync(0xffffffffu, acc.s[k], 4); acc.q[k] += __shfl_xor_sync(0xffffffffu, acc.q[k], 4); }
+        }
+        const int row = PH > 64 ? ph >> 1 : ph;
+        if (PH <= 64 || !(ph & 1)) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) { ss[row][qd * 8 + k] = acc.s[k]; sq[row][qd * 8 + k] = acc.q[k]; }
+        }
+    }
+    __syncthreads();
+    const int c = threadIdx.x & 31, which = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
+    double (*src)[33] = which ? sq : ss;
+    /* GR partial sums a (channel, sum), one of each thread, added in order by the first 64 threads */
+    auto groups = [&](double t, double *dst) {
+        __syncthreads();
+        src[grp][c] = t;
+        __syncthreads();
+        if (threadIdx.x < 64) { double v = src[0][c]; for (int k = 1; k < GR; k++) v += src[k][c]; dst[threadIdx.x] = v; }
+    };
+    {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 64 / GR; k++) t += src[grp * (64 / GR) + k][c];
+        groups(t, mine);
+    }
+    if (CL > 1) {                                            /* the blocks are a cluster */
+        cluster_sync_all();
+        double t = 0.0;
+        if (threadIdx.x < 64) {
+            const uint32_t at = smem_u32(mine) + threadIdx.x * 8;
+            for (int r = 0; r < CL; r++) t += cluster_ldd(cluster_addr(at, (uint32_t)r));
+        }
+        cluster_arrive();                                    /* no block's memory is read after this; everyone waits for everyone before leaving */
+        if (threadIdx.x < 64) ss[which][c] = t;
+    } else if (B > 1) {
+        double *part = a.part + (size_t)g * B * 64;
+        if (threadIdx.x < 64) { __stcg(part + rank * 64 + threadIdx.x, mine[threadIdx.x]); __threadfence(); }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(&g_norm_count[2 * g], 1u);
+            const long long t0 = clock64();
+            unsigned seen;
+            for (;;) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&g_norm_count[2 * g]) : "memory");
+                if (seen >= (unsigned)B) break;
+                if (clock64() - t0 > 4000000000ll) { if (atomicCAS(a.err, 0, 10) == 0) { a.err[1] = (int)blockIdx.x; a.err[2] = (int)seen; } break; }
+            }
+            if (atomicAdd(&g_norm_count[2 * g + 1], 1u) == (unsigned)B - 1u) { g_norm_count[2 * g] = 0u; g_norm_count[2 * g + 1] = 0u; }
+        }
+        __syncthreads();
+        double t = 0.0;
+#pragma unroll 4
+        for (int k = grp; k < B; k += GR) t += __ldcg(part + k * 64 + (which << 5) + c);
+        groups(t, mine);
+        __syncthreads();
+        if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x];
+    } else { __syncthreads(); if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x]; }
+    __syncthreads();
+    if (threadIdx.x < 32) sc[c] = coef_of(ss[0][c], ss[1][c], (double)S, a.eps, nullptr, nullptr, 0);
+    __syncthreads();
+    float ca[8], cb[8]; bool live[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) { const float2 ab = sc[qd * 8 + k]; ca[k] = ab.x; cb[k] = ab.y; live[k] = true; }
+    const float slope = a.act == 2 ? 0.01f : 1.f;
+    const int H = a.H, W = a.W, pow2 = S2D && !(W & (W - 1)) && !(H & (H - 1)), wsh = pow2 ? __ffs(W) - 1 : -1, hsh = pow2 ? __ffs(H) - 1 : 0;
+    const size_t drow = (size_t)n * a.nb_dst + a.b0 + blk;
+    uint8_t *qb; int qs;
+    if (BITS == 8 && a.split) { qb = a.q + (drow * 2 + (qd >> 1)) * S * 16 + (qd & 1) * 8; qs = 16; }
+    else if (BITS == 8) { qb = a.q + drow * S * 32 + qd * 8; qs = 32; }
+    else { qb = a.q + drow * S * 16 + qd * 4; qs = 16; }
+    uint8_t *qsc = a.q + (size_t)N * a.nb_dst * S * RB + drow * S;
+    auto put = [&](const uint4 &r, unsigned v) {
+        uint4 o; unsigned w0, w1;
+        const unsigned sb = apply_row<BITS, true, true>(r, ca, cb, slope, live, o, w0, w1);
+        if (v < S) {
+            if (BITS == 8) *(uint2 *)(qb + (size_t)v * qs) = make_uint2(w0, w1); else *(unsigned *)(qb + (size_t)v * qs) = w0;
+            if (qd == 0) qsc[v] = (uint8_t)sb;
+            if (S2D) s2d_store<BITS>(a.q2, N, nb, n, blk, qd, v, S, H, W, wsh, hsh, a.split, w0, w1, sb);
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < ROWS; u++) put(raw[u], vox(u / 4, u & 3));
+    if (CL > 1) cluster_wait();
+}
+/* whether clusters of 16 blocks of a variant can be launched, looked up once per device */
+template <int BITS, bool S2D, int ROWS, int NT> bool norm_sixteen() {
+    static int have[16];
+    int d = 0; cudaGetDevice(&d); d &= 15;
+    if (!have[d]) {
+        const void *k = (const void *)in_norm_k<BITS, S2D, ROWS, NT>;
+        cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
+        cudaLaunchAttribute at; memset(&at, 0, sizeof at);
+        at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = 16; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(16); cfg.blockDim = dim3(NT); cfg.attrs = &at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) n = 0;
+        cudaGetLastError();
+        have[d] = n > 0 ? 1 : -1;
+    }
+    return have[d] > 0;
+}
+template <int BITS, bool S2D, int ROWS, int NT> bool norm_go(NormArgs &a, int B, int cl, int nb, int N) {
+    a.cl = cl;
+    /* small tensors: fewer rows a thread */
+    a.vp = (size_t)B * NT > a.S ? (unsigned)(((size_t)a.S + B * (NT / 4) - 1) / ((size_t)B * (NT / 4))) * (NT / 4) : NT;
+    umx_launch_cluster(in_norm_k<BITS, S2D, ROWS, NT>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3((unsigned)cl, 1, 1), dim3(NT), 0, a);
+    return true;
+}
+template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N) {
+    const size_t S = a.S;
+    /* a cluster a group while a thread of it has at most four (eight) rows */
+    if (S <= 256) return norm_go<BITS, S2D, 4, 256>(a, 1, 1, nb, N);
+    if (S <= 1024) return norm_go<BITS, S2D, 4, 256>(a, 8, 8, nb, N);
+    if (S <= 4096 && norm_sixteen<BITS, S2D, 4, 256>()) return norm_go<BITS, S2D, 4, 256>(a, 16, 16, nb, N);
+    if (S <= 4096) return norm_go<BITS, S2D, 8, 256>(a, 8, 8, nb, N);
+    /* one block a multiprocessor, dealt to the groups, each of at most 1024 voxels */
+    static int sms_of[16];
+    int d = 0; cudaGetDevice(&d); d &= 15;
+    if (!sms_of[d]) { int v = 1; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d); sms_of[d] = v; }
+    long long B = sms_of[d] / ((long long)nb * N);
+    const long long most = (long long)((S + 127) / 128);    /* a row a thread */
+    if (B > most) B = most;
+    if (B < 1 || (size_t)B * 1024 < S) return false;
+    return (size_t)B * 512 >= S ? norm_go<BITS, S2D, 4, 512>(a, (int)B, 1, nb, N) : norm_go<BITS, S2D, 8, 512>(a, (int)B, 1, nb, N);
+}
+}   // namespace
+/* statistics, coefficients (gamma 1, beta 0) and apply of a blocked fp16 tensor of a multiple of 32 channels in one launch; part: scratch of
+   umx_stats_doubles doubles.  Launches on one device must not overlap (they share the counters).  1: not this tensor; the caller takes
+   umx_in_stats_coef and umx_in_apply. */
+extern "C" int umx_in_norm_apply(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout) {
+    const size_t S = (size_t)D * H * W;
+    if (!umx_ready("umx_in_norm_apply") || !S || !N || (C & 31) || S >= (size_t)1 << 31 || !q || (q_s2d && ((D | H | W) & 1)) || (long long)N * (C / 32) > 4096) return 1;
+    NormArgs a; memset(&a, 0, sizeof a);
+    a.x = (const uint4 *)x; a.H = H; a.W = W; a.S = (unsigned)S; a.eps = eps; a.act = act; a.q = (uint8_t *)q; a.nb_dst = nb_dst ? nb_dst : C / 32; a.b0 = nb_dst ? b0 : 0;
+    a.q2 = (uint8_t *)q_s2d; a.split = layout == UMX_LAYOUT_SPLIT; a.part = part; a.err = umx_errflag();
+    if (!a.err) return -1;
+    const bool done = bits == 8 ? (q_s2d ? norm_pick<8, true>(a, C / 32, N) : norm_pick<8, false>(a, C / 32, N)) : (q_s2d ? norm_pick<4, true>(a, C / 32, N) : norm_pick<4, false>(a, C / 32, N));
+    if (!done) return 1;
+    g_umx_launches++;
+    UMX_CK("umx_in_norm_apply");
+    return 0;
+}
+void umx_norm_counts_reset(void) { void *p = nullptr; if (cudaGetSymbolAddress(&p, g_norm_count) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 2 * 4096); }

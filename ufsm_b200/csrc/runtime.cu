@@ -31,6 +31,7 @@ int umx_ready(const char *where) {
 static int *g_flag[16];
 void umx_conv_r_tickets_reset(void);
 void umx_stat_tickets_reset(void);
+void umx_norm_counts_reset(void);
 extern "C" const char *lp_check(void) {
     int d = -1;
     if (!g_has_err && cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 16 && g_flag[d]) umx_errflag_read();   /* a kernel's bounded wait that gave up */
@@ -151,7 +152,7 @@ int umx_errflag_read(void) {
         umx_latch_msg(b);
         /* blocks that gave up left without drawing their tickets: zero the ticket counters of the kernels that finalise from the last block,
            so that later launches count from zero again, then clear the flag */
-        umx_conv_r_tickets_reset(); umx_stat_tickets_reset();
+        umx_conv_r_tickets_reset(); umx_stat_tickets_reset(); umx_norm_counts_reset();
         cudaMemset(f, 0, 256);
     }
     return h[0];

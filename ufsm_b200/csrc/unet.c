@@ -16,6 +16,7 @@
 
 void umx_u8_to_h16(const uint8_t *x, size_t n, void *y);
 int umx_has_error(void);
+int umx_in_norm_apply(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout);
 void umx_h16_to_prob_u8(const void *x, size_t n, uint8_t *y);
 void umx_blend_add_fx(const float *logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0, const float *w1d, long long *acc, long long *wsum);
 void umx_emit_fx(const long long *acc, const long long *wsum, const uint8_t *mode, int want, int nh, int V, int zext, int za, int zb, int ya, int yb, int fmt, void *out);
@@ -137,6 +138,13 @@ static void conv_norm(umx_unet *u, const umx_conv *c, const void *x, int xflag, 
     /* UMX_STATS_EPILOGUE=1 in the environment: InstanceNorm sums in the conv's epilogue (see umx_conv_fwd_norm); off by default */
     static int epi = -1;
     if (epi < 0) { const char *e = getenv("UMX_STATS_EPILOGUE"); epi = e && *e == '1'; }
+    if (!epi) {      /* statistics, coefficients and apply in one launch */
+        umx_conv_fwd(c, x, N, D, D, D, u->ybuf, UMX_OUT_H16B, 0, 0, 0, nullptr, xflag ? xflag : UMX_X_SPLIT);
+        if (umx_in_norm_apply(u->ybuf, N, C, D, D, D, 1e-5f, 2, u->part, q, bits, nb_dst, b0, q_s2d, UMX_LAYOUT_SPLIT) == 0) return;
+        umx_in_stats_coef(u->ybuf, N, C, D, D, D, nullptr, nullptr, 1e-5f, u->part, u->coef);
+        umx_in_apply(u->ybuf, u->coef, N, C, D, D, D, 2, q, bits, nb_dst, b0, q_s2d, nullptr, UMX_LAYOUT_SPLIT);
+        return;
+    }
     umx_conv_fwd_norm(c, x, N, D, D, D, u->ybuf, u->part, nullptr, nullptr, 1e-5f, u->coef, (xflag ? xflag : UMX_X_SPLIT) | (epi ? UMX_STATS_EPILOGUE : 0));
     umx_in_apply(u->ybuf, u->coef, N, C, D, D, D, 2, q, bits, nb_dst, b0, q_s2d, nullptr, UMX_LAYOUT_SPLIT);
 }
