@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     uint32_t *tmem_slot = (uint32_t *)(smem_raw + 512);
     volatile int *abort_flag = (volatile int *)(smem_raw + 516);
     uint8_t *stages = smem_raw + 1024;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int R = a.ring;
     const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_cp = bar_tma + 16 * R, bar_empty = bar_tma + 24 * R, bar_acc = bar_tma + 32 * R;
 
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = uni(*tmem_slot);
     const int nbuf = R < 3 ? R : 3;               /* TMEM scale buffers in use */
     /* with a ring of two the stage that waits for the scale thread is the stage the MMAs need next: the MMA thread copies for itself (128 -> 128 on
        32^3, two blocks a multiprocessor: 19.1 us, 20.6 with the scale thread between) */
@@ -112,14 +112,14 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     auto stage_live = [&](int st) -> bool { if (a.taps != 27) return true; const int zi = z + st % 3 - 1; return zi >= 0 && zi < a.D; };
     auto stage_items = [&](int st) -> int { return a.taps == 27 ? 9 : min(4, a.nki - 4 * st); };
 
-    /* a stage's A and B scales from shared memory to TMEM buffer buf (one thread) */
-    auto copy_scales = [&](int st, uint32_t so, int buf) {
+    /* a stage's A and B scales from shared memory to TMEM buffer buf (one warp) */
+    auto copy_scales = [&](int st, uint32_t so, int buf, uint32_t lead) {
         const uint32_t sf_hi = desc_hi(128), sb0 = smem_u32(stages), sfa_lo = desc_lo(sb0 + a.offSFA, 0) + so, sfb_lo = desc_lo(sb0 + a.offSFB, 0) + so;
         const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
         const int nq = a.taps == 27 ? a.nquad : (stage_items(st) + a.ipq - 1) / a.ipq;
         for (int q = 0; q < nq; q++) {
-            utccp_32x128b(sfa_t + 4 * q, desc_make(sfa_lo + 32u * q, sf_hi));
-            utccp_32x128b(sfb_t + 4 * q, desc_make(sfb_lo + 32u * q, sf_hi));
+            utccp_32x128b(sfa_t + 4 * q, desc_make(sfa_lo + 32u * q, sf_hi), lead);
+            utccp_32x128b(sfb_t + 4 * q, desc_make(sfb_lo + 32u * q, sf_hi), lead);
         }
     };
 
@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        /* ---------------- MMA issue: one thread; everything that does not change with the stage is worked out before the loop ---------------- */
-        if (lane == 0) {
+        /* ---------------- MMA issue: one warp, of which one lane issues; everything that does not change with the stage is worked out before the loop ---------------- */
+        {
+            const uint32_t lead = elect_one();
             int it = 0, s = 0, ph = 0; bool ok = true;
             const uint32_t sb0 = smem_u32(stages), sstep = (uint32_t)a.stage_bytes >> 4;
             const uint32_t b_hi = desc_hi(128), a_hi = a.taps == 27 ? desc_hi(160) : desc_hi(128);
@@ -183,41 +184,42 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 const uint32_t so = (uint32_t)s * sstep;
                 const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
                 if (own_copies) {
-                    if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 3, st); ok = false; break; }
-                    if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 2, st); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 2, st); ok = false; break; }
                     tc_fence_after();
-                    copy_scales(st, so, buf);
+                    copy_scales(st, so, buf, lead);
                 } else {
                     /* the scale thread passed the stage's load barrier before it copied the scales, so codes and weights have landed too */
-                    if (!mbar_wait(bar_cp + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 3, st); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_cp + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
                     tc_fence_after();
                 }
-                if (a.taps == 27) issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9);
-                else issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, stage_items(st));
-                umma_commit(bar_empty + 8 * s);
+                if (a.taps == 27) issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9, lead);
+                else issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, stage_items(st), lead);
+                umma_commit(bar_empty + 8 * s, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
                 if (++buf == nbuf) buf = 0;
             }
-            umma_commit(bar_acc);   /* also after a give-up: the epilogue must not wait for its full limit */
+            umma_commit(bar_acc, lead);   /* also after a give-up: the epilogue must not wait for its full limit */
         }
     } else if (warp == 6) {
         /* ---------------- scale copies: one thread brings a stage's A and B scales from shared memory to one of nbuf TMEM buffers.  A tcgen05.cp costs
            the thread that issues it some 40 clocks and the tensor pipe next to nothing, so it is kept out of the MMA thread (a stage of nine N = 128
            MMAs: 1050 clocks with the six copies in it, 576 of them arithmetic). ---------------- */
-        if (lane == 0 && !own_copies) {
+        if (!own_copies) {
+            const uint32_t lead = elect_one();
             const uint32_t sstep = (uint32_t)a.stage_bytes >> 4;
             int it = 0, s = 0, ph = 0, s3 = 0, ph3 = 0, buf = 0;
             for (int st = st_lo; st < st_hi; st++) {
                 if (!stage_live(st)) continue;
-                if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 2, st); break; }
-                if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit)) { raise(a, abort_flag, 4, st); break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 2, st); break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 4, st); break; }
                 if (it >= nbuf) {                /* the MMAs that read this buffer (nbuf stages back; nbuf <= ring, so that barrier is at most one phase ahead) */
-                    if (!mbar_wait(bar_empty + 8 * s3, ph3, abort_flag, kWaitLimit)) { raise(a, abort_flag, 7, st); break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s3, ph3, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 7, st); break; }
                     if (++s3 == R) { s3 = 0; ph3 ^= 1; }
                 }
                 tc_fence_after();
-                copy_scales(st, (uint32_t)s * sstep, buf);
-                umma_commit(bar_cp + 8 * s);
+                copy_scales(st, (uint32_t)s * sstep, buf, lead);
+                umma_commit(bar_cp + 8 * s, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
                 if (++buf == nbuf) buf = 0;
             }

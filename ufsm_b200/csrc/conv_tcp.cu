@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
     uint32_t *tmem_slot = (uint32_t *)(smem_raw + 768);
     volatile int *abort_flag = (volatile int *)(smem_raw + 772);
     uint8_t *wsm = smem_raw + a.off_w, *stages = smem_raw + a.off_ring;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int R = a.ring, NS = a.nslot;
     const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_accf = bar_tma + 24 * R, bar_acce = bar_accf + 8 * kMaxSlotsP, bar_w = bar_acce + 8 * kMaxSlotsP;
     constexpr int IPQ = BITS == 8 ? 4 : 2, NQ = 4 / IPQ;      /* K items a scale quad, quads a stage */
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = uni(*tmem_slot);
     const long long j0 = a.jobs * (long long)blockIdx.x / (long long)gridDim.x, j1 = a.jobs * ((long long)blockIdx.x + 1) / (long long)gridDim.x;
 
     if (warp == 0) {
@@ -108,16 +108,18 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
             }
         }
     } else if (warp == 1) {
-        /* ---------------- MMA issue ---------------- */
-        if (lane == 0) {
-            bool ok = mbar_wait(bar_w, 0, abort_flag, kWaitLimitP);
-            if (!ok) raise_p(a, abort_flag, 6, 0);
+        /* ---------------- MMA issue (the warp runs the loop, one lane issues) ---------------- */
+        {
+            const uint32_t lead = elect_one();
+            const bool ok0 = mbar_wait(bar_w, 0, abort_flag, kWaitLimitP);
+            bool ok = __all_sync(0xffffffffu, ok0);
+            if (!ok && lane == 0) raise_p(a, abort_flag, 6, 0);
             tc_fence_after();
             const uint32_t wbase = smem_u32(wsm), sf_hi = desc_hi(128), a_hi = desc_hi(128), b_hi = desc_hi(128);
             const uint32_t idesc_b = (BITS == 8 ? idesc_mxf8(0, 0, 0) : idesc_mxf4(0, 0, 0));
             if (ok) {
                 const int nsf = a.ntiles * a.ngroups * NQ;
-                for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi));
+                for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi), lead);
             }
             const uint32_t a_lo0 = desc_lo(smem_u32(stages), 2048), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
             const uint32_t b_lo0 = desc_lo(wbase, (uint32_t)a.ntp * 16), b_item = 2u * (uint32_t)a.ntp, b_tile = (uint32_t)a.nki * b_item;
@@ -126,26 +128,26 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
             while (ok && job < j1) {
                 const int n_cur = min(a.ntp, a.cop - ntile * a.ntp);
                 const uint32_t idn = idesc_b | ((uint32_t)(n_cur >> 3) << 17), d = tmem + (uint32_t)(slot * a.ntp);
-                if (!mbar_wait(bar_acce + 8 * slot, (uint32_t)(sph ^ 1), abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 7, it); break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_acce + 8 * slot, (uint32_t)(sph ^ 1), abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 7, it); break; }
                 for (int g = 0; g < a.ngroups; g++) {
-                    if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 3, it); ok = false; break; }
-                    if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 2, it); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 3, it); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 2, it); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = tmem + (uint32_t)a.sfa_base + ((uint32_t)it & 1u) * 8u;
                     const uint32_t sfb_t = tmem + (uint32_t)a.sfb_base + (uint32_t)((ntile * a.ngroups + g) * NQ * 4);
                     const uint32_t bb = b_lo0 + (uint32_t)ntile * b_tile + (uint32_t)(4 * g) * b_item;
                     const int items = min(4, a.nki - 4 * g);
 #pragma unroll
-                    for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi));
+                    for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi), lead);
 #pragma unroll
                     for (int j = 0; j < 4; j++) if (j < items) {
                         const int q = j / IPQ, id = (j % IPQ) * (4 / IPQ);
                         const uint32_t idesc = idn | ((uint32_t)id << 4) | ((uint32_t)id << 29), acc = (g == 0 && j == 0) ? 0u : 1u;
                         const uint64_t ad = desc_make(a_lo + (uint32_t)j * 256u, a_hi), bd = desc_make(bb + (uint32_t)j * b_item, b_hi);
-                        if (BITS == 8) umma_mxf8(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q); else umma_mxf4(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q);
+                        if (BITS == 8) umma_mxf8(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead); else umma_mxf4(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead);
                     }
-                    if (g == a.ngroups - 1) umma_commit(bar_accf + 8 * slot);
-                    umma_commit(bar_empty + 8 * s);
+                    if (g == a.ngroups - 1) umma_commit(bar_accf + 8 * slot, lead);
+                    umma_commit(bar_empty + 8 * s, lead);
                     it++; if (++s == R) { s = 0; ph ^= 1; }
                 }
                 if (++slot == NS) { slot = 0; sph ^= 1; }

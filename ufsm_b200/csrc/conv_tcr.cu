@@ -11,20 +11,20 @@
 
 
    What bounds this kernel.  An M = 128, N = 96, K = 32 MMA occupies the tensor pipe for 56 clocks (48 of arithmetic; its 4 KB A tile and
-   3 KB B tile exceed what shared memory delivers in 48), and one thread cannot issue tcgen05.mma faster than one per 54 clocks whatever
-   N is; a scale copy or a commit costs the thread that issues it another 30 to 130 clocks while it takes next to nothing from the
-   pipe.  So the MMA thread issues nothing but MMAs and one commit per stage, and every role's per-stage program is kept short: (1) the
+   3 KB B tile exceed what shared memory delivers in 48).  One warp runs the MMA loop with uniform values and one elected lane issues: issued by
+   a lone thread, with operands moved to uniform registers one by one, a stage of nine MMAs took 1190 clocks on 128 -> 64 channels, 64^3 (80.7 us
+   the conv, 60.0 now).  A commit costs its issuer another 60 clocks, so there is one per stage, and every role's per-stage program is kept short: (1) the
    producer thread tracks slots and parities incrementally (no division) and hands the MMA thread a record with everything
    precomputed: TMEM addresses, the N field of the instruction descriptor, B descriptor and B scale addresses, the barriers to wait
-   for; (2) the MMA thread's stage is three PTX blocks of three MMAs whose operands are a record field plus an immediate; (3)
+   for; (2) the MMA warp's stage is three PTX blocks of three MMAs whose operands are a record field plus an immediate; (3)
    accumulators are never "fresh": the epilogue zeroes a slot after reading it, so every MMA accumulates; (4) the A scale factors are
    gathered from a TMA-staged window in shared memory with no bounds logic (voxels outside the volume arrive as zero codes with scale
-   byte 0) and copied to TMEM by the scale warps themselves, whose commit is what the MMA thread waits for; (5) the MMA thread's single
+   byte 0) and copied to TMEM by the scale warps themselves, whose commit is what the MMA warp waits for; (5) the MMA warp's single
    commit per stage lands on the stage's `empty` barrier; the scale warps, which wait for that barrier anyway before they reuse a TMEM
    scale buffer, pass the completion of output planes on to the epilogue's accumulator-full barriers; (6) two blocks share a
    multiprocessor when the weights are small enough: one block's waits are the other's issue time.
 
-   Roles (256 threads): warp 0 lane 0 producer (records + TMA), warp 1 lane 0 MMA issue (the warp allocates TMEM), warps 2-3 scale
+   Roles (256 threads): warp 0 lane 0 producer (records + TMA), warp 1 MMA issue (and TMEM), warps 2-3 scale
    layout, scale copies and completion relay (alternate stages), warps 4-7 epilogue.  All waits are bounded as in conv_mx_k. */
 #include "conv_epi.cuh"
 #include "tc_ptx.cuh"
@@ -67,7 +67,7 @@ struct ConvRArgs {
     int ring, stage_bytes, offSW, offSFA;
     int w_bytes, w_codes, nquad, gt, goff1, goff2, nslot;
     int tmem_cols, sfa_base, sfa_cols, sfb_base; /* TMEM: accumulator slots from 0, two A scale buffers, B scales */
-    int off_rec, off_bias, off_stage, off_w, off_ring;   /* off_stage: 2 KB per epilogue warp and 32-channel chunk, the fp16 output rows on their way to coalesced stores */
+    int off_rec, off_bias, off_stage, off_w, off_ring;   /* off_stage (with statistics): 2 KB per epilogue warp and 32-channel chunk, the fp16 output rows on their way to coalesced stores */
     int fast_h16;                                /* output is the fp16 blocked tensor of a plain conv: the short epilogue */
     /* InstanceNorm statistics taken in that epilogue (coef != NULL): fp64 sums of the stored fp16 values and of their squares, written once per
        sample and block into part [n][gcol][cop][2]; the last block of a column tile to finish adds the blocks' entries in block order and
@@ -98,10 +98,9 @@ __device__ __forceinline__ void raise_r(const ConvRArgs &a, volatile int *abort_
 }
 /* Three of the nine (dy, dx) MMAs of a group in one PTX block: tap j reads the A view a_lo + (j / 3) * 10 + j % 3 and the B image
    b_lo + j * BSTEP; the scale sets come in quads of four (fp8) or two (fp4) taps.  Everything that depends on the tap is an immediate, so
-   between two MMAs the issuing thread runs a handful of independent integer instructions that the assembler is free to hoist: a lone
-   thread runs dependent scalar code at four to five clocks an instruction, and every clock it spends between MMAs the tensor pipe idles. */
+   between two MMAs the warp runs a handful of independent uniform instructions that the assembler is free to hoist; `lead` is 1 in the lane that issues. */
 template <int BITS, int BSTEP, int SFBQ, int J0>
-__device__ __forceinline__ void mma3(uint32_t d, uint32_t idn, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t sfa, uint32_t sfb) {
+__device__ __forceinline__ void mma3(uint32_t d, uint32_t idn, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t sfa, uint32_t sfb, uint32_t lead) {
     constexpr int IPQ = BITS == 8 ? 4 : 2;
 #define UMX_TAP(j) "n"(((j) / 3) * 10 + (j) % 3), "n"((j) * BSTEP), "n"(((((j) % IPQ) * (4 / IPQ)) << 4) | ((((j) % IPQ) * (4 / IPQ)) << 29)), "n"(4 * ((j) / IPQ)), "n"(((j) / IPQ) * SFBQ)
 #define UMX_MMA_TEXT(KIND, o)                                                                                        \
@@ -109,25 +108,25 @@ __device__ __forceinline__ void mma3(uint32_t d, uint32_t idn, uint32_t a_lo, ui
     "add.u32 tb, %4, %" UMX_STR(UMX_ADD1(o)) ";\n\tmov.b64 db, {tb, %5};\n\t"                                      \
     "or.b32 ti, %1, %" UMX_STR(UMX_ADD2(o)) ";\n\t"                                                                   \
     "add.u32 sa, %6, %" UMX_STR(UMX_ADD3(o)) ";\n\tadd.u32 sb, %7, %" UMX_STR(UMX_ADD4(o)) ";\n\t"                  \
-    "tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, ti, [sa], [sb], p;\n\t"
+    "@pl tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, ti, [sa], [sb], p;\n\t"
     if constexpr (BITS == 8) {
-        asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 ta, tb, ti, sa, sb;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        asm volatile("{\n\t.reg .pred p, pl;\n\t.reg .b32 ta, tb, ti, sa, sb;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %1, 0;\n\tsetp.ne.b32 pl, %23, 0;\n\t"
                      UMX_MMA_TEXT("mxf8f6f4.block_scale", 8) UMX_MMA_TEXT("mxf8f6f4.block_scale", 13) UMX_MMA_TEXT("mxf8f6f4.block_scale", 18) "}"
-                     ::"r"(d), "r"(idn), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(sfa), "r"(sfb), UMX_TAP(J0), UMX_TAP(J0 + 1), UMX_TAP(J0 + 2) : "memory");
+                     ::"r"(d), "r"(idn), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(sfa), "r"(sfb), UMX_TAP(J0), UMX_TAP(J0 + 1), UMX_TAP(J0 + 2), "r"(lead) : "memory");
     } else {
-        asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 ta, tb, ti, sa, sb;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        asm volatile("{\n\t.reg .pred p, pl;\n\t.reg .b32 ta, tb, ti, sa, sb;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %1, 0;\n\tsetp.ne.b32 pl, %23, 0;\n\t"
                      UMX_MMA_TEXT("mxf4.block_scale.scale_vec::2X", 8) UMX_MMA_TEXT("mxf4.block_scale.scale_vec::2X", 13) UMX_MMA_TEXT("mxf4.block_scale.scale_vec::2X", 18) "}"
-                     ::"r"(d), "r"(idn), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(sfa), "r"(sfb), UMX_TAP(J0), UMX_TAP(J0 + 1), UMX_TAP(J0 + 2) : "memory");
+                     ::"r"(d), "r"(idn), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(sfa), "r"(sfb), UMX_TAP(J0), UMX_TAP(J0 + 1), UMX_TAP(J0 + 2), "r"(lead) : "memory");
     }
 #undef UMX_TAP
 #undef UMX_MMA_TEXT
 }
 /* the nine (dy, dx) MMAs of one group into the accumulator window at d (idn: the instruction descriptor with the window's N) */
-template <int BITS, int NT> __device__ __forceinline__ void issue_group(uint32_t d, uint32_t idn, uint32_t bb, uint32_t sfb, uint32_t a_lo, uint32_t a_hi, uint32_t b_hi, uint32_t sfa_t) {
+template <int BITS, int NT> __device__ __forceinline__ void issue_group(uint32_t d, uint32_t idn, uint32_t bb, uint32_t sfb, uint32_t a_lo, uint32_t a_hi, uint32_t b_hi, uint32_t sfa_t, uint32_t lead) {
     constexpr int BSTEP = 2 * 3 * NT, SFBQ = 4 * ((3 * NT + 127) / 128 + (2 * NT + 127) / 128 + (NT + 127) / 128);
-    mma3<BITS, BSTEP, SFBQ, 0>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb);
-    mma3<BITS, BSTEP, SFBQ, 3>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb);
-    mma3<BITS, BSTEP, SFBQ, 6>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb);
+    mma3<BITS, BSTEP, SFBQ, 0>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb, lead);
+    mma3<BITS, BSTEP, SFBQ, 3>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb, lead);
+    mma3<BITS, BSTEP, SFBQ, 6>(d, idn, a_lo, a_hi, bb, b_hi, sfa_t, sfb, lead);
 }
 /* the block's piece of the plane list, u in [u0, u1) with u = (sample * tiles + tile) * D + z, cut into runs along z */
 struct Piece { long long u, u1; };
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     StageRec *recs = (StageRec *)(smem_raw + a.off_rec);
     float *bias_s = (float *)(smem_raw + a.off_bias);
     uint8_t *wsm = smem_raw + a.off_w, *stages = smem_raw + a.off_ring;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int R = a.ring, NS = a.nslot;
     /* barriers: tma[R] (codes + scale window landed), sf[R] (A scales laid out), empty[R], accumulator full / empty per slot, weights */
     const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_accf = bar_tma + 24 * R, bar_acce = bar_accf + 8 * kMaxSlots, bar_w = bar_acce + 8 * kMaxSlots, bar_red = bar_w + 8;
@@ -197,7 +196,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = uni(*tmem_slot);
     Piece piece = piece_of_block(a);
 
     if (warp == 0) {
@@ -253,10 +252,14 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             }
         }
     } else if (warp == 1) {
-        /* ---------------- MMA issue: one thread follows the records; a stage is straight-line code ---------------- */
-        if (lane == 0) {
+        /* ---------------- MMA issue: one warp follows the records; a stage is straight-line code.  The whole warp runs the loop and one lane issues:
+           a record passes through a shuffle, so that the operands of an MMA are known to be the same in every lane and its address arithmetic stays in
+           the uniform registers that the instruction reads, instead of being moved there operand by operand ---------------- */
+        {
+            const uint32_t lead = elect_one();
             bool ok = mbar_wait(bar_w, 0, abort_flag, kWaitLimitR);
-            if (!ok) raise_r(a, abort_flag, 6, 0);
+            if (!ok && lane == 0) raise_r(a, abort_flag, 6, 0);
+            ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
             const uint32_t wbase = smem_u32(wsm);
             const uint32_t a_hi = desc_hi(160), b_hi = desc_hi(128);
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             if (ok) {
                 /* the B scale factors of every (input block, tap quad, image, 128-row group): copied to TMEM once */
                 const int nsf = a.nki * a.nquad * a.gt;
-                for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi));
+                for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi), lead);
             }
             const uint32_t a_lo0 = desc_lo(smem_u32(stages), 2880), a_step = (uint32_t)a.stage_bytes >> 4;
             const uint32_t sfa_t0 = tmem + (uint32_t)a.sfa_base, sfa_cols = (uint32_t)a.sfa_cols;
@@ -272,21 +275,22 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             while (ok) {
                 /* the stage's A scales are in TMEM (the scale warp's copies have completed); that warp passed the stage's load barrier before
                    it laid the scales out, so the codes have landed too */
-                if (!mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 3, it, bar_sf + 8 * s - bar_tma, ph); break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 3, it, bar_sf + 8 * s - bar_tma, ph); break; }
                 /* the whole record goes to registers before anything is committed: committing `empty` hands the stage, record included, back to the producer */
                 const uint4 *r = (const uint4 *)(recs + s);
-                const uint4 g1 = r[0], g2 = r[1], wc = r[2]; const uint32_t last = r[3].x;
+                const uint4 g1 = uni(r[0]), g2 = uni(r[1]), wc = uni(r[2]); const uint32_t last = uni(r[3].x);
                 if (wc.x) {   /* a plane that starts here: its slot must have been read out and zeroed by the epilogue */
-                    if (!mbar_wait(wc.x & 0x7fffffffu, wc.x >> 31, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 7, it, (wc.x & 0x7fffffffu) - bar_tma, wc.x >> 31); break; }
-                    if (wc.y && !mbar_wait(wc.y & 0x7fffffffu, wc.y >> 31, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 7, it); break; }
+                    bool got = mbar_wait(wc.x & 0x7fffffffu, wc.x >> 31, abort_flag, kWaitLimitR);
+                    if (got && wc.y) got = mbar_wait(wc.y & 0x7fffffffu, wc.y >> 31, abort_flag, kWaitLimitR);
+                    if (!__all_sync(0xffffffffu, got)) { if (lane == 0) raise_r(a, abort_flag, 7, it, (wc.x & 0x7fffffffu) - bar_tma, wc.x >> 31); break; }
                 }
                 tc_fence_after();
                 const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = sfa_t0 + ((uint32_t)it & 1u) * sfa_cols;
-                issue_group<BITS, 32 * NCH>(g1.x, g1.y, g1.z, g1.w, a_lo, a_hi, b_hi, sfa_t);
-                if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, g2.z, g2.w, a_lo, a_hi, b_hi, sfa_t);
+                issue_group<BITS, 32 * NCH>(g1.x, g1.y, g1.z, g1.w, a_lo, a_hi, b_hi, sfa_t, lead);
+                if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, g2.z, g2.w, a_lo, a_hi, b_hi, sfa_t, lead);
                 /* the one commit of a stage: "stage s has been consumed".  The producer reuses the ring slot on it, the scale warps reuse the
                    stage's TMEM scale buffer on it and pass the news that output planes are complete on to the epilogue */
-                umma_commit(bar_empty + 8 * s);
+                umma_commit(bar_empty + 8 * s, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
                 if (last) break;
             }
@@ -306,7 +310,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
            barrier of both kinds in order, also for the stages the other warp works on: a warp that skipped a phase of a barrier could
            later take a wait for phase k + 2 as satisfied while the barrier is still in phase k + 1 (the parity reads the same). */
         const int sfw = warp - 2;
-        const uint32_t sf_hi = desc_hi(128);
+        const uint32_t sf_hi = desc_hi(128), lead = elect_one(), sfa_lo0 = desc_lo(smem_u32(stages) + (uint32_t)a.offSFA, 0), sstep = (uint32_t)a.stage_bytes >> 4;
         const uint32_t sfa_t = tmem + (uint32_t)a.sfa_base + (uint32_t)sfw * (uint32_t)a.sfa_cols;      /* this warp's stages all have parity sfw */
         int it = 0, s = 0, ph = 0, s2 = 0, ph2 = 0; bool ok = true;
         int done = 0;                       /* output planes completed by all stages before the current one */
@@ -324,7 +328,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             const Run rn = next_run(a, piece);
             const int x0 = (rn.txy % a.tiles_x) * 8;
             const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
-            const int xo = (x0 - 1) - (((x0 - 1) >> 4) << 4);     /* 7 or 15 */
+            const int off = (lane >> 3) * 32 + (lane & 7) + (x0 - 1) - (((x0 - 1) >> 4) << 4), sh = (off & 3) * 8;      /* the three dx of a row are neighbours: two words and a funnel shift */
             for (int zi = zlo; zi <= zhi && ok; zi++) {
                 /* planes that the last stage of this input plane completes: the plane below it, and the volume's last plane with it */
                 const int nc = (zi - 1 >= rn.zb ? 1 : 0) + ((zi == a.D - 1 && rn.ze == a.D) ? 1 : 0);
@@ -339,20 +343,23 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         continue;
                     }
                     uint8_t *stg = stages + (size_t)cs * a.stage_bytes;
-                    const uint8_t *sw = stg + a.offSW;
                     uint32_t *sfa = (uint32_t *)(stg + a.offSFA);
+                    const uint32_t *sw = (const uint32_t *)(stg + a.offSW + (off & ~3));
                     uint32_t wq[4][5];
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        const int r = q * 32 + lane;
-                        const uint8_t *p = sw + (r >> 3) * 32 + (r & 7) + xo;
+                        uint32_t t[3], u[3];          /* bytes 0..2: the scales of dx = 0, 1, 2 */
 #pragma unroll
-                        for (int t = 0; t < 5; t++) wq[q][t] = 0u;
-#pragma unroll
-                        for (int j = 0; j < 9; j++) {
-                            const uint32_t b0 = p[(j / 3) * 32 + j % 3];
-                            if (BITS == 8) wq[q][j >> 2] |= b0 << (8 * (j & 3));
-                            else { const uint32_t b1 = p[576 + (j / 3) * 32 + j % 3]; wq[q][j >> 1] |= (b0 | (b1 << 8)) << (16 * (j & 1)); }
+                        for (int dy = 0; dy < 3; dy++) {
+                            const uint32_t *p = sw + q * 32 + dy * 8;
+                            t[dy] = __funnelshift_r(p[0], p[1], sh);
+                            if (BITS == 4) u[dy] = __funnelshift_r(p[144], p[145], sh);
+                        }
+                        if (BITS == 8) {              /* taps 0-3, 4-7, 8 */
+                            wq[q][0] = __byte_perm(t[0], t[1], 0x4210); wq[q][1] = __byte_perm(t[1], t[2], 0x5421); wq[q][2] = (t[2] >> 16) & 0xffu;
+                        } else {                      /* pairs (block 2 ki, block 2 ki + 1) of taps 0 1, 2 3, 4 5, 6 7, 8 */
+                            wq[q][0] = __byte_perm(t[0], u[0], 0x5140); wq[q][1] = __byte_perm(__byte_perm(t[0], u[0], 0x0062), __byte_perm(t[1], u[1], 0x0040), 0x5410);
+                            wq[q][2] = __byte_perm(t[1], u[1], 0x6251); wq[q][3] = __byte_perm(t[2], u[2], 0x5140); wq[q][4] = __byte_perm(t[2], u[2], 0x0062) & 0xffffu;
                         }
                     }
                     /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
@@ -365,13 +372,11 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     done += ncs;
                     it++; if (++s == R) { s = 0; ph ^= 1; }
                     __syncwarp();
-                    if (lane == 0) {
-                        tc_fence_after();
-                        const uint32_t src = desc_lo(smem_u32(sfa), 0);
+                    tc_fence_after();
+                    const uint32_t src = sfa_lo0 + (uint32_t)cs * sstep;
 #pragma unroll
-                        for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make(src + 32u * q, sf_hi));
-                        umma_commit(bar_sf + 8 * cs);
-                    }
+                    for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make(src + 32u * q, sf_hi), lead);
+                    umma_commit(bar_sf + 8 * cs, lead);
                     __syncwarp();
                 }
             }
@@ -473,8 +478,33 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 tmem_ld_wait();
                 tmem_zero32(tcol);
                 if (NCH > 1) tmem_zero32(tcol + 32);
-                if (a.fast_h16) {
-                    /* fp16 blocked output [n][block][voxel][32]: bias, one rounding; the zeroing of the slot completes meanwhile */
+                if (a.fast_h16 && !STATS) {
+                    /* fp16 blocked output [n][block][voxel][32]: bias, one rounding.  A thread has a whole row of 64 bytes and stores it as two full sectors: passing
+                       the rows through shared memory for 512-byte runs took a tenth of its bandwidth, which the MMA operands need (64 -> 64 MX-fp4 on 64^3 20.9 us,
+                       18.5 this way; 32 -> 32 MX-fp8 on 128^3 68.9 and 68.0) */
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_acce + 8 * slot);          /* the slot is free once it is in registers and zeroed */
+                    uint8_t *pv = (uint8_t *)a.e.y + (((size_t)rn.n * a.e.nb_dst + a.e.b0 + ctile * NCH) * S + ((size_t)z * a.H + oy) * a.W + ox) * 64;
+#pragma unroll
+                    for (int jc = 0; jc < NCH; jc++) {
+                        const float4 *bs = (const float4 *)(bias_s + jc * 32);
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            uint32_t h[8];
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                const float4 b0 = bs[4 * k + t];
+                                const __half2 x0 = __floats2half2_rn(__fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t]), b0.x), __fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t + 1]), b0.y));
+                                const __half2 x1 = __floats2half2_rn(__fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t + 2]), b0.z), __fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t + 3]), b0.w));
+                                h[2 * t] = *(const uint32_t *)&x0; h[2 * t + 1] = *(const uint32_t *)&x1;
+                            }
+                            if (row_ok) asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(pv + (size_t)jc * S * 64 + k * 32), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7]) : "memory");
+                        }
+                    }
+                } else if (a.fast_h16) {
+                    /* the same with the statistics, which are taken where a warp re-reads its rows; the zeroing of the slot completes meanwhile */
                     __syncwarp();                               /* the previous plane's rows have been read out of the staging buffer */
 #pragma unroll
                     for (int jc = 0; jc < NCH; jc++) {
@@ -502,7 +532,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                             const uint4 v = *(const uint4 *)(stg_r + jc * 2048 + i * 512);
                             const bool in = sy + i < a.H;
                             if (in) *(uint4 *)(pz + (size_t)jc * S * 64 + (size_t)i * row_b) = v;
-                            if (STATS && in) {
+                            if (in) {
                                 const __half2 *hp = (const __half2 *)&v;
 #pragma unroll
                                 for (int t = 0; t < 4; t++) {
@@ -647,13 +677,13 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     a.tiles_x = (W + 7) / 8; a.tiles = a.tiles_x * ((H + 15) / 16);
     a.units = (long long)N * a.tiles * D;
     a.nquad = c->nquad;
-    a.fast_h16 = e.out_mode == UMX_OUT_H16B && !e.tconv;
+    a.fast_h16 = e.out_mode == UMX_OUT_H16B && !e.tconv && (want_coef || !((size_t)e.y & 31));      /* stores of 32 bytes */
     if (want_coef && (!a.fast_h16 || !part || g.ncol > 64)) return 0;
     a.cop = c->cop;
     /* the codes and the scale window are TMA destinations (128-byte aligned) */
     a.offSW = 5888; a.offSFA = a.offSW + (c->bits == 8 ? 640 : 1152);
     a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
-    a.off_rec = 1024; a.off_bias = a.off_rec + 12 * 64; a.off_stage = 2048; a.off_red = a.off_stage; a.off_w = a.off_stage + 8192 * (g.nt == 32 ? 1 : 2); a.off_ring = (a.off_w + a.w_bytes + 1023) & ~1023;
+    a.off_rec = 1024; a.off_bias = a.off_rec + 12 * 64; a.off_stage = 2048; a.off_red = a.off_stage; a.off_w = a.off_stage + (want_coef ? 8192 * (g.nt == 32 ? 1 : 2) : 0); a.off_ring = (a.off_w + a.w_bytes + 1023) & ~1023;
     int dev = 0, sms = 148; cudaGetDevice(&dev);
     { static int sms_of[16]; if (!sms_of[dev & 15]) { int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); sms_of[dev & 15] = v; } sms = sms_of[dev & 15]; }   /* looked up once per device */
     /* two blocks a multiprocessor when shared memory (113 KB each) and TMEM (256 columns each) allow */

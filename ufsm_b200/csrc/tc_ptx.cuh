@@ -15,6 +15,18 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
+/* tcgen05 instructions read their operands from uniform registers.  Issued from a branch that one lane takes, each operand is a per-thread value that
+   has to be moved there (128 -> 64 channels on 64^3: a stage of nine MMAs 1190 clocks, 850 this way); so the whole warp runs the loop of a role that
+   issues them, its values are uniform, and only the instruction itself is predicated on the elected lane (`lead`). */
+/* lane 0's value, which the compiler then knows to be the same in the whole warp */
+__device__ __forceinline__ uint32_t uni(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint4 uni(uint4 v) { return make_uint4(uni(v.x), uni(v.y), uni(v.z), uni(v.w)); }
+/* 1 in one lane of a converged warp, 0 in the others */
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok)::"memory");
+    return ok;
+}
 /* the same with a suspend-time hint: the hardware parks the thread until the phase completes or about `ns` nanoseconds have passed, so a
    waiting warp issues one instruction per `ns` instead of spinning through the issue slots the working warps need */
 __device__ __forceinline__ uint32_t mbar_try_hint(uint32_t bar, uint32_t parity, uint32_t ns) {
@@ -83,20 +95,24 @@ __device__ __forceinline__ uint32_t idesc_mxf8(int n, int sfa_id, int sfb_id) { 
 __device__ __forceinline__ uint32_t idesc_mxf4(int n, int sfa_id, int sfb_id) {   /* E2M1 x E2M1, K = 64, two scales per row */
     return ((uint32_t)sfb_id << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24) | ((uint32_t)sfa_id << 29);
 }
-__device__ __forceinline__ void umma_mxf8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
+__device__ __forceinline__ void umma_mxf8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb, uint32_t lead) {
+    asm volatile("{\n\t.reg .pred p, pl;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 pl, %7, 0;\n\t"
+                 "@pl tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb), "r"(lead) : "memory");
 }
-__device__ __forceinline__ void umma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
+__device__ __forceinline__ void umma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb, uint32_t lead) {
+    asm volatile("{\n\t.reg .pred p, pl;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 pl, %7, 0;\n\t"
+                 "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb), "r"(lead) : "memory");
 }
 /* 32 lanes x 128 bits of shared memory (512 contiguous bytes described by sdesc) -> the same 4 columns of all four 32-lane quarters */
-__device__ __forceinline__ void utccp_32x128b(uint32_t tmem, uint64_t sdesc) { asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(sdesc) : "memory"); }
+__device__ __forceinline__ void utccp_32x128b(uint32_t tmem, uint64_t sdesc, uint32_t lead) {
+    asm volatile("{\n\t.reg .pred pl;\n\tsetp.ne.b32 pl, %2, 0;\n\t@pl tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem), "l"(sdesc), "r"(lead) : "memory");
+}
 /* arrive on an mbarrier once every tcgen05 operation this thread issued so far has completed */
-__device__ __forceinline__ void umma_commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t lead = 1u) {
+    asm volatile("{\n\t.reg .pred pl;\n\tsetp.ne.b32 pl, %1, 0;\n\t@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead) : "memory");
+}
 /* 32 consecutive fp32 columns of this warp's 32 TMEM lanes: register k of lane l = (lane base + l, column base + k) */
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
@@ -128,7 +144,7 @@ __device__ __forceinline__ uint64_t desc_make(uint32_t lo, uint32_t hi) { return
    item j reads A at a_lo + a_step(j), B at b_lo + j * b_step; fp8: four items a scale quad (scale id = j % 4); fp4: two (id = 2 (j % 2)) */
 template <int BITS, int ITEMS, bool TAPS3>
 __device__ __forceinline__ void issue_items(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t b_step, uint32_t a_step1,
-                                            uint32_t idesc0, uint32_t sfa_t, uint32_t sfb_t, bool fresh, int nitems) {
+                                            uint32_t idesc0, uint32_t sfa_t, uint32_t sfb_t, bool fresh, int nitems, uint32_t lead) {
 #pragma unroll
     for (int j = 0; j < ITEMS; j++) {
         if (j < nitems) {
@@ -138,8 +154,8 @@ __device__ __forceinline__ void issue_items(uint32_t d_tmem, uint32_t a_lo, uint
             const uint64_t ad = desc_make(a_lo + aoff, a_hi), bd = desc_make(b_lo + (uint32_t)j * b_step, b_hi);
             const uint32_t idesc = idesc0 | ((uint32_t)id << 4) | ((uint32_t)id << 29);
             const uint32_t acc = (fresh && j == 0) ? 0u : 1u;
-            if (BITS == 8) umma_mxf8(d_tmem, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q);
-            else umma_mxf4(d_tmem, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q);
+            if (BITS == 8) umma_mxf8(d_tmem, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead);
+            else umma_mxf4(d_tmem, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead);
         }
     }
 }
