@@ -17,11 +17,11 @@
 
    Scale factors.  tcgen05 block-scaled MMAs read scales from TMEM: row r of a 128-row operand at lane r % 32, column r / 32,
    byte = scale id.  The scale of an A row depends on the tap (it is the shifted voxel's), so four epilogue warps gather, per
-   stage, the nine shifted scale sets from the scale plane into that layout in shared memory, and the MMA thread copies them to
+   stage, the nine shifted scale sets from the scale plane into that layout in shared memory, and the MMA warp copies them to
    TMEM with tcgen05.cp before issuing the stage's MMAs.  Out-of-range voxels get scale 1 (their codes are zero).
 
-   Roles (224 threads): warp 0 lane 0 = TMA producer; warp 1 = TMEM allocation, lane 0 = MMA issue; warp 6 lane 0 = scale copies; warps 2-5 = scale gather,
-   then the epilogue (tcgen05.ld of 32 channels per voxel = one MX block per thread: bias, fp16 store or MX requantisation;
+   Roles (192 threads): warp 0 = TMA producer; warp 1 = TMEM allocation, scale copies and MMA issue; warps 2-5 = scale gather, then the epilogue
+   (tcgen05.ld of 32 channels per voxel = one MX block per thread: bias, fp16 store or MX requantisation;
    InstanceNorm partial sums are taken by a separate pass over the stored output).  Every wait is bounded; a wait that gives up records (code, block, stage) in a device
    flag, raises a block-wide abort flag and the block tears down normally. */
 #include "conv_epi.cuh"
@@ -31,9 +31,9 @@
 
 namespace {
 
-constexpr int kThreads = 224;
+constexpr int kThreads = 192;
 constexpr int kTmemCols = 256;
-constexpr int kSfBase = 128;        /* TMEM columns: [0, 128) accumulators, then up to three scale buffers of 40 (A 20 | B 20) */
+constexpr int kSfBase = 128;        /* TMEM columns: [0, 128) accumulators, then two scale buffers of 40 (A 20 | B 20) */
 constexpr long long kWaitLimit = 4000000000ll;   /* clock cycles (about two seconds) */
 
 struct ConvArgs {
@@ -69,13 +69,13 @@ template <int BITS>
 __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__ CUtensorMap map0, const ConvArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     /* control block, then the stage ring at the next 1024-byte boundary */
-    uint64_t *bars = (uint64_t *)smem_raw;                       /* ring each: tma full, scales in shared memory, scales in TMEM, empty; then accumulator full */
+    uint64_t *bars = (uint64_t *)smem_raw;                       /* ring each: tma full, scales laid out, empty; then accumulator full */
     uint32_t *tmem_slot = (uint32_t *)(smem_raw + 512);
     volatile int *abort_flag = (volatile int *)(smem_raw + 516);
     uint8_t *stages = smem_raw + 1024;
     const int warp = (int)uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int R = a.ring;
-    const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_cp = bar_tma + 16 * R, bar_empty = bar_tma + 24 * R, bar_acc = bar_tma + 32 * R;
+    const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_acc = bar_tma + 24 * R;
 
     const int txy = blockIdx.x, tx = txy % a.tiles_x, ty = txy / a.tiles_x;
     const int z = blockIdx.y;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     }
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 4); mbar_init(bar_cp + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
+        for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 4); mbar_init(bar_empty + 8 * i, 1); }
         mbar_init(bar_acc, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -103,16 +103,13 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = uni(*tmem_slot);
-    const int nbuf = R < 3 ? R : 3;               /* TMEM scale buffers in use */
-    /* with a ring of two the stage that waits for the scale thread is the stage the MMAs need next: the MMA thread copies for itself (128 -> 128 on
-       32^3, two blocks a multiprocessor: 19.1 us, 20.6 with the scale thread between) */
-    const bool own_copies = R < 3;
-
     /* a stage is live unless it is a 3^3 stage whose input plane lies outside the volume (it would add zeros) */
     auto stage_live = [&](int st) -> bool { if (a.taps != 27) return true; const int zi = z + st % 3 - 1; return zi >= 0 && zi < a.D; };
     auto stage_items = [&](int st) -> int { return a.taps == 27 ? 9 : min(4, a.nki - 4 * st); };
 
-    /* a stage's A and B scales from shared memory to TMEM buffer buf (one warp) */
+    /* a stage's A and B scales from shared memory to TMEM buffer buf.  Copies and MMAs of one thread run in issue order, so two buffers are enough and no
+       barrier guards them; with uniform operands a copy costs the warp a few clocks (as a role of its own it cost a barrier round trip a stage: 128 -> 128 on
+       32^3 18.0 us against 16.6, 256 -> 128 28.4 against 26.1) */
     auto copy_scales = [&](int st, uint32_t so, int buf, uint32_t lead) {
         const uint32_t sf_hi = desc_hi(128), sb0 = smem_u32(stages), sfa_lo = desc_lo(sb0 + a.offSFA, 0) + so, sfb_lo = desc_lo(sb0 + a.offSFB, 0) + so;
         const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
@@ -125,12 +122,14 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
 
     if (warp == 0) {
         /* ---------------- TMA producer ---------------- */
-        if (lane == 0) {
-            tma_prefetch_desc(&map0);
+        {
+            const uint32_t lead = elect_one();
+            if (lead) tma_prefetch_desc(&map0);
             const uint8_t *wbase = a.wpk + (size_t)ntile * a.nst * a.w_stage_bytes;
             auto put_weights = [&](int st, int s) {
                 const uint32_t bar = bar_tma + 8 * s;
                 const int abytes = a.taps == 27 ? 5760 : stage_items(st) * 4096;
+                if (!lead) return;
                 mbar_expect_tx(bar, (uint32_t)(abytes + a.w_stage_bytes));
                 bulk_g2s(smem_u32(stages + (size_t)s * a.stage_bytes + a.offW), wbase + (size_t)st * a.w_stage_bytes, (uint32_t)a.w_stage_bytes, bar);
             };
@@ -138,21 +137,20 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
             int early = 0;
             for (int st = st_lo; st < st_hi && early < R; st++) if (stage_live(st)) put_weights(st, early++);
             pdl_wait();                          /* from here on this thread touches activations */
-            int it = 0;
+            int it = 0, s = 0, ph = 0;
             for (int st = st_lo; st < st_hi; st++) {
                 if (!stage_live(st)) continue;
-                const int s = it % R, ph = (it / R) & 1;
                 uint8_t *sb = stages + (size_t)s * a.stage_bytes;
                 const uint32_t bar = bar_tma + 8 * s;
                 const int items = stage_items(st);
                 if (it >= early) {
-                    if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 1, st); break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 1, st); break; }
                     put_weights(st, s);
                 }
                 /* two 16-byte-wide planes per K item (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1) */
                 if (a.taps == 27) {
                     const int ki = st / 3, zi = z + st % 3 - 1;
-                    tma_load_4d(smem_u32(sb + a.offA), &map0, bar, (x0 - 1) * 16, y0 - 1, zi, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki);
+                    tma_load_4d(smem_u32(sb + a.offA), &map0, bar, (x0 - 1) * 16, y0 - 1, zi, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki, lead);
                 } else {
                     for (int j = 0; j < items; j++) {
                         const int ki = 4 * st + j;
@@ -160,12 +158,12 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                             /* K item ki = tap * a.nit + i: fp8: block i (its two half planes); fp4: blocks 2 i and 2 i + 1 (the second may lie past the
                                sample's last block: its weights are zero and its scale is read as 1) */
                             const int tap = ki / a.nit, blk = ki - tap * a.nit;
-                            tma_load_5d(smem_u32(sb + a.offA + j * 4096), &map0, bar, 0, 2 * x0 + tap % 3 - 1, 2 * y0 + (tap / 3) % 3 - 1, 2 * z + tap / 9 - 1, BITS == 8 ? (n * a.nbi + blk) * 2 : n * a.nbi + 2 * blk);
+                            tma_load_5d(smem_u32(sb + a.offA + j * 4096), &map0, bar, 0, 2 * x0 + tap % 3 - 1, 2 * y0 + (tap / 3) % 3 - 1, 2 * z + tap / 9 - 1, BITS == 8 ? (n * a.nbi + blk) * 2 : n * a.nbi + 2 * blk, lead);
                         } else
-                        tma_load_4d(smem_u32(sb + a.offA + j * 4096), &map0, bar, x0 * 16, y0, z, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki);
+                        tma_load_4d(smem_u32(sb + a.offA + j * 4096), &map0, bar, x0 * 16, y0, z, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki, lead);
                     }
                 }
-                it++;
+                it++; if (++s == R) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
@@ -183,46 +181,17 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 if (!stage_live(st)) continue;
                 const uint32_t so = (uint32_t)s * sstep;
                 const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
-                if (own_copies) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 2, st); ok = false; break; }
-                    tc_fence_after();
-                    copy_scales(st, so, buf, lead);
-                } else {
-                    /* the scale thread passed the stage's load barrier before it copied the scales, so codes and weights have landed too */
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_cp + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
-                    tc_fence_after();
-                }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 2, st); ok = false; break; }
+                tc_fence_after();
+                copy_scales(st, so, buf, lead);
                 if (a.taps == 27) issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9, lead);
                 else issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, stage_items(st), lead);
                 umma_commit(bar_empty + 8 * s, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
-                if (++buf == nbuf) buf = 0;
+                buf ^= 1;
             }
             umma_commit(bar_acc, lead);   /* also after a give-up: the epilogue must not wait for its full limit */
-        }
-    } else if (warp == 6) {
-        /* ---------------- scale copies: one thread brings a stage's A and B scales from shared memory to one of nbuf TMEM buffers.  A tcgen05.cp costs
-           the thread that issues it some 40 clocks and the tensor pipe next to nothing, so it is kept out of the MMA thread (a stage of nine N = 128
-           MMAs: 1050 clocks with the six copies in it, 576 of them arithmetic). ---------------- */
-        if (!own_copies) {
-            const uint32_t lead = elect_one();
-            const uint32_t sstep = (uint32_t)a.stage_bytes >> 4;
-            int it = 0, s = 0, ph = 0, s3 = 0, ph3 = 0, buf = 0;
-            for (int st = st_lo; st < st_hi; st++) {
-                if (!stage_live(st)) continue;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 2, st); break; }
-                if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 4, st); break; }
-                if (it >= nbuf) {                /* the MMAs that read this buffer (nbuf stages back; nbuf <= ring, so that barrier is at most one phase ahead) */
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s3, ph3, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 7, st); break; }
-                    if (++s3 == R) { s3 = 0; ph3 ^= 1; }
-                }
-                tc_fence_after();
-                copy_scales(st, (uint32_t)s * sstep, buf, lead);
-                umma_commit(bar_cp + 8 * s, lead);
-                it++; if (++s == R) { s = 0; ph ^= 1; }
-                if (++buf == nbuf) buf = 0;
-            }
         }
     } else {
         /* ---------------- scale gather, then epilogue ---------------- */

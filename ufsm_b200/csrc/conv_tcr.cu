@@ -14,18 +14,19 @@
    3 KB B tile exceed what shared memory delivers in 48).  One warp runs the MMA loop with uniform values and one elected lane issues: issued by
    a lone thread, with operands moved to uniform registers one by one, a stage of nine MMAs took 1190 clocks on 128 -> 64 channels, 64^3 (80.7 us
    the conv, 60.0 now).  A commit costs its issuer another 60 clocks, so there is one per stage, and every role's per-stage program is kept short: (1) the
-   producer thread tracks slots and parities incrementally (no division) and hands the MMA thread a record with everything
+   producer tracks slots and parities incrementally (no division) and hands the MMA warp a record with everything
    precomputed: TMEM addresses, the N field of the instruction descriptor, B descriptor and B scale addresses, the barriers to wait
    for; (2) the MMA warp's stage is three PTX blocks of three MMAs whose operands are a record field plus an immediate; (3)
    accumulators are never "fresh": the epilogue zeroes a slot after reading it, so every MMA accumulates; (4) the A scale factors are
    gathered from a TMA-staged window in shared memory with no bounds logic (voxels outside the volume arrive as zero codes with scale
-   byte 0) and copied to TMEM by the scale warps themselves, whose commit is what the MMA warp waits for; (5) the MMA warp's single
-   commit per stage lands on the stage's `empty` barrier; the scale warps, which wait for that barrier anyway before they reuse a TMEM
-   scale buffer, pass the completion of output planes on to the epilogue's accumulator-full barriers; (6) two blocks share a
-   multiprocessor when the weights are small enough: one block's waits are the other's issue time.
+   byte 0), as far ahead of the MMAs as the ring is deep, and copied to TMEM by the MMA warp (copies and MMAs of one thread run in issue order,
+   so nothing guards the two buffers; copied by the gathering warps, which had to wait for the MMAs of two stages back, 64 -> 64 on 64^3 took
+   26.8 us, 25.8 this way); (5) the MMA warp's single commit per stage lands on the stage's `empty` barrier; a relay passes the completion of
+   output planes on to the epilogue's accumulator-full barriers; (6) two blocks share a multiprocessor when the weights are small enough: one
+   block's waits are the other's issue time.
 
-   Roles (256 threads): warp 0 lane 0 producer (records + TMA), warp 1 MMA issue (and TMEM), warps 2-3 scale
-   layout, scale copies and completion relay (alternate stages), warps 4-7 epilogue.  All waits are bounded as in conv_mx_k. */
+   Roles (256 threads): warp 0 producer (records + TMA), warp 1 scale copies and MMA issue (and TMEM), warp 2 scale layout, warp 3 completion
+   relay, warps 4-7 epilogue.  All waits are bounded as in conv_mx_k. */
 #include "conv_epi.cuh"
 #include "tc_ptx.cuh"
 #include <stdlib.h>
@@ -78,7 +79,7 @@ struct ConvRArgs {
     int *err;
 };
 
-/* what the MMA thread does for one stage; written by the producer thread */
+/* what the MMA warp does for one stage; written by the producer */
 struct StageRec {
     uint32_t d1, idn1, bb1, sfb1;      /* first group: TMEM accumulator address, instruction descriptor with N, B descriptor low word of tap 0, B scale address */
     uint32_t d2, idn2, bb2, sfb2;      /* second group when the window wraps (idn2 = 0: none) */
@@ -201,8 +202,9 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
 
     if (warp == 0) {
         /* ---------------- producer: stage records and TMA ---------------- */
-        if (lane == 0) {
-            tma_prefetch_desc(&map0); tma_prefetch_desc(&maps);
+        {
+            const uint32_t lead = elect_one();
+            if (lead) { tma_prefetch_desc(&map0); tma_prefetch_desc(&maps); }
             pdl_wait();      /* the only role that reads activations from global memory; every other role's data comes through this thread's loads,
                                 so the weight load, the B scale copies and the zeroing of the accumulators overlap the previous kernel */
             const uint32_t nt = (uint32_t)a.nt, bstep9 = 9u * 2u * 3u * nt;            /* B descriptor step of one input block: nine taps of two halves of 3 nt rows */
@@ -232,20 +234,22 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     const int slot = NS - 1 - pos, n1 = min(cnt, NS - slot), n2 = cnt - n1;
                     const uint32_t g1 = (uint32_t)(dzf == 0 ? 0 : dzf == 1 ? a.goff1 : a.goff2), g2 = (uint32_t)(dzf + n1 == 1 ? a.goff1 : a.goff2);
                     for (int ki = 0; ki < a.nki; ki++) {
-                        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 1, it, bar_empty + 8 * s - bar_tma, ph ^ 1); ok = false; break; }
+                        if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 1, it, bar_empty + 8 * s - bar_tma, ph ^ 1); ok = false; break; }
                         const bool kl = ki == a.nki - 1;
                         const uint32_t bk = b_lo0 + (uint32_t)ki * bstep9, sk = sfb_t0 + (uint32_t)ki * sfb_per_ki;
-                        uint4 *r = (uint4 *)(recs + s);
-                        r[0] = make_uint4(tmem + (uint32_t)slot * nt, idesc_b | (uint32_t)n1 * ntn, bk + (uint32_t)dzf * nt, sk + g1);
-                        r[1] = make_uint4(tmem, n2 ? (idesc_b | (uint32_t)n2 * ntn) : 0u, bk + (uint32_t)(dzf + n1) * nt, sk + g2);
-                        r[2] = make_uint4(ki == 0 ? w0 : 0u, ki == 0 ? w1 : 0u, 0u, 0u);
-                        r[3] = make_uint4((last_run && zi == zhi && kl) ? 1u : 0u, 0u, 0u, 0u);
+                        if (lead) {
+                            uint4 *r = (uint4 *)(recs + s);
+                            r[0] = make_uint4(tmem + (uint32_t)slot * nt, idesc_b | (uint32_t)n1 * ntn, bk + (uint32_t)dzf * nt, sk + g1);
+                            r[1] = make_uint4(tmem, n2 ? (idesc_b | (uint32_t)n2 * ntn) : 0u, bk + (uint32_t)(dzf + n1) * nt, sk + g2);
+                            r[2] = make_uint4(ki == 0 ? w0 : 0u, ki == 0 ? w1 : 0u, 0u, 0u);
+                            r[3] = make_uint4((last_run && zi == zhi && kl) ? 1u : 0u, 0u, 0u, 0u);
+                            mbar_expect_tx(bar_tma + 8 * s, TX);
+                        }
                         const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
-                        mbar_expect_tx(bar, TX);
                         /* codes: two 16-byte-wide planes (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1), 18 rows of 10 voxels;
                            scale bytes: 18 rows of a 32-byte window per block */
-                        tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki);
-                        tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki);
+                        tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki, lead);
+                        tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki, lead);
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
                 }
@@ -269,12 +273,11 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int nsf = a.nki * a.nquad * a.gt;
                 for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi), lead);
             }
-            const uint32_t a_lo0 = desc_lo(smem_u32(stages), 2880), a_step = (uint32_t)a.stage_bytes >> 4;
+            const uint32_t a_lo0 = desc_lo(smem_u32(stages), 2880), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
             const uint32_t sfa_t0 = tmem + (uint32_t)a.sfa_base, sfa_cols = (uint32_t)a.sfa_cols;
             int s = 0, ph = 0, it = 0;
             while (ok) {
-                /* the stage's A scales are in TMEM (the scale warp's copies have completed); that warp passed the stage's load barrier before
-                   it laid the scales out, so the codes have landed too */
+                /* the stage's A scales are laid out; the scale warp passed the stage's load barrier before, so the codes have landed too */
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 3, it, bar_sf + 8 * s - bar_tma, ph); break; }
                 /* the whole record goes to registers before anything is committed: committing `empty` hands the stage, record included, back to the producer */
                 const uint4 *r = (const uint4 *)(recs + s);
@@ -286,103 +289,82 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 }
                 tc_fence_after();
                 const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = sfa_t0 + ((uint32_t)it & 1u) * sfa_cols;
+                /* copies and MMAs of one thread run in issue order, so a buffer is overwritten after the MMAs that read it two stages ago */
+#pragma unroll
+                for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi), lead);
                 issue_group<BITS, 32 * NCH>(g1.x, g1.y, g1.z, g1.w, a_lo, a_hi, b_hi, sfa_t, lead);
                 if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, g2.z, g2.w, a_lo, a_hi, b_hi, sfa_t, lead);
-                /* the one commit of a stage: "stage s has been consumed".  The producer reuses the ring slot on it, the scale warps reuse the
-                   stage's TMEM scale buffer on it and pass the news that output planes are complete on to the epilogue */
+                /* the one commit of a stage: "stage s has been consumed".  The producer reuses the ring slot on it, and the relay passes the news that output
+                   planes are complete on to the epilogue */
                 umma_commit(bar_empty + 8 * s, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
                 if (last) break;
             }
         }
-    } else if (warp < 4) {
-        /* ---------------- A scales: warp 2 takes the even stages, warp 3 the odd ones ----------------
+    } else if (warp == 2) {
+        /* ---------------- A scales ----------------
            The TMA left 18 rows of a 32-byte window of scale bytes (two windows for fp4); row r of the tile needs, for tap (dy, dx), the
-           byte at window row r / 8 + dy, column r % 8 + dx + (x0 - 1 - xa).  Four rows per lane (one per TMEM column of the quad).  The
-           warp lays the nine shifted scale sets out in shared memory in the tcgen05.cp layout, and its lane 0 copies them to the TMEM
-           scale buffer of the stage's parity and commits: the MMA thread waits for that commit and issues nothing but MMAs (a scale copy
-           or a commit costs its issuing thread 30 to 130 clocks, an MMA of N = 96 occupies the tensor pipe for 56).
-
-           The same warps relay completions.  The MMA thread commits once per stage, on the stage's `empty` barrier.  A scale warp
-           waits for that barrier of stage it - 2 before it touches the TMEM scale buffer again (two buffers: the MMAs that read it must
-           have completed), and it knows which output planes that stage completed (the plane below the input plane, and the volume's
-           last plane with it), so it arrives on their accumulator-full barriers, which the epilogue waits on.  Both warps pass every
-           barrier of both kinds in order, also for the stages the other warp works on: a warp that skipped a phase of a barrier could
-           later take a wait for phase k + 2 as satisfied while the barrier is still in phase k + 1 (the parity reads the same). */
-        const int sfw = warp - 2;
-        const uint32_t sf_hi = desc_hi(128), lead = elect_one(), sfa_lo0 = desc_lo(smem_u32(stages) + (uint32_t)a.offSFA, 0), sstep = (uint32_t)a.stage_bytes >> 4;
-        const uint32_t sfa_t = tmem + (uint32_t)a.sfa_base + (uint32_t)sfw * (uint32_t)a.sfa_cols;      /* this warp's stages all have parity sfw */
-        int it = 0, s = 0, ph = 0, s2 = 0, ph2 = 0; bool ok = true;
-        int done = 0;                       /* output planes completed by all stages before the current one */
-        int rel_first = 0, rel_n = 0;       /* the planes this warp's latest stage completes: relayed once that stage's commit has arrived */
-        /* stage j = it - 2 has been consumed: pass its barrier; the warp that laid it out tells the epilogue about its planes */
-        auto pass_empty = [&](bool mine) -> bool {
-            if (!mbar_wait(bar_empty + 8 * s2, ph2, abort_flag, kWaitLimitR)) { if (lane == 0) raise_r(a, abort_flag, 2, it, bar_empty + 8 * s2 - bar_tma, ph2); return false; }
-            if (++s2 == R) { s2 = 0; ph2 ^= 1; }
-            if (mine && lane == 0) {
-                for (int k = 0; k < rel_n; k++) mbar_arrive(bar_accf + 8u * (uint32_t)(NS - 1 - (rel_first + k) % NS));
-            }
-            return true;
-        };
+           byte at window row r / 8 + dy, column r % 8 + dx + (x0 - 1 - xa).  Four rows per lane (one per TMEM column of the quad); the three
+           dx of a row are neighbours, so two words and a funnel shift fetch them.  The warp lays the nine shifted scale sets out in shared
+           memory in the tcgen05.cp layout, as far ahead of the MMAs as the ring is deep. */
+        int it = 0, s = 0, ph = 0; bool ok = true;
         while (piece.u < piece.u1 && ok) {
             const Run rn = next_run(a, piece);
             const int x0 = (rn.txy % a.tiles_x) * 8;
             const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
-            const int off = (lane >> 3) * 32 + (lane & 7) + (x0 - 1) - (((x0 - 1) >> 4) << 4), sh = (off & 3) * 8;      /* the three dx of a row are neighbours: two words and a funnel shift */
-            for (int zi = zlo; zi <= zhi && ok; zi++) {
-                /* planes that the last stage of this input plane completes: the plane below it, and the volume's last plane with it */
-                const int nc = (zi - 1 >= rn.zb ? 1 : 0) + ((zi == a.D - 1 && rn.ze == a.D) ? 1 : 0);
-                for (int ki = 0; ki < a.nki && ok; ki++) {
-                    const bool my = (it & 1) == sfw; const int cs = s, cph = ph;
-                    if (!mbar_wait(bar_tma + 8 * cs, cph, abort_flag, kWaitLimitR)) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * cs, cph); ok = false; break; }
-                    const int ncs = ki == a.nki - 1 ? nc : 0;
-                    if (!my) {
-                        if (it >= 2 && !pass_empty(false)) { ok = false; break; }
-                        done += ncs;
+            const int off = (lane >> 3) * 32 + (lane & 7) + (x0 - 1) - (((x0 - 1) >> 4) << 4), sh = (off & 3) * 8;
+            const int nst = (zhi - zlo + 1) * a.nki;
+            for (int i = 0; i < nst; i++) {
+                if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitR)) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * s, ph); ok = false; break; }
+                uint8_t *stg = stages + (size_t)s * a.stage_bytes;
+                const uint32_t *sw = (const uint32_t *)(stg + a.offSW + (off & ~3));
+                uint32_t *sfa = (uint32_t *)(stg + a.offSFA);
+                uint32_t wq[4][5];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    uint32_t t[3], u[3];          /* bytes 0..2: the scales of dx = 0, 1, 2 */
+#pragma unroll
+                    for (int dy = 0; dy < 3; dy++) {
+                        const uint32_t *p = sw + q * 32 + dy * 8;
+                        t[dy] = __funnelshift_r(p[0], p[1], sh);
+                        if (BITS == 4) u[dy] = __funnelshift_r(p[144], p[145], sh);
+                    }
+                    if (BITS == 8) {              /* taps 0-3, 4-7, 8 */
+                        wq[q][0] = __byte_perm(t[0], t[1], 0x4210); wq[q][1] = __byte_perm(t[1], t[2], 0x5421); wq[q][2] = (t[2] >> 16) & 0xffu;
+                    } else {                      /* pairs (block 2 ki, block 2 ki + 1) of taps 0 1, 2 3, 4 5, 6 7, 8 */
+                        wq[q][0] = __byte_perm(t[0], u[0], 0x5140); wq[q][1] = __byte_perm(__byte_perm(t[0], u[0], 0x0062), __byte_perm(t[1], u[1], 0x0040), 0x5410);
+                        wq[q][2] = __byte_perm(t[1], u[1], 0x6251); wq[q][3] = __byte_perm(t[2], u[2], 0x5140); wq[q][4] = __byte_perm(t[2], u[2], 0x0062) & 0xffffu;
+                    }
+                }
+                /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
+#pragma unroll
+                for (int qd = 0; qd < NQ; qd++) *(uint4 *)(sfa + qd * 128 + lane * 4) = make_uint4(wq[0][qd], wq[1][qd], wq[2][qd], wq[3][qd]);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_sf + 8 * s);
+                it++; if (++s == R) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 3) {
+        /* ---------------- completion relay ----------------
+           The MMA warp commits once per stage, on the stage's `empty` barrier.  This thread passes every one of them in order, knows which
+           output planes a stage completes (the plane below the input plane, and the volume's last plane with it) and arrives on their
+           accumulator-full barriers, which the epilogue waits on. */
+        if (lane == 0) {
+            int it = 0, s = 0, ph = 0, fs = NS - 1; bool ok = true;      /* fs: accumulator slot of the oldest plane not yet complete */
+            while (piece.u < piece.u1 && ok) {
+                const Run rn = next_run(a, piece);
+                const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
+                for (int zi = zlo; zi <= zhi && ok; zi++) {
+                    for (int ki = 0; ki < a.nki; ki++) {
+                        if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 2, it, bar_empty + 8 * s - bar_tma, ph); ok = false; break; }
                         it++; if (++s == R) { s = 0; ph ^= 1; }
-                        continue;
                     }
-                    uint8_t *stg = stages + (size_t)cs * a.stage_bytes;
-                    uint32_t *sfa = (uint32_t *)(stg + a.offSFA);
-                    const uint32_t *sw = (const uint32_t *)(stg + a.offSW + (off & ~3));
-                    uint32_t wq[4][5];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        uint32_t t[3], u[3];          /* bytes 0..2: the scales of dx = 0, 1, 2 */
-#pragma unroll
-                        for (int dy = 0; dy < 3; dy++) {
-                            const uint32_t *p = sw + q * 32 + dy * 8;
-                            t[dy] = __funnelshift_r(p[0], p[1], sh);
-                            if (BITS == 4) u[dy] = __funnelshift_r(p[144], p[145], sh);
-                        }
-                        if (BITS == 8) {              /* taps 0-3, 4-7, 8 */
-                            wq[q][0] = __byte_perm(t[0], t[1], 0x4210); wq[q][1] = __byte_perm(t[1], t[2], 0x5421); wq[q][2] = (t[2] >> 16) & 0xffu;
-                        } else {                      /* pairs (block 2 ki, block 2 ki + 1) of taps 0 1, 2 3, 4 5, 6 7, 8 */
-                            wq[q][0] = __byte_perm(t[0], u[0], 0x5140); wq[q][1] = __byte_perm(__byte_perm(t[0], u[0], 0x0062), __byte_perm(t[1], u[1], 0x0040), 0x5410);
-                            wq[q][2] = __byte_perm(t[1], u[1], 0x6251); wq[q][3] = __byte_perm(t[2], u[2], 0x5140); wq[q][4] = __byte_perm(t[2], u[2], 0x0062) & 0xffffu;
-                        }
-                    }
-                    /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
-#pragma unroll
-                    for (int qd = 0; qd < NQ; qd++) *(uint4 *)(sfa + qd * 128 + lane * 4) = make_uint4(wq[0][qd], wq[1][qd], wq[2][qd], wq[3][qd]);
-                    fence_proxy_async();
-                    /* the scale sets are laid out; before they go to TMEM, the MMAs that read this buffer two stages ago must have completed */
-                    if (it >= 2 && !pass_empty(true)) { ok = false; break; }
-                    rel_first = done; rel_n = ncs;
-                    done += ncs;
-                    it++; if (++s == R) { s = 0; ph ^= 1; }
-                    __syncwarp();
-                    tc_fence_after();
-                    const uint32_t src = sfa_lo0 + (uint32_t)cs * sstep;
-#pragma unroll
-                    for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make(src + 32u * q, sf_hi), lead);
-                    umma_commit(bar_sf + 8 * cs, lead);
-                    __syncwarp();
+                    const int nc = (zi - 1 >= rn.zb ? 1 : 0) + ((zi == a.D - 1 && rn.ze == a.D) ? 1 : 0);
+                    for (int k = 0; k < nc && ok; k++) { mbar_arrive(bar_accf + 8 * fs); fs = fs == 0 ? NS - 1 : fs - 1; }
                 }
             }
         }
-        /* the last two stages: their commits, and the planes of this warp's last stage */
-        for (int k = (it >= 2 ? 2 : it); k > 0 && ok; k--) { const bool my = ((it - k) & 1) == sfw; if (!pass_empty(my)) ok = false; }
     } else {
         /* ---------------- epilogue: one output plane of one tile at a time ---------------- */
         const int q4 = warp & 3, r = q4 * 32 + lane, ry = r >> 3, rx = r & 7;
@@ -453,7 +435,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
         const size_t plane_b = (size_t)a.H * a.W * 64, row_b = (size_t)a.W * 64;
         /* sample being accumulated and the first sample this block has planes of.  Nothing is written to `part` before the block has taken a plane
            out of TMEM: this kernel may have been started while its predecessor in the stream, which can be a conv that shares `part`, was still
-           running, and only the producer thread waits for the predecessor; a plane in TMEM means that wait is over.  So the zero entries of the
+           running, and only the producer waits for the predecessor; a plane in TMEM means that wait is over.  So the zero entries of the
            samples this block has no planes of are written at the end. */
         int n_cur = -1, n_first = -1;
         while (piece.u < piece.u1 && !dead) {
