@@ -14,7 +14,7 @@
    generic one (bias, fp16 / MX / plane-major output, the transposed conv's scatter).
 
    Roles (384 threads): warp 0 lane 0 producer, warp 1 lane 0 MMA issue (the warp allocates TMEM), warp 2 scale layout, warp 3
-   idle, warps 4-11 epilogue (two groups).  All waits are bounded as in conv_mx_k. */
+   idle, warps 4-11 epilogue (two groups, jobs in turn).  All waits are bounded as in conv_mx_k. */
 #include "conv_epi.cuh"
 #include "tc_ptx.cuh"
 #include <stdlib.h>
@@ -31,6 +31,7 @@ struct ConvPArgs {
     int N, nkb, nki, bits, cop, ntp, ntiles, ngroups;
     long long S, rtiles_per_n, jobs;             /* voxels per sample, row tiles per sample, (row tile, column tile) jobs */
     int HW, W;
+    unsigned hw_mul, w_mul; int hw_shift, w_shift;      /* reciprocals of H W and W (fast_div) */
     int ring, stage_bytes, offSW, offSFA, sw_rows;
     int w_bytes, w_codes, nquad, nslot;
     int tmem_cols, sfa_base, sfb_base;
@@ -49,6 +50,19 @@ __device__ __forceinline__ void raise_p(const ConvPArgs &a, volatile int *abort_
     __threadfence_block();
 }
 
+/* n / d for n < 2^31: mul = ceil(2^(31 + l) / d), shift = l - 1 with l = ceil(log2 d) (Granlund and Montgomery, "Division by invariant integers using
+   multiplication"); mul = 0 stands for d = 1 */
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned mul, int shift) { return mul ? __umulhi(n, mul) >> shift : n; }
+/* two fp32 additions in one instruction, each rounded to nearest even */
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+    float2 o;
+    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 r, p, q;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+    return o;
+}
+/* 32 bytes in one store: two neighbouring 16-byte rows, a whole sector where the address is a multiple of 32 */
+__device__ __forceinline__ void st_32b(uint8_t *p, unsigned a, unsigned b, unsigned c, unsigned d, unsigned e, unsigned f, unsigned g, unsigned h) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
+}
 /* EPI: the output mode known at compile time (0: any, read from the arguments; 1: plane-major fp32; 2: plane-major fp16; 3: MX-fp8 split
    layout; 4: the same through the transposed conv's scatter; 5, 6: MX-fp4 likewise), so that the epilogue's code is only what that mode needs */
 template <int BITS, int EPI>
@@ -65,7 +79,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
-        for (int i = 0; i < kMaxSlotsP; i++) { mbar_init(bar_accf + 8 * i, 1); mbar_init(bar_acce + 8 * i, 8); }
+        for (int i = 0; i < kMaxSlotsP; i++) { mbar_init(bar_accf + 8 * i, 1); mbar_init(bar_acce + 8 * i, 4); }
         mbar_init(bar_w, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -177,65 +191,114 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
             it++; if (++s == R) { s = 0; ph ^= 1; }
         }
     } else if (warp >= 4) {
-        /* ---------------- epilogue: two groups of four warps; a job of two 32-column chunks gives one to each group, jobs of one chunk
-           alternate between the groups.  Both groups wait for and release every accumulator slot. ---------------- */
+        /* ---------------- epilogue: two groups of four warps; jobs alternate between them, and so do the accumulator slots (their number is even, so a
+           group sees every phase of its slots' barriers).  A thread has the whole GEMM row of one voxel.  What bounds the MX modes is the instructions of this
+           part (64 -> 32 transposed conv on 64^3: 416 a row of 32 values with two divisions, 64-bit index products and a store of 16 bytes for each
+           half row, 44.4 us; MXP_INS this way, MXP_US us): coordinates come from multiplications by host-made reciprocals, bases are worked out once a job,
+           biases are added in pairs, and a transposed conv's two x neighbours, which share sectors, belong to one job and leave in one store. ---------------- */
         const int q4 = warp & 3, eg = (warp - 4) >> 2, r = q4 * 32 + lane;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
-        int slot = 0, sph = 0, pc = 0; bool dead = false;
-        long long job = j0; int ntile = (int)(j0 % a.ntiles), n = (int)((j0 / a.ntiles) / a.rtiles_per_n), tin = (int)((j0 / a.ntiles) % a.rtiles_per_n);
-        const unsigned Su = (unsigned)a.S, HWu = (unsigned)a.HW, Wu = (unsigned)a.W;
-        for (; job < j1 && !dead; job++, pc++) {
-            const int n_cur = min(a.ntp, a.cop - ntile * a.ntp), nchunk = n_cur >> 5;
-            const bool mine = nchunk > 1 ? true : (pc & 1) == eg;
-            const int jc = nchunk > 1 ? eg : 0;
-            if (!mbar_wait(bar_accf + 8 * slot, (uint32_t)sph, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 5, pc); dead = true; break; }
+        int slot = eg, sph = 0; bool dead = false;
+        const unsigned Su = (unsigned)a.S;
+        long long job = j0 + eg;
+        int ntile = (int)(job % a.ntiles), n = (int)((job / a.ntiles) / a.rtiles_per_n), tin = (int)((job / a.ntiles) % a.rtiles_per_n);
+        for (; job < j1 && !dead; job += 2) {
+            const int n_cur = min(a.ntp, a.cop - ntile * a.ntp), nchunk = n_cur >> 5, cb = ntile * (a.ntp >> 5);
+            if (!mbar_wait(bar_accf + 8 * slot, (uint32_t)sph, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 5, (int)(job - j0)); dead = true; break; }
             tc_fence_after();
-            if (EPI == 7) {
-                /* probability bytes of a plane-major output of at most eight channels (the head): only those accumulator columns leave TMEM; the
-                   byte of fp16(acc + bias) comes from the table of all 65536 fp16 values; a warp's 32 voxels are 32 consecutive bytes of a plane */
+            const uint32_t tcol = tlane + (uint32_t)(slot * a.ntp);
+            const unsigned vo = (unsigned)tin * 128u + (unsigned)r;
+            const bool row_ok = vo < Su;
+            auto release = [&]() { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(bar_acce + 8 * slot); };     /* one arrival per warp: arrivals on one barrier serialise */
+            if (EPI == 7 || ((EPI == 1 || EPI == 2) && a.e.co_real <= 8)) {
+                /* a plane-major output of at most eight channels (the head): only those accumulator columns leave TMEM; a warp's 32 voxels are consecutive
+                   in every plane.  7: probability bytes, the byte of fp16(acc + bias) from the table of all 65536 fp16 values */
                 uint32_t r8[8];
-                if (mine) { tmem_ld8(tlane + (uint32_t)(slot * a.ntp), r8); tmem_ld_wait(); }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_acce + 8 * slot);
-                const unsigned vo = (unsigned)tin * 128u + (unsigned)r;
-                if (mine && vo < Su) {
-                    uint8_t *yo = (uint8_t *)a.e.y + (size_t)n * a.e.co_real * Su + vo;
+                tmem_ld8(tcol, r8); tmem_ld_wait();
+                release();
+                if (row_ok) {
+                    const size_t o = (size_t)n * a.e.co_real * Su + vo;
 #pragma unroll
                     for (int k = 0; k < 8; k++) {
                         if (k < a.e.co_real) {
-                            const __half h = __float2half_rn(__fadd_rn(__uint_as_float(r8[k]), __ldg(a.e.bias + k)));
-                            yo[(size_t)k * Su] = __ldg(a.e.ptab + __half_as_ushort(h));
+                            const float v = __fadd_rn(__uint_as_float(r8[k]), __ldg(a.e.bias + k));
+                            if (EPI == 1) ((float *)a.e.y)[o + (size_t)k * Su] = v;
+                            else if (EPI == 2) ((__half *)a.e.y)[o + (size_t)k * Su] = __float2half_rn(v);
+                            else ((uint8_t *)a.e.y)[o + (size_t)k * Su] = __ldg(a.e.ptab + __half_as_ushort(__float2half_rn(v)));
                         }
                     }
                 }
-                if (++slot == NS) { slot = 0; sph ^= 1; }
-                if (++ntile == a.ntiles) { ntile = 0; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
-                continue;
-            }
-            uint32_t rr[32];
-            if (mine) { tmem_ld32(tlane + (uint32_t)(slot * a.ntp + jc * 32), rr); tmem_ld_wait(); }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_acce + 8 * slot);     /* one arrival per warp: arrivals on one barrier serialise */
-            if (mine) {
-                const unsigned vo = (unsigned)tin * 128u + (unsigned)r;
-                const bool row_ok = vo < Su;
-                const unsigned zu = vo / HWu, rem = vo - zu * HWu, oyu = rem / Wu;
-                float v[32];
+            } else if (EPI >= 3) {
+                /* MX rows.  Column blocks of a transposed conv come as (dz, dy, block, dx): the two chunks of a job are the voxels 2 x and 2 x + 1 of one
+                   output row (neighbours in the 16-byte-wide planes); without one they are two blocks of the same voxel */
+                constexpr bool T = EPI == 4 || EPI == 6, O8 = EPI == 3 || EPI == 4;
+                constexpr int NW = O8 ? 8 : 4;
+                const size_t So = T ? (size_t)Su * 8 : (size_t)Su;
+                int ob = cb; size_t vx = vo;
+                if (T) {
+                    const int pair = cb >> 1, zy = a.e.cob_t == 1 ? pair : pair / a.e.cob_t;
+                    ob = a.e.cob_t == 1 ? 0 : pair - zy * a.e.cob_t;
+                    const unsigned z = fast_div(vo, a.hw_mul, a.hw_shift), rem = vo - z * (unsigned)a.HW, oy = fast_div(rem, a.w_mul, a.w_shift), ox = rem - oy * (unsigned)a.W;
+                    vx = ((size_t)(2 * z + (unsigned)(zy >> 1)) * (unsigned)(2 * a.e.H) + (2 * oy + (unsigned)(zy & 1))) * (unsigned)(2 * a.W) + 2 * ox;
+                }
+                const size_t blk = (size_t)n * a.e.nb_dst + a.e.b0 + ob;
+                uint8_t *pc = (uint8_t *)a.e.y + (O8 ? (2 * blk * So + vx) * 16 : (blk * So + vx) * 16);
+                uint8_t *ps = (uint8_t *)a.e.y + (size_t)a.N * a.e.nb_dst * So * (O8 ? 32 : 16) + blk * So + vx;
+                unsigned w[2][NW], sb[2];
 #pragma unroll
-                for (int k = 0; k < 32; k++) v[k] = __uint_as_float(rr[k]);
-                EpiArgs e = a.e;
-                if (EPI == 1) { e.out_mode = UMX_OUT_PM32; e.tconv = 0; }
-                if (EPI == 2) { e.out_mode = UMX_OUT_PM16; e.tconv = 0; }
-                if (EPI == 3) { e.out_mode = UMX_OUT_MX; e.out_bits = 8; e.y_split = 1; e.tconv = 0; }
-                if (EPI == 4) { e.out_mode = UMX_OUT_MX; e.out_bits = 8; e.y_split = 1; e.tconv = 1; }
-                if (EPI == 5) { e.out_mode = UMX_OUT_MX; e.out_bits = 4; e.tconv = 0; }
-                if (EPI == 6) { e.out_mode = UMX_OUT_MX; e.out_bits = 4; e.tconv = 1; }
-                epi_chunk(e, n, (int)zu, (int)oyu, (int)(rem - oyu * Wu), row_ok, ntile * (a.ntp >> 5) + jc, v);
+                for (int jc = 0; jc < 2; jc++) {
+                    if (jc < nchunk) {
+                        uint32_t rr[32];
+                        tmem_ld32(tcol + (uint32_t)(jc * 32), rr); tmem_ld_wait();
+                        if (jc == nchunk - 1) release();
+                        const float4 *bp = (const float4 *)(a.e.bias + (T ? ob : cb + jc) * 32);
+                        __half2 h[16];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            const float4 b = __ldg(bp + k);
+                            const float2 s0 = add2(make_float2(__uint_as_float(rr[4 * k]), __uint_as_float(rr[4 * k + 1])), make_float2(b.x, b.y));
+                            const float2 s1 = add2(make_float2(__uint_as_float(rr[4 * k + 2]), __uint_as_float(rr[4 * k + 3])), make_float2(b.z, b.w));
+                            h[2 * k] = __floats2half2_rn(s0.x, s0.y); h[2 * k + 1] = __floats2half2_rn(s1.x, s1.y);
+                        }
+                        if (O8) sb[jc] = mx_encode_row32_h8(h, w[jc]);
+                        else {
+                            float v[32];
+#pragma unroll
+                            for (int k = 0; k < 16; k++) { const float2 f = __half22float2(h[k]); v[2 * k] = f.x; v[2 * k + 1] = f.y; }
+                            sb[jc] = mx_encode_row32<4>(v, w[jc]);
+                        }
+                        if (!T && row_ok) {
+                            *(uint4 *)pc = make_uint4(w[jc][0], w[jc][1], w[jc][2], w[jc][3]);
+                            if (O8) *(uint4 *)(pc + So * 16) = make_uint4(w[jc][4 % NW], w[jc][5 % NW], w[jc][6 % NW], w[jc][7 % NW]);
+                            *ps = (uint8_t)sb[jc];
+                            pc += So * (O8 ? 32 : 16); ps += So;
+                        }
+                    }
+                }
+                if (T && row_ok) {
+                    st_32b(pc, w[0][0], w[0][1], w[0][2], w[0][3], w[1][0], w[1][1], w[1][2], w[1][3]);
+                    if (O8) st_32b(pc + So * 16, w[0][4 % NW], w[0][5 % NW], w[0][6 % NW], w[0][7 % NW], w[1][4 % NW], w[1][5 % NW], w[1][6 % NW], w[1][7 % NW]);
+                    *(unsigned short *)ps = (unsigned short)(sb[0] | (sb[1] << 8));
+                }
+            } else {
+                const unsigned z = fast_div(vo, a.hw_mul, a.hw_shift), rem = vo - z * (unsigned)a.HW, oy = fast_div(rem, a.w_mul, a.w_shift);
+                for (int jc = 0; jc < nchunk; jc++) {
+                    uint32_t rr[32];
+                    tmem_ld32(tcol + (uint32_t)(jc * 32), rr); tmem_ld_wait();
+                    if (jc == nchunk - 1) release();
+                    float v[32];
+#pragma unroll
+                    for (int k = 0; k < 32; k++) v[k] = __uint_as_float(rr[k]);
+                    EpiArgs e = a.e;
+                    if (EPI == 1) { e.out_mode = UMX_OUT_PM32; e.tconv = 0; }
+                    if (EPI == 2) { e.out_mode = UMX_OUT_PM16; e.tconv = 0; }
+                    /* the caller's order of a transposed conv's column blocks is (dz, dy, dx, block) */
+                    const int pair = cb >> 1;
+                    epi_chunk(e, n, (int)z, (int)oy, (int)(rem - oy * (unsigned)a.W), row_ok, e.tconv ? (2 * (pair / e.cob_t) + jc) * e.cob_t + pair % e.cob_t : cb + jc, v);
+                }
             }
-            if (++slot == NS) { slot = 0; sph ^= 1; }
-            if (++ntile == a.ntiles) { ntile = 0; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
+            slot += 2; if (slot >= NS) { slot = eg; sph ^= 1; }
+            ntile += 2; while (ntile >= a.ntiles) { ntile -= a.ntiles; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
         }
     }
     /* ---------------- teardown ---------------- */
@@ -257,19 +320,21 @@ __global__ void __launch_bounds__(128) prep_wp_k(const PrepArgs p, uint8_t *wp, 
     if (i >= total) return;
     const int rl = i % ntp, ki = (i / ntp) % p.nki, nt_i = i / (ntp * p.nki), row = nt_i * ntp + rl;
     const bool live = row < p.cop;
-    constexpr int dummy = 0; (void)dummy;
+    /* a transposed conv's column blocks in the order (dz, dy, block, dx): see the epilogue */
+    int src = row;
+    if (p.kind == UMX_TCONV2) { const int pair = row >> 6, zy = pair / p.cob_t; src = ((2 * zy + ((row >> 5) & 1)) * p.cob_t + pair % p.cob_t) * 32 + (row & 31); }
     unsigned w[8]; unsigned sb[2] = {127u, 127u};
     float v[32];
     if (p.bits == 8) {
 #pragma unroll
-        for (int k = 0; k < 32; k++) v[k] = live ? prep_src(p, row, 0, ki, k) : 0.f;
+        for (int k = 0; k < 32; k++) v[k] = live ? prep_src(p, src, 0, ki, k) : 0.f;
         sb[0] = mx_encode_row32<8>(v, w);
     } else {
         unsigned w4[4];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
 #pragma unroll
-            for (int k = 0; k < 32; k++) v[k] = live ? prep_src(p, row, 0, 2 * ki + h, k) : 0.f;
+            for (int k = 0; k < 32; k++) v[k] = live ? prep_src(p, src, 0, 2 * ki + h, k) : 0.f;
             sb[h] = mx_encode_row32<4>(v, w4);
 #pragma unroll
             for (int t = 0; t < 4; t++) w[4 * h + t] = w4[t];
@@ -296,6 +361,10 @@ static int p_geometry(const umx_conv *c, PGeo *g) {
     if (16 + g->ntiles * g->ngroups * g->nq * 4 + 2 * g->ntp > 512) return 0;
     return 1;
 }
+static void recip(unsigned d, unsigned *mul, int *shift) {
+    int l = 0; while ((1ull << l) < d) l++;
+    *mul = l ? (unsigned)(((1ull << (31 + l)) + d - 1) / d) : 0u; *shift = l - 1;
+}
 /* builds the weight image of the streaming kernel from device fp32 weights; NULL when the conv does not qualify */
 uint8_t *umx_conv_p_prepare(const umx_conv *c, const float *w_dev) {
     PGeo g;
@@ -321,6 +390,7 @@ int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *
     if (e.out_mode == UMX_OUT_PROB8 && (e.co_real > 8 || g.ntiles != 1 || e.tconv || !e.ptab)) return 1;     /* the probability epilogue is the head's: one column tile, at most eight channels */       /* the scale plane's rows must be multiples of 16 bytes */
     a.N = N; a.nkb = c->nkb; a.nki = c->nki; a.bits = c->bits; a.cop = c->cop; a.ntp = g.ntp; a.ntiles = g.ntiles; a.ngroups = g.ngroups;
     a.S = (long long)S; a.rtiles_per_n = (long long)((S + 127) / 128); a.jobs = (long long)N * a.rtiles_per_n * g.ntiles; a.HW = H * W; a.W = W;
+    recip((unsigned)(H * W), &a.hw_mul, &a.hw_shift); recip((unsigned)W, &a.w_mul, &a.w_shift);
     a.w_codes = g.w_codes; a.w_bytes = g.w_bytes; a.nquad = g.nq;
     a.sw_rows = c->bits == 8 ? 4 : 8;
     a.offSW = 4 * 4096; a.offSFA = a.offSW + 1024; a.stage_bytes = (a.offSFA + g.nq * 512 + 1023) & ~1023;
@@ -329,6 +399,7 @@ int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *
     const int two = a.off_ring + 3 * a.stage_bytes <= 113 * 1024 && (256 - 16 - sfb_cols) / g.ntp >= 2;
     a.tmem_cols = two ? 256 : 512;
     a.nslot = (a.tmem_cols - 16 - sfb_cols) / g.ntp; if (a.nslot > kMaxSlotsP) a.nslot = kMaxSlotsP;
+    a.nslot &= ~1;
     if (a.nslot < 2) return 1;
     a.sfa_base = a.nslot * g.ntp; a.sfb_base = a.sfa_base + 16;
     a.ring = ((two ? 113 : 227) * 1024 - a.off_ring) / a.stage_bytes; if (a.ring > 8) a.ring = 8;
@@ -363,6 +434,8 @@ int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *
     int epi = 0;
     if (e.out_mode == UMX_OUT_PM32 && !e.tconv) epi = 1;
     else if (e.out_mode == UMX_OUT_PM16 && !e.tconv) epi = 2;
+    /* the pair stores of the transposed conv want a 32-byte aligned tensor (its planes are multiples of 128 voxels); the scale plane then starts on an even address */
+    else if (e.out_mode == UMX_OUT_MX && e.tconv && ((size_t)e.y & 31)) epi = 0;
     else if (e.out_mode == UMX_OUT_MX && e.out_bits == 8 && e.y_split) epi = e.tconv ? 4 : 3;
     else if (e.out_mode == UMX_OUT_MX && e.out_bits == 4) epi = e.tconv ? 6 : 5;
     else if (e.out_mode == UMX_OUT_PROB8) epi = 7;
