@@ -574,10 +574,11 @@ def test_weights_without_a_key_may_change_between_calls(dev):
 
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("N,Cn,D,H,W", [(1, 32, 4, 8, 8), (2, 64, 5, 7, 9), (1, 96, 2, 2, 2), (1, 320, 8, 8, 8), (3, 32, 10, 10, 10), (1, 64, 16, 16, 16), (2, 32, 12, 20, 16), (1, 128, 17, 16, 16),
-                                        (1, 32, 32, 32, 32), (2, 64, 24, 24, 24), (1, 32, 42, 60, 60), (1, 96, 48, 32, 32), (5, 32, 20, 20, 20)])
+                                        (1, 32, 32, 32, 32), (2, 64, 24, 24, 24), (1, 32, 42, 60, 60), (1, 96, 48, 32, 32), (5, 32, 20, 20, 20),
+                                        (1, 64, 64, 64, 64), (2, 32, 40, 44, 48), (1, 32, 84, 84, 85), (1, 32, 86, 86, 84)])
 def test_norm_in_one_launch(dev, bits, N, Cn, D, H, W):
     """statistics, coefficients and apply in one launch: the bytes of the two-launch path at the edges of its forms (one block, a cluster of 8 or 16,
-    blocks that meet through a counter, one or two trips a block, partly filled blocks), with and without the space-to-depth copy, into part
+    blocks that meet through a counter, one or two trips a block or up to six more in shared memory, partly filled blocks), with and without the space-to-depth copy, into part
     of a larger tensor, twice in a row (the counters are cleared); tensors it does not hold return 1 and touch nothing"""
     import ctypes as C
     import ufsm_b200
@@ -598,8 +599,40 @@ def test_norm_in_one_launch(dev, bits, N, Cn, D, H, W):
             got, got2 = DevBuf(N * 2 * nb * S * rb).fill(0xEE), DevBuf(N * nb * S * rb).fill(0xEE)
             rc = fn(yd.ptr, N, Cn, D, H, W, 1e-5, 2, pd.ptr, got.ptr, bits, 2 * nb, nb, got2.ptr if s2d else None, 1)
             ufsm_b200.check()
-            held = S <= 4096 or (148 // (nb * N)) * 1024 >= S
+            held = S <= 4096 or (148 // (nb * N)) * 4096 >= S
             assert rc == (0 if held else 1)
             assert np.array_equal(got.download(), want.download() if held else np.full(got.nbytes, 0xEE, np.uint8))
             if s2d and held:
                 assert np.array_equal(got2.download(), want2.download())
+
+
+@pytest.mark.parametrize("kind,N,Ci,Co,D,H,W,bits", [("tconv2", 1, 32, 24, 1, 4, 4, 8), ("tconv2", 2, 64, 32, 3, 16, 7, 8), ("tconv2", 1, 64, 40, 2, 8, 13, 8), ("tconv2", 1, 32, 96, 5, 9, 16, 4),
+                                                     ("tconv2", 1, 64, 32, 16, 16, 16, 4), ("down2", 1, 32, 32, 3, 16, 5, 8), ("down2", 2, 64, 96, 4, 12, 7, 8), ("conv1", 1, 32, 7, 3, 16, 9, 8),
+                                                     ("conv1", 2, 64, 8, 1, 16, 1, 4), ("conv1", 1, 32, 33, 9, 16, 8, 8)])
+def test_one_tap_epilogues(dev, kind, N, Ci, Co, D, H, W, bits):
+    """the streaming kernel's short epilogues (pair stores of the transposed conv, MX rows, few plane-major channels) against its general one: the same bytes,
+    at partial row tiles, odd widths, one and several column tiles, one and several blocks a sub-voxel group"""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    taps, S, nbi = {"conv1": 1, "down2": 8, "tconv2": 8}[kind], D * H * W, (Ci + 31) // 32 * (8 if kind == "down2" else 1)
+    r, rb, nbo, So = synth.rng(601), 4 * bits, (Co + 31) // 32, S * (8 if kind == "tconv2" else 1)
+    x = DevBuf(data=np.concatenate([r.integers(0, 120, N * nbi * S * rb, dtype=np.uint8), r.integers(120, 130, N * nbi * S, dtype=np.uint8)]))
+    c = G.Conv(kind, synth.kaiming(602, Co, Ci, taps, transposed=(kind == "tconv2")), synth.bias(603, Co, 0.1), Co, Ci, bits)
+
+    def run(nbytes, shift, mode, ob, flags):
+        y = DevBuf(data=np.full(nbytes + shift, 0x5a, np.uint8))
+        assert dev.umx_conv_fwd(c.h, x.ptr, N, D, H, W, y.ptr + shift, mode, ob, 0, 0, None, flags) == 0
+        ufsm_b200.check()
+        return y.download()[shift:]
+    if kind == "conv1":          # fp32 planes of at most eight channels, or more, against the blocked fp16 form
+        pm = run(N * Co * S * 4, 0, 2, 0, 1).view(np.float32).reshape(N, Co, S)
+        h = run(N * nbo * S * 64, 0, 0, 0, 1).view(np.float16).reshape(N, nbo, S, 32).transpose(0, 1, 3, 2).reshape(N, nbo * 32, S)[:, :Co]
+        assert np.array_equal(pm.astype(np.float16).view(np.uint16), h.view(np.uint16))
+        assert np.array_equal(run(N * Co * S * 2, 0, 3, 0, 1).view(np.uint16).reshape(N, Co, S), h.view(np.uint16))
+        return
+    got = run(N * nbo * So * (rb + 1), 0, 1, bits, 3)
+    if kind == "tconv2":         # a tensor that does not start on a 32-byte boundary takes the general epilogue
+        assert np.array_equal(got, run(N * nbo * So * (rb + 1), 16, 1, bits, 3))
+    else:                        # rows of 32 bytes instead of two planes of 16
+        flat = run(N * nbo * So * 33, 0, 1, 8, 1)
+        assert np.array_equal(got[:N * nbo * So * 32].reshape(N * nbo, 2, So, 16).transpose(0, 2, 1, 3).ravel(), flat[:N * nbo * So * 32]) and np.array_equal(got[N * nbo * So * 32:], flat[N * nbo * So * 32:])

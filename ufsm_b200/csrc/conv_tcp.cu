@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
         /* ---------------- epilogue: two groups of four warps; jobs alternate between them, and so do the accumulator slots (their number is even, so a
            group sees every phase of its slots' barriers).  A thread has the whole GEMM row of one voxel.  What bounds the MX modes is the instructions of this
            part (64 -> 32 transposed conv on 64^3: 416 a row of 32 values with two divisions, 64-bit index products and a store of 16 bytes for each
-           half row, 44.4 us; MXP_INS this way, MXP_US us): coordinates come from multiplications by host-made reciprocals, bases are worked out once a job,
+           half row, 44.4 us; 31.7 us this way): coordinates come from multiplications by host-made reciprocals, bases are worked out once a job,
            biases are added in pairs, and a transposed conv's two x neighbours, which share sectors, belong to one job and leave in one store. ---------------- */
         const int q4 = warp & 3, eg = (warp - 4) >> 2, r = q4 * 32 + lane;
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);

@@ -310,13 +310,15 @@ namespace {
 __device__ unsigned g_norm_count[2 * 4096];                  /* per (sample, block): blocks that have left their sums, blocks that have seen them all (the last one clears both) */
 struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl; unsigned vp; double *part; int *err; };      /* vp: voxels of a block's trip, NT / 4 to NT; cl: blocks of a cluster, all B of them, or 1 */
 
-template <int BITS, bool S2D, int ROWS, int NT>
+template <int BITS, bool S2D, int ROWS, int NT, bool STASH>
 __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
     pdl_trigger();
     constexpr int RB = 32 * BITS / 8, PH = NT / 4, GR = NT / 64;
     __shared__ double ss[64][33], sq[64][33];
     __shared__ double mine[64];
     __shared__ float2 sc[32];
+    extern __shared__ __align__(16) uint8_t stash_raw[];
+    uint4 *stash = (uint4 *)stash_raw + threadIdx.x;           /* STASH: [row of a thread][thread] */
     const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, B = gridDim.x, rank = blockIdx.x, CL = a.cl;
     const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
     const unsigned S = a.S, vp = a.vp, step = vp * (unsigned)B, K = (S + step - 1) / step, g = (unsigned)(n * nb + blk);
@@ -332,8 +334,17 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
 #pragma unroll
             for (int u = 0; u < 4; u++) { const unsigned v = vox(k, u); r[u] = v < S ? __ldg(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
         };
+        unsigned kr = 0;                                     /* the trips before those in registers wait in shared memory */
+        if (STASH) {
+            for (; kr + ROWS / 4 < K; kr += ROWS / 4) {
 #pragma unroll
-        for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, k);
+                for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, kr + k);
+#pragma unroll
+                for (int u = 0; u < ROWS; u++) { stat_add(acc, raw[u]); stash[(size_t)(kr * 4 + u) * NT] = raw[u]; }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, kr + k);
 #pragma unroll
         for (int u = 0; u < ROWS; u++) stat_add(acc, raw[u]);
         if (PH > 64) {                                       /* 128 row phases: two neighbouring ones together */
@@ -418,8 +429,16 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
             if (S2D) s2d_store<BITS>(a.q2, N, nb, n, blk, qd, v, S, H, W, wsh, hsh, a.split, w0, w1, sb);
         }
     };
+    unsigned kr = 0;
+    if (STASH) while (kr + ROWS / 4 < K) kr += ROWS / 4;
 #pragma unroll
-    for (int u = 0; u < ROWS; u++) put(raw[u], vox(u / 4, u & 3));
+    for (int u = 0; u < ROWS; u++) put(raw[u], vox(kr + u / 4, u & 3));
+    if (STASH) {
+        for (unsigned k = 0; k < kr; k++) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) put(stash[(size_t)(k * 4 + u) * NT], vox(k, u));
+        }
+    }
     if (CL > 1) cluster_wait();
 }
 /* whether clusters of 16 blocks of a variant can be launched, looked up once per device */
@@ -427,7 +446,7 @@ template <int BITS, bool S2D, int ROWS, int NT> bool norm_sixteen() {
     static int have[16];
     int d = 0; cudaGetDevice(&d); d &= 15;
     if (!have[d]) {
-        const void *k = (const void *)in_norm_k<BITS, S2D, ROWS, NT>;
+        const void *k = (const void *)in_norm_k<BITS, S2D, ROWS, NT, false>;
         cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
         cudaLaunchAttribute at; memset(&at, 0, sizeof at);
         at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = 16; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
@@ -443,7 +462,20 @@ template <int BITS, bool S2D, int ROWS, int NT> bool norm_go(NormArgs &a, int B,
     a.cl = cl;
     /* small tensors: fewer rows a thread */
     a.vp = (size_t)B * NT > a.S ? (unsigned)(((size_t)a.S + B * (NT / 4) - 1) / ((size_t)B * (NT / 4))) * (NT / 4) : NT;
-    umx_launch_cluster(in_norm_k<BITS, S2D, ROWS, NT>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3((unsigned)cl, 1, 1), dim3(NT), 0, a);
+    umx_launch_cluster(in_norm_k<BITS, S2D, ROWS, NT, false>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3((unsigned)cl, 1, 1), dim3(NT), 0, a);
+    return true;
+}
+/* one block a multiprocessor that keeps eight rows a thread in registers and up to kStashTrips x 4 more in shared memory (they come to 226 KB with the sums) */
+constexpr int kStashTrips = 6;
+template <int BITS, bool S2D> bool norm_go_stash(NormArgs &a, int B, int nb, int N) {
+    const void *k = (const void *)in_norm_k<BITS, S2D, 8, 512, true>;
+    static int set[16];
+    int d = 0; cudaGetDevice(&d); d &= 15;
+    if (!set[d]) set[d] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kStashTrips * 4 * 512 * 16) == cudaSuccess ? 1 : -1;
+    if (set[d] < 0) { cudaGetLastError(); return false; }
+    a.cl = 1; a.vp = 512;
+    const unsigned trips = (unsigned)(((size_t)a.S + (size_t)B * 512 - 1) / ((size_t)B * 512)), kept = (trips - 1) / 2 * 2;
+    umx_launch(in_norm_k<BITS, S2D, 8, 512, true>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3(512), (size_t)kept * 4 * 512 * 16, a);
     return true;
 }
 template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N) {
@@ -453,14 +485,15 @@ template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N) {
     if (S <= 1024) return norm_go<BITS, S2D, 4, 256>(a, 8, 8, nb, N);
     if (S <= 4096 && norm_sixteen<BITS, S2D, 4, 256>()) return norm_go<BITS, S2D, 4, 256>(a, 16, 16, nb, N);
     if (S <= 4096) return norm_go<BITS, S2D, 8, 256>(a, 8, 8, nb, N);
-    /* one block a multiprocessor, dealt to the groups, each of at most 1024 voxels */
+    /* one block a multiprocessor, dealt to the groups, each of at most 1024 voxels in registers and 3072 in shared memory */
     static int sms_of[16];
     int d = 0; cudaGetDevice(&d); d &= 15;
     if (!sms_of[d]) { int v = 1; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d); sms_of[d] = v; }
     long long B = sms_of[d] / ((long long)nb * N);
     const long long most = (long long)((S + 127) / 128);    /* a row a thread */
     if (B > most) B = most;
-    if (B < 1 || (size_t)B * 1024 < S) return false;
+    if (B < 1 || (size_t)B * (2 + kStashTrips) * 512 < S) return false;
+    if ((size_t)B * 1024 < S) return norm_go_stash<BITS, S2D>(a, (int)B, nb, N);
     return (size_t)B * 512 >= S ? norm_go<BITS, S2D, 4, 512>(a, (int)B, 1, nb, N) : norm_go<BITS, S2D, 8, 512>(a, (int)B, 1, nb, N);
 }
 }   // namespace
