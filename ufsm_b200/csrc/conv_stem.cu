@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kStemThreads, kStemBlocks) conv_stem_k(const S
             const XT *s0 = in0 ? xn + (ptrdiff_t)gy0 * W + gx0 : xn, *s1 = in1 ? xn + (ptrdiff_t)gy1 * W + gx1 : xn;
             auto fetch = [&](int zp, XT &v0, XT &v1) {
                 const size_t zo = (size_t)min(max(zp, 0), D - 1) * HW;
-                v0 = __ldg(s0 + zo); v1 = __ldg(s1 + zo);
+                v0 = ld_dep(s0 + zo); v1 = ld_dep(s1 + zo);
             };
             auto quant = [&](XT v, bool live) -> unsigned short {
                 if constexpr (U8) return live ? qtab[v] : (unsigned short)0; else return fq_h16_one(v, live);

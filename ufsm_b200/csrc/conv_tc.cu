@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < 9; j++) {
                     const bool in = (inm >> j) & 1u;
-                    raw[j] = in ? __ldg(p + toff[j / 3] + j % 3) : 127u;
-                    if (BITS == 4) raw[9 + j] = in && two ? __ldg(p + S + toff[j / 3] + j % 3) : 127u;
+                    raw[j] = in ? ld_dep(p + toff[j / 3] + j % 3) : 127u;
+                    if (BITS == 4) raw[9 + j] = in && two ? ld_dep(p + S + toff[j / 3] + j % 3) : 127u;
                 }
             } else {
                 const int items = stage_items(st);
@@ -239,12 +239,12 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                         const bool in = row_ok && iz >= 0 && iz < a.Di && iy >= 0 && iy < a.Hi && ix >= 0 && ix < a.Wi;
                         const size_t Si = (size_t)a.Di * a.Hi * a.Wi, vi = ((size_t)iz * a.Hi + iy) * a.Wi + ix;
                         const uint8_t *p = a.x_sc + ((size_t)n * a.nbi + (BITS == 8 ? blk : 2 * blk)) * Si + vi;
-                        if (in) raw[j] = __ldg(p);
-                        if (BITS == 4 && in && 2 * blk + 1 < a.nbi) raw[9 + j] = __ldg(p + Si);
+                        if (in) raw[j] = ld_dep(p);
+                        if (BITS == 4 && in && 2 * blk + 1 < a.nbi) raw[9 + j] = ld_dep(p + Si);
                     } else {
                         const uint8_t *p = a.x_sc + ((size_t)n * a.nkb + (BITS == 8 ? ki : 2 * ki)) * S + vox;
-                        if (row_ok) raw[j] = __ldg(p);
-                        if (BITS == 4 && row_ok && 2 * ki + 1 < a.nkb) raw[9 + j] = __ldg(p + S);
+                        if (row_ok) raw[j] = ld_dep(p);
+                        if (BITS == 4 && row_ok && 2 * ki + 1 < a.nkb) raw[9 + j] = ld_dep(p + S);
                     }
                 }
             }

@@ -18,8 +18,8 @@ namespace {
    grid (runs of voxels, 32-channel blocks, samples) */
 struct GnSlabs { int ns, zs, zo; size_t zhw; };             /* slab-local statistics (gnp_t.ns / zs / zo / zhw, src/nn_lp.h:15-18); ns 0: per sample */
 template <int XK, int BY, int FORM, bool SL>
-__global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ xv, uint8_t *__restrict__ y, int C, int G, size_t S,
-                                                      const float *__restrict__ gamma, const float *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd, int y_split,
+__global__ void __launch_bounds__(256) gn_silu_rows_k(const void *xv, uint8_t *__restrict__ y, int C, int G, size_t S,
+                                                      const float *gamma, const float *beta, const float *mean, const float *rstd, int y_split,
                                                       int c_off, int cpg, const GnSlabs sl, int nb_dst, int b0) {
     pdl_trigger(); pdl_wait();
     const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, T = gridDim.x;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ x
         for (int u = 0; u < 4; u++) {
             const size_t v = vb + u * 64 + ph;
             raw[u] = make_uint2(0u, 0u); sb[u] = 127u;
-            if (v < v1) { raw[u] = qrow_ld<(XK == 4 ? 4 : 8)>(xq, nbk * S + v, q); sb[u] = __ldg(xs + nbk * S + v); }
+            if (v < v1) { raw[u] = qrow_ld<(XK == 4 ? 4 : 8)>(xq, nbk * S + v, q); sb[u] = ld_dep(xs + nbk * S + v); }
         }
     };
     if (MXIN) fetch(va);
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) gn_silu_rows_k(const void *__restrict__ x
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
                     const size_t o = ((size_t)n * C + blk * 32 + q * 8 + k) * S + v;
-                    const float t = (live[k] && v < v1) ? (XK == 0 ? __ldg((const float *)xv + o) : __half2float(__ldg((const __half *)xv + o))) : 0.f;
+                    const float t = (live[k] && v < v1) ? (XK == 0 ? ld_dep((const float *)xv + o) : __half2float(ld_dep((const __half *)xv + o))) : 0.f;
                     if (k & 1) r[u][k >> 1].y = t; else r[u][k >> 1].x = t;
                 }
             }

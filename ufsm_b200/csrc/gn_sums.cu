@@ -45,7 +45,7 @@ __device__ __forceinline__ double slot_get(const double *base, size_t i) {
 /* block = (run of voxels, 32-channel block, sample); PER: runs of PER of a lane's eight channels lie in one group (8, 4, 2 or 1) and are added up
    together, the codes' sum exact in fp32 and their squares in fp64, then one fp64 fma a row and run for the scale */
 template <int BITS, int PER>
-__global__ void __launch_bounds__(256) gn_sums_rows_k(const uint8_t *__restrict__ x, int N, int C, int G, size_t S, double *sums, size_t v0, size_t v1, int n0) {
+__global__ void __launch_bounds__(256) gn_sums_rows_k(const uint8_t *x, int N, int C, int G, size_t S, double *sums, size_t v0, size_t v1, int n0) {
     pdl_trigger(); pdl_wait();
     const int nb = (C + 31) / 32, blk = blockIdx.y, n = n0 + (int)blockIdx.z, q = threadIdx.x & 3, ph = threadIdx.x >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int RB = BITS == 8 ? 32 : 16, NA = 8 / PER;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) gn_sums_rows_k(const uint8_t *__restrict_
         for (int u = 0; u < 4; u++) {
             const size_t v = vb + u * 64 + ph;
             nxt[u] = make_uint2(0u, 0u); nsb[u] = 127u;            /* rows past the end count as zeros */
-            if (v < q1) { nxt[u] = qrow_ld<BITS>(x, rbase + v, q); nsb[u] = __ldg(xs + rbase + v); }
+            if (v < q1) { nxt[u] = qrow_ld<BITS>(x, rbase + v, q); nsb[u] = ld_dep(xs + rbase + v); }
         }
     };
     fetch(q0);
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) gn_sums_rows_k(const uint8_t *__restrict_
 
 /* the same sums of a plane-major fp32 tensor [N][C][S] (a conv's unrounded accumulators): block = (run of voxels, channel, sample); fp64 sums
    (a square of an fp32 value is exact in fp64), a fixed-order reduction in the block, one slot addition per sum */
-__global__ void __launch_bounds__(256) gn_sums_pm32_k(const float *__restrict__ x, int C, int G, size_t S, double *sums, size_t v0, size_t v1) {
+__global__ void __launch_bounds__(256) gn_sums_pm32_k(const float *x, int C, int G, size_t S, double *sums, size_t v0, size_t v1) {
     pdl_trigger(); pdl_wait();
     const int c = blockIdx.y, n = blockIdx.z;
     size_t q0 = S * blockIdx.x / gridDim.x, q1 = S * (blockIdx.x + 1) / gridDim.x;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) gn_sums_pm32_k(const float *__restrict__ 
     if (q1 > v1) q1 = v1;
     const float *p = x + ((size_t)n * C + c) * S;
     double a = 0.0, b = 0.0;
-    for (size_t v = q0 + threadIdx.x; v < q1; v += 256) { const double t = (double)__ldg(p + v); a += t; b = fma(t, t, b); }
+    for (size_t v = q0 + threadIdx.x; v < q1; v += 256) { const double t = (double)ld_dep(p + v); a += t; b = fma(t, t, b); }
     __shared__ double sa[256], sb[256];
     sa[threadIdx.x] = a; sb[threadIdx.x] = b;
     __syncthreads();

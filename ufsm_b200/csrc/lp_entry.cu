@@ -54,7 +54,7 @@ static const void *gn_input(const char *fn, const void *x, int xbf, shape5 xs, g
     return ws;
 }
 int umx_gn_sums_pm32(const float *x, int N, int C, int G, size_t S, double *sums, size_t v0, size_t v1);
-__global__ void f32_to_h16_k(const float *__restrict__ x, __half *__restrict__ y, size_t n) {
+__global__ void f32_to_h16_k(const float *x, __half *__restrict__ y, size_t n) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) y[i] = __float2half_rn(x[i]);
 }
@@ -125,7 +125,7 @@ static void *slab_of(int slot, const void *x, int bf, int N, int C, int D, size_
     return s;
 }
 /* y (fp16 plane-major, n elements) += t */
-__global__ void __launch_bounds__(256) h16_add_k(__half *__restrict__ y, const __half *__restrict__ t, size_t n) {
+__global__ void __launch_bounds__(256) h16_add_k(__half *__restrict__ y, const __half *t, size_t n) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) y[i] = __float2half_rn(__fadd_rn(__half2float(y[i]), __half2float(t[i])));
 }

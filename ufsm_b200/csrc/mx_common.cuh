@@ -50,6 +50,17 @@ static inline void umx_launch_cluster(void (*kern)(KA...), dim3 grid, dim3 clust
 }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+/* A load of what an earlier kernel of the stream wrote, in a kernel launched through umx_launch.  Not __ldg: the non-coherent path may serve a line that an
+   earlier kernel on this multiprocessor left in L1, since the block may have started before its predecessor wrote the data and pdl_wait() orders coherent
+   accesses only (seen: a U-Net whose logits differed from run to run once a norm read its rows that way).  __ldg is for constants. */
+template <typename T> __device__ __forceinline__ T ld_dep(const T *p) {
+    static_assert(sizeof(T) == 1 || sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "1 to 16 bytes");
+    if constexpr (sizeof(T) == 16) { uint4 v; asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)); return *(const T *)&v; }
+    else if constexpr (sizeof(T) == 8) { uint2 v; asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p)); return *(const T *)&v; }
+    else if constexpr (sizeof(T) == 4) { unsigned v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return *(const T *)&v; }
+    else if constexpr (sizeof(T) == 2) { unsigned short v; asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p)); return *(const T *)&v; }
+    else { unsigned v; asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p)); return (T)v; }
+}
 #endif
 
 /* ---- MX arithmetic ---- */

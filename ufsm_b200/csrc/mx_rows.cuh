@@ -7,8 +7,8 @@
 
 /* this lane's codes of row `row`: fp8 in (x, y), fp4 in x */
 template <int BITS> __device__ __forceinline__ uint2 qrow_ld(const uint8_t *__restrict__ codes, size_t row, int q) {
-    if (BITS == 8) return __ldg((const uint2 *)(codes + row * 32) + q);
-    return make_uint2(__ldg((const unsigned *)(codes + row * 16) + q), 0u);
+    if (BITS == 8) return ld_dep((const uint2 *)(codes + row * 32) + q);
+    return make_uint2(ld_dep((const unsigned *)(codes + row * 16) + q), 0u);
 }
 /* codes -> the eight decoded values times the row's scale factor, as four pairs (the fp32 arithmetic of these kernels runs on
    packed pairs, fma.rn.f32x2 and its siblings: half the issue slots of the scalar forms, each half an IEEE operation of its own) */

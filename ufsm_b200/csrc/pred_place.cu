@@ -23,15 +23,15 @@ PlaceBox place_box_of(int D, int W, int hz, int halo, int oz, int oy, int ox, in
    two approximations */
 __device__ __forceinline__ unsigned prob255(float l) { return __float_as_uint(__fadd_rd(fmaxf(__fdividef(255.f, 1.f + __expf(-l)) + 0.5f, 0.f), 8388608.f)) & 0xffu; }
 template <typename LT> __device__ __forceinline__ float logit_at(const LT *lg, size_t k);
-template <> __device__ __forceinline__ float logit_at<float>(const float *lg, size_t k) { return __ldg(lg + k); }
-template <> __device__ __forceinline__ float logit_at<__half>(const __half *lg, size_t k) { return __half2float(__ldg(lg + k)); }
+template <> __device__ __forceinline__ float logit_at<float>(const float *lg, size_t k) { return ld_dep(lg + k); }
+template <> __device__ __forceinline__ float logit_at<__half>(const __half *lg, size_t k) { return __half2float(ld_dep(lg + k)); }
 
 /* MASK 0: material where ct[k] >= iso; 1: where bit k of `bits` is set.  zoff: the window is held from its plane zoff on (a half of a split window).
    A block takes R = 256 / nq whole rows of the box at a time (nq groups of eight x a row), so a thread works out its place once and needs
    one 32-bit division a trip; eight voxels go with one load of their logits, one of their mask bits and one store where these are aligned.
    Bound by latency and issue: 160^3 of a 192^3 window 12.4 us with 64-bit index divisions every four voxels, 7.6 us in this form. */
 template <typename LT, int MASK>
-__global__ void __launch_bounds__(256) pred_place_k(const LT *__restrict__ lg, const uint8_t *__restrict__ ct, const uint32_t *__restrict__ bits, PlaceBox B, int W, int zoff,
+__global__ void __launch_bounds__(256) pred_place_k(const LT *lg, const uint8_t *ct, const uint32_t *bits, PlaceBox B, int W, int zoff,
                                                     int oz, int oy, int ox, int shard, uint8_t *__restrict__ dsh, int iso) {
     pdl_trigger(); pdl_wait();
     const int nq = (B.nx + 7) >> 3, R = nq < 256 ? 256 / nq : 1, tr = (int)threadIdx.x / nq;
@@ -48,11 +48,11 @@ __global__ void __launch_bounds__(256) pred_place_k(const LT *__restrict__ lg, c
             float l[8]; unsigned on = 0u;
             if (n == 8 && !((size_t)(lg + k) & 15)) {
                 if (sizeof(LT) == 2) {
-                    const uint4 r = __ldg((const uint4 *)(lg + k)); const __half2 *h = (const __half2 *)&r;
+                    const uint4 r = ld_dep((const uint4 *)(lg + k)); const __half2 *h = (const __half2 *)&r;
 #pragma unroll
                     for (int j = 0; j < 4; j++) { const float2 f = __half22float2(h[j]); l[2 * j] = f.x; l[2 * j + 1] = f.y; }
                 } else {
-                    const float4 r = __ldg((const float4 *)(lg + k)), t = __ldg((const float4 *)(lg + k) + 1);
+                    const float4 r = ld_dep((const float4 *)(lg + k)), t = ld_dep((const float4 *)(lg + k) + 1);
                     l[0] = r.x; l[1] = r.y; l[2] = r.z; l[3] = r.w; l[4] = t.x; l[5] = t.y; l[6] = t.z; l[7] = t.w;
                 }
             } else {
@@ -61,11 +61,11 @@ __global__ void __launch_bounds__(256) pred_place_k(const LT *__restrict__ lg, c
             }
             if (MASK) {
                 const unsigned sh = (unsigned)(k & 31);
-                on = __ldg(bits + (k >> 5)) >> sh;
-                if (sh + n > 32) on |= __ldg(bits + (k >> 5) + 1) << (32 - sh);
+                on = ld_dep(bits + (k >> 5)) >> sh;
+                if (sh + n > 32) on |= ld_dep(bits + (k >> 5) + 1) << (32 - sh);
             } else {
 #pragma unroll
-                for (int j = 0; j < 8; j++) if (j < n && (int)__ldg(ct + k + j) >= iso) on |= 1u << j;
+                for (int j = 0; j < 8; j++) if (j < n && (int)ld_dep(ct + k + j) >= iso) on |= 1u << j;
             }
             unsigned v[8];
 #pragma unroll
@@ -75,26 +75,26 @@ __global__ void __launch_bounds__(256) pred_place_k(const LT *__restrict__ lg, c
         }
     }
 }
-__global__ void __launch_bounds__(256) pred_out_k(const void *lg, int h16, const uint8_t *__restrict__ ct, size_t n, uint8_t *__restrict__ out) {
+__global__ void __launch_bounds__(256) pred_out_k(const void *lg, int h16, const uint8_t *ct, size_t n, uint8_t *__restrict__ out) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = __ldg(ct + i) ? (uint8_t)prob255(h16 ? logit_at<__half>((const __half *)lg, i) : logit_at<float>((const float *)lg, i)) : (uint8_t)0;
+        out[i] = ld_dep(ct + i) ? (uint8_t)prob255(h16 ? logit_at<__half>((const __half *)lg, i) : logit_at<float>((const float *)lg, i)) : (uint8_t)0;
 }
 /* one 32-voxel word a thread: two 16-byte loads where the bytes are there and aligned, byte compares four at a time */
-__global__ void __launch_bounds__(256) ctmask_k(const uint8_t *__restrict__ ct, size_t n, uint32_t *__restrict__ bits, int t) {
+__global__ void __launch_bounds__(256) ctmask_k(const uint8_t *ct, size_t n, uint32_t *__restrict__ bits, int t) {
     pdl_trigger(); pdl_wait();
     const size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x, i0 = w * 32;
     if (i0 >= n) return;
     uint32_t m = 0;
     if (t > 255) { bits[w] = 0u; return; }
     if (i0 + 32 <= n && !((size_t)(ct + i0) & 15)) {
-        const uint4 u0 = __ldg((const uint4 *)(ct + i0)), u1 = __ldg((const uint4 *)(ct + i0) + 1);
+        const uint4 u0 = ld_dep((const uint4 *)(ct + i0)), u1 = ld_dep((const uint4 *)(ct + i0) + 1);
         const uint32_t v[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w}, tt = (uint32_t)t * 0x01010101u;
 #pragma unroll
         for (int j = 0; j < 8; j++) m |= ((((__vcmpgeu4(v[j], tt) & 0x01010101u) * 0x01020408u) >> 24) & 15u) << (4 * j);
     } else {
         const int cnt = (int)min((size_t)32, n - i0);
-        for (int j = 0; j < cnt; j++) m |= (uint32_t)((int)__ldg(ct + i0 + j) >= t) << j;
+        for (int j = 0; j < cnt; j++) m |= (uint32_t)((int)ld_dep(ct + i0 + j) >= t) << j;
     }
     bits[w] = m;
 }
@@ -119,9 +119,9 @@ __device__ __forceinline__ const uint8_t *fe_row(const FeatherArgs &f, int d, in
 /* four bytes of a row from x on (n of them real) */
 __device__ __forceinline__ unsigned fe_four(const uint8_t *r, int x, int n) {
     const uint8_t *p = r + x;
-    if (n == 4 && !((size_t)p & 3)) return __ldg((const uint32_t *)p);
+    if (n == 4 && !((size_t)p & 3)) return ld_dep((const uint32_t *)p);
     unsigned v = 0u;
-    for (int j = 0; j < n; j++) v |= (unsigned)__ldg(p + j) << (8 * j);
+    for (int j = 0; j < n; j++) v |= (unsigned)ld_dep(p + j) << (8 * j);
     return v;
 }
 /* The output box in up to eight parts by which axes lie in the lower shell (bit 0 x, 1 y, 2 z), so that the windows that reach a voxel are the
@@ -143,12 +143,12 @@ template <int M> __device__ __forceinline__ unsigned fe_mean(const FeatherArgs &
     }
     float wz[2] = {1.f, 1.f}, wy[2] = {1.f, 1.f};
 #pragma unroll
-    for (int k = 0; k < 2; k++) { if (M & 4) wz[k] = __ldg(f.u + k * B + z); if (M & 2) wy[k] = __ldg(f.u + k * B + y); }
+    for (int k = 0; k < 2; k++) { if (M & 4) wz[k] = ld_dep(f.u + k * B + z); if (M & 2) wy[k] = ld_dep(f.u + k * B + y); }
     unsigned v = 0u;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         float wx[2] = {1.f, 1.f};
-        if ((M & 1) && j < n) { wx[0] = __ldg(f.u + x + j); wx[1] = __ldg(f.u + B + x + j); }
+        if ((M & 1) && j < n) { wx[0] = ld_dep(f.u + x + j); wx[1] = ld_dep(f.u + B + x + j); }
         float s = 0.f, w = 0.f;
 #pragma unroll
         for (int d = 0; d < 8; d++) {
@@ -199,14 +199,14 @@ __global__ void __launch_bounds__(256) feather_k(const FeatherArgs f, const Feat
 }
 /* a window's upper slabs, kept for the windows after it (feather_keep, src/predict.c:362-376): one T (byte or four-byte word) a thread, indices of type I */
 template <typename T, typename I>
-__global__ void __launch_bounds__(256) feather_keep_k(const T *__restrict__ e, I S, I B, I SX, I BX, T *__restrict__ zs, T *__restrict__ ys, T *__restrict__ xs) {
+__global__ void __launch_bounds__(256) feather_keep_k(const T *e, I S, I B, I SX, I BX, T *__restrict__ zs, T *__restrict__ ys, T *__restrict__ xs) {
     pdl_trigger(); pdl_wait();
     /* S, B, E in voxels; SX, BX, EX along x in units of T */
     const I E = S + B, EX = SX + BX, nz = B * E * EX, ny = S * B * EX, nx = S * S * BX;
     for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < nz + ny + nx; i += (I)gridDim.x * blockDim.x) {
-        if (i < nz) zs[i] = __ldg(e + S * E * EX + i);
-        else if (i < nz + ny) { const I k = i - nz, r = k / EX, x = k - r * EX, z = r / B, y = r - z * B; ys[k] = __ldg(e + (z * E + S + y) * EX + x); }
-        else { const I k = i - nz - ny, r = k / BX, x = k - r * BX, z = r / S, y = r - z * S; xs[k] = __ldg(e + (z * E + y) * EX + SX + x); }
+        if (i < nz) zs[i] = ld_dep(e + S * E * EX + i);
+        else if (i < nz + ny) { const I k = i - nz, r = k / EX, x = k - r * EX, z = r / B, y = r - z * B; ys[k] = ld_dep(e + (z * E + S + y) * EX + x); }
+        else { const I k = i - nz - ny, r = k / BX, x = k - r * BX, z = r / S, y = r - z * S; xs[k] = ld_dep(e + (z * E + y) * EX + SX + x); }
     }
 }
 

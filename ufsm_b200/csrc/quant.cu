@@ -10,15 +10,15 @@
 __host__ __device__ static inline int mxbw(int C, int force) { return force > 0 ? force : C <= 8 ? 8 : C <= 16 ? 16 : 32; }
 
 template <typename T> __device__ __forceinline__ float ld_as_f32(const T *p);
-template <> __device__ __forceinline__ float ld_as_f32<float>(const float *p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ld_as_f32<__half>(const __half *p) { return __half2float(__ldg(p)); }
-template <> __device__ __forceinline__ float ld_as_f32<__nv_bfloat16>(const __nv_bfloat16 *p) { return __uint_as_float((unsigned)__ldg((const unsigned short *)p) << 16); }
+template <> __device__ __forceinline__ float ld_as_f32<float>(const float *p) { return ld_dep(p); }
+template <> __device__ __forceinline__ float ld_as_f32<__half>(const __half *p) { return __half2float(ld_dep(p)); }
+template <> __device__ __forceinline__ float ld_as_f32<__nv_bfloat16>(const __nv_bfloat16 *p) { return __uint_as_float((unsigned)ld_dep((const unsigned short *)p) << 16); }
 
 /* grid = (voxel chunks, blocks, samples): no index division per row; consecutive threads take consecutive voxels, so the plane-major
    reads and the row writes are both coalesced.  Channels from c2 on come from a second tensor x2 of C - c2 channels (a conv's concat
    input, split_t.x2 / c_split of the reference: the 32-channel blocks run over the concatenated index); c2 = C without one. */
 template <int BITS, typename TI, bool CAT>
-__global__ void __launch_bounds__(256) pm_to_mx_k(const TI *__restrict__ x, uint8_t *__restrict__ y, int N, int C, size_t S, int bw, int split, const TI *__restrict__ x2, int c2) {
+__global__ void __launch_bounds__(256) pm_to_mx_k(const TI *x, uint8_t *__restrict__ y, int N, int C, size_t S, int bw, int split, const TI *x2, int c2) {
     pdl_trigger(); pdl_wait();
     const int nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, rb = bw * BITS / 8;
     const size_t rows = (size_t)N * nb * S, row0 = ((size_t)n * nb + blk) * S;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) pm_to_mx_k(const TI *__restrict__ x, uint
    values converted to fp32.  Bound by latency and the memory rate: 32 channels x 64^3 into MX-fp8 16.4 us at one voxel and 32 predicated
    2-byte loads a thread, 5.6 us in this form. */
 template <int BITS>
-__global__ void __launch_bounds__(128) h16_to_mx_pair_k(const __half *__restrict__ x, uint8_t *__restrict__ y, int N, int C, size_t S, int split) {
+__global__ void __launch_bounds__(128) h16_to_mx_pair_k(const __half *x, uint8_t *__restrict__ y, int N, int C, size_t S, int split) {
     pdl_trigger(); pdl_wait();
     const int nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z;
     constexpr int RB = 32 * BITS / 8;
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128) h16_to_mx_pair_k(const __half *__restrict
     for (size_t v2 = blockIdx.x * (size_t)128 + threadIdx.x; v2 < S2; v2 += (size_t)gridDim.x * 128) {
         unsigned raw[32];
 #pragma unroll
-        for (int k = 0; k < 32; k++) raw[k] = __ldg(xb + (size_t)k * S2 + v2);
+        for (int k = 0; k < 32; k++) raw[k] = ld_dep(xb + (size_t)k * S2 + v2);
         const __half2 *h = (const __half2 *)raw;
         __half2 a2 = __habs2(h[0]);
 #pragma unroll
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) h16_to_mx_pair_k(const __half *__restrict
    bytes a warp.  grid (voxels, blocks, samples).  Rows of 8 or 16 channels take mx_to_pm_k.  64 channels x 48^3 15.0 us with a decode in integer
    arithmetic and three index divisions a row, 5.3 us in this form. */
 template <int BITS>
-__global__ void __launch_bounds__(128) mx32_to_pm_k(const uint8_t *__restrict__ x, float *__restrict__ y, int N, int C, size_t S, int split) {
+__global__ void __launch_bounds__(128) mx32_to_pm_k(const uint8_t *x, float *__restrict__ y, int N, int C, size_t S, int split) {
     pdl_trigger(); pdl_wait();
     const int nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z;
     constexpr int RB = 32 * BITS / 8;
@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(128) mx32_to_pm_k(const uint8_t *__restrict__ 
     for (size_t v = blockIdx.x * (size_t)128 + threadIdx.x; v < S; v += (size_t)gridDim.x * 128) {
         uint4 q[RB / 16];
 #pragma unroll
-        for (int h = 0; h < RB / 16; h++) q[h] = __ldg((const uint4 *)(x + (BITS == 8 && split ? (row0 * 2 + h * S + v) * 16 : (row0 + v) * RB + h * 16)));
-        const float s = mx_scale(__ldg(sc + row0 + v));
+        for (int h = 0; h < RB / 16; h++) q[h] = ld_dep((const uint4 *)(x + (BITS == 8 && split ? (row0 * 2 + h * S + v) * 16 : (row0 + v) * RB + h * 16)));
+        const float s = mx_scale(ld_dep(sc + row0 + v));
         const unsigned *w = (const unsigned *)q;
         float e[32];
 #pragma unroll
@@ -278,14 +278,14 @@ extern "C" void umx_h16b_to_f32(const void *x, int N, int C, size_t S, float *y)
 
 /* MX-fp8 codes between the reference layout [n][blk][voxel][32 B] and the split layout [n][blk][half][voxel][16 B].  grid (voxels, blocks of all
    samples): a thread moves half rows 2 v + h of its block, consecutive threads consecutive 16-byte pieces of the reference layout */
-__global__ void __launch_bounds__(256) relayout8_k(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t blocks, size_t S, int to_split) {
+__global__ void __launch_bounds__(256) relayout8_k(const uint4 *src, uint4 *__restrict__ dst, size_t blocks, size_t S, int to_split) {
     pdl_trigger(); pdl_wait();
     for (size_t b = blockIdx.y; b < blocks; b += gridDim.y) {
         const uint4 *s = src + b * 2 * S; uint4 *d = dst + b * 2 * S;
         for (size_t i = blockIdx.x * (size_t)1024 + threadIdx.x; i < 2 * S; i += (size_t)gridDim.x * 1024) {
             uint4 t[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) { const size_t j = i + 256 * k; if (j < 2 * S) t[k] = __ldg(s + (to_split ? j : (j & 1) * S + (j >> 1))); }
+            for (int k = 0; k < 4; k++) { const size_t j = i + 256 * k; if (j < 2 * S) t[k] = ld_dep(s + (to_split ? j : (j & 1) * S + (j >> 1))); }
 #pragma unroll
             for (int k = 0; k < 4; k++) { const size_t j = i + 256 * k; if (j < 2 * S) d[to_split ? (j & 1) * S + (j >> 1) : j] = t[k]; }
         }
@@ -314,15 +314,15 @@ extern "C" void umx_mx_relayout(const void *src, int bits, int N, int C, size_t 
 /* blocks of an MX tensor (32-wide rows, reference layout, nb_src blocks a sample) to blocks [b0, b0 + nb_src) of one of nb_dst blocks, codes and scale
    bytes in one launch; to_split: MX-fp8 codes into the split layout.  The part of a conv's concat input that needs no transform. */
 template <int RB>
-__global__ void __launch_bounds__(256) mx_blocks_put_k(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int N, int nb_src, int nb_dst, int b0, size_t S, int to_split) {
+__global__ void __launch_bounds__(256) mx_blocks_put_k(const uint8_t *src, uint8_t *__restrict__ dst, int N, int nb_src, int nb_dst, int b0, size_t S, int to_split) {
     pdl_trigger(); pdl_wait();
     const int blk = blockIdx.y, n = blockIdx.z;
     const size_t sb = (size_t)n * nb_src + blk, db = (size_t)n * nb_dst + b0 + blk;
     const uint8_t *ss = src + (size_t)N * nb_src * S * RB + sb * S; uint8_t *ds = dst + (size_t)N * nb_dst * S * RB + db * S;
     const uint4 *s = (const uint4 *)(src + sb * S * RB); uint4 *d = (uint4 *)(dst + db * S * RB);
     for (size_t v = blockIdx.x * (size_t)256 + threadIdx.x; v < S; v += (size_t)gridDim.x * 256) {
-        const uint4 a = __ldg(s + v * (RB / 16)), b = RB == 32 ? __ldg(s + v * 2 + 1) : a;
-        const uint8_t e = __ldg(ss + v);
+        const uint4 a = ld_dep(s + v * (RB / 16)), b = RB == 32 ? ld_dep(s + v * 2 + 1) : a;
+        const uint8_t e = ld_dep(ss + v);
         if (RB == 32 && to_split) { d[v] = a; d[S + v] = b; }
         else if (RB == 32) { d[2 * v] = a; d[2 * v + 1] = b; }
         else d[v] = a;
@@ -342,12 +342,12 @@ void umx_mx_blocks_put(const void *src, int bits, int N, int nb_src, size_t S, v
 /* MX tensors of 16 channels or fewer keep rows of 8 or 16 channels in the reference's storage (src/lp_common.cuh:132-134).  Such a row
    and the 32-wide row holding the same channels followed by zeros have the same amax, hence the same scale byte and the same codes:
    widening and narrowing are copies.  One thread per row. */
-__global__ void __launch_bounds__(256) mx_rewidth_k(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, size_t rows, int rb_src, int rb_dst) {
+__global__ void __launch_bounds__(256) mx_rewidth_k(const uint8_t *src, uint8_t *__restrict__ dst, size_t rows, int rb_src, int rb_dst) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows; i += (size_t)gridDim.x * blockDim.x) {
         const unsigned *s = (const unsigned *)(src + i * rb_src); unsigned *d = (unsigned *)(dst + i * rb_dst);
-        for (int k = 0; k < rb_dst / 4; k++) d[k] = k < rb_src / 4 ? __ldg(s + k) : 0u;
-        dst[rows * rb_dst + i] = __ldg(src + rows * rb_src + i);
+        for (int k = 0; k < rb_dst / 4; k++) d[k] = k < rb_src / 4 ? ld_dep(s + k) : 0u;
+        dst[rows * rb_dst + i] = ld_dep(src + rows * rb_src + i);
     }
 }
 /* x: an MX tensor of C <= 16 channels (one block of 8 or 16 a voxel) -> y: the same tensor with 32-wide rows (to_wide), or back */
@@ -380,7 +380,7 @@ template <int HD> __device__ __forceinline__ float2 round16x2(float a, float b) 
    zero by construction, so only those are measured and encoded.  Bound by instruction issue, a third of it the IEEE square root and division
    a voxel: 192^3 50.8 us with a 32-channel encode and 64-bit index divisions a voxel, 25 us in this form (1 B read, 9 B written). */
 template <int BITS, int HD>
-__global__ void __launch_bounds__(256) pred_input_k(const uint8_t *__restrict__ ct, int W, float mean, float isd, const float *__restrict__ dyo, const float *__restrict__ dxo,
+__global__ void __launch_bounds__(256) pred_input_k(const uint8_t *ct, int W, float mean, float isd, const float *dyo, const float *dxo,
                                                     int axis, int z0, int nz, uint8_t *__restrict__ y) {
     pdl_trigger(); pdl_wait();
     const unsigned plane = (unsigned)W * (unsigned)W;
@@ -401,10 +401,10 @@ __global__ void __launch_bounds__(256) pred_input_k(const uint8_t *__restrict__ 
     uint8_t *yp = y + ((size_t)blockIdx.y * plane + p0) * BITS, *sp = y + (size_t)nz * plane * BITS + (size_t)blockIdx.y * plane + p0;   /* a row is BITS bytes: eight channels */
     const size_t step = (size_t)gridDim.y * plane;
     for (int zl = blockIdx.y; zl < nz; zl += gridDim.y, cp += step, yp += step * BITS, sp += step) {
-        const float oy = __ldg(dyo + z0 + zl), ox = __ldg(dxo + z0 + zl);
+        const float oy = ld_dep(dyo + z0 + zl), ox = ld_dep(dxo + z0 + zl);
         unsigned cv[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) cv[k] = p0 + 32 * k < plane ? __ldg(cp + 32 * k) : 0u;
+        for (int k = 0; k < 4; k++) cv[k] = p0 + 32 * k < plane ? ld_dep(cp + 32 * k) : 0u;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float dy = __fadd_rn(oy, fy[k]), dx = __fadd_rn(ox, fx[k]);
