@@ -57,7 +57,7 @@ __device__ __forceinline__ void stat_add(StatAcc &a, const uint4 &r) {
 __device__ unsigned g_stat_tickets[8192];
 
 template <bool FINAL>
-__global__ void __launch_bounds__(256, 3) in_part_k(const uint4 *__restrict__ y, size_t S, int T, double *__restrict__ part,
+__global__ void __launch_bounds__(256, 3) in_part_k(const uint4 *y, size_t S, int T, double *__restrict__ part,
                                                  int C, const float *gamma, const float *beta, float eps, float *coef) {
     pdl_trigger(); pdl_wait();
     const int t = blockIdx.x, blk = blockIdx.y, n = blockIdx.z, nb = gridDim.y, Cop = nb * 32;
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256, 3) in_part_k(const uint4 *__restrict__ y,
        leaves its start there for the apply (32 channels x 128^3: 35 us, and 37 instead of 41 for the apply; 37 with a contiguous piece a block in ascending order) */
     const size_t sweep = (size_t)T * 256;
     size_t k = (S + sweep - 1) / sweep;
-    auto at = [&](size_t trip, int u) { const size_t v = trip * sweep + (size_t)t * 256 + 64 * u + ph; return v < S ? __ldg(p + v * 4) : make_uint4(0u, 0u, 0u, 0u); };      /* rows past the end add zeros */
+    auto at = [&](size_t trip, int u) { const size_t v = trip * sweep + (size_t)t * 256 + 64 * u + ph; return v < S ? ld_dep(p + v * 4) : make_uint4(0u, 0u, 0u, 0u); };      /* rows past the end add zeros */
     for (; k >= 2; k -= 2) {      /* eight loads in flight */
         const uint4 r0 = at(k - 1, 0), r1 = at(k - 1, 1), r2 = at(k - 1, 2), r3 = at(k - 1, 3), r4 = at(k - 2, 0), r5 = at(k - 2, 1), r6 = at(k - 2, 2), r7 = at(k - 2, 3);
         add(r0); add(r1); add(r2); add(r3); add(r4); add(r5); add(r6); add(r7);
@@ -152,124 +152,164 @@ extern "C" void umx_in_coef(const double *part, int N, int C, int D, int H, int 
     UMX_CK("umx_in_coef");
 }
 
-/* NaN-propagating max of magnitudes in one instruction */
-__device__ __forceinline__ float amax_nan(float a, float v) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(fabsf(v))); return r; }
 
-/* one lane's eight channels of a row (four lanes a row): affine map, LeakyReLU as max(g, slope g), fp16 rounding (o), MX codes (w0, w1) and scale byte.
-   All 32 lanes call it together. */
+/* two fp32 operations in one instruction, each rounded to nearest even */
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
+    float2 o;
+    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 r, {%6, %7};\n\tfma.rn.f32x2 r, p, q, r;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+    return o;
+}
+__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
+    float2 o;
+    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmul.rn.f32x2 r, p, q;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+    return o;
+}
+/* Four lanes a row, eight channels a lane, four rows together: affine map, LeakyReLU, fp16 rounding (o), MX codes (w0, w1).  Returns the scale byte of row
+   qd: the four rows' maxima are reduced so that each lane of the quad ends up with one row's, works that row's scale out and hands it to the other three.
+   Instruction issue bounds the passes that call this where
+   they are not DRAM bound (rows one at a time, each lane working out each scale: with the space-to-depth copy 59 us for 32 channels x 128^3, 52 this way;
+   64^3 x 64 in one launch 20.9, 19.4).
+   LeakyReLU is max(g, slope g) for 0 < slope <= 1; rounding to fp16 is monotonic, so the maximum is taken of the rounded pairs.  mask: channels that are
+   real (FULL: all).  All 32 lanes call it together. */
 template <int BITS, bool COEF, bool FULL>
-__device__ __forceinline__ unsigned apply_row(const uint4 &raw, const float *ca, const float *cb, float slope, const bool *live, uint4 &o, unsigned &w0, unsigned &w1) {
-    const __half2 *hp = (const __half2 *)&raw;
-    __half2 *op = (__half2 *)&o;
+__device__ __forceinline__ unsigned apply4(const uint4 *raw, const float2 *ca, const float2 *cb, float slope, const unsigned *mask, int qd, uint4 *o, unsigned *w0, unsigned *w1) {
+    const float2 sl = make_float2(slope, slope);
+    __half2 am[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float2 t = __half22float2(hp[k]);
-        float g0 = t.x, g1 = t.y;
-        if (COEF) { g0 = __fmaf_rn(g0, ca[2 * k], cb[2 * k]); g1 = __fmaf_rn(g1, ca[2 * k + 1], cb[2 * k + 1]); }
-        g0 = fmaxf(g0, __fmul_rn(slope, g0)); g1 = fmaxf(g1, __fmul_rn(slope, g1));      /* LeakyReLU for 0 < slope <= 1 (NaN stays NaN) */
-        if (!FULL) { if (!live[2 * k]) g0 = 0.f; if (!live[2 * k + 1]) g1 = 0.f; }
-        op[k] = __floats2half2_rn(g0, g1);
-    }
-    /* amax of the stored fp16 values, NaN-propagating, taken on the halves (exact: the conversion to fp32 is monotonic) */
-    __half2 a2 = __hmax2_nan(__hmax2_nan(__habs2(op[0]), __habs2(op[1])), __hmax2_nan(__habs2(op[2]), __habs2(op[3])));
-    const __half a1 = __hmax_nan(__low2half(a2), __high2half(a2));
-    unsigned am = __float_as_uint(__half2float(a1)) & 0x7fffffffu;
-    am = max(am, __shfl_xor_sync(0xffffffffu, am, 1));
-    am = max(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    const mx_sb mq = mx_scale_of(__uint_as_float(am), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
-    const unsigned sb = mq.sb;
-    w1 = 0u;
-    if (BITS == 8 && sb - 112u <= 29u) {
-        /* 2^-e is a normal fp16: scale the halves (exact, or below 2^-14 where E4M3 rounds to zero either way) and convert pairs */
-        const unsigned mh = (142u - sb) << 10, m2 = mh | (mh << 16);
-        const __half2 mm = *(const __half2 *)&m2;
-        unsigned short c0, c1, c2, c3;
-        const __half2 s0 = __hmul2(op[0], mm), s1 = __hmul2(op[1], mm), s2 = __hmul2(op[2], mm), s3 = __hmul2(op[3], mm);
-        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c0) : "r"(*(const unsigned *)&s0));
-        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c1) : "r"(*(const unsigned *)&s1));
-        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c2) : "r"(*(const unsigned *)&s2));
-        asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c3) : "r"(*(const unsigned *)&s3));
-        w0 = (unsigned)c0 | ((unsigned)c1 << 16); w1 = (unsigned)c2 | ((unsigned)c3 << 16);
-    } else {
-        float f[8];
+    for (int u = 0; u < 4; u++) {
+        const __half2 *hp = (const __half2 *)(raw + u);
+        __half2 *op = (__half2 *)(o + u);
 #pragma unroll
-        for (int k = 0; k < 4; k++) { const float2 r = __half22float2(op[k]); f[2 * k] = r.x; f[2 * k + 1] = r.y; }
-        const float m = mq.m;
-        if (BITS == 8) { w0 = cvt_e4m3x4(f[0] * m, f[1] * m, f[2] * m, f[3] * m); w1 = cvt_e4m3x4(f[4] * m, f[5] * m, f[6] * m, f[7] * m); }
-        else w0 = cvt_e2m1x8(f, m);
+        for (int k = 0; k < 4; k++) {
+            float2 g = __half22float2(hp[k]);
+            if (COEF) g = fma2(g, ca[k], cb[k]);
+            const float2 l = mul2(sl, g);
+            op[k] = __hmax2(__floats2half2_rn(g.x, g.y), __floats2half2_rn(l.x, l.y));
+            if (!FULL) *(unsigned *)(op + k) &= mask[k];
+        }
+        /* amax of the stored fp16 values, NaN-propagating, taken on the halves (exact: the conversion to fp32 is monotonic) */
+        am[u] = __hmax2_nan(__hmax2_nan(__habs2(op[0]), __habs2(op[1])), __hmax2_nan(__habs2(op[2]), __habs2(op[3])));
     }
-    return sb;
+    const __half2 p01 = __hmax2_nan(__lows2half2(am[0], am[1]), __highs2half2(am[0], am[1])), p23 = __hmax2_nan(__lows2half2(am[2], am[3]), __highs2half2(am[2], am[3]));
+    const unsigned b01 = *(const unsigned *)&p01, b23 = *(const unsigned *)&p23;
+    unsigned own = qd & 2 ? b23 : b01, t = __shfl_xor_sync(0xffffffffu, qd & 2 ? b01 : b23, 2);
+    __half2 m = __hmax2_nan(*(const __half2 *)&own, *(const __half2 *)&t);
+    own = *(const unsigned *)&m; t = __shfl_xor_sync(0xffffffffu, own, 1);
+    m = __hmax2_nan(m, *(const __half2 *)&t);
+    const float a1 = __half2float(qd & 1 ? __high2half(m) : __low2half(m));
+    const mx_sb mq = mx_scale_of(__uint_as_float(__float_as_uint(a1) & 0x7fffffffu), BITS == 4 ? 1.f / 6.f : 1.f / 448.f);
+    /* what the row's codes need: the factor 2^-e as fp16 where it is a normal one (0: it is not) and the scale byte */
+    const unsigned pack = (mq.sb - 112u <= 29u ? (142u - mq.sb) << 10 : 0u) | (mq.sb << 16);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const unsigned f = __shfl_sync(0xffffffffu, pack, u, 4);
+        const __half2 *op = (const __half2 *)(o + u);
+        w1[u] = 0u;
+        if (BITS == 8 && (f & 0xffffu)) {
+            /* scale the halves (exact, or below 2^-14 where E4M3 rounds to zero either way) and convert pairs */
+            const unsigned m2 = __byte_perm(f, f, 0x1010);
+            const __half2 mm = *(const __half2 *)&m2;
+            unsigned short c0, c1, c2, c3;
+            const __half2 s0 = __hmul2(op[0], mm), s1 = __hmul2(op[1], mm), s2 = __hmul2(op[2], mm), s3 = __hmul2(op[3], mm);
+            asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c0) : "r"(*(const unsigned *)&s0));
+            asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c1) : "r"(*(const unsigned *)&s1));
+            asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c2) : "r"(*(const unsigned *)&s2));
+            asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(c3) : "r"(*(const unsigned *)&s3));
+            w0[u] = (unsigned)c0 | ((unsigned)c1 << 16); w1[u] = (unsigned)c2 | ((unsigned)c3 << 16);
+        } else {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) { const float2 r = __half22float2(op[k]); v[2 * k] = r.x; v[2 * k + 1] = r.y; }
+            const float fm = __uint_as_float((254u - (f >> 16)) << 23);
+            if (BITS == 8) { w0[u] = cvt_e4m3x4(v[0] * fm, v[1] * fm, v[2] * fm, v[3] * fm); w1[u] = cvt_e4m3x4(v[4] * fm, v[5] * fm, v[6] * fm, v[7] * fm); }
+            else w0[u] = cvt_e2m1x8(v, fm);
+        }
+    }
+    return mq.sb;
 }
-/* the same codes into the space-to-depth copy: block (tap * nb + blk) at the coarse voxel; wsh >= 0: W and H are powers of two */
-template <int BITS>
-__device__ __forceinline__ void s2d_store(uint8_t *q2, int N, int nb, int n, int blk, int qd, unsigned v, size_t S, int H, int W, int wsh, int hsh, int split, unsigned w0, unsigned w1, unsigned sb) {
-    constexpr int RB = 32 * BITS / 8;
+/* where a voxel lies in the space-to-depth copy: tap << 28 | coarse voxel (fewer than 2^28 of them); wsh >= 0: W and H are powers of two */
+__device__ __forceinline__ unsigned s2d_where(unsigned v, int H, int W, int wsh, int hsh) {
     unsigned xx, yy, zz;
-    if (wsh >= 0) { xx = v & ((1u << wsh) - 1u); const unsigned t1 = v >> wsh; yy = t1 & ((1u << hsh) - 1u); zz = t1 >> hsh; }      /* W and H powers of two */
-    else { xx = v % (unsigned)W; const unsigned t1 = v / (unsigned)W; yy = t1 % (unsigned)H; zz = t1 / (unsigned)H; }
-    const int tap = ((zz & 1) * 2 + (yy & 1)) * 2 + (xx & 1);
-    const size_t Sc = S / 8, vc = ((size_t)(zz >> 1) * (H >> 1) + (yy >> 1)) * (W >> 1) + (xx >> 1);
-    const size_t ro = (size_t)n * 8 * nb + tap * nb + blk;
-    if (BITS == 8 && split) *(uint2 *)(q2 + ((ro * 2 + (qd >> 1)) * Sc + vc) * 16 + (qd & 1) * 8) = make_uint2(w0, w1);
-    else if (BITS == 8) *(uint2 *)(q2 + (ro * Sc + vc) * 32 + qd * 8) = make_uint2(w0, w1);
-    else *(unsigned *)(q2 + (ro * Sc + vc) * 16 + qd * 4) = w0;
-    if (qd == 0) q2[(size_t)N * 8 * nb * Sc * RB + ro * Sc + vc] = (uint8_t)sb;
+    if (wsh >= 0) { xx = v & ((1u << wsh) - 1u); const unsigned t1 = v >> wsh; yy = t1 & ((1u << hsh) - 1u); zz = t1 >> hsh; }
+    else { const unsigned t1 = v / (unsigned)W; xx = v - t1 * (unsigned)W; zz = t1 / (unsigned)H; yy = t1 - zz * (unsigned)H; }
+    const unsigned tap = ((zz & 1) * 2 + (yy & 1)) * 2 + (xx & 1);
+    return tap << 28 | (((zz >> 1) * (unsigned)(H >> 1) + (yy >> 1)) * (unsigned)(W >> 1) + (xx >> 1));
 }
+/* one (sample, block)'s destinations: codes of the plain tensor and of the space-to-depth copy (block tap * nb + blk at the coarse voxel), each with this lane's
+   offset in a row, and the scale planes; put4 stores four rows, of which row u is voxel v[u], and the scale byte of voxel vo (any of them S or more: not there) */
+template <int BITS, bool S2D>
+struct MxDst {
+    uint8_t *qb, *qsc, *q2, *q2sc; int qs, q2s, H, W, wsh, hsh; size_t tstep, tsc;
+    __device__ __forceinline__ MxDst(uint8_t *q, uint8_t *qd2, int N, int nb, int n, int blk, int nb_dst, int b0, size_t S, int H_, int W_, int split, int qd) : H(H_), W(W_) {
+        constexpr int RB = 32 * BITS / 8;
+        const size_t drow = (size_t)n * nb_dst + b0 + blk, Sc = S / 8, ro = (size_t)n * 8 * nb + blk;
+        const int half = BITS == 8 && split;
+        qs = half ? 16 : RB;
+        qb = q ? q + (half ? (drow * 2 + (qd >> 1)) * S * 16 + (qd & 1) * 8 : drow * S * RB + qd * (RB / 4)) : nullptr;
+        qsc = q ? q + (size_t)N * nb_dst * S * RB + drow * S : nullptr;
+        if (S2D) {
+            const int pow2 = !(W & (W - 1)) && !(H & (H - 1));
+            wsh = pow2 ? __ffs(W) - 1 : -1; hsh = pow2 ? __ffs(H) - 1 : 0;
+            q2s = qs; tstep = (size_t)nb * Sc * RB; tsc = (size_t)nb * Sc;
+            q2 = qd2 + (half ? (ro * 2 + (qd >> 1)) * Sc * 16 + (qd & 1) * 8 : ro * Sc * RB + qd * (RB / 4));
+            q2sc = qd2 + (size_t)N * 8 * nb * Sc * RB + ro * Sc;
+        }
+    }
+    __device__ __forceinline__ void put4(const unsigned *v, unsigned vo, unsigned S, const unsigned *w0, const unsigned *w1, unsigned sb) const {
+        unsigned wo = 0u;
+        if (S2D) { wo = vo < S ? s2d_where(vo, H, W, wsh, hsh) : 0u; if (vo < S) q2sc[(size_t)(wo >> 28) * tsc + (wo & 0x0fffffffu)] = (uint8_t)sb; }
+        if (qb && vo < S) qsc[vo] = (uint8_t)sb;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            unsigned wu = 0u;
+            if (S2D) wu = __shfl_sync(0xffffffffu, wo, u, 4);
+            if (v[u] < S) {
+                if (qb) { if (BITS == 8) *(uint2 *)(qb + (size_t)v[u] * qs) = make_uint2(w0[u], w1[u]); else *(unsigned *)(qb + (size_t)v[u] * qs) = w0[u]; }
+                if (S2D) {
+                    uint8_t *d = q2 + (size_t)(wu >> 28) * tstep + (size_t)(wu & 0x0fffffffu) * q2s;
+                    if (BITS == 8) *(uint2 *)d = make_uint2(w0[u], w1[u]); else *(unsigned *)d = w0[u];
+                }
+            }
+        }
+    }
+};
 
 /* Four threads per voxel row, eight channels (one 16-byte load) each; a block walks a run of voxels of one (sample, block), so the
    sixteen coefficients a thread needs stay in registers.  The row's amax is combined with two shuffles.  grid = (voxel chunks,
-   blocks, samples).  This pass is bound by instruction issue (about ten instructions an element for the affine map, the
-   activation, two roundings and the MX encode), so the variants are compiled apart: COEF (affine map present), FULL (all 32
+   blocks, samples).  This pass is bound by instruction issue (see apply4), so the variants are compiled apart: COEF (affine map present), FULL (all 32
    channels of every block are real), S2D (second, space-to-depth destination). */
 template <int BITS, bool COEF, bool FULL, bool S2D>
-__global__ void __launch_bounds__(256) in_apply_k(const uint4 *__restrict__ x, const float2 *__restrict__ coef, int C, int D, int H, int W, int act,
+__global__ void __launch_bounds__(256) in_apply_k(const uint4 *x, const float2 *coef, int C, int D, int H, int W, int act,
                                                   uint8_t *__restrict__ q, int nb_dst, int b0, uint8_t *__restrict__ q2, uint4 *__restrict__ hout, int split, int T) {
     pdl_trigger(); pdl_wait();
     const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z;
     const size_t S = (size_t)D * H * W;
     const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
-    constexpr int RB = 32 * BITS / 8;
-    float ca[8], cb[8]; bool live[8];
+    float2 ca[4], cb[4]; unsigned mask[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int c = blk * 32 + qd * 8 + k;
-        live[k] = FULL || c < C; ca[k] = 1.f; cb[k] = 0.f;
-        if (COEF && live[k]) { const float2 ab = __ldg(coef + (size_t)n * C + c); ca[k] = ab.x; cb[k] = ab.y; }
+    for (int k = 0; k < 4; k++) {
+        const int c = blk * 32 + qd * 8 + 2 * k;
+        float2 p = make_float2(1.f, 0.f), r = p;
+        if (COEF) { if (FULL || c < C) p = ld_dep(coef + (size_t)n * C + c); if (FULL || c + 1 < C) r = ld_dep(coef + (size_t)n * C + c + 1); }
+        ca[k] = make_float2(p.x, r.x); cb[k] = make_float2(p.y, r.y);
+        mask[k] = FULL ? 0xffffffffu : (c < C ? 0xffffu : 0u) | (c + 1 < C ? 0xffff0000u : 0u);
     }
     const float slope = act == 2 ? 0.01f : 1.f;           /* LeakyReLU as max(g, slope g); slope 1 leaves g as it is */
-    const int pow2 = S2D && !(W & (W - 1)) && !(H & (H - 1)), wsh = pow2 ? __ffs(W) - 1 : -1, hsh = pow2 ? __ffs(H) - 1 : 0;
     const unsigned v0 = (unsigned)(S * blockIdx.x / T), v1 = (unsigned)(S * (blockIdx.x + 1) / T);      /* S < 2^31: 32-bit voxel indices in the loop */
     const uint4 *xp = x + ((size_t)n * nb + blk) * S * 4 + qd;
     uint4 *hp_out = hout ? hout + ((size_t)n * nb + blk) * S * 4 + qd : nullptr;
-    const size_t drow = (size_t)n * nb_dst + b0 + blk;
-    /* destination of this thread's 8 (fp8) or 4 (fp4) code bytes of voxel v: base + v * stride */
-    uint8_t *qb = nullptr; int qs = 0;
-    if (q) {
-        if (BITS == 8 && split) { qb = q + (drow * 2 + (qd >> 1)) * S * 16 + (qd & 1) * 8; qs = 16; }
-        else if (BITS == 8) { qb = q + drow * S * 32 + qd * 8; qs = 32; }
-        else { qb = q + drow * S * 16 + qd * 4; qs = 16; }
-    }
-    uint8_t *qsc = q ? q + (size_t)N * nb_dst * S * RB + drow * S : nullptr;
+    const MxDst<BITS, S2D> dst(q, q2, N, nb, n, blk, nb_dst, b0, S, H, W, split, qd);
     for (unsigned vb = v0; vb < v1; vb += 256) {
         /* four rows a thread per trip, their loads issued together */
-        uint4 raws[4];
+        uint4 raws[4], o[4]; unsigned v[4], w0[4], w1[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) { const unsigned v = vb + u * 64 + ph; raws[u] = v < v1 ? __ldcs(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* the last use of x */
+        for (int u = 0; u < 4; u++) { v[u] = vb + u * 64 + ph; raws[u] = v[u] < v1 ? __ldcs(xp + (size_t)v[u] * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* the last use of x */
+        const unsigned sb = apply4<BITS, COEF, FULL>(raws, ca, cb, slope, mask, qd, o, w0, w1);
+        if (hp_out) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const unsigned v = vb + u * 64 + ph; const bool ok = v < v1;      /* all 32 lanes stay for the shuffles */
-            uint4 o; unsigned w0, w1;
-            const unsigned sb = apply_row<BITS, COEF, FULL>(raws[u], ca, cb, slope, live, o, w0, w1);
-            if (hp_out && ok) hp_out[(size_t)v * 4] = o;
-            if (!ok) continue;
-            if (qb) {
-                if (BITS == 8) *(uint2 *)(qb + (size_t)v * qs) = make_uint2(w0, w1); else *(unsigned *)(qb + (size_t)v * qs) = w0;
-                if (qd == 0) qsc[v] = (uint8_t)sb;
-            }
-            if (S2D) {   /* space-to-depth copy: block (tap * nb + blk) at the coarse voxel */
-                s2d_store<BITS>(q2, N, nb, n, blk, qd, v, S, H, W, wsh, hsh, split, w0, w1, sb);
-            }
+            for (int u = 0; u < 4; u++) if (v[u] < v1) hp_out[(size_t)v[u] * 4] = o[u];
         }
+        dst.put4(v, vb + (unsigned)qd * 64 + ph, v1, w0, w1, sb);
     }
 }
 template <int BITS, bool COEF, bool FULL>
@@ -313,7 +353,7 @@ struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint
 template <int BITS, bool S2D, int ROWS, int NT, bool STASH>
 __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
     pdl_trigger();
-    constexpr int RB = 32 * BITS / 8, PH = NT / 4, GR = NT / 64;
+    constexpr int PH = NT / 4, GR = NT / 64;
     __shared__ double ss[64][33], sq[64][33];
     __shared__ double mine[64];
     __shared__ float2 sc[32];
@@ -332,7 +372,7 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         stat_zero(acc);
         auto load4 = [&](uint4 *r, unsigned k) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) { const unsigned v = vox(k, u); r[u] = v < S ? __ldg(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
+            for (int u = 0; u < 4; u++) { const unsigned v = vox(k, u); r[u] = v < S ? ld_dep(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
         };
         unsigned kr = 0;                                     /* the trips before those in registers wait in shared memory */
         if (STASH) {
@@ -409,34 +449,28 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
     __syncthreads();
     if (threadIdx.x < 32) sc[c] = coef_of(ss[0][c], ss[1][c], (double)S, a.eps, nullptr, nullptr, 0);
     __syncthreads();
-    float ca[8], cb[8]; bool live[8];
+    float2 ca[4], cb[4]; unsigned mask[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++) { const float2 ab = sc[qd * 8 + k]; ca[k] = ab.x; cb[k] = ab.y; live[k] = true; }
+    for (int k = 0; k < 4; k++) { const float2 p = sc[qd * 8 + 2 * k], r = sc[qd * 8 + 2 * k + 1]; ca[k] = make_float2(p.x, r.x); cb[k] = make_float2(p.y, r.y); mask[k] = 0xffffffffu; }
     const float slope = a.act == 2 ? 0.01f : 1.f;
-    const int H = a.H, W = a.W, pow2 = S2D && !(W & (W - 1)) && !(H & (H - 1)), wsh = pow2 ? __ffs(W) - 1 : -1, hsh = pow2 ? __ffs(H) - 1 : 0;
-    const size_t drow = (size_t)n * a.nb_dst + a.b0 + blk;
-    uint8_t *qb; int qs;
-    if (BITS == 8 && a.split) { qb = a.q + (drow * 2 + (qd >> 1)) * S * 16 + (qd & 1) * 8; qs = 16; }
-    else if (BITS == 8) { qb = a.q + drow * S * 32 + qd * 8; qs = 32; }
-    else { qb = a.q + drow * S * 16 + qd * 4; qs = 16; }
-    uint8_t *qsc = a.q + (size_t)N * a.nb_dst * S * RB + drow * S;
-    auto put = [&](const uint4 &r, unsigned v) {
-        uint4 o; unsigned w0, w1;
-        const unsigned sb = apply_row<BITS, true, true>(r, ca, cb, slope, live, o, w0, w1);
-        if (v < S) {
-            if (BITS == 8) *(uint2 *)(qb + (size_t)v * qs) = make_uint2(w0, w1); else *(unsigned *)(qb + (size_t)v * qs) = w0;
-            if (qd == 0) qsc[v] = (uint8_t)sb;
-            if (S2D) s2d_store<BITS>(a.q2, N, nb, n, blk, qd, v, S, H, W, wsh, hsh, a.split, w0, w1, sb);
-        }
+    const MxDst<BITS, S2D> dst(a.q, a.q2, N, nb, n, blk, a.nb_dst, a.b0, S, a.H, a.W, a.split, qd);
+    auto put = [&](const uint4 *r, unsigned k) {             /* the four rows of trip k */
+        uint4 o[4]; unsigned v[4], w0[4], w1[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = vox(k, u);
+        const unsigned sb = apply4<BITS, true, true>(r, ca, cb, slope, mask, qd, o, w0, w1);
+        dst.put4(v, vox(k, qd), S, w0, w1, sb);
     };
     unsigned kr = 0;
     if (STASH) while (kr + ROWS / 4 < K) kr += ROWS / 4;
 #pragma unroll
-    for (int u = 0; u < ROWS; u++) put(raw[u], vox(kr + u / 4, u & 3));
+    for (int k = 0; k < ROWS / 4; k++) put(raw + 4 * k, kr + k);
     if (STASH) {
         for (unsigned k = 0; k < kr; k++) {
+            uint4 r[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) put(stash[(size_t)(k * 4 + u) * NT], vox(k, u));
+            for (int u = 0; u < 4; u++) r[u] = stash[(size_t)(k * 4 + u) * NT];
+            put(r, k);
         }
     }
     if (CL > 1) cluster_wait();
