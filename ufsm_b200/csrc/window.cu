@@ -2,7 +2,7 @@
    the rank's accumulators (the role of k_i3_blend, src/nn_ink3dext.cu:58-73, in the reference).  HBM-bound elementwise passes. */
 #include "mx_common.cuh"
 
-__global__ void __launch_bounds__(256) u8_to_h16_k(const uint8_t *__restrict__ x, __half *__restrict__ y, size_t n) {
+__global__ void __launch_bounds__(256) u8_to_h16_k(const uint8_t *x, __half *__restrict__ y, size_t n) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         y[i] = __float2half_rn(__fdiv_rn((float)x[i], 255.f));
@@ -18,7 +18,7 @@ extern "C" void umx_u8_to_h16(const uint8_t *x, size_t n, void *y) {
 /* one P^3 patch at (z, y, x) of a uint8 volume slab on the device (planes of V x V voxels, z counted from the slab's first plane) -> fp16
    intensities x / 255, the patch contiguous; voxels beyond the volume's y / x extent read as zero.  Eight voxels of a row a thread when
    the rows allow 8-byte loads. */
-__global__ void __launch_bounds__(256) gather_u8_h16_k(const uint8_t *__restrict__ vol, int V, int z, int y, int x, int P, __half *__restrict__ out, int vec) {
+__global__ void __launch_bounds__(256) gather_u8_h16_k(const uint8_t *vol, int V, int z, int y, int x, int P, __half *__restrict__ out, int vec) {
     pdl_trigger(); pdl_wait();
     const size_t plane = (size_t)V * V;
     if (vec) {
@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(256) gather_u8_h16_k(const uint8_t *__restrict
         for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
             const int px = (int)(i % P8) * 8, py = (int)((i / P8) % P), pz = (int)(i / ((size_t)P8 * P));
             uint2 v = make_uint2(0u, 0u);
-            if (y + py < V && x + px + 8 <= V) v = __ldg((const uint2 *)(vol + (size_t)(z + pz) * plane + (size_t)(y + py) * V + x + px));
+            if (y + py < V && x + px + 8 <= V) v = ld_dep((const uint2 *)(vol + (size_t)(z + pz) * plane + (size_t)(y + py) * V + x + px));
             __half2 h[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -56,11 +56,11 @@ extern "C" void umx_gather_u8_h16(const uint8_t *vol_dev, int V, int z, int y, i
    rounds 255 p + 0.5 down; the blended path's k_i3_emit uses round(254 p), which is what this library uses throughout) */
 __device__ __forceinline__ unsigned prob_u8(float l) { return (unsigned)__float2int_rn(__fmul_rn(__fdiv_rn(1.f, __fadd_rn(1.f, expf(-l))), 254.f)) & 0xffu; }
 /* eight values a thread: one 16-byte load, one 8-byte store (x and y 16- and 8-byte aligned); the tail one by one */
-__global__ void __launch_bounds__(256) h16_to_prob_u8_k(const __half *__restrict__ x, uint8_t *__restrict__ y, size_t n) {
+__global__ void __launch_bounds__(256) h16_to_prob_u8_k(const __half *x, uint8_t *__restrict__ y, size_t n) {
     pdl_trigger(); pdl_wait();
     const size_t n8 = n / 8;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-        const uint4 v = __ldg((const uint4 *)x + i);
+        const uint4 v = ld_dep((const uint4 *)x + i);
         const __half2 *h = (const __half2 *)&v;
         unsigned w[2] = {0u, 0u};
 #pragma unroll
@@ -99,8 +99,8 @@ extern "C" void umx_h16_to_prob_u8(const void *x, size_t n, uint8_t *y) {
 /* acc[c][z - zlo][y][x] += w(z) w(y) w(x) logits[c][patch voxel], wsum likewise, for the patch at (z0, y0, x0); one thread per patch
    voxel, channels looped (patches are added one launch at a time, so no two threads touch the same accumulator) */
 template <typename T>
-__global__ void __launch_bounds__(256) blend_add_k(const T *__restrict__ logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0,
-                                                    const float *__restrict__ w1d, float *__restrict__ acc, float *__restrict__ wsum) {
+__global__ void __launch_bounds__(256) blend_add_k(const T *logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0,
+                                                    const float *w1d, float *__restrict__ acc, float *__restrict__ wsum) {
     pdl_trigger(); pdl_wait();
     const size_t PS = (size_t)P * P * P, plane = (size_t)V * V, AS = plane * zext;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < PS; i += (size_t)gridDim.x * blockDim.x) {
@@ -128,21 +128,29 @@ extern "C" void umx_blend_add(const void *logits, int fmt, int nh, int P, int V,
    forwarded in or on which rank forwarded them, so the partial sums of two ranks add up to the single-rank sums bit for bit.
    (|sum| < 2^17; a weight is at least exp(-24) = 2^-34.6, so even the volume's corner voxels keep 11 significant bits of weight.) ---- */
 #define UMX_FX_SCALE 70368744177664.0      /* 2^46 */
-__global__ void __launch_bounds__(256) blend_fx_k(const float *__restrict__ logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0,
-                                                   const float *__restrict__ w1d, long long *__restrict__ acc, long long *__restrict__ wsum) {
+__global__ void __launch_bounds__(256) blend_fx_k(const float *logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0,
+                                                   const float *w1d, long long *__restrict__ acc, long long *__restrict__ wsum) {
     pdl_trigger(); pdl_wait();
-    const size_t PS = (size_t)P * P * P, plane = (size_t)V * V, AS = plane * zext;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < PS; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % P), y = (int)((i / P) % P), z = (int)(i / ((size_t)P * P));
-        const int gz = z0 + z - zlo, gy = y0 + y, gx = x0 + x;
+    /* Latency bound when the channels go one after the other (seven on 64^3: 20 us): eight channels' loads are in flight before the first store */
+    const unsigned PS = (unsigned)P * P * P; const size_t plane = (size_t)V * V, AS = plane * zext;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < PS; i += gridDim.x * blockDim.x) {
+        const unsigned row = i / (unsigned)P, z = row / (unsigned)P, y = row - z * (unsigned)P, x = i - row * (unsigned)P;
+        const int gz = z0 + (int)z - zlo, gy = y0 + (int)y, gx = x0 + (int)x;
         if (gz < 0 || gz >= zext || gy >= V || gx >= V) continue;
         const double w = (double)__fmul_rn(__fmul_rn(w1d[z], w1d[y]), w1d[x]) * UMX_FX_SCALE;      /* the reference's fp32 weight, scaled */
         const size_t gv = (size_t)gz * plane + (size_t)gy * V + gx;
-        for (int c = 0; c < nh; c++) {
-            const double t = w * (double)logits[(size_t)c * PS + i];        /* exact: 24 x 24 bits, the scale a power of two */
-            acc[(size_t)c * AS + gv] += fabs(t) < 9.0e18 ? __double2ll_rn(t) : 0ll;
+        const long long ws = wsum[gv];
+        for (int c0 = 0; c0 < nh; c0 += 8) {
+            float l[8]; long long s[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) { const bool on = c0 + k < nh; l[k] = on ? logits[(size_t)(c0 + k) * PS + i] : 0.f; s[k] = on ? acc[(size_t)(c0 + k) * AS + gv] : 0ll; }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const double t = w * (double)l[k];        /* exact: 24 x 24 bits, the scale a power of two */
+                if (c0 + k < nh) acc[(size_t)(c0 + k) * AS + gv] = s[k] + (fabs(t) < 9.0e18 ? __double2ll_rn(t) : 0ll);
+            }
         }
-        wsum[gv] += __double2ll_rn(w);
+        wsum[gv] = ws + __double2ll_rn(w);
     }
 }
 extern "C" void umx_blend_add_fx(const float *logits, int nh, int P, int V, int zlo, int zext, int z0, int y0, int x0, const float *w1d, long long *acc, long long *wsum) {
@@ -155,7 +163,7 @@ extern "C" void umx_blend_add_fx(const float *logits, int nh, int P, int V, int 
 /* the blended value of the rows (z, y) with mode[z][y] == want, z in [za, zb) of the accumulators' extent and y in [ya, yb): l = sum / weight (in fp64, rounded to
    fp32), then fmt UMX_F16: the logit as fp16; any other fmt (uint8): round(254 p) with p = 1 / (1 + exp(-l)), 255 where no patch covers the voxel
    (k_i3_emit, src/nn_ink3dext.cu:77-100).  out [nh][zext][V][V]. */
-__global__ void __launch_bounds__(256) emit_fx_k(const long long *__restrict__ acc, const long long *__restrict__ wsum, const uint8_t *__restrict__ mode, int want,
+__global__ void __launch_bounds__(256) emit_fx_k(const long long *acc, const long long *wsum, const uint8_t *mode, int want,
                                                   int nh, int V, int zext, int za, int zb, int ya, int yb, int fmt, void *__restrict__ out) {
     pdl_trigger(); pdl_wait();
     const size_t plane = (size_t)V * V, AS = plane * zext, slab = (size_t)(yb - ya) * V, n = (size_t)(zb - za) * slab;
@@ -179,7 +187,7 @@ extern "C" void umx_emit_fx(const long long *acc, const long long *wsum, const u
     UMX_CK("umx_emit_fx");
 }
 /* the same values for a list of rows (z, y), compact: out [row][nh][V] */
-__global__ void __launch_bounds__(256) emit_rows_fx_k(const long long *__restrict__ acc, const long long *__restrict__ wsum, const int *__restrict__ zy, long nrows, int nh, int V, int zext, int fmt, void *__restrict__ out) {
+__global__ void __launch_bounds__(256) emit_rows_fx_k(const long long *acc, const long long *wsum, const int *zy, long nrows, int nh, int V, int zext, int fmt, void *__restrict__ out) {
     pdl_trigger(); pdl_wait();
     const size_t plane = (size_t)V * V, AS = plane * zext, per = (size_t)nh * V, n = (size_t)nrows * per;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -200,7 +208,7 @@ extern "C" void umx_emit_rows_fx(const long long *acc, const long long *wsum, co
 }
 /* rows (z, y) of the accumulators to or from a compact buffer buf [row][nh + 1][V] (the weight sum last): dir 0 copies the rows out, dir 1 adds
    the buffer's rows into the accumulators.  zy: device, 2 ints a row, z relative to the accumulators' first plane. */
-__global__ void __launch_bounds__(256) rows_fx_k(long long *__restrict__ acc, long long *__restrict__ wsum, const int *__restrict__ zy, long nrows, int nh, int V, int zext, int dir, long long *__restrict__ buf) {
+__global__ void __launch_bounds__(256) rows_fx_k(long long *__restrict__ acc, long long *__restrict__ wsum, const int *zy, long nrows, int nh, int V, int zext, int dir, long long *__restrict__ buf) {
     pdl_trigger(); pdl_wait();
     const size_t plane = (size_t)V * V, AS = plane * zext, per = (size_t)(nh + 1) * V, n = (size_t)nrows * per;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
