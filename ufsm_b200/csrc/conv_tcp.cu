@@ -59,10 +59,6 @@ __device__ __forceinline__ float2 add2(float2 x, float2 y) {
     asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 r, p, q;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
     return o;
 }
-/* 32 bytes in one store: two neighbouring 16-byte rows, a whole sector where the address is a multiple of 32 */
-__device__ __forceinline__ void st_32b(uint8_t *p, unsigned a, unsigned b, unsigned c, unsigned d, unsigned e, unsigned f, unsigned g, unsigned h) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
-}
 /* EPI: the output mode known at compile time (0: any, read from the arguments; 1: plane-major fp32; 2: plane-major fp16; 3: MX-fp8 split
    layout; 4: the same through the transposed conv's scatter; 5, 6: MX-fp4 likewise), so that the epilogue's code is only what that mode needs */
 template <int BITS, int EPI>

@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                                 const __half2 x1 = __floats2half2_rn(__fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t + 2]), b0.z), __fadd_rn(__uint_as_float(rr[jc][16 * k + 4 * t + 3]), b0.w));
                                 h[2 * t] = *(const uint32_t *)&x0; h[2 * t + 1] = *(const uint32_t *)&x1;
                             }
-                            if (row_ok) asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(pv + (size_t)jc * S * 64 + k * 32), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7]) : "memory");
+                            if (row_ok) st_32b(pv + (size_t)jc * S * 64 + k * 32, h[0], h[1], h[2], h[3], h[4], h[5], h[6], h[7]);
                         }
                     }
                 } else if (a.fast_h16) {
