@@ -276,10 +276,11 @@ struct MxDst {
 
 /* Four threads per voxel row, eight channels (one 16-byte load) each; a block walks a run of voxels of one (sample, block), so the
    sixteen coefficients a thread needs stay in registers.  The row's amax is combined with two shuffles.  grid = (voxel chunks,
-   blocks, samples).  This pass is bound by instruction issue (see apply4), so the variants are compiled apart: COEF (affine map present), FULL (all 32
+   blocks, samples).  This pass is bound by instruction issue (see apply4) and, at three blocks a multiprocessor, by latency (32 channels x 128^3 36.5 us, 33.3 at
+   four; the 64-channel MX-fp4 pass with its copy on 96^3 47 and 39), so the variants are compiled apart: COEF (affine map present), FULL (all 32
    channels of every block are real), S2D (second, space-to-depth destination). */
 template <int BITS, bool COEF, bool FULL, bool S2D>
-__global__ void __launch_bounds__(256) in_apply_k(const uint4 *x, const float2 *coef, int C, int D, int H, int W, int act,
+__global__ void __launch_bounds__(256, 4) in_apply_k(const uint4 *x, const float2 *coef, int C, int D, int H, int W, int act,
                                                   uint8_t *__restrict__ q, int nb_dst, int b0, uint8_t *__restrict__ q2, uint4 *__restrict__ hout, int split, int T) {
     pdl_trigger(); pdl_wait();
     const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z;
@@ -440,8 +441,13 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         }
         __syncthreads();
         double t = 0.0;
-#pragma unroll 4
-        for (int k = grp; k < B; k += GR) t += __ldcg(part + k * 64 + (which << 5) + c);
+        for (int k = grp; k < B; k += 20 * GR) {             /* one round trip for 148 blocks of 512 threads */
+            double v[20];
+#pragma unroll
+            for (int j = 0; j < 20; j++) v[j] = k + j * GR < B ? __ldcg(part + (k + j * GR) * 64 + (which << 5) + c) : 0.0;
+#pragma unroll
+            for (int j = 0; j < 20; j++) t += v[j];
+        }
         groups(t, mine);
         __syncthreads();
         if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x];
