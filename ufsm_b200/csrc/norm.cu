@@ -441,13 +441,8 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         }
         __syncthreads();
         double t = 0.0;
-        for (int k = grp; k < B; k += 20 * GR) {             /* one round trip for 148 blocks of 512 threads */
-            double v[20];
-#pragma unroll
-            for (int j = 0; j < 20; j++) v[j] = k + j * GR < B ? __ldcg(part + (k + j * GR) * 64 + (which << 5) + c) : 0.0;
-#pragma unroll
-            for (int j = 0; j < 20; j++) t += v[j];
-        }
+#pragma unroll 4
+        for (int k = grp; k < B; k += GR) t += __ldcg(part + k * 64 + (which << 5) + c);
         groups(t, mine);
         __syncthreads();
         if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x];
