@@ -197,3 +197,25 @@ def test_up2_blocks_conv1_ranges_and_add(dev, bits):
     L.lp_add_mx(yd.ptr, x2d.ptr, Shape5(N, Cs, D, H, W), bits, 0)
     ufsm_b200.check()
     assert np.array_equal(yd.download(), want)
+
+
+@pytest.mark.parametrize("bits,Cn,Co,W,gn", [(8, 32, 7, 64, False), (4, 40, 16, 63, False), (8, 64, 3, 65, True)])
+def test_conv1_two_voxels_a_thread(dev, bits, Cn, Co, W, gn):
+    """a volume large enough for two voxels a thread (from 2^18 voxels), full and ragged last blocks, against ranges small enough for one: the same bits"""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf, Shape5, Gnp
+    L = ufsm_b200.lib()
+    D, H = 66, 64
+    S, dt, r = D * H * W, 3 if bits == 8 else 4, synth.rng(401)
+    nb = (Cn + 31) // 32
+    xd = DevBuf(data=np.concatenate([r.integers(0, 120, nb * S * 4 * bits, dtype=np.uint8), r.integers(120, 130, nb * S, dtype=np.uint8)]))
+    wd, bd = DevBuf(data=(r.standard_normal((Co, Cn)) / np.sqrt(Cn)).astype(f32)), DevBuf(data=(0.1 * r.standard_normal(Co)).astype(f32))
+    gp, keep = make_gp(8, gn_params(402, 1, Cn, 8)) if gn else (Gnp(), None)
+    y = DevBuf(Co * S * 4).fill(0xEE)
+    L.lp_conv1_fwd_mx(xd.ptr, dt, Shape5(1, Cn, D, H, W), wd.ptr, bd.ptr, Co, y.ptr, gp)
+    whole = y.download(f32).reshape(Co, S)
+    for vb, nv in ((0, S // 2), (S // 2, S - S // 2)):
+        p = DevBuf(Co * nv * 4).fill(0xEE)
+        assert L.lp_conv1_fwd_mx_r(xd.ptr, dt, Shape5(1, Cn, D, H, W), wd.ptr, bd.ptr, Co, p.ptr, gp, vb, nv, nv) == 0
+        ufsm_b200.check()
+        assert np.array_equal(p.download().view(np.uint32).reshape(Co, nv), np.ascontiguousarray(whole[:, vb:vb + nv]).view(np.uint32))
