@@ -109,3 +109,23 @@ def test_small_grids_in_few_blocks(dev, N, Ci, Co, D, H, W, cap, bits):
     assert np.array_equal(coef, orc.in_coef(orc.in_sums(y.astype(np.float32), N, Co, S), N, Co, S))
     if same_kernel:
         assert np.array_equal(y_free.view(np.uint16), y.view(np.uint16)) and np.array_equal(coef, coef_free)
+
+
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,bits", [(1, 32, 32, 3, 16, 16, 8), (2, 32, 24, 4, 19, 16, 8), (1, 64, 64, 3, 9, 48, 8), (1, 32, 96, 5, 16, 32, 4), (1, 64, 33, 12, 5, 16, 8), (1, 32, 1, 2, 16, 16, 8)])
+def test_plane_major_halves(dev, N, Ci, Co, D, H, W, bits):
+    """the plane-major fp16 epilogue: the values of the blocked fp16 one, at partial tiles, channel counts that end inside a block or a pair, one and several
+    column tiles; an output that is not on a 16-byte boundary takes the general epilogue"""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S, nbi, nbo, r = D * H * W, (Ci + 31) // 32, (Co + 31) // 32, synth.rng(701)
+    x = DevBuf(data=np.concatenate([r.integers(0, 120, N * nbi * S * 4 * bits, dtype=np.uint8), r.integers(118, 128, N * nbi * S, dtype=np.uint8)]))
+    c = G.Conv("conv3", synth.kaiming(702, Co, Ci, 27), synth.bias(703, Co, 0.1), Co, Ci, bits)
+
+    def run(nbytes, shift, mode):
+        y = DevBuf(data=np.full(nbytes + shift, 0x5a, np.uint8))
+        assert dev.umx_conv_fwd(c.h, x.ptr, N, D, H, W, y.ptr + shift, mode, 0, 0, 0, None, 1) == 0
+        ufsm_b200.check()
+        return y.download()[shift:].copy().view(np.uint16)
+    want = run(N * nbo * S * 64, 0, 0).reshape(N, nbo, S, 32).transpose(0, 1, 3, 2).reshape(N, nbo * 32, S)[:, :Co]
+    for shift in (0, 2):
+        assert np.array_equal(run(N * Co * S * 2, shift, 3).reshape(N, Co, S), want)

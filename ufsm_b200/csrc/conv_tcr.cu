@@ -68,8 +68,8 @@ struct ConvRArgs {
     int ring, stage_bytes, offSW, offSFA;
     int w_bytes, w_codes, nquad, gt, goff1, goff2, nslot;
     int tmem_cols, sfa_base, sfa_cols, sfb_base; /* TMEM: accumulator slots from 0, two A scale buffers, B scales */
-    int off_rec, off_bias, off_stage, off_w, off_ring;   /* off_stage (with statistics): 2 KB per epilogue warp and 32-channel chunk, the fp16 output rows on their way to coalesced stores */
-    int fast_h16;                                /* output is the fp16 blocked tensor of a plain conv: the short epilogue */
+    int off_rec, off_bias, off_stage, off_w, off_ring;   /* off_stage (with statistics or a plane-major output): 2 KB per epilogue warp (and 32-channel chunk), the fp16 rows on their way to wide stores */
+    int fast_h16, fast_pm16;                     /* output is the fp16 blocked tensor of a plain conv, or plane-major fp16: the short epilogues */
     /* InstanceNorm statistics taken in that epilogue (coef != NULL): fp64 sums of the stored fp16 values and of their squares, written once per
        sample and block into part [n][gcol][cop][2]; the last block of a column tile to finish adds the blocks' entries in block order and
        turns them into coefficients (a, b) per (sample, channel) */
@@ -526,6 +526,36 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                             }
                         }
                     }
+                } else if (!STATS && a.fast_pm16) {
+                    /* plane-major fp16: a tile row is 16 bytes of a plane.  The warp's 32 voxels pass through shared memory as [channel pair][voxel], so that a lane
+                       stores whole tile rows instead of a 2-byte piece a channel (32 -> 32 on 64^3 20.7 us, 17.1 this way; 64 -> 64 51.4 and 30.4).  On volumes far
+                       beyond L2 half-written sectors bound it (128^3 233 us) */
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_acce + 8 * slot);
+                    uint32_t *sp = (uint32_t *)(smem_raw + a.off_stage + q4 * 2048);
+#pragma unroll
+                    for (int jc = 0; jc < NCH; jc++) {
+                        const float4 *bs = (const float4 *)(bias_s + jc * 32);
+                        __syncwarp();                       /* the rows before have been read */
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            const float4 b0 = bs[k];
+                            const __half2 x0 = __floats2half2_rn(__fadd_rn(__uint_as_float(rr[jc][4 * k]), b0.x), __fadd_rn(__uint_as_float(rr[jc][4 * k + 1]), b0.y));
+                            const __half2 x1 = __floats2half2_rn(__fadd_rn(__uint_as_float(rr[jc][4 * k + 2]), b0.z), __fadd_rn(__uint_as_float(rr[jc][4 * k + 3]), b0.w));
+                            sp[2 * k * 32 + lane] = *(const uint32_t *)&x0; sp[(2 * k + 1) * 32 + lane] = *(const uint32_t *)&x1;
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const int q = i * 32 + lane, pair = q >> 2, y = sy + (q & 3), c = (ctile * NCH + jc) * 32 + 2 * pair;
+                            const uint4 u = *(const uint4 *)(sp + pair * 32 + (q & 3) * 8), v = *(const uint4 *)(sp + pair * 32 + (q & 3) * 8 + 4);
+                            __half *d = (__half *)a.e.y + ((size_t)rn.n * a.e.co_real + c) * S + ((size_t)z * a.H + y) * a.W + x0t;
+                            if (y < a.H && c < a.e.co_real) *(uint4 *)d = make_uint4(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.z, u.w, 0x5410), __byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410));
+                            if (y < a.H && c + 1 < a.e.co_real) *(uint4 *)(d + S) = make_uint4(__byte_perm(u.x, u.y, 0x7632), __byte_perm(u.z, u.w, 0x7632), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));
+                        }
+                    }
                 } else {
                     tmem_st_wait();
                     tc_fence_before();
@@ -660,12 +690,13 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     a.units = (long long)N * a.tiles * D;
     a.nquad = c->nquad;
     a.fast_h16 = e.out_mode == UMX_OUT_H16B && !e.tconv && (want_coef || !((size_t)e.y & 31));      /* stores of 32 bytes */
+    a.fast_pm16 = e.out_mode == UMX_OUT_PM16 && !e.tconv && !((size_t)e.y & 15);        /* W is a multiple of 16: tile rows are aligned and whole */
     if (want_coef && (!a.fast_h16 || !part || g.ncol > 64)) return 0;
     a.cop = c->cop;
     /* the codes and the scale window are TMA destinations (128-byte aligned) */
     a.offSW = 5888; a.offSFA = a.offSW + (c->bits == 8 ? 640 : 1152);
     a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
-    a.off_rec = 1024; a.off_bias = a.off_rec + 12 * 64; a.off_stage = 2048; a.off_red = a.off_stage; a.off_w = a.off_stage + (want_coef ? 8192 * (g.nt == 32 ? 1 : 2) : 0); a.off_ring = (a.off_w + a.w_bytes + 1023) & ~1023;
+    a.off_rec = 1024; a.off_bias = a.off_rec + 12 * 64; a.off_stage = 2048; a.off_red = a.off_stage; a.off_w = a.off_stage + (want_coef ? 8192 * (g.nt == 32 ? 1 : 2) : a.fast_pm16 ? 8192 : 0); a.off_ring = (a.off_w + a.w_bytes + 1023) & ~1023;
     int dev = 0, sms = 148; cudaGetDevice(&dev);
     { static int sms_of[16]; if (!sms_of[dev & 15]) { int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); sms_of[dev & 15] = v; } sms = sms_of[dev & 15]; }   /* looked up once per device */
     /* two blocks a multiprocessor when shared memory (113 KB each) and TMEM (256 columns each) allow */
