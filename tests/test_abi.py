@@ -84,6 +84,23 @@ def test_network_sizes():
     assert abs(L.umx_unet_flops(C.byref(cfg)) / 1e9 - 1012.8) < 0.5     # the benchmark's figure for one 128^3 patch
 
 
+def test_upsample_tile_rows_are_exact():
+    """the upsample finds a staged row's plane, line and place by multiplication: every row of every tile its search can return"""
+    L = ufsm_b200.lib()
+    buf, seen = (C.c_int * (3 * 896))(), 0
+    for ux in range(1, 34):
+        for uy in range(0, 34):
+            for uz in range(0, 14):
+                n = (uz + 1) * (uy + 1) * (ux + 1)
+                ok = 2 <= ux <= 32 and 1 <= uy <= 64 // ux and 1 <= uz <= 12 and n <= 896
+                assert L.umx_up2_tile_rows(uz, uy, ux, buf) == (n if ok else 0)
+                if ok:
+                    seen += 1
+                    s, hx, hyx = np.arange(n), ux + 1, (ux + 1) * (uy + 1)
+                    assert np.array_equal(np.ctypeslib.as_array(buf)[:3 * n].reshape(n, 3), np.stack([s // hyx, s % hyx // hx, s % hx], 1)), (uz, uy, ux)
+    assert seen > 1000
+
+
 def test_no_cpu_fallback():
     """Without a B200 a compute entry must latch an error, not compute something."""
     import torch

@@ -109,6 +109,51 @@ def test_up2_fwd_mx(dev, xbits, ybits, gn, shape):
         assert bad == 0, "%d of %d bytes differ" % (bad, want.size)
 
 
+# the tiles whose last staged rows a reciprocal of 16 bits puts into the next plane
+@pytest.mark.parametrize("bits,tile,shape,gn", [(8, (10, 8, 8), (1, 32, 54, 54, 54), False), (4, (10, 8, 8), (1, 256, 36, 15, 28), False), (8, (9, 16, 4), (1, 160, 32, 31, 25), False),
+                                                (4, (9, 16, 4), (1, 160, 40, 30, 19), True), (8, (9, 4, 16), (1, 160, 32, 24, 30), True), (8, (10, 26, 2), (1, 160, 27, 25, 37), False),
+                                                (8, (10, 2, 26), (1, 320, 37, 21, 25), True)])
+def test_up2_tiles_of_many_rows(dev, bits, tile, shape, gn):
+    """grids whose tile stages 850 rows or more: every fine voxel is its own cell's.  The decoder form of the conv entry upsamples through the same kernel: the
+    conv of the upsampled tensor as a plain concat part"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf, Shape5, Gnp, Split
+    L = dev
+    N, Cn, D, H, W = shape
+    S, dt, G = D * H * W, 3 if bits == 8 else 4, 8
+    L.umx_up2_tile.restype, L.umx_up2_tile.argtypes = None, [C.c_int] * 3 + [C.c_size_t, C.c_int, C.c_void_p]
+    t = (C.c_int * 3)()
+    L.umx_up2_tile(D, H, W, N * Cn // 32, gn, t)
+    assert tuple(t) == tile
+    mx = orc.pm_to_mx((synth.rng(111).standard_normal(N * Cn * S) * 2).astype(f32), 0, N, Cn, S, bits)
+    dq = orc.mx_to_pm(mx, bits, N, Cn, S)
+    gp, keep = Gnp(), None
+    if gn:
+        pr = gn_params(112, N, Cn, G)
+        gp, keep = make_gp(G, pr)
+        dq = orc.gn_silu(dq, N, Cn, S, G, *pr, 1)
+    want = orc.pm_to_mx(orc.up2(dq, N, Cn, D, H, W), 0, N, Cn, 8 * S, bits)
+    xd, yd = DevBuf(data=mx), DevBuf(want.size).fill(0xEE)
+    L.lp_up2_fwd_mx(xd.ptr, dt, Shape5(N, Cn, D, H, W), yd.ptr, dt, gp)
+    ufsm_b200.check()
+    bad = np.count_nonzero(yd.download() != want)
+    assert bad <= (2e-4 * want.size if gn else 0), "%d of %d bytes differ" % (bad, want.size)      # with the activation as in test_up2_fwd_mx
+    if gn:
+        L.lp_up2_fwd_mx(xd.ptr, dt, Shape5(N, Cn, D, H, W), yd.ptr, dt, Gnp())
+    C2, Co, r = 32, 32, synth.rng(113)
+    x2 = DevBuf(data=np.concatenate([r.integers(0, 120, N * 8 * S * 4 * bits, dtype=np.uint8), r.integers(120, 130, N * 8 * S, dtype=np.uint8)]))
+    wd, bd = DevBuf(data=synth.kaiming(114, Co, Cn + C2, 27)), DevBuf(data=synth.bias(115, Co, 0.1))
+    fn, ys = L.lp_conv_fwd_f8 if bits == 8 else L.lp_conv_fwd_f4, []
+    for x, up in ((xd, 1), (yd, 0)):
+        sp = Split()
+        sp.x2, sp.c_split, sp.up = x2.ptr, Cn, up
+        ys.append(DevBuf(N * Co * 8 * S * 2).fill(0xEE))
+        fn(x.ptr, dt, Shape5(N, Cn + C2, 2 * D, 2 * H, 2 * W), wd.ptr, bd.ptr, Co, ys[-1].ptr, 2, Gnp(), None, 0, sp)
+    ufsm_b200.check()
+    assert np.array_equal(ys[0].download(), ys[1].download())
+
+
 @pytest.mark.parametrize("bits,Ci,Co,N,h16,gn", [(8, 32, 7, 1, False, False), (4, 64, 16, 2, False, False), (8, 40, 3, 1, True, False), (8, 64, 32, 2, False, False), (8, 64, 7, 2, False, True), (4, 96, 10, 1, False, True),
                                                    (8, 16, 7, 2, False, False), (4, 8, 3, 1, True, True)])          # rows of 16 / 8 channels
 def test_conv1_fwd_mx(dev, bits, Ci, Co, N, h16, gn):
