@@ -572,6 +572,37 @@ def test_weights_without_a_key_may_change_between_calls(dev):
         assert np.array_equal(g.download(), wnt)
 
 
+@pytest.mark.parametrize("bits,Ci,Co", [(8, 32, 32), (4, 64, 96), (8, 96, 160)])
+def test_weights_written_by_the_kernel_before(dev, bits, Ci, Co):
+    """a conv without split_t.wkey whose weights and bias another kernel of the library (lp_mx8_to_f32, which lets its successor start early) has just
+    written: eight sets in one buffer, queued without a wait, against handles made from the same values"""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf, Shape5, Gnp, Split
+    D, H, W, n, r = 2, 8, 16, Ci * 27, synth.rng(701)
+    S = D * H * W
+    codes = r.integers(0, 256, (8, Co * n), dtype=np.uint8)
+    codes[(codes & 0x7f) == 0x7f] = 0                        # no NaN codes
+    sets = [DevBuf(data=np.concatenate([c, r.integers(122, 126, Co // 32 * n, dtype=np.uint8)])) for c in codes]
+    bcodes = [DevBuf(data=np.concatenate([r.integers(0, 120, Co, dtype=np.uint8), np.full(Co // 32, 120, np.uint8)])) for _ in codes]
+    mx = orc.pm_to_mx(synth.act_h16(702, Ci * S), 2, 1, Ci, S, bits, 32)
+    xd, wd, bd = DevBuf(data=mx), DevBuf(Co * n * 4).fill(0), DevBuf(Co * 4).fill(0)
+    ys = [DevBuf(Co * S * 2).fill(0xEE) for _ in codes]
+    fn = dev.lp_conv_fwd_f8 if bits == 8 else dev.lp_conv_fwd_f4
+    ufsm_b200.check()
+    for s, t, y in zip(sets, bcodes, ys):
+        dev.lp_mx8_to_f32(t.ptr, 1, Co, 1, bd.ptr)
+        dev.lp_mx8_to_f32(s.ptr, 1, Co, n, wd.ptr)
+        fn(xd.ptr, 3 if bits == 8 else 4, Shape5(1, Ci, D, H, W), wd.ptr, bd.ptr, Co, y.ptr, 2, Gnp(), None, 0, Split())
+    ufsm_b200.check()
+    for s, t, y in zip(sets, bcodes, ys):
+        dev.lp_mx8_to_f32(t.ptr, 1, Co, 1, bd.ptr)
+        dev.lp_mx8_to_f32(s.ptr, 1, Co, n, wd.ptr)
+        ufsm_b200.check()
+        c = G.Conv("conv3", wd.download(np.float32), bd.download(np.float32), Co, Ci, bits)
+        assert np.array_equal(y.download(), c.fwd(mx, 1, D, H, W, G.OUT_PM16)[0])
+        c.free()
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("N,Cn,D,H,W", [(1, 32, 4, 8, 8), (2, 64, 5, 7, 9), (1, 96, 2, 2, 2), (1, 320, 8, 8, 8), (3, 32, 10, 10, 10), (1, 64, 16, 16, 16), (2, 32, 12, 20, 16), (1, 128, 17, 16, 16),
                                         (1, 32, 32, 32, 32), (2, 64, 24, 24, 24), (1, 32, 42, 60, 60), (1, 96, 48, 32, 32), (5, 32, 20, 20, 20),

@@ -18,14 +18,14 @@ __global__ void __launch_bounds__(128) prep_w27_k(const PrepArgs p, const RImage
     constexpr int CI = BITS == 8 ? 32 : 64, RUN = CI * 27;
     __shared__ float sm[4][RUN];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x, ki = blockIdx.y * 4 + warp;
-    if (blockIdx.y == 0 && threadIdx.x == 0 && p.bias_p) p.bias_p[row] = (p.bias && row < p.co) ? p.bias[row] : 0.f;
+    if (blockIdx.y == 0 && threadIdx.x == 0 && p.bias_p) p.bias_p[row] = (p.bias && row < p.co) ? ld_dep(p.bias + row) : 0.f;
     const int nitem = (p.ci + CI - 1) / CI;                   /* K items a tap */
     if (ki >= nitem) return;
     float *s = sm[warp];
     const int have = row < p.co ? min(CI, p.ci - ki * CI) * 27 : 0;
     const float *src = p.w + ((size_t)row * p.ci + (size_t)ki * CI) * 27;
 #pragma unroll 9
-    for (int i = lane; i < RUN; i += 32) s[i] = i < have ? __ldg(src + i) : 0.f;
+    for (int i = lane; i < RUN; i += 32) s[i] = i < have ? ld_dep(src + i) : 0.f;      /* the caller's weights may come from the kernel just ahead */
     __syncwarp();
     if (lane >= 27) return;
     const int tap = lane;
