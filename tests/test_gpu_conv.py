@@ -637,6 +637,32 @@ def test_norm_in_one_launch(dev, bits, N, Cn, D, H, W):
                 assert np.array_equal(got2.download(), want2.download())
 
 
+@pytest.mark.parametrize("sms,wait", [(148, 0), (296, 0), (500, 200000)])
+@pytest.mark.parametrize("bits,N,Cn,D,H,W,s2d", [(8, 1, 32, 24, 20, 22, True), (4, 2, 64, 32, 32, 32, False), (8, 1, 64, 40, 44, 48, True), (4, 1, 32, 84, 84, 85, False)])
+def test_norm_in_one_launch_rests_on_no_residency(dev, sms, wait, bits, N, Cn, D, H, W, s2d):
+    """blocks that do not wait (all but a group's last leave their rows to it) or that wait in turn because there are more of them than fit the device: the bytes of
+    the two-launch path, three times in a row on the same counters, and then the plain call"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S, nb, rb = D * H * W, Cn // 32, 32 * bits // 8 + 1
+    sig = [C.c_void_p] + [C.c_int] * 5 + [C.c_float, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int]
+    on, fn = dev.umx_in_norm_apply_on, dev.umx_in_norm_apply
+    on.restype, on.argtypes, fn.restype, fn.argtypes = C.c_int, sig + [C.c_int, C.c_longlong], C.c_int, sig
+    yd, pd, cd = DevBuf(data=synth.act_h16(511, N * Cn * S)), DevBuf(dev.umx_stats_doubles(N, Cn, D, H, W) * 8), DevBuf(N * Cn * 8)
+    want, want2, got, got2 = (DevBuf(N * nb * S * rb) for _ in range(4))
+    dev.umx_in_stats_coef(yd.ptr, N, Cn, D, H, W, None, None, 1e-5, pd.ptr, cd.ptr)
+    dev.umx_in_apply(yd.ptr, cd.ptr, N, Cn, D, H, W, 2, want.ptr, bits, 0, 0, want2.ptr if s2d else None, None, 1)
+    for k in range(4):
+        got.fill(0xEE), got2.fill(0xEE)
+        args = (yd.ptr, N, Cn, D, H, W, 1e-5, 2, pd.ptr, got.ptr, bits, 0, 0, got2.ptr if s2d else None, 1)
+        assert (on(*args, sms, wait) if k < 3 else fn(*args)) == 0
+        ufsm_b200.check()
+        assert np.array_equal(got.download(), want.download()), k
+        if s2d:
+            assert np.array_equal(got2.download(), want2.download()), k
+
+
 @pytest.mark.parametrize("kind,N,Ci,Co,D,H,W,bits", [("tconv2", 1, 32, 24, 1, 4, 4, 8), ("tconv2", 2, 64, 32, 3, 16, 7, 8), ("tconv2", 1, 64, 40, 2, 8, 13, 8), ("tconv2", 1, 32, 96, 5, 9, 16, 4),
                                                      ("tconv2", 1, 64, 32, 16, 16, 16, 4), ("down2", 1, 32, 32, 3, 16, 5, 8), ("down2", 2, 64, 96, 4, 12, 7, 8), ("conv1", 1, 32, 7, 3, 16, 9, 8),
                                                      ("conv1", 2, 64, 8, 1, 16, 1, 4), ("conv1", 1, 32, 33, 9, 16, 8, 8)])

@@ -343,13 +343,19 @@ extern "C" void umx_in_apply(const void *x, const float *coef, int N, int C, int
    take two launches: read again in one launch they were no faster (32 channels x 128^3 87 us against 79).
    Two launches are each a chain of a load, a reduction and a store behind a device-wide wait, which is what bounds them on the deep levels and on
    small patches: 8^3 x 320 channels 10 us, 16^3 x 256 14, 32^3 x 128 16, with the space-to-depth copy 26; in one launch 5.5, 7, 9 and 11.
-   Blocks wait for one another through the counter only when the launch has at most one block a multiprocessor: they are all resident once the
-   kernels before them have drained, and no later kernel of the stream starts before all of them have (pdl_trigger).  (Clusters do not give
-   that: of 36 clusters of eight that the occupancy query allows, 32 were scheduled.)  The wait is bounded all the same.  Sums are fp64 in a
-   fixed order: rows of a thread, row phases, blocks. ---- */
+   A launch has at most one block a multiprocessor, so its blocks are resident together once the kernels before them have drained, and the wait at the
+   counter is short.  Nothing rests on that (another process may hold part of the device): a block that has waited for kNormWait leaves its rows to
+   whichever block of its group arrives last, which by then waits for nobody, and ends.  Every block therefore ends, and the result is the same
+   either way.  (A cooperative launch, which guarantees residency, cannot overlap the end of its predecessor: 4 us for the four of the 32^3
+   three-level network, 19 for the eight of the 96^3 four-level one, where this form costs nothing.  Clusters do not give it: of 36 clusters of
+   eight that the occupancy query allows, 32 were scheduled.)  Sums are fp64 in a fixed order: rows of a thread, row phases, blocks. ---- */
 namespace {
-__device__ unsigned g_norm_count[2 * 4096];                  /* per (sample, block): blocks that have left their sums, blocks that have seen them all (the last one clears both) */
-struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl; unsigned vp; double *part; int *err; };      /* vp: voxels of a block's trip, NT / 4 to NT; cl: blocks of a cluster, all B of them, or 1 */
+constexpr int kNormBlocks = 1024, kNormPart = 512;            /* blocks of a launch that meet through the counter, at most; of a (sample, block), which is the room in part */
+constexpr long long kNormWait = 200000;                      /* clock cycles (0.1 ms) */
+/* per (sample, block): blocks that have left their sums | blocks that have left their rows << 16; blocks that need neither word any more (the last one clears both) */
+__device__ unsigned g_norm_count[2 * 4096];
+__device__ unsigned g_norm_left[kNormBlocks];                /* per (sample, block): 1 + rank of the blocks that have left their rows, zero between launches */
+struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl; unsigned vp; long long wait; double *part; int *err; };      /* vp: voxels of a block's trip, NT / 4 to NT; cl: blocks of a cluster, all B of them, or 1 */
 
 template <int BITS, bool S2D, int ROWS, int NT, bool STASH>
 __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
@@ -364,8 +370,10 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
     const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
     const unsigned S = a.S, vp = a.vp, step = vp * (unsigned)B, K = (S + step - 1) / step, g = (unsigned)(n * nb + blk);
     const uint4 *xp = a.x + ((size_t)n * nb + blk) * S * 4 + qd;
-    /* row u of this thread in trip k of its block; S where there is none */
-    auto vox = [&](unsigned k, int u) { const unsigned v = k * step + (unsigned)rank * vp + (unsigned)PH * u + (unsigned)ph; return k < K && (unsigned)PH * u < vp && v < S ? v : S; };
+    /* row u of this thread in trip k of block r; S where there is none */
+    auto vox_of = [&](int r, unsigned k, int u) { const unsigned v = k * step + (unsigned)r * vp + (unsigned)PH * u + (unsigned)ph; return k < K && (unsigned)PH * u < vp && v < S ? v : S; };
+    auto vox = [&](unsigned k, int u) { return vox_of(rank, k, u); };
+    unsigned left = 0;                                       /* blocks of the group whose rows are this block's to do as well */
     pdl_wait();
     uint4 raw[ROWS];
     {
@@ -427,19 +435,31 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         double *part = a.part + (size_t)g * B * 64;
         if (threadIdx.x < 64) { __stcg(part + rank * 64 + threadIdx.x, mine[threadIdx.x]); __threadfence(); }
         __syncthreads();
+        __shared__ unsigned others;
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(&g_norm_count[2 * g], 1u);
-            const long long t0 = clock64();
-            unsigned seen;
-            for (;;) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&g_norm_count[2 * g]) : "memory");
-                if (seen >= (unsigned)B) break;
-                if (clock64() - t0 > 4000000000ll) { if (atomicCAS(a.err, 0, 10) == 0) { a.err[1] = (int)blockIdx.x; a.err[2] = (int)seen; } break; }
+            unsigned *cnt = &g_norm_count[2 * g], w = atomicAdd(cnt, 1u) + 1u, rest = 0u;
+            if ((w & 0xffffu) == (unsigned)B) rest = w >> 16;         /* the last to arrive: nobody leaves rows behind after this */
+            else {
+                const long long t0 = clock64();
+                for (;;) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(w) : "l"(cnt) : "memory");
+                    if ((w & 0xffffu) == (unsigned)B) break;
+                    if (clock64() - t0 < a.wait) continue;
+                    if (atomicCAS(cnt, w, w + 0x10000u) == w) {       /* not all here: the rows are the last block's */
+                        asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(&g_norm_left[g * B + (w >> 16)]), "r"((unsigned)rank + 1u) : "memory");
+                        rest = ~0u;
+                        break;
+                    }
+                }
             }
-            if (atomicAdd(&g_norm_count[2 * g + 1], 1u) == (unsigned)B - 1u) { g_norm_count[2 * g] = 0u; g_norm_count[2 * g + 1] = 0u; }
+            __threadfence();
+            if (atomicAdd(&cnt[1], 1u) == (unsigned)B - 1u) { cnt[0] = 0u; cnt[1] = 0u; }
+            others = rest;
         }
         __syncthreads();
+        left = others;
+        if (left == ~0u) return;
         double t = 0.0;
 #pragma unroll 4
         for (int k = grp; k < B; k += GR) t += __ldcg(part + k * 64 + (which << 5) + c);
@@ -475,6 +495,27 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         }
     }
     if (CL > 1) cluster_wait();
+    for (unsigned i = 0; i < left; i++) {                    /* rows of blocks that could not wait; read again */
+        __shared__ unsigned whose;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned r = 0u;                                 /* the block has announced itself and writes its rank next */
+            const long long t0 = clock64();
+            while (!r && clock64() - t0 < 4000000000ll) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(r) : "l"(&g_norm_left[g * B + i]) : "memory");
+            if (!r && atomicCAS(a.err, 0, 10) == 0) { a.err[1] = (int)blockIdx.x; a.err[2] = (int)i; }
+            g_norm_left[g * B + i] = 0u;
+            whose = r;
+        }
+        __syncthreads();
+        const int r = (int)whose - 1;
+        for (unsigned k = 0; r >= 0 && k < K; k++) {
+            uint4 x4[4], o[4]; unsigned v[4], w0[4], w1[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) { v[u] = vox_of(r, k, u); x4[u] = v[u] < S ? ld_dep(xp + (size_t)v[u] * 4) : make_uint4(0u, 0u, 0u, 0u); }
+            const unsigned sb = apply4<BITS, true, true>(x4, ca, cb, slope, mask, qd, o, w0, w1);
+            dst.put4(v, vox_of(r, k, qd), S, w0, w1, sb);
+        }
+    }
 }
 /* whether clusters of 16 blocks of a variant can be launched, looked up once per device */
 template <int BITS, bool S2D, int ROWS, int NT> bool norm_sixteen() {
@@ -513,7 +554,7 @@ template <int BITS, bool S2D> bool norm_go_stash(NormArgs &a, int B, int nb, int
     umx_launch(in_norm_k<BITS, S2D, 8, 512, true>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3(512), (size_t)kept * 4 * 512 * 16, a);
     return true;
 }
-template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N) {
+template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N, int sms) {
     const size_t S = a.S;
     /* a cluster a group while a thread of it has at most four (eight) rows */
     if (S <= 256) return norm_go<BITS, S2D, 4, 256>(a, 1, 1, nb, N);
@@ -521,31 +562,41 @@ template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N) {
     if (S <= 4096 && norm_sixteen<BITS, S2D, 4, 256>()) return norm_go<BITS, S2D, 4, 256>(a, 16, 16, nb, N);
     if (S <= 4096) return norm_go<BITS, S2D, 8, 256>(a, 8, 8, nb, N);
     /* one block a multiprocessor, dealt to the groups, each of at most 1024 voxels in registers and 3072 in shared memory */
-    static int sms_of[16];
-    int d = 0; cudaGetDevice(&d); d &= 15;
-    if (!sms_of[d]) { int v = 1; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d); sms_of[d] = v; }
-    long long B = sms_of[d] / ((long long)nb * N);
+    if (sms > kNormBlocks) sms = kNormBlocks;
+    long long B = sms / ((long long)nb * N);
     const long long most = (long long)((S + 127) / 128);    /* a row a thread */
     if (B > most) B = most;
+    if (B > kNormPart) B = kNormPart;
     if (B < 1 || (size_t)B * (2 + kStashTrips) * 512 < S) return false;
     if ((size_t)B * 1024 < S) return norm_go_stash<BITS, S2D>(a, (int)B, nb, N);
     return (size_t)B * 512 >= S ? norm_go<BITS, S2D, 4, 512>(a, (int)B, 1, nb, N) : norm_go<BITS, S2D, 8, 512>(a, (int)B, 1, nb, N);
 }
 }   // namespace
-/* statistics, coefficients (gamma 1, beta 0) and apply of a blocked fp16 tensor of a multiple of 32 channels in one launch; part: scratch of
-   umx_stats_doubles doubles.  Launches on one device must not overlap (they share the counters).  1: not this tensor; the caller takes
-   umx_in_stats_coef and umx_in_apply. */
-extern "C" int umx_in_norm_apply(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout) {
+/* umx_in_norm_apply dealt out for sms multiprocessors, its blocks waiting for one another for `wait` clock cycles */
+extern "C" int umx_in_norm_apply_on(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout, int sms, long long wait) {
     const size_t S = (size_t)D * H * W;
     if (!umx_ready("umx_in_norm_apply") || !S || !N || (C & 31) || S >= (size_t)1 << 31 || !q || (q_s2d && ((D | H | W) & 1)) || (long long)N * (C / 32) > 4096) return 1;
     NormArgs a; memset(&a, 0, sizeof a);
     a.x = (const uint4 *)x; a.H = H; a.W = W; a.S = (unsigned)S; a.eps = eps; a.act = act; a.q = (uint8_t *)q; a.nb_dst = nb_dst ? nb_dst : C / 32; a.b0 = nb_dst ? b0 : 0;
-    a.q2 = (uint8_t *)q_s2d; a.split = layout == UMX_LAYOUT_SPLIT; a.part = part; a.err = umx_errflag();
+    a.q2 = (uint8_t *)q_s2d; a.split = layout == UMX_LAYOUT_SPLIT; a.wait = wait; a.part = part; a.err = umx_errflag();
     if (!a.err) return -1;
-    const bool done = bits == 8 ? (q_s2d ? norm_pick<8, true>(a, C / 32, N) : norm_pick<8, false>(a, C / 32, N)) : (q_s2d ? norm_pick<4, true>(a, C / 32, N) : norm_pick<4, false>(a, C / 32, N));
+    const bool done = bits == 8 ? (q_s2d ? norm_pick<8, true>(a, C / 32, N, sms) : norm_pick<8, false>(a, C / 32, N, sms)) : (q_s2d ? norm_pick<4, true>(a, C / 32, N, sms) : norm_pick<4, false>(a, C / 32, N, sms));
     if (!done) return 1;
     g_umx_launches++;
     UMX_CK("umx_in_norm_apply");
     return 0;
 }
-void umx_norm_counts_reset(void) { void *p = nullptr; if (cudaGetSymbolAddress(&p, g_norm_count) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 2 * 4096); }
+/* statistics, coefficients (gamma 1, beta 0) and apply of a blocked fp16 tensor of a multiple of 32 channels in one launch; part: scratch of
+   umx_stats_doubles doubles.  Launches on one device must not overlap (they share the counters).  1: not this tensor; the caller takes
+   umx_in_stats_coef and umx_in_apply. */
+extern "C" int umx_in_norm_apply(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout) {
+    static int sms_of[16];
+    int d = 0; cudaGetDevice(&d); d &= 15;
+    if (!sms_of[d]) { int v = 1; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d); sms_of[d] = v; }
+    return umx_in_norm_apply_on(x, N, C, D, H, W, eps, act, part, q, bits, nb_dst, b0, q_s2d, layout, sms_of[d], kNormWait);
+}
+void umx_norm_counts_reset(void) {
+    void *p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_norm_count) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 2 * 4096);
+    if (cudaGetSymbolAddress(&p, g_norm_left) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * kNormBlocks);
+}
