@@ -101,6 +101,41 @@ def test_upsample_tile_rows_are_exact():
     assert seen > 1000
 
 
+def test_norm_plan_keeps_a_sample_its_own():
+    """the one-launch norm: what fixes the order of a sample's sums (the shares, their trips, the voxels of a trip) does not depend on the batch, every share has
+    its block, and a launch has at most one block a multiprocessor and as many trips as a block can hold"""
+    L = ufsm_b200.lib()
+    L.umx_norm_plan.restype, L.umx_norm_plan.argtypes = None, [C.c_size_t] + [C.c_int] * 4 + [C.c_void_p]
+    out, r, seen = (C.c_int * 8)(), np.random.default_rng(3), set()
+
+    def plan(*a):
+        L.umx_norm_plan(*a, out)
+        return tuple(out)
+    sizes = [1, 255, 256, 257, 1024, 1025, 4096, 4097, 8000, 16 ** 3, 24 ** 3, 32 ** 3, 64 ** 3, 148 * 4096, 148 * 4096 + 1, 96 ** 3] + [int(2 ** r.uniform(0, 21)) for _ in range(300)]
+    for S in sizes:
+        for nb in (1, 2, 3, 4, 8, 10, 74, 148, 149):
+            for sms in (148, 132, 20, 600):
+                one = plan(S, nb, 1, sms, 1)
+                assert one[0] == (1 if S <= 4096 or min(sms // nb, 511) * 4096 >= S else 0)
+                for N in (1, 2, 3, 4, 5, 7, 16, 200):
+                    held, blocks, cl, ranks, per, vp, trips, most = plan(S, nb, N, sms, 1)
+                    assert (held == 0) == (one[0] == 0)
+                    if not held:
+                        continue
+                    assert (ranks, vp, trips) == (one[3], one[5], one[6]) and ranks * vp * trips >= S
+                    if S <= 4096:
+                        assert held == 1 and blocks == cl == ranks <= 16 and per == 1 and vp <= 256 and trips == most == 1
+                        continue
+                    assert cl == 1 and vp == 512 and ranks <= 511 and (ranks - 1) * vp < S
+                    seen.add((held, per > 1, most > 2))
+                    if held == 1:
+                        assert blocks * nb * N <= sms and blocks * per >= ranks and most <= 8 and per <= 4
+                        # the trips of each block, counted one by one
+                        count = np.bincount(np.arange(0, S, vp) // vp % ranks % blocks, minlength=blocks)
+                        assert count.max() == count[0] == most
+    assert {(1, False, False), (1, False, True), (1, True, False), (1, True, True)} <= seen and any(s[0] == 2 for s in seen)
+
+
 def test_no_cpu_fallback():
     """Without a B200 a compute entry must latch an error, not compute something."""
     import torch

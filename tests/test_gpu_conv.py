@@ -663,6 +663,34 @@ def test_norm_in_one_launch_rests_on_no_residency(dev, sms, wait, bits, N, Cn, D
             assert np.array_equal(got2.download(), want2.download()), k
 
 
+# shares of one trip and of several, one to four of them a block; batches that take two launches (32 and 64 channels x 64^3); a cluster (16^3)
+@pytest.mark.parametrize("bits,N,Cn,D,H,W,s2d", [(8, 4, 32, 32, 32, 32, True), (4, 3, 96, 20, 24, 28, True), (8, 3, 32, 64, 64, 64, False), (4, 2, 64, 64, 64, 64, True), (8, 5, 32, 17, 19, 23, False), (4, 3, 64, 16, 16, 16, True)])
+def test_norm_of_a_sample_is_its_own(dev, bits, N, Cn, D, H, W, s2d):
+    """values of 40 binary orders, whose fp64 sums round: partial sums, codes and scales of each sample of a batch are those of the sample alone"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S, nb, rb, r = D * H * W, Cn // 32, 32 * bits // 8, synth.rng(521)
+    fn, plan, out = dev.umx_in_norm_apply, dev.umx_norm_plan, (C.c_int * 8)()
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p] + [C.c_int] * 5 + [C.c_float, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int]
+    plan.restype, plan.argtypes = None, [C.c_size_t] + [C.c_int] * 4 + [C.c_void_p]
+    plan(S, nb, N, 148, 1, out)
+    y = (r.standard_normal(N * Cn * S) * np.exp2(r.integers(-24, 13, N * Cn * S))).astype(np.float16).reshape(N, -1)
+
+    def run(v, n):
+        yd, pd = DevBuf(data=v), DevBuf(dev.umx_stats_doubles(n, Cn, D, H, W) * 8).fill(0)
+        q, q2 = DevBuf(n * nb * S * (rb + 1)).fill(0xEE), DevBuf(n * nb * S * (rb + 1)).fill(0xEE)
+        assert fn(yd.ptr, n, Cn, D, H, W, 1e-5, 2, pd.ptr, q.ptr, bits, 0, 0, q2.ptr if s2d else None, 1) == 0
+        ufsm_b200.check()
+        sums = pd.download(np.uint64)[:n * nb * out[3] * 64].reshape(n, -1)
+        parts = [q.download()[:n * nb * S * rb], q.download()[n * nb * S * rb:], q2.download()[:n * nb * S * rb], q2.download()[n * nb * S * rb:]]
+        return [sums] + [p.reshape(n, -1) for p in parts]
+    whole = run(y, N)
+    for n in range(N):
+        for got, want in zip(whole, run(y[n], 1)):
+            assert np.array_equal(got[n], want[0])
+
+
 @pytest.mark.parametrize("kind,N,Ci,Co,D,H,W,bits", [("tconv2", 1, 32, 24, 1, 4, 4, 8), ("tconv2", 2, 64, 32, 3, 16, 7, 8), ("tconv2", 1, 64, 40, 2, 8, 13, 8), ("tconv2", 1, 32, 96, 5, 9, 16, 4),
                                                      ("tconv2", 1, 64, 32, 16, 16, 16, 4), ("down2", 1, 32, 32, 3, 16, 5, 8), ("down2", 2, 64, 96, 4, 12, 7, 8), ("conv1", 1, 32, 7, 3, 16, 9, 8),
                                                      ("conv1", 2, 64, 8, 1, 16, 1, 4), ("conv1", 1, 32, 33, 9, 16, 8, 8)])

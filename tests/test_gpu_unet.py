@@ -56,6 +56,19 @@ def test_unet_batch_and_determinism(dev):
     u.free()
 
 
+@pytest.mark.parametrize("P,cw,bits", [(32, [32, 64, 128], (8, 8, 8)), (64, [32, 64], (8, 4, 8))])
+def test_unet_batch_on_grids_whose_norms_meet_in_memory(dev, P, cw, bits):
+    """batches of 2 to 4 patches large enough that the blocks of a norm meet through global memory: each patch's logits are those of the patch alone"""
+    x = np.stack([ct_patch(21 + i, P ** 3) for i in range(4)])
+    u = G.Unet(G.make_cfg(P, cw, 7, bits), synth.unet_weights(22, cw), 4)
+    alone = [u.forward(v, 1) for v in x]
+    for N in (2, 3, 4):
+        got = u.forward(x[:N].reshape(-1), N).reshape(N, -1)
+        for i in range(N):
+            assert np.array_equal(got[i], alone[i])
+    u.free()
+
+
 def test_unet_queued_host_entry(dev):
     """umx_unet_submit_host / umx_unet_wait: five patches in flight through the two slots give the bytes of the synchronous entry."""
     import ctypes as C

@@ -348,94 +348,133 @@ extern "C" void umx_in_apply(const void *x, const float *coef, int N, int C, int
    whichever block of its group arrives last, which by then waits for nobody, and ends.  Every block therefore ends, and the result is the same
    either way.  (A cooperative launch, which guarantees residency, cannot overlap the end of its predecessor: 4 us for the four of the 32^3
    three-level network, 19 for the eight of the 96^3 four-level one, where this form costs nothing.  Clusters do not give it: of 36 clusters of
-   eight that the occupancy query allows, 32 were scheduled.)  Sums are fp64 in a fixed order: rows of a thread, row phases, blocks. ---- */
+   eight that the occupancy query allows, 32 were scheduled.)  Sums are fp64 in a fixed order: rows of a thread, row phases, shares.  The shares are those of
+   a launch with one sample, whatever the batch (norm_plan), so a sample's bytes are its own: a block of a launch with several samples does several shares one
+   after the other (MULTI), and a batch that is too much for one launch takes the same sums in a launch of their own (in_share_k) and in_apply_k. ---- */
 namespace {
-constexpr int kNormBlocks = 1024, kNormPart = 512;            /* blocks of a launch that meet through the counter, at most; of a (sample, block), which is the room in part */
+/* blocks of a launch that meet through the counter, at most; shares of a (sample, block), for which part has room and for the coefficients; shares of a block, for which shared memory has */
+constexpr int kNormBlocks = 1024, kNormPart = 511, kNormPer = 4;
 constexpr long long kNormWait = 200000;                      /* clock cycles (0.1 ms) */
 /* per (sample, block): blocks that have left their sums | blocks that have left their rows << 16; blocks that need neither word any more (the last one clears both) */
 __device__ unsigned g_norm_count[2 * 4096];
 __device__ unsigned g_norm_left[kNormBlocks];                /* per (sample, block): 1 + rank of the blocks that have left their rows, zero between launches */
-struct NormArgs { const uint4 *x; int H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl; unsigned vp; long long wait; double *part; int *err; };      /* vp: voxels of a block's trip, NT / 4 to NT; cl: blocks of a cluster, all B of them, or 1 */
+/* ranks: shares of a (sample, block), of which a block takes rank, rank + B, ...; vp: voxels of a share's trip, NT / 4 to NT; step: of all shares' together; trips: of
+   a share at most; cl: blocks of a cluster, all B of them, or 1 */
+struct NormArgs { const uint4 *x; int N, H, W; unsigned S; float eps; int act; uint8_t *q; int nb_dst, b0; uint8_t *q2; int split; int cl, ranks; unsigned vp, step, trips; long long wait; double *part; int *err; };
 
-template <int BITS, bool S2D, int ROWS, int NT, bool STASH>
+/* The trips of a block, NT voxels (four rows a thread) each: those of its first share, of the next, ...  Trip k of share r begins at voxel k step + r vp; trips past
+   the end of the tensor are not there (they come last in a share, and every share has a first one). */
+constexpr unsigned kNoTrip = 0x80000000u;
+struct NormTrips {
+    unsigned v, k, r;                                        /* first voxel of the trip, kNoTrip when there are no more; number in its share; share */
+    __device__ __forceinline__ NormTrips(const NormArgs &a, unsigned rank) : v(rank * a.vp), k(0u), r(rank) {}
+    __device__ __forceinline__ void next(const NormArgs &a, unsigned B) {
+        k++;
+        v += a.step;
+        if (k == a.trips || v >= a.S) { k = 0u; r += B; v = r < (unsigned)a.ranks ? r * a.vp : kNoTrip; }
+    }
+};
+/* A warp's sums of one share into shared memory, as [sum or sum of squares][channel].  The lanes that hold the same channels halve what they hold three
+   times, each keeping one half and adding what the other held of it: no barrier, and a sixteenth of the shared memory traffic of 16 doubles a thread.  With it
+   and shares of 512 voxels or more 32 channels x 32^3 take 6.8 us (8.2 before), 64 x 64^3 17.8 (18.7), and a second share a block costs 32 x 64^3 x 2 samples
+   0.8 us of 19.5; with a barrier and the wide form it cost 4. */
+__device__ __forceinline__ void warp_sums(const StatAcc &acc, double *to) {
+    const int lane = threadIdx.x & 31;
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) { const bool up = lane & 16; const double o = __shfl_xor_sync(0xffffffffu, up ? acc.s[k] : acc.q[k], 16); v[k] = (up ? acc.q[k] : acc.s[k]) + o; }
+#pragma unroll
+    for (int k = 0; k < 4; k++) { const bool up = lane & 8; const double o = __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + 4], 8); v[k] = (up ? v[k + 4] : v[k]) + o; }
+#pragma unroll
+    for (int k = 0; k < 2; k++) { const bool up = lane & 4; const double o = __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + 2], 4); v[k] = (up ? v[k + 2] : v[k]) + o; }
+    *(double2 *)&to[((lane >> 4) << 5) + (lane & 3) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2] = make_double2(v[0], v[1]);
+}
+/* the n rows of place threadIdx.x & 63, added in order */
+template <int N> __device__ __forceinline__ double rows_sum(const double (*red)[64]) {
+    double t = red[0][threadIdx.x & 63];
+#pragma unroll
+    for (int k = 1; k < N; k++) t += red[k][threadIdx.x & 63];
+    return t;
+}
+/* the sums of all shares, on the first 64 threads */
+template <int NT> __device__ __forceinline__ double shares_sum(const double *part, int ranks, double (*red)[64]) {
+    double t = 0.0;
+#pragma unroll 4
+    for (int k = threadIdx.x >> 6; k < ranks; k += NT / 64) t += __ldcg(part + k * 64 + (threadIdx.x & 63));
+    red[threadIdx.x >> 6][threadIdx.x & 63] = t;
+    __syncthreads();
+    return threadIdx.x < 64 ? rows_sum<NT / 64>(red) : 0.0;
+}
+template <int BITS, bool S2D, int ROWS, int NT, bool STASH, bool MULTI>
 __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
     pdl_trigger();
-    constexpr int PH = NT / 4, GR = NT / 64;
-    __shared__ double ss[64][33], sq[64][33];
+    constexpr int PH = NT / 4, NW = NT / 32;
+    __shared__ __align__(16) double red[MULTI ? kNormPer : 1][NW][64];
     __shared__ double mine[64];
     __shared__ float2 sc[32];
     extern __shared__ __align__(16) uint8_t stash_raw[];
     uint4 *stash = (uint4 *)stash_raw + threadIdx.x;           /* STASH: [row of a thread][thread] */
-    const int N = gridDim.z, nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, B = gridDim.x, rank = blockIdx.x, CL = a.cl;
-    const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
-    const unsigned S = a.S, vp = a.vp, step = vp * (unsigned)B, K = (S + step - 1) / step, g = (unsigned)(n * nb + blk);
+    const int nb = gridDim.y, blk = blockIdx.y, n = blockIdx.z, B = gridDim.x, rank = blockIdx.x, CL = a.cl;
+    const int qd = threadIdx.x & 3, ph = threadIdx.x >> 2, warp = threadIdx.x >> 5;
+    const unsigned S = a.S, g = blockIdx.z * (unsigned)nb + (unsigned)blk;
     const uint4 *xp = a.x + ((size_t)n * nb + blk) * S * 4 + qd;
-    /* row u of this thread in trip k of block r; S where there is none */
-    auto vox_of = [&](int r, unsigned k, int u) { const unsigned v = k * step + (unsigned)r * vp + (unsigned)PH * u + (unsigned)ph; return k < K && (unsigned)PH * u < vp && v < S ? v : S; };
-    auto vox = [&](unsigned k, int u) { return vox_of(rank, k, u); };
+    double *part = a.part + (size_t)(n * nb + blk) * a.ranks * 64;
     unsigned left = 0;                                       /* blocks of the group whose rows are this block's to do as well */
+    StatAcc acc;
+    stat_zero(acc);
     pdl_wait();
     uint4 raw[ROWS];
-    {
-        StatAcc acc;
-        stat_zero(acc);
-        auto load4 = [&](uint4 *r, unsigned k) {
+    unsigned at[ROWS / 4];                                   /* where the trips in raw begin */
+    bool turn[ROWS / 4];                                     /* MULTI: the trip begins another share */
+    NormTrips tr(a, (unsigned)rank);
+    unsigned kept = 0;                                       /* rows of a thread that wait in shared memory: those before the ones in registers */
+    int cur = 0;                                             /* the block's share that is being added up */
+    /* voxel of this thread's row u of the trip that begins at v; S or more: none */
+    auto vox = [&](unsigned v, int u) { return NT == 512 || (unsigned)(PH * u) < a.vp ? v + (unsigned)(PH * u + ph) : S; };
+    auto load4 = [&](uint4 *r, unsigned v) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) { const unsigned v = vox(k, u); r[u] = v < S ? ld_dep(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
-        };
-        unsigned kr = 0;                                     /* the trips before those in registers wait in shared memory */
-        if (STASH) {
-            for (; kr + ROWS / 4 < K; kr += ROWS / 4) {
-#pragma unroll
-                for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, kr + k);
-#pragma unroll
-                for (int u = 0; u < ROWS; u++) { stat_add(acc, raw[u]); stash[(size_t)(kr * 4 + u) * NT] = raw[u]; }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < ROWS / 4; k++) load4(raw + 4 * k, kr + k);
-#pragma unroll
-        for (int u = 0; u < ROWS; u++) stat_add(acc, raw[u]);
-        if (PH > 64) {                                       /* 128 row phases: two neighbouring ones together */
-#pragma unroll
-            for (int k = 0; k < 8; k++) { acc.s[k] += __shfl_xor_sync(0xffffffffu, acc.s[k], 4); acc.q[k] += __shfl_xor_sync(0xffffffffu, acc.q[k], 4); }
-        }
-        const int row = PH > 64 ? ph >> 1 : ph;
-        if (PH <= 64 || !(ph & 1)) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) { ss[row][qd * 8 + k] = acc.s[k]; sq[row][qd * 8 + k] = acc.q[k]; }
-        }
-    }
-    __syncthreads();
-    const int c = threadIdx.x & 31, which = (threadIdx.x >> 5) & 1, grp = threadIdx.x >> 6;
-    double (*src)[33] = which ? sq : ss;
-    /* GR partial sums a (channel, sum), one of each thread, added in order by the first 64 threads */
-    auto groups = [&](double t, double *dst) {
-        __syncthreads();
-        src[grp][c] = t;
-        __syncthreads();
-        if (threadIdx.x < 64) { double v = src[0][c]; for (int k = 1; k < GR; k++) v += src[k][c]; dst[threadIdx.x] = v; }
+        for (int u = 0; u < 4; u++) { const unsigned w = vox(v, u); r[u] = w < S ? ld_dep(xp + (size_t)w * 4) : make_uint4(0u, 0u, 0u, 0u); }      /* rows past the end add zeros */
     };
-    {
-        double t = 0.0;
+    auto load = [&]() {
 #pragma unroll
-        for (int k = 0; k < 64 / GR; k++) t += src[grp * (64 / GR) + k][c];
-        groups(t, mine);
+        for (int k = 0; k < ROWS / 4; k++) {
+            at[k] = tr.v; turn[k] = MULTI && !tr.k && tr.v != kNoTrip && kept + k;
+            load4(raw + 4 * k, tr.v);
+            if (tr.v != kNoTrip) tr.next(a, (unsigned)B);
+        }
+    };
+    load();
+    if (STASH) while (tr.v != kNoTrip) {
+#pragma unroll
+        for (int u = 0; u < ROWS; u++) {
+            if (MULTI && !(u & 3) && turn[u / 4]) { warp_sums(acc, red[cur++][warp]); stat_zero(acc); }
+            stat_add(acc, raw[u]);
+            stash[(size_t)(kept + u) * NT] = raw[u];
+        }
+        kept += ROWS;
+        load();
     }
+#pragma unroll
+    for (int u = 0; u < ROWS; u++) {
+        if (MULTI && !(u & 3) && turn[u / 4]) { warp_sums(acc, red[cur++][warp]); stat_zero(acc); }
+        stat_add(acc, raw[u]);
+    }
+    warp_sums(acc, red[cur][warp]);
+    __syncthreads();
+    double tot = 0.0;                                        /* of the first 64 threads: over all shares */
     if (CL > 1) {                                            /* the blocks are a cluster */
+        if (threadIdx.x < 64) mine[threadIdx.x] = rows_sum<NW>(red[0]);
         cluster_sync_all();
-        double t = 0.0;
         if (threadIdx.x < 64) {
-            const uint32_t at = smem_u32(mine) + threadIdx.x * 8;
-            for (int r = 0; r < CL; r++) t += cluster_ldd(cluster_addr(at, (uint32_t)r));
+            const uint32_t at0 = smem_u32(mine) + threadIdx.x * 8;
+            for (int r = 0; r < CL; r++) tot += cluster_ldd(cluster_addr(at0, (uint32_t)r));
         }
         cluster_arrive();                                    /* no block's memory is read after this; everyone waits for everyone before leaving */
-        if (threadIdx.x < 64) ss[which][c] = t;
     } else if (B > 1) {
-        double *part = a.part + (size_t)g * B * 64;
-        if (threadIdx.x < 64) { __stcg(part + rank * 64 + threadIdx.x, mine[threadIdx.x]); __threadfence(); }
-        __syncthreads();
+        const int j = threadIdx.x >> 6;                      /* 64 threads a share */
+        if (j <= cur) { __stcg(part + (rank + j * B) * 64 + (threadIdx.x & 63), rows_sum<NW>(red[j])); __threadfence(); }
         __shared__ unsigned others;
+        __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             unsigned *cnt = &g_norm_count[2 * g], w = atomicAdd(cnt, 1u) + 1u, rest = 0u;
@@ -460,38 +499,34 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
         __syncthreads();
         left = others;
         if (left == ~0u) return;
-        double t = 0.0;
-#pragma unroll 4
-        for (int k = grp; k < B; k += GR) t += __ldcg(part + k * 64 + (which << 5) + c);
-        groups(t, mine);
-        __syncthreads();
-        if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x];
-    } else { __syncthreads(); if (threadIdx.x < 64) ss[which][c] = mine[threadIdx.x]; }
+        tot = shares_sum<NT>(part, a.ranks, red[0]);
+    } else if (threadIdx.x < 64) tot = rows_sum<NW>(red[0]);
+    if (threadIdx.x < 64) red[0][0][threadIdx.x] = tot;
     __syncthreads();
-    if (threadIdx.x < 32) sc[c] = coef_of(ss[0][c], ss[1][c], (double)S, a.eps, nullptr, nullptr, 0);
+    if (threadIdx.x < 32) sc[threadIdx.x] = coef_of(red[0][0][threadIdx.x], red[0][0][32 + threadIdx.x], (double)S, a.eps, nullptr, nullptr, 0);
     __syncthreads();
     float2 ca[4], cb[4]; unsigned mask[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) { const float2 p = sc[qd * 8 + 2 * k], r = sc[qd * 8 + 2 * k + 1]; ca[k] = make_float2(p.x, r.x); cb[k] = make_float2(p.y, r.y); mask[k] = 0xffffffffu; }
     const float slope = a.act == 2 ? 0.01f : 1.f;
-    const MxDst<BITS, S2D> dst(a.q, a.q2, N, nb, n, blk, a.nb_dst, a.b0, S, a.H, a.W, a.split, qd);
-    auto put = [&](const uint4 *r, unsigned k) {             /* the four rows of trip k */
+    const MxDst<BITS, S2D> dst(a.q, a.q2, a.N, nb, n, blk, a.nb_dst, a.b0, S, a.H, a.W, a.split, qd);
+    auto put = [&](const uint4 *r, unsigned w) {             /* the four rows of the trip that begins at w */
         uint4 o[4]; unsigned v[4], w0[4], w1[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = vox(k, u);
+        for (int u = 0; u < 4; u++) v[u] = vox(w, u);
         const unsigned sb = apply4<BITS, true, true>(r, ca, cb, slope, mask, qd, o, w0, w1);
-        dst.put4(v, vox(k, qd), S, w0, w1, sb);
+        dst.put4(v, vox(w, qd), S, w0, w1, sb);
     };
-    unsigned kr = 0;
-    if (STASH) while (kr + ROWS / 4 < K) kr += ROWS / 4;
 #pragma unroll
-    for (int k = 0; k < ROWS / 4; k++) put(raw + 4 * k, kr + k);
+    for (int k = 0; k < ROWS / 4; k++) if (at[k] != kNoTrip) put(raw + 4 * k, at[k]);
     if (STASH) {
-        for (unsigned k = 0; k < kr; k++) {
+        NormTrips w(a, (unsigned)rank);
+        for (unsigned k = 0; k < kept; k += 4) {
             uint4 r[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) r[u] = stash[(size_t)(k * 4 + u) * NT];
-            put(r, k);
+            for (int u = 0; u < 4; u++) r[u] = stash[(size_t)(k + u) * NT];
+            put(r, w.v);
+            w.next(a, (unsigned)B);
         }
     }
     if (CL > 1) cluster_wait();
@@ -507,22 +542,53 @@ __global__ void __launch_bounds__(NT) in_norm_k(const NormArgs a) {
             whose = r;
         }
         __syncthreads();
-        const int r = (int)whose - 1;
-        for (unsigned k = 0; r >= 0 && k < K; k++) {
-            uint4 x4[4], o[4]; unsigned v[4], w0[4], w1[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) { v[u] = vox_of(r, k, u); x4[u] = v[u] < S ? ld_dep(xp + (size_t)v[u] * 4) : make_uint4(0u, 0u, 0u, 0u); }
-            const unsigned sb = apply4<BITS, true, true>(x4, ca, cb, slope, mask, qd, o, w0, w1);
-            dst.put4(v, vox_of(r, k, qd), S, w0, w1, sb);
+        if (!whose) continue;
+        for (NormTrips w(a, whose - 1u); w.v != kNoTrip; w.next(a, (unsigned)B)) {
+            uint4 r[4];
+            load4(r, w.v);
+            put(r, w.v);
         }
     }
+}
+/* The statistics alone, for a batch that is more than one launch holds: a block a share, the sums and their order those of in_norm_k; the block of a (sample,
+   block) that comes last makes the coefficients.  The last sample comes first: it is what the conv before left in L2.  With the apply 64 channels x 64^3 x 2
+   samples take 32.0 us, 35.5 with in_part_k, 40.4 in one launch a sample. */
+__global__ void __launch_bounds__(512, 2) in_share_k(const NormArgs a, float2 *coef) {
+    pdl_trigger();
+    __shared__ __align__(16) double red[16][64];
+    __shared__ unsigned last;
+    const int nb = gridDim.y, blk = blockIdx.y, n = gridDim.z - 1 - blockIdx.z, rank = blockIdx.x, qd = threadIdx.x & 3, ph = threadIdx.x >> 2;
+    const unsigned S = a.S, g = (unsigned)(n * nb + blk);
+    const uint4 *xp = a.x + (size_t)g * S * 4 + qd;
+    double *part = a.part + (size_t)g * a.ranks * 64;
+    StatAcc acc;
+    stat_zero(acc);
+    pdl_wait();
+    for (NormTrips tr(a, (unsigned)rank); tr.v != kNoTrip; tr.next(a, (unsigned)a.ranks)) {
+        uint4 r[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) { const unsigned v = tr.v + 128u * u + (unsigned)ph; r[u] = v < S ? ld_dep(xp + (size_t)v * 4) : make_uint4(0u, 0u, 0u, 0u); }
+#pragma unroll
+        for (int u = 0; u < 4; u++) stat_add(acc, r[u]);
+    }
+    warp_sums(acc, red[threadIdx.x >> 5]);
+    __syncthreads();
+    if (threadIdx.x < 64) { __stcg(part + rank * 64 + threadIdx.x, rows_sum<16>(red)); __threadfence(); }
+    __syncthreads();
+    if (threadIdx.x == 0) { last = atomicAdd(&g_norm_count[2 * g], 1u) == (unsigned)a.ranks - 1u; if (last) g_norm_count[2 * g] = 0u; __threadfence(); }
+    __syncthreads();
+    if (!last) return;
+    const double tot = shares_sum<512>(part, a.ranks, red);
+    if (threadIdx.x < 64) red[0][threadIdx.x] = tot;
+    __syncthreads();
+    if (threadIdx.x < 32) coef[(size_t)g * 32 + threadIdx.x] = coef_of(red[0][threadIdx.x], red[0][32 + threadIdx.x], (double)S, a.eps, nullptr, nullptr, 0);
 }
 /* whether clusters of 16 blocks of a variant can be launched, looked up once per device */
 template <int BITS, bool S2D, int ROWS, int NT> bool norm_sixteen() {
     static int have[16];
     int d = 0; cudaGetDevice(&d); d &= 15;
     if (!have[d]) {
-        const void *k = (const void *)in_norm_k<BITS, S2D, ROWS, NT, false>;
+        const void *k = (const void *)in_norm_k<BITS, S2D, ROWS, NT, false, false>;
         cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
         cudaLaunchAttribute at; memset(&at, 0, sizeof at);
         at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = 16; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
@@ -534,54 +600,80 @@ template <int BITS, bool S2D, int ROWS, int NT> bool norm_sixteen() {
     }
     return have[d] > 0;
 }
-template <int BITS, bool S2D, int ROWS, int NT> bool norm_go(NormArgs &a, int B, int cl, int nb, int N) {
-    a.cl = cl;
-    /* small tensors: fewer rows a thread */
-    a.vp = (size_t)B * NT > a.S ? (unsigned)(((size_t)a.S + B * (NT / 4) - 1) / ((size_t)B * (NT / 4))) * (NT / 4) : NT;
-    umx_launch_cluster(in_norm_k<BITS, S2D, ROWS, NT, false>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3((unsigned)cl, 1, 1), dim3(NT), 0, a);
-    return true;
-}
 /* one block a multiprocessor that keeps eight rows a thread in registers and up to kStashTrips x 4 more in shared memory (they come to 226 KB with the sums) */
 constexpr int kStashTrips = 6;
-template <int BITS, bool S2D> bool norm_go_stash(NormArgs &a, int B, int nb, int N) {
-    const void *k = (const void *)in_norm_k<BITS, S2D, 8, 512, true>;
+/* How a tensor is dealt out.  ranks, vp and trips (of a share, at most), which fix the order of the sums, follow from one sample; per (shares of a block, at
+   most), blocks and all (trips of a block, at most) from the batch.  held 0: not in this form, 1: in one launch, 2: one sample would be, the batch takes
+   in_share_k and in_apply_k */
+struct NormPlan { int held, blocks, cl, ranks, per, vp, trips, all; };
+NormPlan norm_plan(size_t S, int nb, int N, int sms, bool sixteen) {
+    NormPlan p = {1, 1, 1, 1, 1, 256, 1, 1};
+    if (S <= 4096) {                                         /* a block, or a cluster while a thread of it has at most four (eight) rows */
+        p.blocks = p.cl = p.ranks = S <= 256 ? 1 : S <= 1024 || !sixteen ? 8 : 16;
+        if ((size_t)p.ranks * 256 > S) p.vp = (int)((S + p.ranks * 64 - 1) / (size_t)(p.ranks * 64)) * 64;
+        p.trips = (int)((S + (size_t)p.ranks * p.vp - 1) / ((size_t)p.ranks * p.vp));
+        p.all = p.trips;
+        return p;
+    }
+    /* one block a multiprocessor, dealt to the (sample, block) pairs, each of at most 1024 voxels in registers and 3072 in shared memory */
+    if (sms > kNormBlocks) sms = kNormBlocks;
+    long long r = sms / nb;
+    if (r > kNormPart) r = kNormPart;
+    if (r < 1 || (size_t)r * (2 + kStashTrips) * 512 < S) { p.held = 0; return p; }
+    p.vp = 512;
+    p.trips = (int)((S + (size_t)r * 512 - 1) / ((size_t)r * 512));
+    /* no share without a voxel; a multiple of four where that does not cost a trip (it deals out well to two and four samples) */
+    p.ranks = p.trips == 1 ? (int)((S + 511) / 512) : (size_t)(r & ~3ll) * 512 * p.trips >= S ? (int)(r & ~3ll) : (int)r;
+    /* trips of the first block, which has most: of a share all but the last, and that one where it begins before the end */
+    const int fit = sms / (nb * N);
+    p.held = 2;
+    if (fit < 1) return p;
+    p.per = (p.ranks + fit - 1) / fit; p.blocks = (p.ranks + p.per - 1) / p.per; p.all = 0;
+    for (int s = 0; s < p.ranks; s += p.blocks) p.all += p.trips - (((long long)(p.trips - 1) * p.ranks + s) * 512 >= (long long)S);
+    if (p.per <= kNormPer && p.all <= 2 + kStashTrips) p.held = 1;
+    return p;
+}
+template <int BITS, bool S2D, int ROWS, int NT> void norm_go(const NormArgs &a, int B, int nb) {
+    umx_launch_cluster(in_norm_k<BITS, S2D, ROWS, NT, false, false>, dim3((unsigned)B, (unsigned)nb, (unsigned)a.N), dim3((unsigned)a.cl, 1, 1), dim3(NT), 0, a);
+}
+template <int BITS, bool S2D, bool MULTI> bool norm_go_wide(const NormArgs &a, const NormPlan &p, int nb) {
+    const dim3 grid((unsigned)p.blocks, (unsigned)nb, (unsigned)a.N);
+    const int kept = (p.all - 1) / 2 * 2;                     /* trips in shared memory, two in registers */
+    if (!kept) { umx_launch(in_norm_k<BITS, S2D, 8, 512, false, MULTI>, grid, dim3(512), 0, a); return true; }
     static int set[16];
     int d = 0; cudaGetDevice(&d); d &= 15;
-    if (!set[d]) set[d] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kStashTrips * 4 * 512 * 16) == cudaSuccess ? 1 : -1;
+    if (!set[d]) set[d] = cudaFuncSetAttribute((const void *)in_norm_k<BITS, S2D, 8, 512, true, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStashTrips * 4 * 512 * 16) == cudaSuccess ? 1 : -1;
     if (set[d] < 0) { cudaGetLastError(); return false; }
-    a.cl = 1; a.vp = 512;
-    const unsigned trips = (unsigned)(((size_t)a.S + (size_t)B * 512 - 1) / ((size_t)B * 512)), kept = (trips - 1) / 2 * 2;
-    umx_launch(in_norm_k<BITS, S2D, 8, 512, true>, dim3((unsigned)B, (unsigned)nb, (unsigned)N), dim3(512), (size_t)kept * 4 * 512 * 16, a);
+    umx_launch(in_norm_k<BITS, S2D, 8, 512, true, MULTI>, grid, dim3(512), (size_t)kept * 4 * 512 * 16, a);
     return true;
 }
-template <int BITS, bool S2D> bool norm_pick(NormArgs &a, int nb, int N, int sms) {
-    const size_t S = a.S;
-    /* a cluster a group while a thread of it has at most four (eight) rows */
-    if (S <= 256) return norm_go<BITS, S2D, 4, 256>(a, 1, 1, nb, N);
-    if (S <= 1024) return norm_go<BITS, S2D, 4, 256>(a, 8, 8, nb, N);
-    if (S <= 4096 && norm_sixteen<BITS, S2D, 4, 256>()) return norm_go<BITS, S2D, 4, 256>(a, 16, 16, nb, N);
-    if (S <= 4096) return norm_go<BITS, S2D, 8, 256>(a, 8, 8, nb, N);
-    /* one block a multiprocessor, dealt to the groups, each of at most 1024 voxels in registers and 3072 in shared memory */
-    if (sms > kNormBlocks) sms = kNormBlocks;
-    long long B = sms / ((long long)nb * N);
-    const long long most = (long long)((S + 127) / 128);    /* a row a thread */
-    if (B > most) B = most;
-    if (B > kNormPart) B = kNormPart;
-    if (B < 1 || (size_t)B * (2 + kStashTrips) * 512 < S) return false;
-    if ((size_t)B * 1024 < S) return norm_go_stash<BITS, S2D>(a, (int)B, nb, N);
-    return (size_t)B * 512 >= S ? norm_go<BITS, S2D, 4, 512>(a, (int)B, 1, nb, N) : norm_go<BITS, S2D, 8, 512>(a, (int)B, 1, nb, N);
+/* 1: in one launch; 2: the caller launches in_share_k and the apply; 0: not this tensor */
+template <int BITS, bool S2D> int norm_pick(NormArgs &a, int nb, int sms) {
+    const NormPlan p = norm_plan(a.S, nb, a.N, sms, a.S > 1024 && a.S <= 4096 && norm_sixteen<BITS, S2D, 4, 256>());
+    a.cl = p.cl; a.ranks = p.ranks; a.vp = (unsigned)p.vp; a.step = (unsigned)(p.ranks * p.vp); a.trips = (unsigned)p.trips;
+    if (p.held != 1) return p.held;
+    if (a.S <= 4096) { if (p.trips == 1) norm_go<BITS, S2D, 4, 256>(a, p.blocks, nb); else norm_go<BITS, S2D, 8, 256>(a, p.blocks, nb); return 1; }
+    if (p.all == 1) { norm_go<BITS, S2D, 4, 512>(a, p.blocks, nb); return 1; }
+    return p.per > 1 ? norm_go_wide<BITS, S2D, true>(a, p, nb) : norm_go_wide<BITS, S2D, false>(a, p, nb);
 }
 }   // namespace
+/* the plan of a tensor: held, blocks, cluster, shares, shares a block, voxels a trip, trips a share, trips a block */
+extern "C" void umx_norm_plan(size_t S, int nb, int N, int sms, int sixteen, int *out) { const NormPlan p = norm_plan(S, nb, N, sms, sixteen != 0); memcpy(out, &p, sizeof p); }
 /* umx_in_norm_apply dealt out for sms multiprocessors, its blocks waiting for one another for `wait` clock cycles */
 extern "C" int umx_in_norm_apply_on(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout, int sms, long long wait) {
     const size_t S = (size_t)D * H * W;
     if (!umx_ready("umx_in_norm_apply") || !S || !N || (C & 31) || S >= (size_t)1 << 31 || !q || (q_s2d && ((D | H | W) & 1)) || (long long)N * (C / 32) > 4096) return 1;
     NormArgs a; memset(&a, 0, sizeof a);
-    a.x = (const uint4 *)x; a.H = H; a.W = W; a.S = (unsigned)S; a.eps = eps; a.act = act; a.q = (uint8_t *)q; a.nb_dst = nb_dst ? nb_dst : C / 32; a.b0 = nb_dst ? b0 : 0;
+    a.x = (const uint4 *)x; a.N = N; a.H = H; a.W = W; a.S = (unsigned)S; a.eps = eps; a.act = act; a.q = (uint8_t *)q; a.nb_dst = nb_dst ? nb_dst : C / 32; a.b0 = nb_dst ? b0 : 0;
     a.q2 = (uint8_t *)q_s2d; a.split = layout == UMX_LAYOUT_SPLIT; a.wait = wait; a.part = part; a.err = umx_errflag();
     if (!a.err) return -1;
-    const bool done = bits == 8 ? (q_s2d ? norm_pick<8, true>(a, C / 32, N, sms) : norm_pick<8, false>(a, C / 32, N, sms)) : (q_s2d ? norm_pick<4, true>(a, C / 32, N, sms) : norm_pick<4, false>(a, C / 32, N, sms));
-    if (!done) return 1;
+    const int form = bits == 8 ? (q_s2d ? norm_pick<8, true>(a, C / 32, sms) : norm_pick<8, false>(a, C / 32, sms)) : (q_s2d ? norm_pick<4, true>(a, C / 32, sms) : norm_pick<4, false>(a, C / 32, sms));
+    if (!form) return 1;
+    if (form == 2) {
+        float2 *coef = (float2 *)(part + (size_t)N * (C / 32) * a.ranks * 64);      /* behind the sums: a place of 64 doubles a (sample, block) is left */
+        umx_launch(in_share_k, dim3((unsigned)a.ranks, (unsigned)(C / 32), (unsigned)N), dim3(512), 0, a, coef);
+        umx_in_apply(x, (const float *)coef, N, C, D, H, W, act, q, bits, nb_dst, b0, q_s2d, nullptr, layout);      /* counts itself */
+    }
     g_umx_launches++;
     UMX_CK("umx_in_norm_apply");
     return 0;
