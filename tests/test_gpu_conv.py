@@ -691,6 +691,26 @@ def test_norm_of_a_sample_is_its_own(dev, bits, N, Cn, D, H, W, s2d):
             assert np.array_equal(got[n], want[0])
 
 
+@pytest.mark.parametrize("N,D,H,W", [(4101, 2, 3, 2), (4101, 17, 16, 16)])
+def test_norm_of_more_samples_than_counters(dev, N, D, H, W):
+    """more than 4096 (sample, block) pairs, in a cluster a pair and in two launches: the codes and scales of the sample alone, for every sample"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S, bits = D * H * W, 4
+    fn = dev.umx_in_norm_apply
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p] + [C.c_int] * 5 + [C.c_float, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int]
+    y = synth.act_h16(531, 32 * S)
+
+    def run(n):
+        yd, pd, q = DevBuf(data=np.tile(y, n)), DevBuf(dev.umx_stats_doubles(n, 32, D, H, W) * 8), DevBuf(n * S * 17)
+        assert fn(yd.ptr, n, 32, D, H, W, 1e-5, 2, pd.ptr, q.ptr, bits, 0, 0, None, 1) == 0
+        ufsm_b200.check()
+        return q.download()
+    one, many = run(1), run(N)
+    assert (many[:N * S * 16].reshape(N, -1) == one[:S * 16]).all() and (many[N * S * 16:].reshape(N, -1) == one[S * 16:]).all()
+
+
 @pytest.mark.parametrize("kind,N,Ci,Co,D,H,W,bits", [("tconv2", 1, 32, 24, 1, 4, 4, 8), ("tconv2", 2, 64, 32, 3, 16, 7, 8), ("tconv2", 1, 64, 40, 2, 8, 13, 8), ("tconv2", 1, 32, 96, 5, 9, 16, 4),
                                                      ("tconv2", 1, 64, 32, 16, 16, 16, 4), ("down2", 1, 32, 32, 3, 16, 5, 8), ("down2", 2, 64, 96, 4, 12, 7, 8), ("conv1", 1, 32, 7, 3, 16, 9, 8),
                                                      ("conv1", 2, 64, 8, 1, 16, 1, 4), ("conv1", 1, 32, 33, 9, 16, 8, 8)])

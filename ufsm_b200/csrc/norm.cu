@@ -352,11 +352,12 @@ extern "C" void umx_in_apply(const void *x, const float *coef, int N, int C, int
    a launch with one sample, whatever the batch (norm_plan), so a sample's bytes are its own: a block of a launch with several samples does several shares one
    after the other (MULTI), and a batch that is too much for one launch takes the same sums in a launch of their own (in_share_k) and in_apply_k. ---- */
 namespace {
-/* blocks of a launch that meet through the counter, at most; shares of a (sample, block), for which part has room and for the coefficients; shares of a block, for which shared memory has */
-constexpr int kNormBlocks = 1024, kNormPart = 511, kNormPer = 4;
+/* blocks of a launch that meet through the counter, at most; shares of a (sample, block), for which part has room and for the coefficients; shares of a block, for which shared memory has; (sample,
+   block) pairs that meet */
+constexpr int kNormBlocks = 1024, kNormPart = 511, kNormPer = 4, kNormPairs = 4096;
 constexpr long long kNormWait = 200000;                      /* clock cycles (0.1 ms) */
 /* per (sample, block): blocks that have left their sums | blocks that have left their rows << 16; blocks that need neither word any more (the last one clears both) */
-__device__ unsigned g_norm_count[2 * 4096];
+__device__ unsigned g_norm_count[2 * kNormPairs];
 __device__ unsigned g_norm_left[kNormBlocks];                /* per (sample, block): 1 + rank of the blocks that have left their rows, zero between launches */
 /* ranks: shares of a (sample, block), of which a block takes rank, rank + B, ...; vp: voxels of a share's trip, NT / 4 to NT; step: of all shares' together; trips: of
    a share at most; cl: blocks of a cluster, all B of them, or 1 */
@@ -662,7 +663,7 @@ extern "C" void umx_norm_plan(size_t S, int nb, int N, int sms, int sixteen, int
 /* umx_in_norm_apply dealt out for sms multiprocessors, its blocks waiting for one another for `wait` clock cycles */
 extern "C" int umx_in_norm_apply_on(const void *x, int N, int C, int D, int H, int W, float eps, int act, double *part, void *q, int bits, int nb_dst, int b0, void *q_s2d, int layout, int sms, long long wait) {
     const size_t S = (size_t)D * H * W;
-    if (!umx_ready("umx_in_norm_apply") || !S || !N || (C & 31) || S >= (size_t)1 << 31 || !q || (q_s2d && ((D | H | W) & 1)) || (long long)N * (C / 32) > 4096) return 1;
+    if (!umx_ready("umx_in_norm_apply") || !S || !N || (C & 31) || S >= (size_t)1 << 31 || !q || (q_s2d && ((D | H | W) & 1)) || C / 32 > kNormPairs) return 1;
     NormArgs a; memset(&a, 0, sizeof a);
     a.x = (const uint4 *)x; a.N = N; a.H = H; a.W = W; a.S = (unsigned)S; a.eps = eps; a.act = act; a.q = (uint8_t *)q; a.nb_dst = nb_dst ? nb_dst : C / 32; a.b0 = nb_dst ? b0 : 0;
     a.q2 = (uint8_t *)q_s2d; a.split = layout == UMX_LAYOUT_SPLIT; a.wait = wait; a.part = part; a.err = umx_errflag();
@@ -671,7 +672,12 @@ extern "C" int umx_in_norm_apply_on(const void *x, int N, int C, int D, int H, i
     if (!form) return 1;
     if (form == 2) {
         float2 *coef = (float2 *)(part + (size_t)N * (C / 32) * a.ranks * 64);      /* behind the sums: a place of 64 doubles a (sample, block) is left */
-        umx_launch(in_share_k, dim3((unsigned)a.ranks, (unsigned)(C / 32), (unsigned)N), dim3(512), 0, a, coef);
+        const int nb = C / 32, most = kNormPairs / nb;        /* samples a launch: a counter a (sample, block) */
+        for (int n = 0; n < N; n += most) {
+            NormArgs b = a;
+            b.x += (size_t)n * nb * S * 4; b.part += (size_t)n * nb * a.ranks * 64;
+            umx_launch(in_share_k, dim3((unsigned)a.ranks, (unsigned)nb, (unsigned)(N - n < most ? N - n : most)), dim3(512), 0, b, coef + (size_t)n * C);
+        }
         umx_in_apply(x, (const float *)coef, N, C, D, H, W, act, q, bits, nb_dst, b0, q_s2d, nullptr, layout);      /* counts itself */
     }
     g_umx_launches++;
@@ -689,6 +695,6 @@ extern "C" int umx_in_norm_apply(const void *x, int N, int C, int D, int H, int 
 }
 void umx_norm_counts_reset(void) {
     void *p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_norm_count) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 2 * 4096);
+    if (cudaGetSymbolAddress(&p, g_norm_count) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * 2 * kNormPairs);
     if (cudaGetSymbolAddress(&p, g_norm_left) == cudaSuccess && p) cudaMemset(p, 0, sizeof(unsigned) * kNormBlocks);
 }
