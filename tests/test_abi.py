@@ -101,6 +101,23 @@ def test_upsample_tile_rows_are_exact():
     assert seen > 1000
 
 
+def test_upsample_tile_is_the_cheapest():
+    """the upsample's tile search skips what cannot win: the tile, and the one of equals, that a look at every tile finds (cost model of up2_tile)"""
+    L = ufsm_b200.lib()
+    L.umx_up2_tile.restype, L.umx_up2_tile.argtypes = None, [C.c_int] * 3 + [C.c_size_t, C.c_int, C.c_void_p]
+    t = np.array([(x, y, z) for x in range(2, 33) for y in range(1, 64 // x + 1) for z in range(1, 13) if (x + 1) * (y + 1) * (z + 1) <= 896])
+    x, y, z = t.T
+    trips, r, out = ((x + 1) * (y + 1) * (z + 1) + 63) // 64, np.random.default_rng(4), (C.c_int * 3)()
+    grids = [(1, 1, 1), (2, 3, 5), (8, 8, 8), (48, 48, 48), (54, 54, 54), (128, 128, 128)] + [tuple(int(2 ** r.uniform(0, 8)) for _ in range(3)) for _ in range(400)]
+    for D, H, W in grids:
+        for nbk, gn in ((1, 0), (2, 1), (int(2 ** r.uniform(0, 8)), int(r.integers(2)))):
+            blocks = ((D + z) // z) * ((H + y) // y) * ((W + x) // x) * nbk
+            whole, rest = blocks // 296, blocks % 296
+            cost = (1000.0 + 800.0 * z + (150.0 if gn else 70.0) * trips) * (whole + np.where(rest == 0, 0.0, np.where(rest <= 148, 0.65, 1.0)))
+            L.umx_up2_tile(D, H, W, nbk, gn, out)
+            assert tuple(out) == tuple(int(v) for v in t[np.argmin(cost)][::-1]), (D, H, W, nbk, gn)
+
+
 def test_norm_plan_keeps_a_sample_its_own():
     """the one-launch norm: what fixes the order of a sample's sums (the shares, their trips, the voxels of a trip) does not depend on the batch, every share has
     its block, and a launch has at most one block a multiprocessor and as many trips as a block can hold"""
