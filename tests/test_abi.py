@@ -153,6 +153,17 @@ def test_norm_plan_keeps_a_sample_its_own():
     assert {(1, False, False), (1, False, True), (1, True, False), (1, True, True)} <= seen and any(s[0] == 2 for s in seen)
 
 
+def test_zeroing_kernel_only_on_the_devices_own_memory():
+    """nn_zero takes its kernel for 16-byte pieces of the current device's memory (type 2) alone; another device's (which need not be mapped), pinned (1), managed
+    (3) and unregistered (0) memory go to memset"""
+    L = ufsm_b200.lib()
+    f = L.umx_zero_by_kernel
+    f.restype, f.argtypes = C.c_int, [C.c_int, C.c_int, C.c_int, C.c_size_t, C.c_size_t]
+    assert f(2, 0, 0, 4096, 64) and f(2, 3, 3, 16, 16)
+    for other in [(2, 1, 0, 4096, 64), (2, 0, 1, 4096, 64), (1, 0, 0, 4096, 64), (3, 0, 0, 4096, 64), (0, -2, 0, 4096, 64), (2, 0, 0, 4104, 64), (2, 0, 0, 4096, 60), (2, 0, 0, 4096, 0)]:
+        assert not f(*other), other
+
+
 def test_no_cpu_fallback():
     """Without a B200 a compute entry must latch an error, not compute something."""
     import torch

@@ -155,3 +155,24 @@ def test_h16_pairs_of_voxels(dev, bits, N, Cn, S):
     assert np.array_equal(G.quantise_pm(x, 2, N, Cn, S, bits, wide32=True), want)
     assert np.array_equal(G.from_split(G.quantise_pm(x, 2, N, Cn, S, bits, wide32=True, layout=1), N, Cn, S, bits), want)
     assert np.array_equal(G.dequantise(want, bits, N, Cn, S), orc.mx_to_pm(want, bits, N, Cn, S), equal_nan=True)
+
+
+@pytest.mark.parametrize("shift,bytes_", [(0, 16), (0, 4096 * 16 * 148 + 16), (16, 4096), (4, 100), (0, 33), (0, 0)])
+def test_zero(dev, shift, bytes_):
+    """nn_zero on device memory (16-byte pieces, odd addresses and sizes, nothing) and on pinned host memory: those bytes and no others"""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    n = shift + bytes_ + 32
+    want = np.full(n, 0xEE, np.uint8)
+    want[shift:shift + bytes_] = 0
+    b = DevBuf(n).fill(0xEE)
+    dev.nn_zero(b.ptr + shift, bytes_)
+    assert np.array_equal(b.download(), want)
+    h = dev.nn_malloc_host(n)
+    v = np.ctypeslib.as_array(C.cast(h, C.POINTER(C.c_uint8)), (n,))
+    v[:] = 0xEE
+    dev.nn_zero(h + shift, bytes_)
+    ufsm_b200.check()
+    assert np.array_equal(v, want)
+    dev.nn_free_host(h)

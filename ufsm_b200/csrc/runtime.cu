@@ -54,21 +54,28 @@ extern "C" void *nn_malloc(size_t bytes) {
     return p;
 }
 extern "C" void nn_free(void *p) { if (p) cudaFree(p); }
-/* A kernel of the library's own launch chain (programmatic launch: it is scheduled while its predecessor drains) where memset would break the chain:
-   3.7 us between two kernels, 2 in this form.  Devices the library has no kernels for take memset. */
+/* A kernel of the library's own launch chain (programmatic launch: it is scheduled while its predecessor drains) where memset would break the chain, which
+   costs about 1 us.  Memory that is not the current device's own (another device's, which may not be mapped here, managed, host or unknown memory), odd
+   addresses and devices the library has no kernels for take memset. */
 __global__ void __launch_bounds__(256) zero_k(uint4 *p, size_t n) {
     pdl_trigger(); pdl_wait();
     for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
 }
+extern "C" int umx_zero_by_kernel(int memory_type, int memory_device, int device, size_t addr, size_t bytes) {
+    return memory_type == cudaMemoryTypeDevice && memory_device == device && !((addr | bytes) & 15) && bytes;
+}
 extern "C" void nn_zero(void *p, size_t bytes) {
     int d = -1;
-    if (!(((size_t)p | bytes) & 15) && bytes && cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 16 && g_ready[d] > 0) {
+    cudaPointerAttributes at; memset(&at, 0, sizeof at);
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();      /* memset says what it thinks of it */
+    if (cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 16 && g_ready[d] > 0 && umx_zero_by_kernel(at.type, at.device, d, (size_t)p, bytes)) {
         size_t g = (bytes / 16 + 255) / 256; if (g > 148u * 16u) g = 148u * 16u;
         umx_launch(zero_k, dim3((unsigned)g), dim3(256), 0, (uint4 *)p, bytes / 16);
         UMX_CK("nn_zero");
         return;
     }
-    cudaError_t e = cudaMemset(p, 0, bytes); if (e != cudaSuccess) umx_latch("nn_zero", e); }
+    cudaError_t e = cudaMemset(p, 0, bytes); if (e != cudaSuccess) umx_latch("nn_zero", e);
+}
 extern "C" void nn_h2d(void *dst, const void *src, size_t bytes) { cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice); if (e != cudaSuccess) umx_latch("nn_h2d", e); }
 extern "C" void nn_d2h(void *dst, const void *src, size_t bytes) { cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost); if (e != cudaSuccess) umx_latch("nn_d2h", e); }
 extern "C" void nn_sync(void) {
