@@ -53,12 +53,6 @@ __device__ __forceinline__ void raise_p(const ConvPArgs &a, volatile int *abort_
 /* n / d for n < 2^31: mul = ceil(2^(31 + l) / d), shift = l - 1 with l = ceil(log2 d) (Granlund and Montgomery, "Division by invariant integers using
    multiplication"); mul = 0 stands for d = 1 */
 __device__ __forceinline__ unsigned fast_div(unsigned n, unsigned mul, int shift) { return mul ? __umulhi(n, mul) >> shift : n; }
-/* two fp32 additions in one instruction, each rounded to nearest even */
-__device__ __forceinline__ float2 add2(float2 x, float2 y) {
-    float2 o;
-    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 r, p, q;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-    return o;
-}
 /* EPI: the output mode known at compile time (0: any, read from the arguments; 1: plane-major fp32; 2: plane-major fp16; 3: MX-fp8 split
    layout; 4: the same through the transposed conv's scatter; 5, 6: MX-fp4 likewise), so that the epilogue's code is only what that mode needs */
 template <int BITS, int EPI>
@@ -252,8 +246,8 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
                             const float4 b = __ldg(bp + k);
-                            const float2 s0 = add2(make_float2(__uint_as_float(rr[4 * k]), __uint_as_float(rr[4 * k + 1])), make_float2(b.x, b.y));
-                            const float2 s1 = add2(make_float2(__uint_as_float(rr[4 * k + 2]), __uint_as_float(rr[4 * k + 3])), make_float2(b.z, b.w));
+                            const float2 s0 = __fadd2_rn(make_float2(__uint_as_float(rr[4 * k]), __uint_as_float(rr[4 * k + 1])), make_float2(b.x, b.y));
+                            const float2 s1 = __fadd2_rn(make_float2(__uint_as_float(rr[4 * k + 2]), __uint_as_float(rr[4 * k + 3])), make_float2(b.z, b.w));
                             h[2 * k] = __floats2half2_rn(s0.x, s0.y); h[2 * k + 1] = __floats2half2_rn(s1.x, s1.y);
                         }
                         if (O8) sb[jc] = mx_encode_row32_h8(h, w[jc]);

@@ -153,17 +153,6 @@ extern "C" void umx_in_coef(const double *part, int N, int C, int D, int H, int 
 }
 
 
-/* two fp32 operations in one instruction, each rounded to nearest even */
-__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
-    float2 o;
-    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 r, {%6, %7};\n\tfma.rn.f32x2 r, p, q, r;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
-    return o;
-}
-__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
-    float2 o;
-    asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmul.rn.f32x2 r, p, q;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(o.x), "=f"(o.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-    return o;
-}
 /* Four lanes a row, eight channels a lane, four rows together: affine map, LeakyReLU, fp16 rounding (o), MX codes (w0, w1).  Returns the scale byte of row
    qd: the four rows' maxima are reduced so that each lane of the quad ends up with one row's, works that row's scale out and hands it to the other three.
    Instruction issue bounds the passes that call this where
@@ -182,8 +171,8 @@ __device__ __forceinline__ unsigned apply4(const uint4 *raw, const float2 *ca, c
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             float2 g = __half22float2(hp[k]);
-            if (COEF) g = fma2(g, ca[k], cb[k]);
-            const float2 l = mul2(sl, g);
+            if (COEF) g = __ffma2_rn(g, ca[k], cb[k]);
+            const float2 l = __fmul2_rn(sl, g);
             op[k] = __hmax2(__floats2half2_rn(g.x, g.y), __floats2half2_rn(l.x, l.y));
             if (!FULL) *(unsigned *)(op + k) &= mask[k];
         }
