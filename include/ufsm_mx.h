@@ -162,7 +162,7 @@ int umx_conv_fwd(const umx_conv *c, const void *x, int N, int D, int H, int W, v
    fp64 sums of the stored fp16 values and of their squares, which are exact for a sample of any realistic size, so the coefficients are
    those of the pass, whatever the batch, the number of multiprocessors or the way the planes fall to the blocks.  The epilogue's extra
    work (a conversion and two fp64 operations per element) costs more than the pass saves on the benchmark's layers (measured: the
-   level-0 conv goes from 72 to 120 us, the pass takes 33), which is why it is not the default. */
+   level-0 conv goes from 67 to 106 us, conv and pass together take 97), which is why it is not the default. */
 int umx_conv_fwd_norm(const umx_conv *c, const void *x, int N, int D, int H, int W, void *y, double *part, const float *gamma, const float *beta, float eps, float *coef, int flags);
 size_t umx_stats_doubles(int N, int co, int D, int H, int W);   /* size of part for a conv output on that grid */
 /* testing aid (no counterpart in the reference): at most `cap` thread blocks per column tile in the resident-weight 3^3 kernel (0: as many as

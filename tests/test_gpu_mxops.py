@@ -80,7 +80,7 @@ def test_slab_local_groupnorm_in_up2_and_conv1(dev, bits):
     assert orc.rel_l2(yd.download(f32).reshape(N, Co, S), want) < 1e-5
 
 
-# the second shape spans several tiles of the kernel on every axis (4 x 4 x 16 cells of the dual grid), with ragged last tiles
+# small grids, which choose tiles of one cell along z: several tiles along z and x (the first shape along every axis), with ragged last ones; tall tiles: test_up2_tiles_of_many_rows
 @pytest.mark.parametrize("shape", [(2, 40, 5, 3, 5, 7), (1, 64, 8, 6, 9, 35), (2, 16, 2, 3, 5, 7), (1, 8, 1, 2, 6, 5)])      # the last two: rows of 16 / 8 channels
 @pytest.mark.parametrize("xbits,ybits,gn", [(8, 8, False), (4, 4, False), (8, 4, False), (4, 8, False), (8, 8, True), (4, 4, True)])
 def test_up2_fwd_mx(dev, xbits, ybits, gn, shape):

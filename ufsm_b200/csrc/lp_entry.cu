@@ -322,7 +322,7 @@ static int conv_fwd(const char *fn, int bits, const void *x, int xbf, shape5 xs,
         const float *wc = w, *bc = b;
         if (pad_in || pad_out) {
             const size_t nw = (size_t)cout_c * cin * 27;
-            float *wp = (float *)umx_ws(5, (nw + cout_c) * sizeof(float));     /* slot 5 is also the general kernel's K-split scratch: the preparation reads it ahead of that kernel in the stream */
+            float *wp = (float *)umx_ws(5, (nw + cout_c) * sizeof(float));     /* read by the preparation alone, ahead of the conv in the stream */
             if (!wp) return 0;
             w_expand_k<<<(unsigned)((nw + 255) / 256), 256>>>(w, b, wp, wp + nw, cout, Ci, 27, pad_in ? Cx : Ci, pad_in ? up32(Cx) : Ci, cin, Ox, OxP, cout_c);
             wc = wp; bc = wp + nw;

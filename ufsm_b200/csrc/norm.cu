@@ -329,9 +329,9 @@ extern "C" void umx_in_apply(const void *x, const float *coef, int N, int C, int
 /* ---- statistics, coefficients and apply in one launch: what a conv of the U-Net is followed by.  B blocks share a (sample, 32-channel block).
    A block adds up its share of the voxels, the blocks' sums meet (small tensors: a cluster, through distributed shared memory; others: through
    global memory and a counter), and the values are transformed where they are, in registers (ROWS rows a thread).  Tensors too large for that
-   take two launches: read again in one launch they were no faster (32 channels x 128^3 87 us against 79).
+   take two launches (32 channels x 128^3 66.8 us); read again in one launch they were no faster (87 us against 79 for two at the time).
    Two launches are each a chain of a load, a reduction and a store behind a device-wide wait, which is what bounds them on the deep levels and on
-   small patches: 8^3 x 320 channels 10 us, 16^3 x 256 14, 32^3 x 128 16, with the space-to-depth copy 26; in one launch 5.5, 7, 9 and 11.
+   small patches: 8^3 x 320 channels 10.7 us, 16^3 x 256 11.0, 32^3 x 128 14.3, with the space-to-depth copy 16.5; in one launch 5.9, 5.7, 8.0 and 9.0.
    A launch has at most one block a multiprocessor, so its blocks are resident together once the kernels before them have drained, and the wait at the
    counter is short.  Nothing rests on that (another process may hold part of the device): a block that has waited for kNormWait leaves its rows to
    whichever block of its group arrives last, which by then waits for nobody, and ends.  Every block therefore ends, and the result is the same
