@@ -615,7 +615,7 @@ NormPlan norm_plan(size_t S, int nb, int N, int sms, bool sixteen) {
     /* no share without a voxel; a multiple of four where that does not cost a trip (it deals out well to two and four samples) */
     p.ranks = p.trips == 1 ? (int)((S + 511) / 512) : (size_t)(r & ~3ll) * 512 * p.trips >= S ? (int)(r & ~3ll) : (int)r;
     /* trips of the first block, which has most: of a share all but the last, and that one where it begins before the end */
-    const int fit = sms / (nb * N);
+    const int fit = (int)(sms / ((long long)nb * N));
     p.held = 2;
     if (fit < 1) return p;
     p.per = (p.ranks + fit - 1) / fit; p.blocks = (p.ranks + p.per - 1) / p.per; p.all = 0;
