@@ -168,7 +168,7 @@ size_t umx_stats_doubles(int N, int co, int D, int H, int W);   /* size of part 
 /* testing aid (no counterpart in the reference): at most `cap` thread blocks per column tile in the resident-weight 3^3 kernel (0: as many as
    the device holds), so that a small volume is cut into the several-planes-a-block pieces that otherwise only 64^3 and larger volumes see */
 void umx_conv_r_block_cap(int cap);
-int umx_conv_last_kernel(void);          /* which kernel the last umx_conv_fwd on this thread's process launched: 0 general, 1 resident-weight 3^3, 2 one-tap streaming, 3 tap-packed one-channel 3^3; -1 none yet */
+int umx_conv_last_kernel(void);          /* which kernel the last umx_conv_fwd on this thread's process launched: 0 general, 1 resident-weight 3^3, 2 one-tap streaming, 3 tap-packed one-channel 3^3, 4 resident-weight 3^3 stride 2; -1 none yet */
 /* coef [n][C][2] (device floats): a = gamma rstd, b = beta - mean a from the partial sums (k_in_coef, src/nn_xnet.cu:1565-1570);
    gamma / beta device arrays or NULL (1 / 0) */
 void umx_in_coef(const double *part, int N, int C, int D, int H, int W, const float *gamma, const float *beta, float eps, float *coef);

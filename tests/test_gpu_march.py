@@ -129,3 +129,25 @@ def test_plane_major_halves(dev, N, Ci, Co, D, H, W, bits):
     want = run(N * nbo * S * 64, 0, 0).reshape(N, nbo, S, 32).transpose(0, 1, 3, 2).reshape(N, nbo * 32, S)[:, :Co]
     for shift in (0, 2):
         assert np.array_equal(run(N * Co * S * 2, shift, 3).reshape(N, Co, S), want)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,cap", [
+    (1, 32, 64, 41, 37, 19, 2),        # odd grid, runs of many planes: windows that wrap around the slot ring, pieces of several runs
+    (2, 64, 96, 24, 33, 8, 3),         # even depth (the last plane completes on an odd input plane), 32-channel column tiles, pieces that cross samples
+    (1, 32, 32, 1, 40, 50, 0),         # one input plane: a stage that starts and completes its output
+    (1, 160, 40, 9, 16, 16, 1),        # the widest input in MX-fp8, one block a column tile
+    (2, 33, 64, 7, 5, 3, 0),           # grids smaller than a tile, a second input block of one channel
+])
+def test_stride2_runs_and_wraps(dev, N, Ci, Co, D, H, W, cap, bits):
+    """The resident-weight stride-2 kernel on exact operands (every product and partial sum representable): the oracle's bits, whatever the pieces."""
+    x = exact_operands(331, (N, Ci, D, H, W), 1).reshape(-1)
+    w = exact_operands(332, (Co, Ci, 27), 1)
+    b = (synth.rng(333).integers(-8, 8, Co) * 0.5).astype(np.float32)
+    mx, want = orc.conv_case("conv3s2", x, w, b, N, Ci, D, H, W, Co, bits)
+    dev.umx_conv_r_block_cap(cap)
+    try:
+        got = run("conv3s2", mx, w, b, N, Ci, D, H, W, Co, bits, want_kernel=4)
+    finally:
+        dev.umx_conv_r_block_cap(0)
+    assert np.array_equal(got, want), "%d of %d differ" % (np.count_nonzero(got != want), want.size)

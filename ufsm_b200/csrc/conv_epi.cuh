@@ -6,7 +6,7 @@ struct umx_conv {
     int kind, co, ci, bits;
     int taps, nkb, nki, cop, cob_t, nt, ntiles_n, nst, items_max, ipq, nquad, w_stage_bytes;
     uint8_t *wpk; float *bias_p;
-    uint8_t *wr;                    /* weight image of the z-marching kernel, or NULL */
+    uint8_t *wr;                    /* weight image of the z-marching kernel (3^3, or 3^3 stride 2), or NULL */
     uint8_t *wp;                    /* weight image of the one-tap streaming kernel, or NULL */
     uint8_t *wstem;                 /* weight tile of the tap-packed one-channel kernel, or NULL */
     const float *w_src, *b_src;     /* set in a conv that lives for one call (umx_conv_per_call): its images are made in scratch when a kernel asks for them */
@@ -23,10 +23,16 @@ struct EpiArgs {
 };
 
 /* v: the 32 fp32 accumulators of GEMM row (n, z, oy, ox), 32-column block cb_g.  Adds the bias, rounds as the output mode asks (v keeps
-   the values as stored, which is what the statistics are taken from) and writes the row if it lies inside the volume. */
-__device__ __forceinline__ void epi_chunk(const EpiArgs &a, int n, int z, int oy, int ox, bool row_ok, int cb_g, float *v) {
+   the values as stored, which is what the statistics are taken from) and writes the row if it lies inside the volume.  OWN: the block's 32 biases are in `own`, which
+   the caller has read (a bias that a kernel just ahead may have written does not go through the non-coherent path). */
+template <bool OWN = false>
+__device__ __forceinline__ void epi_chunk(const EpiArgs &a, int n, int z, int oy, int ox, bool row_ok, int cb_g, float *v, const float *own = nullptr) {
     const size_t S = (size_t)a.D * a.H * a.W;
-    {
+    if (OWN) {
+        const float4 *bp = (const float4 *)own;
+#pragma unroll
+        for (int k = 0; k < 8; k++) { const float4 b = bp[k]; v[4 * k] = __fadd_rn(v[4 * k], b.x); v[4 * k + 1] = __fadd_rn(v[4 * k + 1], b.y); v[4 * k + 2] = __fadd_rn(v[4 * k + 2], b.z); v[4 * k + 3] = __fadd_rn(v[4 * k + 3], b.w); }
+    } else {
         const float4 *bp = (const float4 *)(a.bias + cb_g * 32);
 #pragma unroll
         for (int k = 0; k < 8; k++) { const float4 b = __ldg(bp + k); v[4 * k] = __fadd_rn(v[4 * k], b.x); v[4 * k + 1] = __fadd_rn(v[4 * k + 1], b.y); v[4 * k + 2] = __fadd_rn(v[4 * k + 2], b.z); v[4 * k + 3] = __fadd_rn(v[4 * k + 3], b.w); }
@@ -96,9 +102,10 @@ __device__ __forceinline__ void epi_chunk(const EpiArgs &a, int n, int z, int oy
     }
 }
 
-/* geometry of the z-marching kernel's weight image (conv_tcr.cu), one image per column tile of nt channels */
+/* geometry of the z-marching kernels' weight images (conv_tcr.cu, conv_s2.cu), one image per column tile of nt channels; 0 when the kernel does not take the conv */
 struct RImageGeo { int nt, ncol, w_bytes, w_codes, gt, goff1, goff2; };
 int umx_conv_r_image(const umx_conv *c, RImageGeo *o);
+int umx_conv_s2_image(const umx_conv *c, RImageGeo *o);
 
 /* ---- weight preparation of the one-tap convs: where GEMM row `row`, tap `tap`, K block `kb`, element k comes from ---- */
 struct PrepArgs {

@@ -1,5 +1,5 @@
 /* Weight preparation of the 27-tap convs: fp32 weights [co][ci][27] -> the shared-memory images of the general kernel (UMX_CONV3, UMX_CONV3S2) and
-   of the z-marching kernel (UMX_CONV3), quantised per (row, tap, 32 input channels) as the reference's prep_w8_k / prep_w4_k
+   of the z-marching ones (conv_tcr.cu, conv_s2.cu), quantised per (row, tap, 32 input channels) as the reference's prep_w8_k / prep_w4_k
    (src/lp_f8fwd.cu:54-71, src/lp_f4fwd.cu:53-66).
 
    A warp owns one (output row, K item of 32 or 64 input channels): its weights are one contiguous run of 27 floats a channel, which comes into
@@ -53,11 +53,14 @@ __global__ void __launch_bounds__(128) prep_w27_k(const PrepArgs p, const RImage
         else *(unsigned short *)(sf + q * 512 + l * 16 + c * 4 + (j & 1) * 2) = (unsigned short)(sb[0] | (sb[1] << 8));
     }
     if (r.wr) {
-        const int nt = r.nt, R3 = 3 * nt, ct = row / nt, cl = row - ct * nt, dz = tap / 9, j = tap % 9, rw = dz * nt + cl;
+        const int nt = r.nt, R3 = 3 * nt, ct = row / nt, cl = row - ct * nt, dz = tap / 9, j = tap % 9;
+        /* the rows of a tap in the order dz = 0, 1, 2, with scale images from each of them on; stride 2: dz = 0, 2, 1, with images of (0, 2), 2 and 1 */
+        const bool s2 = p.kind == UMX_CONV3S2;
+        const int rw = (s2 ? (3 - dz) % 3 : dz) * nt + cl;
         uint8_t *wr = r.wr + (size_t)ct * r.w_bytes, *base = wr + (size_t)(ki * 9 + j) * 2 * R3 * 16;
         *(uint4 *)(base + (size_t)rw * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         *(uint4 *)(base + (size_t)(R3 + rw) * 16) = make_uint4(w[4], w[5], w[6], w[7]);
-        for (int d = 0; d <= dz; d++) {
+        for (int d = s2 && dz == 1 ? 2 : 0; d <= (s2 ? (3 - dz) % 3 : dz); d++) {
             const int rr = rw - d * nt, g = rr >> 7, col = (rr & 127) >> 5, l = rr & 31, gb = d == 0 ? 0 : d == 1 ? r.goff1 : r.goff2;
             if (BITS == 8) wr[r.w_codes + ((ki * r.nquad + (j >> 2)) * r.gt + gb + g) * 512 + l * 16 + col * 4 + (j & 3)] = (uint8_t)sb[0];
             else *(unsigned short *)(wr + r.w_codes + ((ki * r.nquad + (j >> 1)) * r.gt + gb + g) * 512 + l * 16 + col * 4 + (j & 1) * 2) = (unsigned short)(sb[0] | (sb[1] << 8));
@@ -69,7 +72,7 @@ __global__ void __launch_bounds__(128) prep_w27_k(const PrepArgs p, const RImage
 
 /* p.wpk: the general kernel's image or NULL; wr: the z-marching kernel's or NULL; p.bias_p: the padded bias or NULL */
 void umx_prep_w27(const PrepArgs &p, uint8_t *wr, int nt, int w_bytes, int w_codes, int gt, int goff1, int goff2) {
-    const RImage r = {wr, nt, w_bytes, w_codes, p.nquad, gt, goff1, goff2};
+    const RImage r = {wr, nt, w_bytes, w_codes, p.bits == 8 ? 3 : 5, gt, goff1, goff2};      /* scale quads of nine taps */
     const int nitem = (p.ci + (p.bits == 8 ? 31 : 63)) / (p.bits == 8 ? 32 : 64);
     const dim3 grid((unsigned)p.cop, (unsigned)((nitem + 3) / 4));
     if (p.bits == 8) umx_launch(prep_w27_k<8>, grid, dim3(128), 0, p, r); else umx_launch(prep_w27_k<4>, grid, dim3(128), 0, p, r);

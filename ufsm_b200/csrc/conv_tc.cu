@@ -417,6 +417,10 @@ int umx_conv_fwd_stem(const umx_conv *c, const void *x, int src8, int N, int D, 
 int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *enc, int N, int D, int H, int W, const EpiArgs &e);
 const uint8_t *umx_prob_table(void);
 void umx_mx_codes_to_split(const void *x, size_t blocks, size_t S, void *y);
+int umx_conv_s2_takes(const umx_conv *c);
+int umx_conv_fwd_s2(const umx_conv *c, const void *x, int split, const uint8_t *x_sc, void *enc, int N, int Di, int Hi, int Wi, const EpiArgs &e);
+/* the z-marching image of either kind */
+static int march_image(const umx_conv *c, RImageGeo *o) { return c->kind == UMX_CONV3S2 ? umx_conv_s2_image(c, o) : umx_conv_r_image(c, o); }
 
 
 /* the fields of a conv that follow from its kind and sizes */
@@ -458,7 +462,7 @@ static umx_conv *conv_build(int kind, const float *w_dev, const float *bias_dev,
     const PrepArgs p = prep_args(c, w_dev, bias_dev);
     if (kind == UMX_CONV3 || kind == UMX_CONV3S2) {
         RImageGeo g; memset(&g, 0, sizeof g);
-        if (kind == UMX_CONV3 && umx_conv_r_image(c, &g)) {
+        if (march_image(c, &g)) {
             c->wr = (uint8_t *)nn_malloc((size_t)g.w_bytes * g.ncol);
             if (!c->wr) { umx_conv_free(c); return nullptr; }
             cudaMemset(c->wr, 127, (size_t)g.w_bytes * g.ncol);
@@ -491,7 +495,7 @@ static bool image_for_call(umx_conv *c, int which) {
     if (!c->w_src) return false;
     c->bias_p = (float *)umx_ws(15, (size_t)c->cop * 4);
     RImageGeo g; memset(&g, 0, sizeof g);
-    if (which) { if (!umx_conv_r_image(c, &g)) return false; c->wr = (uint8_t *)umx_ws(14, (size_t)g.w_bytes * g.ncol); }
+    if (which) { if (!march_image(c, &g)) return false; c->wr = (uint8_t *)umx_ws(14, (size_t)g.w_bytes * g.ncol); }
     else c->wpk = (uint8_t *)umx_ws(13, wpk_bytes(c));
     if (!c->bias_p || (which ? !c->wr : !c->wpk)) return false;
     PrepArgs p = prep_args(c, c->w_src, c->b_src);
@@ -589,6 +593,24 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     a.e.y = y; a.e.y_split = (flags & UMX_Y_SPLIT) != 0; a.err = umx_errflag();
     if (out_mode == UMX_OUT_PROB8) { a.e.ptab = umx_prob_table(); if (!a.e.ptab) return -1; }
     if (!a.err) return -1;
+    /* algorithmic work: 2 x output voxels x real input channels x real output channels x taps (no credit for padding) */
+    const double flops = 2.0 * (double)N * S * (c->kind == UMX_DOWN2 ? 8.0 : 1.0) * c->ci * (double)c->co * (c->kind == UMX_TCONV2 ? 8.0 : 1.0) * ((c->taps == 27 || s2) ? 27.0 : 1.0);
+    static int force_v1 = -1;
+    if (force_v1 < 0) { const char *ev = getenv("UMX_CONV_V1"); force_v1 = ev && *ev && *ev != '0'; }
+    if (s2 && !force_v1 && umx_conv_s2_takes(c) && image_for_call((umx_conv *)c, 1)) {
+        umx_plain_launch = 0;                               /* this kernel reads weights made for the call behind its dependency wait */
+        a.e.bias = c->bias_p;
+        const int pid = umx_prof_open(flops);
+        const int rc = umx_conv_fwd_s2(c, x, c->bits == 8 && (flags & UMX_X_SPLIT), a.x_sc, (void *)enc, N, Dx, Hx, Wx, a.e);
+        if (rc <= 0) {
+            umx_prof_close(pid);
+            g_umx_launches++; g_last_kernel = 4;
+            UMX_CK("umx_conv_fwd");
+            if (rc == 0 && nrm) umx_in_stats_coef(y, N, c->co, D, H, W, nrm->gamma, nrm->beta, nrm->eps, part, nrm->coef);
+            else if (rc == 0 && part) umx_in_part(y, N, c->co, D, H, W, part);
+            return rc;
+        }
+    }
     /* tensor map over the activation codes seen as 16-byte-wide planes [plane][z][y][x * 16 B]: fp8 in the split layout has two planes a
        block, fp4 one.  A box is (10 or 8 voxels) x (18 or 16 rows) x 1 plane of z x 2 planes; voxels outside the volume read as zero. */
     if (c->bits == 8 && !(flags & UMX_X_SPLIT)) {   /* reference layout: re-lay the codes into scratch first */
@@ -613,12 +635,8 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         const CUresult r0 = enc(&m0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)x, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) { char b[160]; snprintf(b, sizeof b, "umx_conv_fwd: cuTensorMapEncodeTiled failed (%d) for %d x %d x %d x %d, %d blocks", (int)r0, N, D, H, W, c->nkb); umx_latch_msg(b); return -1; }
     }
-    /* algorithmic work: 2 x output voxels x real input channels x real output channels x taps (no credit for padding) */
-    const double flops = 2.0 * (double)N * S * (c->kind == UMX_DOWN2 ? 8.0 : 1.0) * c->ci * (double)c->co * (c->kind == UMX_TCONV2 ? 8.0 : 1.0) * ((c->taps == 27 || s2) ? 27.0 : 1.0);
-    static int force_v1 = -1;
-    if (force_v1 < 0) { const char *ev = getenv("UMX_CONV_V1"); force_v1 = ev && *ev && *ev != '0'; }
     /* InstanceNorm statistics are a separate pass over the stored output (umx_in_part below) */
-    if (!force_v1 && (c->wr || (c->w_src && c->kind == UMX_CONV3 && umx_conv_r_takes(c, a.x_sc, N, D, H, W, a.e) && image_for_call((umx_conv *)c, 1)))) {   /* resident weights: the persistent z-marching kernel, when the geometry allows */
+    if (!force_v1 && c->kind == UMX_CONV3 && (c->wr || (c->w_src && umx_conv_r_takes(c, a.x_sc, N, D, H, W, a.e) && image_for_call((umx_conv *)c, 1)))) {   /* resident weights: the persistent z-marching kernel, when the geometry allows */
         const int pid = umx_prof_open(flops);
         a.e.bias = c->bias_p;
         int rc = (nrm && (flags & UMX_STATS_EPILOGUE)) ? umx_conv_fwd_r(c, a.x_sc, &m0, (void *)enc, N, D, H, W, a.e, part, nrm->gamma, nrm->beta, nrm->eps, nrm->coef) : 1;

@@ -667,6 +667,7 @@ static int r_geometry(const umx_conv *c, RGeo *g) {
    slot windows and several-planes-a-block regime that otherwise only volumes with thousands of tile planes reach */
 static int g_r_block_cap = 0;
 extern "C" void umx_conv_r_block_cap(int cap) { g_r_block_cap = cap > 0 ? cap : 0; }
+int umx_conv_r_cap(void) { return g_r_block_cap; }                /* the stride-2 kernel's too */
 /* Weight image of the z-marching kernel (made by umx_prep_w27): codes [input item][dy dx][k half][dz * nt + channel][16 B], then the B scale
    bytes in the TMEM scale layout per (input item, tap quad, first dz of the MMA, 128-row group): byte (lane, column, id) = row 128 g + 32
    column + lane counted from that dz's first row, tap 4 q + id (fp8) or tap 2 q + id / 2, block id % 2 (fp4).  A block-scaled MMA wants its
