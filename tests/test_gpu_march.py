@@ -151,3 +151,39 @@ def test_stride2_runs_and_wraps(dev, N, Ci, Co, D, H, W, cap, bits):
     finally:
         dev.umx_conv_r_block_cap(0)
     assert np.array_equal(got, want), "%d of %d differ" % (np.count_nonzero(got != want), want.size)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,cap", [
+    (1, 32, 32, 33, 17, 13, 2),        # rows of every alignment, runs of many planes
+    (2, 64, 64, 12, 31, 21, 3),        # two input blocks, 64-channel tiles, pieces that cross samples
+    (1, 96, 32, 9, 18, 35, 2),         # three input blocks: in MX-fp4 the second item's second block is not there
+    (2, 32, 64, 40, 5, 3, 1),          # a grid narrower than a tile
+    (1, 1, 32, 20, 16, 30, 1),         # even width, one channel
+])
+def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
+    """Scale planes whose rows are not multiples of 16 bytes: the scale warp gathers its window.  Random operands within 1e-3 of the oracle (the order of the fp32 sums is the only
+    freedom), exact operands the oracle's bits; fp16 plane-major and MX outputs equal to those of the fp32 output."""
+    S = D * H * W
+    x = synth.rng(341).standard_normal(N * Ci * S).astype(np.float32) * np.exp2(synth.rng(344).integers(-6, 7, N * Ci * S)).astype(np.float32)
+    w, b = synth.kaiming(342, Co, Ci, 27), synth.bias(343, Co, 0.1)
+    mx, want = orc.conv_case("conv3", x, w, b, N, Ci, D, H, W, Co, bits)
+    xe = exact_operands(345, (N, Ci, D, H, W), 1).reshape(-1)
+    we = exact_operands(346, (Co, Ci, 27), 1)
+    mxe, wante = orc.conv_case("conv3", xe, we, None, N, Ci, D, H, W, Co, bits)
+    dev.umx_conv_r_block_cap(cap)
+    try:
+        got = run("conv3", mx, w, b, N, Ci, D, H, W, Co, bits)
+        gote = run("conv3", mxe, we, None, N, Ci, D, H, W, Co, bits)
+        c = G.Conv("conv3", w, b, Co, Ci, bits)
+        h16, _ = c.fwd(mx, N, D, H, W, G.OUT_PM16)
+        q, _ = c.fwd(mx, N, D, H, W, G.OUT_MXRAW, 8)
+        assert dev.umx_conv_last_kernel() == 1
+        c.free()
+    finally:
+        dev.umx_conv_r_block_cap(0)
+    e = orc.rel_l2(got, want)
+    assert np.isfinite(got).all() and e < TOL, "relative L2 %.3g" % e
+    assert np.array_equal(gote, wante), "%d of %d differ" % (np.count_nonzero(gote != wante), wante.size)
+    assert np.array_equal(h16.view(np.float16).reshape(-1), got.astype(np.float16).reshape(-1))
+    assert np.array_equal(q, orc.blocked_to_mx(orc.pm_to_blocked(got, N, Co, S), 8, N, Co, S))

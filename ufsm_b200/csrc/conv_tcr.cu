@@ -74,7 +74,8 @@ struct ConvRArgs {
        sample and block into part [n][gcol][cop][2]; the last block of a column tile to finish adds the blocks' entries in block order and
        turns them into coefficients (a, b) per (sample, channel) */
     double *part; float *coef; const float *gamma, *beta; float eps; int cop, off_red;
-    const uint8_t *wr;
+    const uint8_t *wr, *x_sc;
+    int gather, w_dep;                           /* see GATHER; the weights and the bias were written by a kernel just ahead in the stream */
     EpiArgs e;
     int *err;
 };
@@ -160,8 +161,9 @@ __device__ __forceinline__ double lanes8_sum(double v, int p4, int p2, int p1) {
 __device__ unsigned g_conv_tickets[64];      /* one per column tile; the block that draws the last ticket finalises and resets it */
 
 /* NCH: 32-channel chunks of the column tile (1: two blocks per multiprocessor and at most 128 registers; 2: one block, more registers);
-   STATS: the epilogue also takes the InstanceNorm sums */
-template <int BITS, int NCH, bool STATS>
+   STATS: the epilogue also takes the InstanceNorm sums; GATHER: the scale warp fetches its window of scale bytes itself, for scale planes whose rows TMA does not
+   take (W not a multiple of 16) */
+template <int BITS, int NCH, bool STATS, bool GATHER>
 __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap maps, const ConvRArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint64_t *bars = (uint64_t *)smem_raw;
@@ -175,7 +177,9 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     /* barriers: tma[R] (codes + scale window landed), sf[R] (A scales laid out), empty[R], accumulator full / empty per slot, weights */
     const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_accf = bar_tma + 24 * R, bar_acce = bar_accf + 8 * kMaxSlots, bar_w = bar_acce + 8 * kMaxSlots, bar_red = bar_w + 8;
     constexpr int NQ = BITS == 8 ? 3 : 5;                  /* A scale quads per stage */
-    constexpr uint32_t TX = 5760u + (BITS == 8 ? 576u : 1152u);
+    constexpr int GB = BITS == 8 ? 54 : 108, GN = (GB + 31) / 32;          /* words of the gathered scale window, of a lane */
+    auto win_at = [](int i) { return i / 54 * 576 + (i % 54) / 3 * 32 + i % 3 * 4; };      /* where word i lies in the stage's window */
+    constexpr uint32_t TX = 5760u + (GATHER ? 0u : BITS == 8 ? 576u : 1152u);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < R; i++) { mbar_init(bar_tma + 8 * i, 1); mbar_init(bar_sf + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
@@ -186,10 +190,11 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
         fence_proxy_async();
     }
     const int ctile = (int)blockIdx.x / a.gcol;
-    if ((int)threadIdx.x < a.nt) bias_s[threadIdx.x] = a.e.bias[ctile * a.nt + threadIdx.x];
+    if (!a.w_dep && (int)threadIdx.x < a.nt) bias_s[threadIdx.x] = a.e.bias[ctile * a.nt + threadIdx.x];
     pdl_trigger();
     if (threadIdx.x == 0) {
-        /* the weight image is a constant of the layer: it may load while the previous kernel of the stream is still running */
+        /* the weight image of a prepared layer is a constant: it may load while the previous kernel of the stream is still running */
+        if (a.w_dep) pdl_wait();
         mbar_expect_tx(bar_w, (uint32_t)a.w_bytes);
         for (int o = 0; o < a.w_bytes; o += 32768) bulk_g2s(smem_u32(wsm + o), a.wr + (size_t)ctile * a.w_bytes + o, (uint32_t)min(32768, a.w_bytes - o), bar_w);
     }
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         /* codes: two 16-byte-wide planes (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1), 18 rows of 10 voxels;
                            scale bytes: 18 rows of a 32-byte window per block */
                         tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki, lead);
-                        tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki, lead);
+                        if (!GATHER) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki, lead);
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
                 }
@@ -308,41 +313,107 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
            dx of a row are neighbours, so two words and a funnel shift fetch them.  The warp lays the nine shifted scale sets out in shared
            memory in the tcgen05.cp layout, as far ahead of the MMAs as the ring is deep. */
         int it = 0, s = 0, ph = 0; bool ok = true;
-        while (piece.u < piece.u1 && ok) {
-            const Run rn = next_run(a, piece);
-            const int x0 = (rn.txy % a.tiles_x) * 8;
-            const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
-            const int off = (lane >> 3) * 32 + (lane & 7) + (x0 - 1) - (((x0 - 1) >> 4) << 4), sh = (off & 3) * 8;
-            const int nst = (zhi - zlo + 1) * a.nki;
-            for (int i = 0; i < nst; i++) {
-                if (!mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitR)) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * s, ph); ok = false; break; }
-                uint8_t *stg = stages + (size_t)s * a.stage_bytes;
-                const uint32_t *sw = (const uint32_t *)(stg + a.offSW + (off & ~3));
-                uint32_t *sfa = (uint32_t *)(stg + a.offSFA);
-                uint32_t wq[4][5];
+        /* one stage: window -> scale sets; off: this lane's first byte of the window, gw: the window's bytes (GATHER) */
+        auto lay = [&](int off, const unsigned *gw) {
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * s, ph); ok = false; return; }
+            uint8_t *stg = stages + (size_t)s * a.stage_bytes;
+            if (GATHER) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    uint32_t t[3], u[3];          /* bytes 0..2: the scales of dx = 0, 1, 2 */
-#pragma unroll
-                    for (int dy = 0; dy < 3; dy++) {
-                        const uint32_t *p = sw + q * 32 + dy * 8;
-                        t[dy] = __funnelshift_r(p[0], p[1], sh);
-                        if (BITS == 4) u[dy] = __funnelshift_r(p[144], p[145], sh);
-                    }
-                    if (BITS == 8) {              /* taps 0-3, 4-7, 8 */
-                        wq[q][0] = __byte_perm(t[0], t[1], 0x4210); wq[q][1] = __byte_perm(t[1], t[2], 0x5421); wq[q][2] = (t[2] >> 16) & 0xffu;
-                    } else {                      /* pairs (block 2 ki, block 2 ki + 1) of taps 0 1, 2 3, 4 5, 6 7, 8 */
-                        wq[q][0] = __byte_perm(t[0], u[0], 0x5140); wq[q][1] = __byte_perm(__byte_perm(t[0], u[0], 0x0062), __byte_perm(t[1], u[1], 0x0040), 0x5410);
-                        wq[q][2] = __byte_perm(t[1], u[1], 0x6251); wq[q][3] = __byte_perm(t[2], u[2], 0x5140); wq[q][4] = __byte_perm(t[2], u[2], 0x0062) & 0xffffu;
-                    }
+                for (int k = 0; k < GN; k++) {
+                    const int i = 32 * k + lane;
+                    if (i < GB) *(unsigned *)(stg + a.offSW + win_at(i)) = __funnelshift_r(gw[4 * k], gw[4 * k + 1], gw[4 * k + 2]) & gw[4 * k + 3];
                 }
-                /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
-#pragma unroll
-                for (int qd = 0; qd < NQ; qd++) *(uint4 *)(sfa + qd * 128 + lane * 4) = make_uint4(wq[0][qd], wq[1][qd], wq[2][qd], wq[3][qd]);
-                fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_sf + 8 * s);
-                it++; if (++s == R) { s = 0; ph ^= 1; }
+            }
+            const int sh = (off & 3) * 8;
+            const uint32_t *sw = (const uint32_t *)(stg + a.offSW + (off & ~3));
+            uint32_t *sfa = (uint32_t *)(stg + a.offSFA);
+            uint32_t wq[4][5];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint32_t t[3], u[3];          /* bytes 0..2: the scales of dx = 0, 1, 2 */
+#pragma unroll
+                for (int dy = 0; dy < 3; dy++) {
+                    const uint32_t *p = sw + q * 32 + dy * 8;
+                    t[dy] = __funnelshift_r(p[0], p[1], sh);
+                    if (BITS == 4) u[dy] = __funnelshift_r(p[144], p[145], sh);
+                }
+                if (BITS == 8) {              /* taps 0-3, 4-7, 8 */
+                    wq[q][0] = __byte_perm(t[0], t[1], 0x4210); wq[q][1] = __byte_perm(t[1], t[2], 0x5421); wq[q][2] = (t[2] >> 16) & 0xffu;
+                } else {                      /* pairs (block 2 ki, block 2 ki + 1) of taps 0 1, 2 3, 4 5, 6 7, 8 */
+                    wq[q][0] = __byte_perm(t[0], u[0], 0x5140); wq[q][1] = __byte_perm(__byte_perm(t[0], u[0], 0x0062), __byte_perm(t[1], u[1], 0x0040), 0x5410);
+                    wq[q][2] = __byte_perm(t[1], u[1], 0x6251); wq[q][3] = __byte_perm(t[2], u[2], 0x5140); wq[q][4] = __byte_perm(t[2], u[2], 0x0062) & 0xffffu;
+                }
+            }
+            /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
+#pragma unroll
+            for (int qd = 0; qd < NQ; qd++) *(uint4 *)(sfa + qd * 128 + lane * 4) = make_uint4(wq[0][qd], wq[1][qd], wq[2][qd], wq[3][qd]);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_sf + 8 * s);
+            it++; if (++s == R) { s = 0; ph ^= 1; }
+        };
+        const int off0 = (lane >> 3) * 32 + (lane & 7);
+        if (!GATHER) {
+            while (piece.u < piece.u1 && ok) {
+                const Run rn = next_run(a, piece);
+                const int x0 = (rn.txy % a.tiles_x) * 8;
+                const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
+                const int off = off0 + (x0 - 1) - (((x0 - 1) >> 4) << 4);
+                const int nst = (zhi - zlo + 1) * a.nki;
+                for (int i = 0; i < nst && ok; i++) lay(off, nullptr);
+            }
+        } else {
+            /* The window is 18 rows of 10 bytes (two of them for fp4): of each the three words that begin at its first byte, every one put together from the two aligned words
+               it lies in, and bytes outside the row cleared (scale byte 0, under zero codes).  A lane has GN words and asks for them two stages ahead of their use.  Byte by byte
+               this warp was the slowest role in the 64-channel MX-fp4 tiles. */
+            pdl_wait();
+            Run rn; int zi = 1, zhi = 0, ki = 0; bool live = false; const uint8_t *base = nullptr;
+            unsigned keep[GN];                   /* the bytes of word k that lie in the volume */
+            int offs[GN];
+            const size_t S = (size_t)a.D * a.H * a.W;
+#pragma unroll
+            for (int k = 0; k < GN; k++) { const int i = (32 * k + lane) % 54; offs[k] = (i / 3) * a.W + i % 3 * 4; }
+            auto open = [&]() {
+                live = piece.u < piece.u1;
+                if (!live) return;
+                rn = next_run(a, piece);
+                zi = max(0, rn.zb - 1); zhi = min(a.D - 1, rn.ze); ki = 0;
+                const int x0 = (rn.txy % a.tiles_x) * 8 - 1, y0 = (rn.txy / a.tiles_x) * 16 - 1;
+                base = a.x_sc + (ptrdiff_t)y0 * a.W + x0;
+#pragma unroll
+                for (int k = 0; k < GN; k++) {
+                    const int i = (32 * k + lane) % 54, y = y0 + i / 3, x = x0 + i % 3 * 4;
+                    keep[k] = 0u;
+#pragma unroll
+                    for (int t = 0; t < 4; t++) if (x + t >= 0 && x + t < a.W && i % 3 * 4 + t < 10) keep[k] |= 0xffu << (8 * t);
+                    if (32 * k + lane >= GB || y < 0 || y >= a.H) keep[k] = 0u;
+                }
+            };
+            auto fetch = [&](unsigned *g) {
+                if (!live) return;
+                const uint8_t *p = base + ((size_t)rn.n * a.nkb + (BITS == 8 ? ki : 2 * ki)) * S + (size_t)zi * a.H * a.W;
+                const bool two = BITS == 4 && 2 * ki + 1 < a.nkb;
+#pragma unroll
+                for (int k = 0; k < GN; k++) {
+                    const bool second = 32 * k + lane >= 54;                     /* fp4: the window of the item's second block, which may not be there (zero weights) */
+                    const uint8_t *q = p + (second ? S : 0) + offs[k];
+                    const unsigned sh = (unsigned)(size_t)q & 3u, m = !second || two ? keep[k] : 0u;
+                    const unsigned *w = (const unsigned *)(q - sh);
+                    /* an aligned word is read only where it has a byte that is kept; put together in lay, when they have come */
+                    g[4 * k] = m << (8 * sh) ? ld_dep(w) : 0u; g[4 * k + 1] = sh && m >> (32 - 8 * sh) ? ld_dep(w + 1) : 0u;
+                    g[4 * k + 2] = 8 * sh; g[4 * k + 3] = m;
+                }
+                if (++ki == a.nki) { ki = 0; if (++zi > zhi) open(); }
+            };
+            unsigned g0[4 * GN], g1[4 * GN];
+            open();
+            bool l0 = live; fetch(g0);
+            bool l1 = live; fetch(g1);
+            while (ok && l0) {
+                lay(off0, g0); l0 = live; fetch(g0);
+                if (!ok || !l1) break;
+                lay(off0, g1); l1 = live; fetch(g1);
             }
         }
     } else if (warp == 3) {
@@ -378,6 +449,12 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
         tc_fence_before();
         __syncwarp();
         if (lane == 0) for (int sl = 0; sl < NS; sl++) mbar_arrive(bar_acce + 8 * sl);     /* one arrival per warp: arrivals on one barrier serialise */
+        if (a.w_dep) {                                          /* every warp writes the same values */
+            pdl_wait();
+#pragma unroll
+            for (int jc = 0; jc < NCH; jc++) bias_s[jc * 32 + lane] = ld_dep(a.e.bias + ctile * a.nt + jc * 32 + lane);
+            __syncwarp();
+        }
         int pcm = 0, pph = 0, pc = 0; bool dead = false;        /* pcm = plane count mod slots, pph = its wrap parity */
         const size_t S = (size_t)a.D * a.H * a.W;
         constexpr bool stats = STATS;
@@ -566,7 +643,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         float v[32];
 #pragma unroll
                         for (int k = 0; k < 32; k++) v[k] = __uint_as_float(rr[jc][k]);
-                        epi_chunk(a.e, rn.n, z, oy, ox, row_ok, ctile * NCH + jc, v);
+                        epi_chunk<true>(a.e, rn.n, z, oy, ox, row_ok, ctile * NCH + jc, v, bias_s + jc * 32);
                     }
                 }
                 if (++pcm == NS) { pcm = 0; pph ^= 1; }
@@ -683,7 +760,8 @@ int umx_conv_r_image(const umx_conv *c, RImageGeo *o) {
 static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e, int want_coef, const double *part, ConvRArgs &a, int *grid) {
     memset(&a, 0, sizeof a);
     RGeo g;
-    if (!r_geometry(c, &g) || (W & 15) || ((size_t)x_sc & 15)) return 0;      /* the scale window needs rows that are multiples of 16 bytes */
+    if (!r_geometry(c, &g)) return 0;
+    a.gather = (W & 15) || ((size_t)x_sc & 15);      /* TMA takes the scale plane only in rows that are multiples of 16 bytes */
     a.w_codes = g.w_codes; a.w_bytes = g.w_bytes; a.gt = g.gt; a.goff1 = g.goff1 * 4; a.goff2 = g.goff2 * 4;   /* TMEM column offsets of the dz >= 1, 2 images */
     a.tmem_cols = g.tmem_cols; a.nslot = g.nslot; a.sfa_base = g.sfa_base; a.sfa_cols = g.sfa_cols; a.sfb_base = g.sfb_base;
     a.N = N; a.D = D; a.H = H; a.W = W; a.nkb = c->nkb; a.nki = c->nki; a.bits = c->bits; a.nt = g.nt; a.ncol = g.ncol;
@@ -691,8 +769,8 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     a.units = (long long)N * a.tiles * D;
     a.nquad = c->nquad;
     a.fast_h16 = e.out_mode == UMX_OUT_H16B && !e.tconv && (want_coef || !((size_t)e.y & 31));      /* stores of 32 bytes */
-    a.fast_pm16 = e.out_mode == UMX_OUT_PM16 && !e.tconv && !((size_t)e.y & 15);        /* W is a multiple of 16: tile rows are aligned and whole */
-    if (want_coef && (!a.fast_h16 || !part || g.ncol > 64)) return 0;
+    a.fast_pm16 = e.out_mode == UMX_OUT_PM16 && !e.tconv && !((size_t)e.y & 15) && !(W & 7);        /* tile rows are aligned and whole */
+    if (want_coef && (!a.fast_h16 || !part || g.ncol > 64 || a.gather)) return 0;
     a.cop = c->cop;
     /* the codes and the scale window are TMA destinations (128-byte aligned) */
     a.offSW = 5888; a.offSFA = a.offSW + (c->bits == 8 ? 640 : 1152);
@@ -710,7 +788,12 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     if (g_r_block_cap && slots > g_r_block_cap) slots = g_r_block_cap;
     /* A block pays two halo planes per run: with fewer than eight planes a block (counted for one sample, so that the choice of kernel does not
        depend on the batch) the general kernel is faster.  Volumes with fewer planes than blocks are left here: nothing to gain either way. */
-    { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 0; }
+    { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 0;
+      /* The scale warp that gathers costs 3 to 8 % in MX-fp8 and 6 to 27 in MX-fp4 against the TMA window, and a piece's start, so few planes, and a column tile that re-reads the
+         input, are the general kernel's.  General kernel and this one, us: 32 -> 32 fp4 on 33 x 31 x 30 (264 planes) 6.9 and 9.0, on 36^3 (540) 14.5 and 11.6, on 63 x 61 x 66 45 and
+         17; fp8 64 -> 32 on 80 x 80 x 84 112 and 43; 64 columns, fp4 128 -> 64 plane-major on 36^3 23.0 and 24.6, on 40 x 35 x 42 (720) 33.0 and 29.0; two column tiles, fp8 32 -> 128 on
+         63 x 61 x 66 91 and 124. */
+      if (a.gather && (g.ncol > 1 || 2 * units1 < (g.nt == 32 ? 7ll : 9ll) * (slots < sms ? slots : sms))) return 0; }
     a.gcol = (int)(a.units < slots ? a.units : slots); if (a.gcol > 512) a.gcol = 512;
     *grid = a.gcol * g.ncol;
     return 1;
@@ -734,36 +817,43 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     int dev = 0; cudaGetDevice(&dev);
     const size_t S = (size_t)D * H * W;
     CUtensorMap ms; memset(&ms, 0, sizeof ms);
-    {
+    if (!a.gather) {
         const cuuint64_t gd[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N * c->nkb};
         const cuuint64_t gs[3] = {(cuuint64_t)W, (cuuint64_t)W * H, (cuuint64_t)S};
         const cuuint32_t box[4] = {32, 18, 1, (cuuint32_t)(c->bits == 8 ? 1 : 2)}, es[4] = {1, 1, 1, 1};
         const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) return 1;                        /* e.g. a scale plane that is not 16-byte aligned: take the general kernel */
     }
-    a.wr = c->wr; a.e = e; a.err = umx_errflag();
+    a.wr = c->wr; a.x_sc = x_sc; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
     static int attr_set[16];
     if (!attr_set[dev & 15]) {
-        const void *ks[8] = {(const void *)conv_mxr_k<8, 1, false>, (const void *)conv_mxr_k<8, 2, false>, (const void *)conv_mxr_k<4, 1, false>, (const void *)conv_mxr_k<4, 2, false>,
-                             (const void *)conv_mxr_k<8, 1, true>, (const void *)conv_mxr_k<8, 2, true>, (const void *)conv_mxr_k<4, 1, true>, (const void *)conv_mxr_k<4, 2, true>};
-        for (int i = 0; i < 8; i++) {
+        const void *ks[12] = {(const void *)conv_mxr_k<8, 1, false, false>, (const void *)conv_mxr_k<8, 2, false, false>, (const void *)conv_mxr_k<4, 1, false, false>, (const void *)conv_mxr_k<4, 2, false, false>,
+                              (const void *)conv_mxr_k<8, 1, true, false>, (const void *)conv_mxr_k<8, 2, true, false>, (const void *)conv_mxr_k<4, 1, true, false>, (const void *)conv_mxr_k<4, 2, true, false>,
+                              (const void *)conv_mxr_k<8, 1, false, true>, (const void *)conv_mxr_k<8, 2, false, true>, (const void *)conv_mxr_k<4, 1, false, true>, (const void *)conv_mxr_k<4, 2, false, true>};
+        for (int i = 0; i < 12; i++) {
             const cudaError_t er = cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
         }
         attr_set[dev & 15] = 1;
     }
-    const int variant = (coef ? 4 : 0) | (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+    const int variant = (coef ? 4 : a.gather ? 8 : 0) | (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+#define UMX_R_GO(B, NC, ST, GA) umx_launch(conv_mxr_k<B, NC, ST, GA>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break
     switch (variant) {
-    case 0: umx_launch(conv_mxr_k<8, 1, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 1: umx_launch(conv_mxr_k<8, 2, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 2: umx_launch(conv_mxr_k<4, 1, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 3: umx_launch(conv_mxr_k<4, 2, false>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 4: umx_launch(conv_mxr_k<8, 1, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 5: umx_launch(conv_mxr_k<8, 2, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    case 6: umx_launch(conv_mxr_k<4, 1, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
-    default: umx_launch(conv_mxr_k<4, 2, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break;
+    case 0: UMX_R_GO(8, 1, false, false);
+    case 1: UMX_R_GO(8, 2, false, false);
+    case 2: UMX_R_GO(4, 1, false, false);
+    case 3: UMX_R_GO(4, 2, false, false);
+    case 4: UMX_R_GO(8, 1, true, false);
+    case 5: UMX_R_GO(8, 2, true, false);
+    case 6: UMX_R_GO(4, 1, true, false);
+    case 7: UMX_R_GO(4, 2, true, false);
+    case 8: UMX_R_GO(8, 1, false, true);
+    case 9: UMX_R_GO(8, 2, false, true);
+    case 10: UMX_R_GO(4, 1, false, true);
+    default: UMX_R_GO(4, 2, false, true);
     }
+#undef UMX_R_GO
     return 0;
 }

@@ -23,9 +23,6 @@ void umx_prof_close(int id);
    likes to let its own successor be scheduled.  What is gained is the launch latency (and, in the conv kernels, the prologue: barrier
    set-up, TMEM allocation, weight loads) of some 80 dependent launches per forward.  UMX_PDL=0 in the environment turns it off. ---- */
 int umx_pdl(void);
-/* > 0 while the next launches must wait for everything before them in the stream (a conv whose weight images were prepared just ahead of it
-   reads them before its pdl_wait) */
-extern thread_local int umx_plain_launch;
 #ifdef __CUDACC__
 #include <string.h>
 template <typename... KA, typename... A>
@@ -34,7 +31,7 @@ static inline void umx_launch(void (*kern)(KA...), dim3 grid, dim3 block, size_t
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = 0;
     cudaLaunchAttribute at[1]; memset(at, 0, sizeof at);
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
-    if (umx_pdl() && !umx_plain_launch) { cfg.attrs = at; cfg.numAttrs = 1; }
+    if (umx_pdl()) { cfg.attrs = at; cfg.numAttrs = 1; }
     cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
 }
 /* the same in clusters of blocks */
@@ -45,7 +42,7 @@ static inline void umx_launch_cluster(void (*kern)(KA...), dim3 grid, dim3 clust
     cudaLaunchAttribute at[2]; memset(at, 0, sizeof at);
     at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = cluster.x; at[0].val.clusterDim.y = cluster.y; at[0].val.clusterDim.z = cluster.z;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = umx_pdl() && !umx_plain_launch ? 2 : 1;
+    cfg.attrs = at; cfg.numAttrs = umx_pdl() ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
 }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
