@@ -89,27 +89,26 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
     const long long j0 = a.jobs * (long long)blockIdx.x / (long long)gridDim.x, j1 = a.jobs * ((long long)blockIdx.x + 1) / (long long)gridDim.x;
 
     if (warp == 0) {
-        /* ---------------- producer ---------------- */
-        if (lane == 0) {
-            tma_prefetch_desc(&map0); tma_prefetch_desc(&maps);
-            pdl_wait();      /* the only role that reads activations from global memory; every other role's data comes through this thread's loads,
-                                so the weight load, the B scale copies and the zeroing of the accumulators overlap the previous kernel */
-            int s = 0, ph = 0, it = 0; bool ok = true;
-            /* job = (row tile, column tile), column tile fastest; the indices advance incrementally (no division per job) */
-            int ntile = (int)(j0 % a.ntiles), n = (int)((j0 / a.ntiles) / a.rtiles_per_n), tin = (int)((j0 / a.ntiles) % a.rtiles_per_n);
-            for (long long job = j0; job < j1 && ok; job++) {
-                const int cx = tin * 256, pl0 = BITS == 8 ? n * a.nkb * 2 : n * a.nkb, cs = tin * 128, pls = n * a.nkb;
-                for (int g = 0; g < a.ngroups; g++) {
-                    if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 1, it); ok = false; break; }
-                    const int items = min(4, a.nki - 4 * g);
-                    const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
-                    mbar_expect_tx(bar, (uint32_t)(items * 4096 + a.sw_rows * 128));
-                    for (int j = 0; j < items; j++) tma_load_2d(sb + j * 4096, &map0, bar, cx, pl0 + 2 * (4 * g + j));
-                    tma_load_2d(sb + a.offSW, &maps, bar, cs, pls + a.sw_rows * g);
-                    it++; if (++s == R) { s = 0; ph ^= 1; }
-                }
-                if (++ntile == a.ntiles) { ntile = 0; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
+        /* ---------------- producer: the whole warp runs the loop on uniform values, one lane issues ---------------- */
+        const uint32_t lead = elect_one();
+        if (lead) { tma_prefetch_desc(&map0); tma_prefetch_desc(&maps); }
+        pdl_wait();      /* the only role that reads activations from global memory; every other role's data comes through these loads, so the weight load and the B scale copies
+                            overlap the previous kernel */
+        int s = 0, ph = 0, it = 0; bool ok = true;
+        /* job = (row tile, column tile), column tile fastest; the indices advance incrementally (no division per job) */
+        int ntile = (int)(j0 % a.ntiles), n = (int)((j0 / a.ntiles) / a.rtiles_per_n), tin = (int)((j0 / a.ntiles) % a.rtiles_per_n);
+        for (long long job = j0; job < j1 && ok; job++) {
+            const int cx = tin * 256, pl0 = BITS == 8 ? n * a.nkb * 2 : n * a.nkb, cs = tin * 128, pls = n * a.nkb;
+            for (int g = 0; g < a.ngroups; g++) {
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 1, it); ok = false; break; }
+                const int items = min(4, a.nki - 4 * g);
+                const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
+                if (lead) mbar_expect_tx(bar, (uint32_t)(items * 4096 + a.sw_rows * 128));
+                for (int j = 0; j < items; j++) tma_load_2d(sb + j * 4096, &map0, bar, cx, pl0 + 2 * (4 * g + j), lead);
+                tma_load_2d(sb + a.offSW, &maps, bar, cs, pls + a.sw_rows * g, lead);
+                it++; if (++s == R) { s = 0; ph ^= 1; }
             }
+            if (++ntile == a.ntiles) { ntile = 0; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
         }
     } else if (warp == 1) {
         /* ---------------- MMA issue (the warp runs the loop, one lane issues) ---------------- */
@@ -135,8 +134,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_acce + 8 * slot, (uint32_t)(sph ^ 1), abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 7, it); break; }
                 for (int g = 0; g < a.ngroups; g++) {
                     if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 3, it); ok = false; break; }
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 2, it); ok = false; break; }
-                    tc_fence_after();
+                    tc_fence_after();                            /* the scale warp passed the stage's load barrier before: the codes have landed too */
                     const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = tmem + (uint32_t)a.sfa_base + ((uint32_t)it & 1u) * 8u;
                     const uint32_t sfb_t = tmem + (uint32_t)a.sfb_base + (uint32_t)((ntile * a.ngroups + g) * NQ * 4);
                     const uint32_t bb = b_lo0 + (uint32_t)ntile * b_tile + (uint32_t)(4 * g) * b_item;
@@ -150,8 +148,9 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
                         const uint64_t ad = desc_make(a_lo + (uint32_t)j * 256u, a_hi), bd = desc_make(bb + (uint32_t)j * b_item, b_hi);
                         if (BITS == 8) umma_mxf8(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead); else umma_mxf4(d, ad, bd, idesc, acc, sfa_t + 4 * q, sfb_t + 4 * q, lead);
                     }
-                    if (g == a.ngroups - 1) umma_commit(bar_accf + 8 * slot, lead);
-                    umma_commit(bar_empty + 8 * s, lead);
+                    /* one commit a stage: a second one right behind it costs this warp 135 clocks.  The last stage of a job completes its accumulators, and the epilogue, which waits for
+                       those, passes the stage back to the producer */
+                    umma_commit(g == a.ngroups - 1 ? bar_accf + 8 * slot : bar_empty + 8 * s, lead);
                     it++; if (++s == R) { s = 0; ph ^= 1; }
                 }
                 if (++slot == NS) { slot = 0; sph ^= 1; }
@@ -190,11 +189,14 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
         const uint32_t tlane = tmem + ((uint32_t)(q4 * 32) << 16);
         int slot = eg, sph = 0; bool dead = false;
         const unsigned Su = (unsigned)a.S;
+        int last_s = ((eg + 1) * a.ngroups - 1) % R;                 /* ring slot of the last stage of this group's job */
         long long job = j0 + eg;
         int ntile = (int)(job % a.ntiles), n = (int)((job / a.ntiles) / a.rtiles_per_n), tin = (int)((job / a.ntiles) % a.rtiles_per_n);
         for (; job < j1 && !dead; job += 2) {
             const int n_cur = min(a.ntp, a.cop - ntile * a.ntp), nchunk = n_cur >> 5, cb = ntile * (a.ntp >> 5);
             if (!mbar_wait(bar_accf + 8 * slot, (uint32_t)sph, abort_flag, kWaitLimitP)) { raise_p(a, abort_flag, 5, (int)(job - j0)); dead = true; break; }
+            if (q4 == 0 && lane == 0) mbar_arrive(bar_empty + 8 * last_s);
+            for (last_s += 2 * a.ngroups; last_s >= R;) last_s -= R;
             tc_fence_after();
             const uint32_t tcol = tlane + (uint32_t)(slot * a.ntp);
             const unsigned vo = (unsigned)tin * 128u + (unsigned)r;
