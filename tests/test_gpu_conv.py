@@ -71,6 +71,22 @@ def test_conv3_stride2_parity(dev, N, Ci, Co, D, H, W, bits):
     assert np.array_equal(got, run_pm32("conv3s2", mx, w, b, N, Ci, D, H, W, Co, bits, split=False))    # reference-layout input
 
 
+@pytest.mark.parametrize("N,Ci,Co,D,H,W", [
+    (1, 32, 32, 3, 19, 11),            # general kernel, ragged tiles
+    (2, 256, 128, 3, 16, 16),          # K split over a cluster
+    (2, 64, 96, 5, 18, 16),            # batch, three column tiles
+    (1, 32, 32, 40, 40, 45),           # z-marching kernel, gathered scale window
+    (1, 64, 64, 24, 48, 32),           # z-marching kernel, scale window by TMA
+])
+def test_conv3_reads_the_reference_layout(dev, N, Ci, Co, D, H, W):
+    """MX-fp8 codes in 32-byte rows and in the split layout: the same products in the same order, the same bits."""
+    x = synth.rng(51).standard_normal(N * Ci * D * H * W).astype(np.float32)
+    w, b = synth.kaiming(52, Co, Ci, 27), synth.bias(53, Co, 0.1)
+    mx = orc.pm_to_mx(x, 0, N, Ci, D * H * W, 8)
+    got = run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8, split=False)
+    assert np.isfinite(got).all() and np.array_equal(got, run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8))
+
+
 @pytest.mark.parametrize("Ci,Co,ybf", [(32, 32, 3), (64, 40, 4), (96, 64, 3), (8, 16, 4), (16, 32, 3)])
 def test_lp_conv_fwd_s2_mxfp4_input(dev, Ci, Co, ybf):
     """lp_conv_fwd_s2_f8 on an MX-fp4 tensor computes in MX-fp4 and says so (returns 3: src/lp_s2.cu:652-716), also for inputs and outputs of

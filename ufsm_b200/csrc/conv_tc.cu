@@ -54,6 +54,7 @@ struct ConvArgs {
     int ksplit;
     /* 3^3 stride-2 pad-1 conv: K item = (tap, input block), each item's A tile is its own strided TMA load from the input grid Di x Hi x Wi */
     int s2, nbi, nit, Di, Hi, Wi;       /* stride-2 conv: blocks of the input tensor, K items per tap, input grid */
+    int ref, half;                      /* 3^3 on MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load; bytes between the halves of a stage's A */
     EpiArgs e;
     int *err;
 };
@@ -151,7 +152,8 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 /* two 16-byte-wide planes per K item (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1) */
                 if (a.taps == 27) {
                     const int ki = st / 3, zi = z + st % 3 - 1;
-                    tma_load_4d(smem_u32(sb + a.offA), &map0, bar, (x0 - 1) * 16, y0 - 1, zi, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki, lead);
+                    if (BITS == 8 && a.ref) { tma_load_5d(smem_u32(sb + a.offA), &map0, bar, 0, x0 - 1, y0 - 1, zi, n * a.nkb + ki, lead); tma_load_5d(smem_u32(sb + a.offA) + 2944, &map0, bar, 16, x0 - 1, y0 - 1, zi, n * a.nkb + ki, lead); }
+                    else tma_load_4d(smem_u32(sb + a.offA), &map0, bar, (x0 - 1) * 16, y0 - 1, zi, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki, lead);
                 } else {
                     for (int j = 0; j < items; j++) {
                         const int ki = 4 * st + j;
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
             int it = 0, s = 0, ph = 0; bool ok = true;
             const uint32_t sb0 = smem_u32(stages), sstep = (uint32_t)a.stage_bytes >> 4;
             const uint32_t b_hi = desc_hi(128), a_hi = a.taps == 27 ? desc_hi(160) : desc_hi(128);
-            const uint32_t a_lo0 = desc_lo(sb0 + a.offA, a.taps == 27 ? 2880 : 2048), b_lo0 = desc_lo(sb0 + a.offW, (uint32_t)a.nt * 16);
+            const uint32_t a_lo0 = desc_lo(sb0 + a.offA, (uint32_t)a.half), b_lo0 = desc_lo(sb0 + a.offW, (uint32_t)a.nt * 16);
             const uint32_t idesc0 = BITS == 8 ? idesc_mxf8(n_cur, 0, 0) : idesc_mxf4(n_cur, 0, 0);
             const uint32_t bstep = (uint32_t)a.nt * 2;
             int buf = 0;
@@ -408,7 +410,7 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 }   // namespace
 
 int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e);
-int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, void *enc, int N, int D, int H, int W, const EpiArgs &e,
+int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, int ref, void *enc, int N, int D, int H, int W, const EpiArgs &e,
                    double *part, const float *gamma, const float *beta, float eps, float *coef);
 extern "C" void umx_in_stats_coef(const void *y, int N, int C, int D, int H, int W, const float *gamma, const float *beta, float eps, double *part, float *coef);
 void umx_in_part(const void *y, int N, int C, int D, int H, int W, double *part);
@@ -572,7 +574,7 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     a.N = N; a.D = D; a.H = H; a.W = W; a.nkb = c->nkb; a.nki = c->nki; a.taps = c->taps; a.bits = c->bits;
     a.cop = c->cop; a.nt = c->nt; a.ntiles_n = c->ntiles_n; a.tiles_x = ceil_div(W, 8); a.tiles_y = ceil_div(H, 16);
     a.w_stage_bytes = c->w_stage_bytes; a.nst = c->nst; a.items_max = c->items_max; a.ipq = c->ipq; a.nquad = c->nquad;
-    const int abytes = c->taps == 27 ? 5760 : 4 * 4096;
+    const int abytes = c->taps == 27 ? 2944 + 2880 : 4 * 4096;
     auto up128 = [](int v) { return (v + 127) & ~127; };
     a.offW = 0; a.offSFB = c->items_max * c->nt * 32; a.offA = up128(c->w_stage_bytes); a.offSFA = a.offA + up128(abytes);
     a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
@@ -613,7 +615,11 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     }
     /* tensor map over the activation codes seen as 16-byte-wide planes [plane][z][y][x * 16 B]: fp8 in the split layout has two planes a
        block, fp4 one.  A box is (10 or 8 voxels) x (18 or 16 rows) x 1 plane of z x 2 planes; voxels outside the volume read as zero. */
-    if (c->bits == 8 && !(flags & UMX_X_SPLIT)) {   /* reference layout: re-lay the codes into scratch first */
+    /* MX-fp8 in the reference's layout: a 3^3 conv loads the two halves of the 32-byte rows apart; a one-tap conv has its codes re-laid into scratch first.  32 -> 32 on
+       7 x 9 x 11 11.1 us with a relayout pass ahead, 7.0 this way, on 64^3 17.4 and 13.3, on 128^3 88 and 63; 256 -> 256 on 15 x 18 x 20 26.7 and 24.5: pieces of 16 bytes hold neither kernel up. */
+    a.ref = c->bits == 8 && !(flags & UMX_X_SPLIT) && c->taps == 27;
+    a.half = a.ref ? 2944 : c->taps == 27 ? 2880 : 2048;
+    if (c->bits == 8 && !(flags & UMX_X_SPLIT) && !a.ref) {
         void *ws = umx_ws(1, umx_mx_bytes32(8, N, nbx * 32, Sx));
         if (!ws) return -1;
         umx_mx_codes_to_split(x, (size_t)N * nbx, Sx, ws);         /* the scale plane stays where it is */
@@ -627,6 +633,11 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         const cuuint32_t box[5] = {16, 16, 32, 1, 2}, es[5] = {1, 2, 2, 1, 1};
         const CUresult r0 = enc(&m0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)x, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) { char b[160]; snprintf(b, sizeof b, "umx_conv_fwd: cuTensorMapEncodeTiled failed (%d) for the stride-2 map of %d x %d x %d x %d, %d blocks", (int)r0, N, Dx, Hx, Wx, nbx); umx_latch_msg(b); return -1; }
+    } else if (a.ref) {
+        const cuuint64_t gd[5] = {32, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N * c->nkb}, gs[4] = {32, (cuuint64_t)W * 32, (cuuint64_t)W * H * 32, (cuuint64_t)S * 32};
+        const cuuint32_t box[5] = {16, 10, 18, 1, 1}, es[5] = {1, 1, 1, 1, 1};
+        const CUresult r0 = enc(&m0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)x, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r0 != CUDA_SUCCESS) { char b[160]; snprintf(b, sizeof b, "umx_conv_fwd: cuTensorMapEncodeTiled failed (%d) for %d x %d x %d x %d, %d blocks of 32-byte rows", (int)r0, N, D, H, W, c->nkb); umx_latch_msg(b); return -1; }
     } else {
         const cuuint32_t bx = c->taps == 27 ? 10 : 8, by = c->taps == 27 ? 18 : 16;
         const cuuint64_t gd[4] = {(cuuint64_t)W * 16, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N * c->nkb * (c->bits == 8 ? 2 : 1)};
@@ -639,9 +650,9 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     if (!force_v1 && c->kind == UMX_CONV3 && (c->wr || (c->w_src && umx_conv_r_takes(c, a.x_sc, N, D, H, W, a.e) && image_for_call((umx_conv *)c, 1)))) {   /* resident weights: the persistent z-marching kernel, when the geometry allows */
         const int pid = umx_prof_open(flops);
         a.e.bias = c->bias_p;
-        int rc = (nrm && (flags & UMX_STATS_EPILOGUE)) ? umx_conv_fwd_r(c, a.x_sc, &m0, (void *)enc, N, D, H, W, a.e, part, nrm->gamma, nrm->beta, nrm->eps, nrm->coef) : 1;
+        int rc = (nrm && (flags & UMX_STATS_EPILOGUE)) ? umx_conv_fwd_r(c, a.x_sc, &m0, a.ref, (void *)enc, N, D, H, W, a.e, part, nrm->gamma, nrm->beta, nrm->eps, nrm->coef) : 1;
         const bool fused = rc == 0;
-        if (rc > 0) rc = umx_conv_fwd_r(c, a.x_sc, &m0, (void *)enc, N, D, H, W, a.e, nullptr, nullptr, nullptr, 0.f, nullptr);
+        if (rc > 0) rc = umx_conv_fwd_r(c, a.x_sc, &m0, a.ref, (void *)enc, N, D, H, W, a.e, nullptr, nullptr, nullptr, 0.f, nullptr);
         if (rc <= 0) {
             umx_prof_close(pid);
             g_umx_launches++; g_last_kernel = 1;

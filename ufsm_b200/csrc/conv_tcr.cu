@@ -75,6 +75,7 @@ struct ConvRArgs {
        turns them into coefficients (a, b) per (sample, channel) */
     double *part; float *coef; const float *gamma, *beta; float eps; int cop, off_red;
     const uint8_t *wr, *x_sc;
+    int ref;                                     /* MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load, the halves 2944 bytes apart in a stage */
     int gather, w_dep;                           /* see GATHER; the weights and the bias were written by a kernel just ahead in the stream */
     EpiArgs e;
     int *err;
@@ -253,7 +254,8 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
                         /* codes: two 16-byte-wide planes (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1), 18 rows of 10 voxels;
                            scale bytes: 18 rows of a 32-byte window per block */
-                        tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki, lead);
+                        if (BITS == 8 && a.ref) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + ki, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + ki, lead); }
+                        else tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki, lead);
                         if (!GATHER) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki, lead);
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int nsf = a.nki * a.nquad * a.gt;
                 for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi), lead);
             }
-            const uint32_t a_lo0 = desc_lo(smem_u32(stages), 2880), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
+            const uint32_t a_lo0 = desc_lo(smem_u32(stages), BITS == 8 && a.ref ? 2944u : 2880u), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
             const uint32_t sfa_t0 = tmem + (uint32_t)a.sfa_base, sfa_cols = (uint32_t)a.sfa_cols;
             int s = 0, ph = 0, it = 0;
             while (ok) {
@@ -803,11 +805,11 @@ int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H
     ConvRArgs a; int grid;
     return r_plan(c, x_sc, N, D, H, W, e, 0, nullptr, a, &grid);
 }
-/* x_sc: the MX tensor's scale plane; m0: tensor map over its codes (fp8 in the split layout); enc: the driver's tensor-map encoder (for the scale plane).
+/* x_sc: the MX tensor's scale plane; m0: tensor map over its codes (fp8 in the split layout; ref: in the reference's); enc: the driver's tensor-map encoder (for the scale plane).
    Returns 1 when this kernel does not apply to the geometry (the caller then takes the general kernel), 0 after a launch, -1 on error. */
 /* coef != NULL (only with the blocked fp16 output): InstanceNorm coefficients are produced by the same launch; part then holds N x (blocks per
    column tile, at most 512) x cop x 2 doubles of scratch */
-int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, void *enc_v, int N, int D, int H, int W, const EpiArgs &e,
+int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, int ref, void *enc_v, int N, int D, int H, int W, const EpiArgs &e,
                    double *part, const float *gamma, const float *beta, float eps, float *coef) {
     typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -824,7 +826,7 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
         const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) return 1;                        /* e.g. a scale plane that is not 16-byte aligned: take the general kernel */
     }
-    a.wr = c->wr; a.x_sc = x_sc; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
+    a.wr = c->wr; a.x_sc = x_sc; a.ref = ref; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
     static int attr_set[16];
