@@ -66,6 +66,7 @@ struct ConvRArgs {
     int tiles_x, tiles, ncol, gcol;              /* column tiles of nt channels; blocks per column tile */
     long long units;                             /* N x tiles x D output planes of one tile, split evenly over the grid */
     int ring, stage_bytes, offSW, offSFA;
+    int ips, item_bytes;                         /* input items of a stage (one plane's; the last stage of a plane may have fewer), bytes of one's codes, window and scales */
     int w_bytes, w_codes, nquad, gt, goff1, goff2, nslot;
     int tmem_cols, sfa_base, sfa_cols, sfb_base; /* TMEM: accumulator slots from 0, two A scale buffers, B scales */
     int off_rec, off_bias, off_stage, off_w, off_ring;   /* off_stage (with statistics or a plane-major output): 2 KB per epilogue warp (and 32-channel chunk), the fp16 rows on their way to wide stores */
@@ -86,7 +87,7 @@ struct StageRec {
     uint32_t d1, idn1, bb1, sfb1;      /* first group: TMEM accumulator address, instruction descriptor with N, B descriptor low word of tap 0, B scale address */
     uint32_t d2, idn2, bb2, sfb2;      /* second group when the window wraps (idn2 = 0: none) */
     uint32_t wait0, wait1;             /* accumulator-empty barriers to pass first: address | parity << 31 (0: none) */
-    uint32_t commit0, commit1;         /* accumulator-full barriers to commit after the stage (0: none) */
+    uint32_t items, pad0;              /* input items of the stage */
     uint32_t last, pad[3];
 };
 static_assert(sizeof(StageRec) == 64, "stage record is 64 bytes");
@@ -163,8 +164,8 @@ __device__ unsigned g_conv_tickets[64];      /* one per column tile; the block t
 
 /* NCH: 32-channel chunks of the column tile (1: two blocks per multiprocessor and at most 128 registers; 2: one block, more registers);
    STATS: the epilogue also takes the InstanceNorm sums; GATHER: the scale warp fetches its window of scale bytes itself, for scale planes whose rows TMA does not
-   take (W not a multiple of 16) */
-template <int BITS, int NCH, bool STATS, bool GATHER>
+   take (W not a multiple of 16); MULTI: a stage holds up to a.ips input items of its plane (see r_plan), else one */
+template <int BITS, int NCH, bool STATS, bool GATHER, bool MULTI>
 __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap maps, const ConvRArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint64_t *bars = (uint64_t *)smem_raw;
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     float *bias_s = (float *)(smem_raw + a.off_bias);
     uint8_t *wsm = smem_raw + a.off_w, *stages = smem_raw + a.off_ring;
     const int warp = (int)uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int R = a.ring, NS = a.nslot;
+    const int R = a.ring, NS = a.nslot, ips = MULTI ? a.ips : 1;
     /* barriers: tma[R] (codes + scale window landed), sf[R] (A scales laid out), empty[R], accumulator full / empty per slot, weights */
     const uint32_t bar_tma = smem_u32(bars), bar_sf = bar_tma + 8 * R, bar_empty = bar_tma + 16 * R, bar_accf = bar_tma + 24 * R, bar_acce = bar_accf + 8 * kMaxSlots, bar_w = bar_acce + 8 * kMaxSlots, bar_red = bar_w + 8;
     constexpr int NQ = BITS == 8 ? 3 : 5;                  /* A scale quads per stage */
@@ -239,24 +240,27 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     }
                     const int slot = NS - 1 - pos, n1 = min(cnt, NS - slot), n2 = cnt - n1;
                     const uint32_t g1 = (uint32_t)(dzf == 0 ? 0 : dzf == 1 ? a.goff1 : a.goff2), g2 = (uint32_t)(dzf + n1 == 1 ? a.goff1 : a.goff2);
-                    for (int ki = 0; ki < a.nki; ki++) {
+                    for (int ki = 0; ki < a.nki; ki += ips) {
                         if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 1, it, bar_empty + 8 * s - bar_tma, ph ^ 1); ok = false; break; }
-                        const bool kl = ki == a.nki - 1;
+                        const int nit = MULTI ? min(ips, a.nki - ki) : 1;
+                        const bool kl = ki + nit == a.nki;
                         const uint32_t bk = b_lo0 + (uint32_t)ki * bstep9, sk = sfb_t0 + (uint32_t)ki * sfb_per_ki;
                         if (lead) {
                             uint4 *r = (uint4 *)(recs + s);
                             r[0] = make_uint4(tmem + (uint32_t)slot * nt, idesc_b | (uint32_t)n1 * ntn, bk + (uint32_t)dzf * nt, sk + g1);
                             r[1] = make_uint4(tmem, n2 ? (idesc_b | (uint32_t)n2 * ntn) : 0u, bk + (uint32_t)(dzf + n1) * nt, sk + g2);
-                            r[2] = make_uint4(ki == 0 ? w0 : 0u, ki == 0 ? w1 : 0u, 0u, 0u);
+                            r[2] = make_uint4(ki == 0 ? w0 : 0u, ki == 0 ? w1 : 0u, (uint32_t)nit, 0u);
                             r[3] = make_uint4((last_run && zi == zhi && kl) ? 1u : 0u, 0u, 0u, 0u);
-                            mbar_expect_tx(bar_tma + 8 * s, TX);
+                            mbar_expect_tx(bar_tma + 8 * s, TX * (uint32_t)nit);
                         }
-                        const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
+                        uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes); const uint32_t bar = bar_tma + 8 * s;
                         /* codes: two 16-byte-wide planes (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1), 18 rows of 10 voxels;
                            scale bytes: 18 rows of a 32-byte window per block */
-                        if (BITS == 8 && a.ref) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + ki, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + ki, lead); }
-                        else tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * ki, lead);
-                        if (!GATHER) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + ki : pls + 2 * ki, lead);
+                        for (int k = ki; k < ki + (MULTI ? nit : 1); k++, sb += (uint32_t)a.item_bytes) {
+                            if (BITS == 8 && a.ref) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + k, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + k, lead); }
+                            else tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * k, lead);
+                            if (!GATHER) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + k : pls + 2 * k, lead);
+                        }
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
                 }
@@ -282,6 +286,8 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             }
             const uint32_t a_lo0 = desc_lo(smem_u32(stages), BITS == 8 && a.ref ? 2944u : 2880u), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
             const uint32_t sfa_t0 = tmem + (uint32_t)a.sfa_base, sfa_cols = (uint32_t)a.sfa_cols;
+            const uint32_t i_step = (uint32_t)a.item_bytes >> 4, bstep9 = 9u * 2u * 3u * 32u * NCH, sfb_step = (uint32_t)(a.nquad * a.gt * 4);
+            uint32_t item = 0;
             int s = 0, ph = 0, it = 0;
             while (ok) {
                 /* the stage's A scales are laid out; the scale warp passed the stage's load barrier before, so the codes have landed too */
@@ -295,12 +301,25 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     if (!__all_sync(0xffffffffu, got)) { if (lane == 0) raise_r(a, abort_flag, 7, it, (wc.x & 0x7fffffffu) - bar_tma, wc.x >> 31); break; }
                 }
                 tc_fence_after();
-                const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = sfa_t0 + ((uint32_t)it & 1u) * sfa_cols;
-                /* copies and MMAs of one thread run in issue order, so a buffer is overwritten after the MMAs that read it two stages ago */
+                /* copies and MMAs of one thread run in issue order, so a buffer is overwritten after the MMAs that read it two items ago */
+                if (!MULTI) {
+                    const uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, sfa_t = sfa_t0 + ((uint32_t)it & 1u) * sfa_cols;
 #pragma unroll
-                for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi), lead);
-                issue_group<BITS, 32 * NCH>(g1.x, g1.y, g1.z, g1.w, a_lo, a_hi, b_hi, sfa_t, lead);
-                if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, g2.z, g2.w, a_lo, a_hi, b_hi, sfa_t, lead);
+                    for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi), lead);
+                    issue_group<BITS, 32 * NCH>(g1.x, g1.y, g1.z, g1.w, a_lo, a_hi, b_hi, sfa_t, lead);
+                    if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, g2.z, g2.w, a_lo, a_hi, b_hi, sfa_t, lead);
+                } else {
+                    uint32_t a_lo = a_lo0 + (uint32_t)s * a_step, bb1 = g1.z, sf1 = g1.w, bb2 = g2.z, sf2 = g2.w;
+                    for (uint32_t i = 0; i < wc.z; i++) {
+                        const uint32_t sfa_t = sfa_t0 + (item & 1u) * sfa_cols;
+                        item++;
+#pragma unroll
+                        for (int q = 0; q < NQ; q++) utccp_32x128b(sfa_t + 4 * q, desc_make((a_lo & 0xffffu) + sfa_off + 32u * q, sf_hi), lead);
+                        issue_group<BITS, 32 * NCH>(g1.x, g1.y, bb1, sf1, a_lo, a_hi, b_hi, sfa_t, lead);
+                        if (g2.y) issue_group<BITS, 32 * NCH>(g2.x, g2.y, bb2, sf2, a_lo, a_hi, b_hi, sfa_t, lead);
+                        a_lo += i_step; bb1 += bstep9; bb2 += bstep9; sf1 += sfb_step; sf2 += sfb_step;
+                    }
+                }
                 /* the one commit of a stage: "stage s has been consumed".  The producer reuses the ring slot on it, and the relay passes the news that output
                    planes are complete on to the epilogue */
                 umma_commit(bar_empty + 8 * s, lead);
@@ -316,9 +335,10 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
            memory in the tcgen05.cp layout, as far ahead of the MMAs as the ring is deep. */
         int it = 0, s = 0, ph = 0; bool ok = true;
         /* one stage: window -> scale sets; off: this lane's first byte of the window, gw: the window's bytes (GATHER) */
-        auto lay = [&](int off, const unsigned *gw) {
+        auto lay = [&](int off, int nit, const unsigned *gw) {
             if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * s, ph); ok = false; return; }
             uint8_t *stg = stages + (size_t)s * a.stage_bytes;
+            for (int i = 0; i < (MULTI ? nit : 1); i++, stg += a.item_bytes) {
             if (GATHER) {
 #pragma unroll
                 for (int k = 0; k < GN; k++) {
@@ -350,6 +370,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             /* quad qd: word (lane, column) = row 32 * column + lane; a lane's four columns are 16 contiguous bytes: one store */
 #pragma unroll
             for (int qd = 0; qd < NQ; qd++) *(uint4 *)(sfa + qd * 128 + lane * 4) = make_uint4(wq[0][qd], wq[1][qd], wq[2][qd], wq[3][qd]);
+            }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_sf + 8 * s);
@@ -362,8 +383,8 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int x0 = (rn.txy % a.tiles_x) * 8;
                 const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
                 const int off = off0 + (x0 - 1) - (((x0 - 1) >> 4) << 4);
-                const int nst = (zhi - zlo + 1) * a.nki;
-                for (int i = 0; i < nst && ok; i++) lay(off, nullptr);
+                for (int zi = zlo; zi <= zhi && ok; zi++)
+                    for (int ki = 0; ki < a.nki && ok; ki += ips) lay(off, MULTI ? min(ips, a.nki - ki) : 1, nullptr);
             }
         } else {
             /* The window is 18 rows of 10 bytes (two of them for fp4): of each the three words that begin at its first byte, every one put together from the two aligned words
@@ -413,9 +434,9 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             bool l0 = live; fetch(g0);
             bool l1 = live; fetch(g1);
             while (ok && l0) {
-                lay(off0, g0); l0 = live; fetch(g0);
+                lay(off0, 1, g0); l0 = live; fetch(g0);
                 if (!ok || !l1) break;
-                lay(off0, g1); l1 = live; fetch(g1);
+                lay(off0, 1, g1); l1 = live; fetch(g1);
             }
         }
     } else if (warp == 3) {
@@ -429,7 +450,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const Run rn = next_run(a, piece);
                 const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
                 for (int zi = zlo; zi <= zhi && ok; zi++) {
-                    for (int ki = 0; ki < a.nki; ki++) {
+                    for (int ki = 0; ki < a.nki; ki += ips) {
                         if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, kWaitLimitR)) { raise_r(a, abort_flag, 2, it, bar_empty + 8 * s - bar_tma, ph); ok = false; break; }
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
@@ -776,13 +797,21 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     a.cop = c->cop;
     /* the codes and the scale window are TMA destinations (128-byte aligned) */
     a.offSW = 5888; a.offSFA = a.offSW + (c->bits == 8 ? 640 : 1152);
-    a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
+    a.item_bytes = a.offSFA + c->nquad * 512;                          /* a multiple of 128 */
+    a.stage_bytes = (a.item_bytes + 1023) & ~1023;
     a.off_rec = 1024; a.off_bias = a.off_rec + 12 * 64; a.off_stage = 2048; a.off_red = a.off_stage; a.off_w = a.off_stage + (want_coef ? 8192 * (g.nt == 32 ? 1 : 2) : a.fast_pm16 ? 8192 : 0); a.off_ring = (a.off_w + a.w_bytes + 1023) & ~1023;
     int dev = 0, sms = 148; cudaGetDevice(&dev);
     { static int sms_of[16]; if (!sms_of[dev & 15]) { int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); sms_of[dev & 15] = v; } sms = sms_of[dev & 15]; }   /* looked up once per device */
     /* two blocks a multiprocessor when shared memory (113 KB each) and TMEM (256 columns each) allow */
     const int two = g.tmem_cols == 256 && a.off_ring + 4 * a.stage_bytes <= 113 * 1024;
     const int room = (two ? 113 : 227) * 1024 - a.off_ring;
+    /* Input items of a stage: what the MMA warp does once a stage (its barrier, record and commit, some 380 clocks) is as much as half of an item's MMAs, so a stage takes as many items
+       of its plane as leave three stages, at most four, where a block has four planes or more (with fewer, the first MMAs wait for more bytes than that is worth: 64 -> 64 on 32^3
+       12.7 us, 13.6 with two).  With one item and this way, us, 128 -> 64 on 64^3 63.9 and 56.9, 96 -> 32 on 64^3 31.8 and 30.2, 64 -> 32 on 128^3 115.6 and 112.1; MX-fp4 128 -> 64 on
+       64^3 31.3 and 30.3. */
+    a.ips = 1;
+    if (!a.gather && !want_coef && a.units * g.ncol >= 4ll * sms * (two ? 2 : 1)) for (int k = 2; k <= 4 && k <= a.nki; k++) if (3 * k * a.item_bytes <= room) a.ips = k;
+    if (a.ips > 1) a.stage_bytes = a.ips * a.item_bytes;
     a.ring = room / a.stage_bytes; if (a.ring > 12) a.ring = 12;
     if (a.ring < 3) return 0;
     long long slots = (long long)sms * (two ? 2 : 1) / g.ncol;      /* blocks per column tile */
@@ -831,31 +860,25 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
     static int attr_set[16];
     if (!attr_set[dev & 15]) {
-        const void *ks[12] = {(const void *)conv_mxr_k<8, 1, false, false>, (const void *)conv_mxr_k<8, 2, false, false>, (const void *)conv_mxr_k<4, 1, false, false>, (const void *)conv_mxr_k<4, 2, false, false>,
-                              (const void *)conv_mxr_k<8, 1, true, false>, (const void *)conv_mxr_k<8, 2, true, false>, (const void *)conv_mxr_k<4, 1, true, false>, (const void *)conv_mxr_k<4, 2, true, false>,
-                              (const void *)conv_mxr_k<8, 1, false, true>, (const void *)conv_mxr_k<8, 2, false, true>, (const void *)conv_mxr_k<4, 1, false, true>, (const void *)conv_mxr_k<4, 2, false, true>};
-        for (int i = 0; i < 12; i++) {
+#define UMX_R_KS(ST, GA, MU) (const void *)conv_mxr_k<8, 1, ST, GA, MU>, (const void *)conv_mxr_k<8, 2, ST, GA, MU>, (const void *)conv_mxr_k<4, 1, ST, GA, MU>, (const void *)conv_mxr_k<4, 2, ST, GA, MU>
+        const void *ks[16] = {UMX_R_KS(false, false, false), UMX_R_KS(true, false, false), UMX_R_KS(false, true, false), UMX_R_KS(false, false, true)};
+#undef UMX_R_KS
+        for (int i = 0; i < 16; i++) {
             const cudaError_t er = cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
         }
         attr_set[dev & 15] = 1;
     }
-    const int variant = (coef ? 4 : a.gather ? 8 : 0) | (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
-#define UMX_R_GO(B, NC, ST, GA) umx_launch(conv_mxr_k<B, NC, ST, GA>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break
-    switch (variant) {
-    case 0: UMX_R_GO(8, 1, false, false);
-    case 1: UMX_R_GO(8, 2, false, false);
-    case 2: UMX_R_GO(4, 1, false, false);
-    case 3: UMX_R_GO(4, 2, false, false);
-    case 4: UMX_R_GO(8, 1, true, false);
-    case 5: UMX_R_GO(8, 2, true, false);
-    case 6: UMX_R_GO(4, 1, true, false);
-    case 7: UMX_R_GO(4, 2, true, false);
-    case 8: UMX_R_GO(8, 1, false, true);
-    case 9: UMX_R_GO(8, 2, false, true);
-    case 10: UMX_R_GO(4, 1, false, true);
-    default: UMX_R_GO(4, 2, false, true);
-    }
+    const int variant = (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+#define UMX_R_GO(ST, GA, MU) do { switch (variant) { \
+        case 0: umx_launch(conv_mxr_k<8, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
+        case 1: umx_launch(conv_mxr_k<8, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
+        case 2: umx_launch(conv_mxr_k<4, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
+        default: umx_launch(conv_mxr_k<4, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); } } while (0)
+    if (coef) UMX_R_GO(true, false, false);
+    else if (a.gather) UMX_R_GO(false, true, false);
+    else if (a.ips > 1) UMX_R_GO(false, false, true);
+    else UMX_R_GO(false, false, false);
 #undef UMX_R_GO
     return 0;
 }
