@@ -805,18 +805,18 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     /* two blocks a multiprocessor when shared memory (113 KB each) and TMEM (256 columns each) allow */
     const int two = g.tmem_cols == 256 && a.off_ring + 4 * a.stage_bytes <= 113 * 1024;
     const int room = (two ? 113 : 227) * 1024 - a.off_ring;
+    long long slots = (long long)sms * (two ? 2 : 1) / g.ncol;      /* blocks per column tile */
+    if (slots < 1) return 0;
+    if (g_r_block_cap && slots > g_r_block_cap) slots = g_r_block_cap;
     /* Input items of a stage: what the MMA warp does once a stage (its barrier, record and commit, some 380 clocks) is as much as half of an item's MMAs, so a stage takes as many items
        of its plane as leave three stages, at most four, where a block has four planes or more (with fewer, the first MMAs wait for more bytes than that is worth: 64 -> 64 on 32^3
        12.7 us, 13.6 with two).  With one item and this way, us, 128 -> 64 on 64^3 63.9 and 56.9, 96 -> 32 on 64^3 31.8 and 30.2, 64 -> 32 on 128^3 115.6 and 112.1; MX-fp4 128 -> 64 on
        64^3 31.3 and 30.3. */
     a.ips = 1;
-    if (!a.gather && !want_coef && a.units * g.ncol >= 4ll * sms * (two ? 2 : 1)) for (int k = 2; k <= 4 && k <= a.nki; k++) if (3 * k * a.item_bytes <= room) a.ips = k;
+    if (!a.gather && !want_coef && a.units >= 4 * slots) for (int k = 2; k <= 4 && k <= a.nki; k++) if (3 * k * a.item_bytes <= room) a.ips = k;
     if (a.ips > 1) a.stage_bytes = a.ips * a.item_bytes;
     a.ring = room / a.stage_bytes; if (a.ring > 12) a.ring = 12;
     if (a.ring < 3) return 0;
-    long long slots = (long long)sms * (two ? 2 : 1) / g.ncol;      /* blocks per column tile */
-    if (slots < 1) return 0;
-    if (g_r_block_cap && slots > g_r_block_cap) slots = g_r_block_cap;
     /* A block pays two halo planes per run: with fewer than eight planes a block (counted for one sample, so that the choice of kernel does not
        depend on the batch) the general kernel is faster.  Volumes with fewer planes than blocks are left here: nothing to gain either way. */
     { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 0;
