@@ -187,3 +187,26 @@ def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
     assert np.array_equal(gote, wante), "%d of %d differ" % (np.count_nonzero(gote != wante), wante.size)
     assert np.array_equal(h16.view(np.float16).reshape(-1), got.astype(np.float16).reshape(-1))
     assert np.array_equal(q, orc.blocked_to_mx(orc.pm_to_blocked(got, N, Co, S), 8, N, Co, S))
+
+
+@pytest.mark.parametrize("kind,want_kernel,W", [("conv3", 1, 16), ("conv3", 1, 13), ("conv3s2", 4, 16)])
+def test_nan_scales_stay_in_their_sample(dev, kind, want_kernel, W):
+    """MX-fp4 with an odd number of blocks: the last item's second block has zero weights, and its scales are not those of the next sample (0xff, of a block with a NaN, would make NaN
+    of zero codes times zero weights)."""
+    N, Ci, Co, D, H = 2, 96, 32, 6, 16
+    S = D * H * W
+    x = synth.rng(351).standard_normal(N * Ci * S).astype(np.float32)
+    xn = x.copy()
+    xn[Ci * S:] = np.nan
+    w, b = synth.kaiming(352, Co, Ci, 27), synth.bias(353, Co, 0.1)
+    mx, want = orc.conv_case(kind, x, w, b, N, Ci, D, H, W, Co, 4)
+    mxn, _ = orc.conv_case(kind, xn, w, b, N, Ci, D, H, W, Co, 4)
+    dev.umx_conv_r_block_cap(1)
+    try:
+        got = run(kind, mx, w, b, N, Ci, D, H, W, Co, 4, want_kernel)
+        gotn = run(kind, mxn, w, b, N, Ci, D, H, W, Co, 4, want_kernel)
+    finally:
+        dev.umx_conv_r_block_cap(0)
+    half = got.size // 2
+    assert np.isfinite(got).all() and np.array_equal(got.reshape(-1)[:half], gotn.reshape(-1)[:half])
+    assert np.isnan(gotn.reshape(-1)[half:]).any()

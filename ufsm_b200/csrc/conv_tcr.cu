@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         for (int k = ki; k < ki + (MULTI ? nit : 1); k++, sb += (uint32_t)a.item_bytes) {
                             if (BITS == 8 && a.ref) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + k, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + k, lead); }
                             else tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * k, lead);
-                            if (!GATHER) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? pls + k : pls + 2 * k, lead);
+                            if (!GATHER) tma_load_5d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? k : 2 * k, rn.n, lead);
                         }
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
@@ -849,10 +849,11 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     const size_t S = (size_t)D * H * W;
     CUtensorMap ms; memset(&ms, 0, sizeof ms);
     if (!a.gather) {
-        const cuuint64_t gd[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N * c->nkb};
-        const cuuint64_t gs[3] = {(cuuint64_t)W, (cuuint64_t)W * H, (cuuint64_t)S};
-        const cuuint32_t box[4] = {32, 18, 1, (cuuint32_t)(c->bits == 8 ? 1 : 2)}, es[4] = {1, 1, 1, 1};
-        const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        /* samples as a dimension of their own: the second block of a MX-fp4 item past the last one reads the fill, not the next sample's scales (whose NaN would come through the zero weights) */
+        const cuuint64_t gd[5] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)c->nkb, (cuuint64_t)N};
+        const cuuint64_t gs[4] = {(cuuint64_t)W, (cuuint64_t)W * H, (cuuint64_t)S, (cuuint64_t)S * c->nkb};
+        const cuuint32_t box[5] = {32, 18, 1, (cuuint32_t)(c->bits == 8 ? 1 : 2), 1}, es[5] = {1, 1, 1, 1, 1};
+        const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) return 1;                        /* e.g. a scale plane that is not 16-byte aligned: take the general kernel */
     }
     a.wr = c->wr; a.x_sc = x_sc; a.ref = ref; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
