@@ -210,3 +210,37 @@ def test_nan_scales_stay_in_their_sample(dev, kind, want_kernel, W):
     half = got.size // 2
     assert np.isfinite(got).all() and np.array_equal(got.reshape(-1)[:half], gotn.reshape(-1)[:half])
     assert np.isnan(gotn.reshape(-1)[half:]).any()
+
+
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,bits,kernels", [
+    (3, 32, 96, 24, 20, 32, 8, (0, 1)),       # several column tiles: one wave of the general kernel's blocks alone, more in the batch
+    (3, 32, 96, 24, 20, 32, 4, (0, 1)),
+    (2, 96, 96, 24, 20, 32, 8, (0, 0)),       # MX-fp8 of several input items: an order of its own, so by one sample
+    (2, 64, 256, 24, 20, 32, 8, (1, 1)),      # more than one wave alone
+    (2, 96, 96, 24, 20, 32, 4, (0, 1)),       # a padded item
+    (4, 32, 32, 33, 31, 30, 8, (0, 1)),       # rows that TMA does not take
+    (4, 64, 32, 33, 31, 30, 8, (0, 0)),
+    (4, 64, 32, 33, 31, 30, 4, (0, 1)),
+    (8, 128, 128, 20, 16, 16, 8, (0, 0)),     # K split alone, so split in the batch too
+])
+def test_a_batch_may_take_the_other_kernel(dev, N, Ci, Co, D, H, W, bits, kernels):
+    """In MX-fp4 and with one input item the general kernel and the z-marching kernel add in one order, so that the choice between them may follow the batch: a sample's bits are those it
+    has alone."""
+    S = D * H * W
+    x = synth.rng(361).standard_normal(N * Ci * S).astype(np.float32) * np.exp2(synth.rng(362).integers(-6, 7, N * Ci * S)).astype(np.float32)
+    w, b = synth.kaiming(363, Co, Ci, 27), synth.bias(364, Co, 0.1)
+    got = run("conv3", orc.pm_to_mx(x, 0, N, Ci, S, bits, 32), w, b, N, Ci, D, H, W, Co, bits, kernels[1])
+    alone = run("conv3", orc.pm_to_mx(x[-Ci * S:], 0, 1, Ci, S, bits, 32), w, b, 1, Ci, D, H, W, Co, bits, kernels[0])
+    assert np.isfinite(got).all() and np.array_equal(got.reshape(N, -1)[-1], alone.reshape(-1))
+
+
+@pytest.mark.parametrize("Ci,bits,kernel", [(64, 8, 0), (32, 8, 1), (64, 4, 1)])
+def test_network_layers_keep_their_order_of_sums(dev, Ci, bits, kernel):
+    """Rows that TMA does not take, blocked halves out (a network's layer): several MX-fp8 input items are added item by item, by the general kernel, at every size."""
+    N, Co, D, H, W = 1, 32, 40, 64, 40
+    S = D * H * W
+    x = synth.rng(371).standard_normal(N * Ci * S).astype(np.float32)
+    c = G.Conv("conv3", synth.kaiming(372, Co, Ci, 27), synth.bias(373, Co, 0.1), Co, Ci, bits)
+    y, _ = c.fwd(orc.pm_to_mx(x, 0, N, Ci, S, bits, 32), N, D, H, W, G.OUT_H16B)
+    assert dev.umx_conv_last_kernel() == kernel and np.isfinite(y.view(np.float16)).all()
+    c.free()

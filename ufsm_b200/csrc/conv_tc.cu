@@ -105,8 +105,16 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = uni(*tmem_slot);
-    /* a stage is live unless it is a 3^3 stage whose input plane lies outside the volume (it would add zeros) */
-    auto stage_live = [&](int st) -> bool { if (a.taps != 27) return true; const int zi = z + st % 3 - 1; return zi >= 0 && zi < a.D; };
+    /* The order of a 3^3 block's stages (each the nine (dy, dx) of an input item and a dz): in MX-fp4 dz outermost, which is the z-marching kernel's order, so that the two give the same bits
+       and the choice between them may follow the batch; in MX-fp8 the items outermost.  A conv of one item has the two orders in one.  (MX-fp4 sums are exact in fp32 over many octaves of
+       scales, so its order seldom shows; in MX-fp8 it shows in the last bit, and a network of convs makes 3 to 7 % of that in its logits: codes next to a rounding boundary.) */
+    const int first_dz = a.taps == 27 && z == 0, last_dz = a.taps == 27 ? (z == a.D - 1 ? 1 : 2) : 0;       /* stages whose input plane lies outside the volume would add zeros: left out */
+    const int nshare = st_hi - st_lo, st_step = a.taps == 27 ? 3 : 1, st_first = st_lo + first_dz;
+    const int nlive = a.taps == 27 ? nshare / 3 * (last_dz - first_dz + 1) : nshare;
+    auto next_stage = [&](int st) -> int {
+        if (BITS == 8) return a.taps == 27 && st % 3 == last_dz ? st + 3 - (last_dz - first_dz) : st + 1;
+        st += st_step; return st < st_hi ? st : st - nshare + 1;
+    };
     auto stage_items = [&](int st) -> int { return a.taps == 27 ? 9 : min(4, a.nki - 4 * st); };
 
     /* a stage's A and B scales from shared memory to TMEM buffer buf.  Copies and MMAs of one thread run in issue order, so two buffers are enough and no
@@ -137,11 +145,10 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
             };
             /* the weights of the first ring's stages are constants of a prepared layer: they load while the previous kernel of the stream is still running */
             int early = 0;
-            if (!WDEP) for (int st = st_lo; st < st_hi && early < R; st++) if (stage_live(st)) put_weights(st, early++);
+            if (!WDEP) for (int st = st_first; early < min(nlive, R); st = next_stage(st)) put_weights(st, early++);
             pdl_wait();                          /* from here on this thread touches activations */
-            int it = 0, s = 0, ph = 0;
-            for (int st = st_lo; st < st_hi; st++) {
-                if (!stage_live(st)) continue;
+            int s = 0, ph = 0;
+            for (int it = 0, st = st_first; it < nlive; it++, st = next_stage(st)) {
                 uint8_t *sb = stages + (size_t)s * a.stage_bytes;
                 const uint32_t bar = bar_tma + 8 * s;
                 const int items = stage_items(st);
@@ -166,22 +173,21 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                         tma_load_4d(smem_u32(sb + a.offA + j * 4096), &map0, bar, x0 * 16, y0, z, BITS == 8 ? (n * a.nkb + ki) * 2 : n * a.nkb + 2 * ki, lead);
                     }
                 }
-                it++; if (++s == R) { s = 0; ph ^= 1; }
+                if (++s == R) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
         /* ---------------- MMA issue: one warp, of which one lane issues; everything that does not change with the stage is worked out before the loop ---------------- */
         {
             const uint32_t lead = elect_one();
-            int it = 0, s = 0, ph = 0; bool ok = true;
+            int s = 0, ph = 0; bool ok = true;
             const uint32_t sb0 = smem_u32(stages), sstep = (uint32_t)a.stage_bytes >> 4;
             const uint32_t b_hi = desc_hi(128), a_hi = a.taps == 27 ? desc_hi(160) : desc_hi(128);
             const uint32_t a_lo0 = desc_lo(sb0 + a.offA, (uint32_t)a.half), b_lo0 = desc_lo(sb0 + a.offW, (uint32_t)a.nt * 16);
             const uint32_t idesc0 = BITS == 8 ? idesc_mxf8(n_cur, 0, 0) : idesc_mxf4(n_cur, 0, 0);
             const uint32_t bstep = (uint32_t)a.nt * 2;
             int buf = 0;
-            for (int st = st_lo; st < st_hi && ok; st++) {
-                if (!stage_live(st)) continue;
+            for (int it = 0, st = st_first; it < nlive && ok; it++, st = next_stage(st)) {
                 const uint32_t so = (uint32_t)s * sstep;
                 const uint32_t sfa_t = tmem + kSfBase + buf * 40, sfb_t = sfa_t + 20;
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_sf + 8 * s, ph, abort_flag, kWaitLimit))) { if (lane == 0) raise(a, abort_flag, 3, st); ok = false; break; }
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 if (a.taps == 27) issue_items<BITS, 9, true>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 0, idesc0, sfa_t, sfb_t, it == 0, 9, lead);
                 else issue_items<BITS, 4, false>(tmem, a_lo0 + so, a_hi, b_lo0 + so, b_hi, bstep, 256, idesc0, sfa_t, sfb_t, it == 0, stage_items(st), lead);
                 umma_commit(bar_empty + 8 * s, lead);
-                it++; if (++s == R) { s = 0; ph ^= 1; }
+                if (++s == R) { s = 0; ph ^= 1; }
                 buf ^= 1;
             }
             umma_commit(bar_acc, lead);   /* also after a give-up: the epilogue must not wait for its full limit */
@@ -252,12 +258,10 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 }
             }
         };
-        auto next_live = [&](int st) { while (st < st_hi && !stage_live(st)) st++; return st; };
-        int it = 0;
-        int st = next_live(st_lo);
-        if (st < st_hi) load_scales(st);
-        while (st < st_hi) {
-            const int s = it % R, ph = (it / R) & 1, nst = next_live(st + 1);
+        load_scales(st_first);
+        for (int it = 0, st = st_first, nxt; it < nlive; it++, st = nxt) {
+            const int s = it % R, ph = (it / R) & 1;
+            nxt = next_stage(st);
             uint32_t wq[5] = {0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu};
             const int nj = a.taps == 27 ? 9 : 4;
 #pragma unroll
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
                 if (BITS == 8) wq[j >> 2] = (wq[j >> 2] & ~(0xffu << (8 * (j & 3)))) | (raw[j] << (8 * (j & 3)));
                 else wq[j >> 1] = (wq[j >> 1] & ~(0xffffu << (16 * (j & 1)))) | ((raw[j] | (raw[9 + j] << 8)) << (16 * (j & 1)));
             }
-            if (nst < st_hi) load_scales(nst);
+            if (it + 1 < nlive) load_scales(nxt);
             if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimit)) { raise(a, abort_flag, 4, st); break; }
             uint32_t *sfa = (uint32_t *)(stages + (size_t)s * a.stage_bytes + a.offSFA);
             /* quad q: word (lane, column) = row 32 * column + lane -> this thread's word is at lane * 4 + quarter */
@@ -275,8 +279,6 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_sf + 8 * s);        /* one arrival a warp: arrivals on one barrier serialise */
-            it++;
-            st = nst;
         }
         /* ---- epilogue ---- */
         if (!mbar_wait(bar_acc, 0, abort_flag, kWaitLimit)) raise(a, abort_flag, 5, 0);
@@ -410,6 +412,7 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 }   // namespace
 
 int umx_conv_r_takes(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e);
+
 int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0, int ref, void *enc, int N, int D, int H, int W, const EpiArgs &e,
                    double *part, const float *gamma, const float *beta, float eps, float *coef);
 extern "C" void umx_in_stats_coef(const void *y, int N, int C, int D, int H, int W, const float *gamma, const float *beta, float eps, double *part, float *coef);
@@ -525,6 +528,32 @@ int umx_stats_chunks(int D, int H, int W);
    one entry per block */
 extern "C" size_t umx_stats_doubles(int N, int co, int D, int H, int W) { (void)D; (void)H; (void)W; return (size_t)N * 512 * (size_t)(ceil_div(co, 32) * 32) * 2; }
 
+static int up128(int v) { return (v + 127) & ~127; }
+/* bytes of the general kernel's stage: weights and their scales, A, A scales */
+static int stage_layout(const umx_conv *c, int *offA, int *offSFA) {
+    *offA = up128(c->w_stage_bytes);
+    *offSFA = *offA + up128(c->taps == 27 ? 2944 + 2880 : 4 * 4096);
+    return (*offSFA + c->nquad * 512 + 1023) & ~1023;
+}
+/* K split of the general kernel for the layers with fewer tiles than multiprocessors (the deep levels); chosen from one sample's geometry (the grid of GEMM rows) so that a sample's
+   result does not depend on the batch it is in */
+int umx_conv_ksplit(const umx_conv *c, int D, int H, int W, int sms) {
+    static int no_split = -1;
+    if (no_split < 0) { const char *ev = getenv("UMX_KSPLIT"); no_split = ev && *ev == '0'; }
+    int offA, offSFA;
+    const int stage_bytes = stage_layout(c, &offA, &offSFA);
+    const long long blocks1 = (long long)ceil_div(W, 8) * ceil_div(H, 16) * D * c->ntiles_n;
+    const int units = c->taps == 27 ? c->nki : c->nst;
+    long long ks = blocks1 > 0 ? sms / blocks1 : 1;
+    if (ks > units) ks = units;
+    if (ks > c->nst / 6) ks = c->nst / 6;              /* at least six stages a share: shorter shares cost more in the reduction than they save */
+    /* at most as many parts as 16 KB pieces fit the shallow ring, whatever ring this launch has, so that the split does not change with the batch
+       (never more than six, a portable cluster) */
+    int rs = 100 * 1024 / stage_bytes; if (rs > 8) rs = 8; if (rs < 2) rs = 2;
+    const long long cap = (long long)rs * stage_bytes / 16384; if (ks > cap) ks = cap;
+    return !no_split && ks >= 2 && ks <= 8 ? (int)ks : 1;
+}
+
 static int g_last_kernel = -1;
 extern "C" int umx_conv_last_kernel(void) { return g_last_kernel; }
 struct NormArgs { const float *gamma, *beta; float eps; float *coef; };
@@ -574,10 +603,8 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
     a.N = N; a.D = D; a.H = H; a.W = W; a.nkb = c->nkb; a.nki = c->nki; a.taps = c->taps; a.bits = c->bits;
     a.cop = c->cop; a.nt = c->nt; a.ntiles_n = c->ntiles_n; a.tiles_x = ceil_div(W, 8); a.tiles_y = ceil_div(H, 16);
     a.w_stage_bytes = c->w_stage_bytes; a.nst = c->nst; a.items_max = c->items_max; a.ipq = c->ipq; a.nquad = c->nquad;
-    const int abytes = c->taps == 27 ? 2944 + 2880 : 4 * 4096;
-    auto up128 = [](int v) { return (v + 127) & ~127; };
-    a.offW = 0; a.offSFB = c->items_max * c->nt * 32; a.offA = up128(c->w_stage_bytes); a.offSFA = a.offA + up128(abytes);
-    a.stage_bytes = (a.offSFA + c->nquad * 512 + 1023) & ~1023;
+    a.offW = 0; a.offSFB = c->items_max * c->nt * 32;
+    a.stage_bytes = stage_layout(c, &a.offA, &a.offSFA);
     static int sms_of[16];                                  /* multiprocessors, looked up once per device */
     int d0 = 0; cudaGetDevice(&d0); d0 &= 15;
     if (!sms_of[d0]) { int v = 148; cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d0); sms_of[d0] = v; }
@@ -696,23 +723,7 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         if (e != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", e); return -1; }
         smem_set[dev] = 227 * 1024;
     }
-    /* K split for the layers with fewer tiles than multiprocessors (the deep levels); chosen from one sample's geometry so that a sample's
-       result does not depend on the batch it is in */
-    a.ksplit = 1;
-    {
-        static int no_split = -1;
-        if (no_split < 0) { const char *ev = getenv("UMX_KSPLIT"); no_split = ev && *ev == '0'; }
-        const long long blocks1 = (long long)a.tiles_x * a.tiles_y * D * a.ntiles_n, tiles_all = blocks1 * N;
-        const int units = c->taps == 27 ? c->nki : c->nst;
-        long long ks = blocks1 > 0 ? sms / blocks1 : 1;
-        if (ks > units) ks = units;
-        if (ks > c->nst / 6) ks = c->nst / 6;              /* at least six stages a share: shorter shares cost more in the reduction than they save */
-        if (ks > 16) ks = 16;
-        /* at most as many parts as 16 KB pieces fit the shallow ring, whatever ring this launch has, so that the split does not change with the batch
-           (never more than six, a portable cluster) */
-        { int rs = 100 * 1024 / a.stage_bytes; if (rs > 8) rs = 8; if (rs < 2) rs = 2; const long long cap = (long long)rs * a.stage_bytes / 16384; if (ks > cap) ks = cap; }
-        if (!no_split && ks >= 2 && ks <= 8 && tiles_all <= 8192) a.ksplit = (int)ks;
-    }
+    a.ksplit = (long long)N * a.tiles_x * a.tiles_y * D * a.ntiles_n <= 8192 ? umx_conv_ksplit(c, D, H, W, sms) : 1;
     const dim3 grid(a.tiles_x * a.tiles_y, D, N * a.ntiles_n * a.ksplit);
     const int pid = umx_prof_open(flops);
     /* the parts need 16 KB a 32-column chunk of the ring */

@@ -779,6 +779,7 @@ int umx_conv_r_image(const umx_conv *c, RImageGeo *o) {
     o->nt = g.nt; o->ncol = g.ncol; o->w_bytes = g.w_bytes; o->w_codes = g.w_codes; o->gt = g.gt; o->goff1 = g.goff1; o->goff2 = g.goff2;
     return 1;
 }
+int umx_conv_ksplit(const umx_conv *c, int D, int H, int W, int sms);       /* conv_tc.cu */
 /* the launch of this geometry, everything but the operands; 0 when the kernel does not apply */
 static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, int W, const EpiArgs &e, int want_coef, const double *part, ConvRArgs &a, int *grid) {
     memset(&a, 0, sizeof a);
@@ -817,14 +818,23 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     if (a.ips > 1) a.stage_bytes = a.ips * a.item_bytes;
     a.ring = room / a.stage_bytes; if (a.ring > 12) a.ring = 12;
     if (a.ring < 3) return 0;
-    /* A block pays two halo planes per run: with fewer than eight planes a block (counted for one sample, so that the choice of kernel does not
-       depend on the batch) the general kernel is faster.  Volumes with fewer planes than blocks are left here: nothing to gain either way. */
-    { const long long units1 = (long long)a.tiles * D; if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots) return 0;
-      /* The scale warp that gathers costs 3 to 8 % in MX-fp8 and 6 to 27 in MX-fp4 against the TMA window, and a piece's start, so few planes, and a column tile that re-reads the
-         input, are the general kernel's.  General kernel and this one, us: 32 -> 32 fp4 on 33 x 31 x 30 (264 planes) 6.9 and 9.0, on 36^3 (540) 14.5 and 11.6, on 63 x 61 x 66 45 and
-         17; fp8 64 -> 32 on 80 x 80 x 84 112 and 43; 64 columns, fp4 128 -> 64 plane-major on 36^3 23.0 and 24.6, on 40 x 35 x 42 (720) 33.0 and 29.0; two column tiles, fp8 32 -> 128 on
-         63 x 61 x 66 91 and 124. */
-      if (a.gather && (g.ncol > 1 || 2 * units1 < (g.nt == 32 ? 7ll : 9ll) * (slots < sms ? slots : sms))) return 0; }
+    /* What the general kernel does with the call.  In MX-fp4, or with one input item, it adds in this kernel's order (a dz at a time, the items within it) unless it splits K, which it does by
+       one sample's geometry: the bits are the same, and the choice follows all samples' planes.  Otherwise it follows from one sample's, so that the result does not depend on the batch; and the
+       layers of a network (blocked halves) stay with the order that they have at that size: the last bit of the sums decides codes next to a rounding boundary, which the layers behind make
+       0.05 (three levels) to 0.07 (four) of the logits, relative L2. */
+    const long long units1 = (long long)a.tiles * D;
+    const bool same = (c->bits == 4 || c->nki == 1) && umx_conv_ksplit(c, D, H, W, sms) == 1, keep = !same && e.out_mode == UMX_OUT_H16B;
+    const long long planes = same ? a.units : units1;
+    /* A block here pays two halo planes a run and loads its weights first, so with several column tiles and fewer than eight planes a block the general kernel is faster while one wave of
+       its blocks, two a multiprocessor, holds the call, and slower once it takes a second.  General kernel and this one, us, fp8 / fp4: 32 -> 128 on 32^3 (256 of its blocks) 9.2 and 11.3 /
+       9.4 and 10.6, two samples (512) 16.7 and 15.7 / 17.7 and 14.3; 64 -> 256 on 24 x 20 x 32 (384) 19.4 and 15.4 / 16.5 and 12.6; 32 -> 96 on 32^3 (256) 8.2 and 9.0, two samples 15.0 and
+       11.6 / 16.3 and 11.5; 128 -> 128 on 24 x 20 x 32, two samples, fp4 22.3 and 14.6.  Volumes with fewer planes than blocks are left here: nothing to gain either way. */
+    if (g.ncol > 1 && units1 >= slots && units1 < 8 * slots && (keep || planes * ((c->cop + 127) / 128) <= 2 * sms)) return 0;
+    /* The scale warp that gathers costs 3 to 8 % in MX-fp8 and 6 to 27 in MX-fp4 against the TMA window, and a piece's start, so few planes, and a column tile that re-reads the
+       input, are the general kernel's.  General kernel and this one, us: 32 -> 32 fp4 on 33 x 31 x 30 (264 planes) 6.9 and 9.0, on 36^3 (540) 14.5 and 11.6, on 63 x 61 x 66 45 and
+       17; fp8 64 -> 32 on 80 x 80 x 84 112 and 43; 64 columns, fp4 128 -> 64 plane-major on 36^3 23.0 and 24.6, on 40 x 35 x 42 (720) 33.0 and 29.0; two column tiles, fp8 32 -> 128 on
+       63 x 61 x 66 91 and 124. */
+    if (a.gather && (keep || g.ncol > 1 || 2 * planes < (g.nt == 32 ? 7ll : 9ll) * (slots < sms ? slots : sms))) return 0;
     a.gcol = (int)(a.units < slots ? a.units : slots); if (a.gcol > 512) a.gcol = 512;
     *grid = a.gcol * g.ncol;
     return 1;
