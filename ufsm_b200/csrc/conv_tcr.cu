@@ -76,7 +76,6 @@ struct ConvRArgs {
        turns them into coefficients (a, b) per (sample, channel) */
     double *part; float *coef; const float *gamma, *beta; float eps; int cop, off_red;
     const uint8_t *wr, *x_sc;
-    int ref;                                     /* MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load, the halves 2944 bytes apart in a stage */
     int gather, w_dep;                           /* see GATHER; the weights and the bias were written by a kernel just ahead in the stream */
     EpiArgs e;
     int *err;
@@ -164,8 +163,10 @@ __device__ unsigned g_conv_tickets[64];      /* one per column tile; the block t
 
 /* NCH: 32-channel chunks of the column tile (1: two blocks per multiprocessor and at most 128 registers; 2: one block, more registers);
    STATS: the epilogue also takes the InstanceNorm sums; GATHER: the scale warp fetches its window of scale bytes itself, for scale planes whose rows TMA does not
-   take (W not a multiple of 16); MULTI: a stage holds up to a.ips input items of its plane (see r_plan), else one */
-template <int BITS, int NCH, bool STATS, bool GATHER, bool MULTI>
+   take (W not a multiple of 16); MULTI: a stage holds up to a.ips input items of its plane (see r_plan), else one; REF:
+   MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load, the halves 2944 bytes apart in a stage (as a branch on an argument it cost the split layout 1.3 % on
+   32 -> 32, 64^3) */
+template <int BITS, int NCH, bool STATS, bool GATHER, bool MULTI, bool REF = false>
 __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap maps, const ConvRArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint64_t *bars = (uint64_t *)smem_raw;
@@ -257,9 +258,10 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                         /* codes: two 16-byte-wide planes (fp8: the halves of block ki; fp4: blocks 2 ki and 2 ki + 1), 18 rows of 10 voxels;
                            scale bytes: 18 rows of a 32-byte window per block */
                         for (int k = ki; k < ki + (MULTI ? nit : 1); k++, sb += (uint32_t)a.item_bytes) {
-                            if (BITS == 8 && a.ref) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + k, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + k, lead); }
+                            if (REF) { tma_load_5d(sb, &map0, bar, 0, x0 - 1, cy, zi, pls + k, lead); tma_load_5d(sb + 2944, &map0, bar, 16, x0 - 1, cy, zi, pls + k, lead); }
                             else tma_load_4d(sb, &map0, bar, cx, cy, zi, pl0 + 2 * k, lead);
-                            if (!GATHER) tma_load_5d(sb + a.offSW, &maps, bar, xa, cy, zi, BITS == 8 ? k : 2 * k, rn.n, lead);
+                            if (!GATHER && BITS == 8) tma_load_4d(sb + a.offSW, &maps, bar, xa, cy, zi, pls + k, lead);
+                            if (!GATHER && BITS == 4) tma_load_5d(sb + a.offSW, &maps, bar, xa, cy, zi, 2 * k, rn.n, lead);
                         }
                         it++; if (++s == R) { s = 0; ph ^= 1; }
                     }
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int nsf = a.nki * a.nquad * a.gt;
                 for (int i = 0; i < nsf; i++) utccp_32x128b(tmem + a.sfb_base + i * 4, desc_make(desc_lo(wbase + a.w_codes + i * 512, 0), sf_hi), lead);
             }
-            const uint32_t a_lo0 = desc_lo(smem_u32(stages), BITS == 8 && a.ref ? 2944u : 2880u), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
+            const uint32_t a_lo0 = desc_lo(smem_u32(stages), REF ? 2944u : 2880u), a_step = (uint32_t)a.stage_bytes >> 4, sfa_off = (uint32_t)a.offSFA >> 4;
             const uint32_t sfa_t0 = tmem + (uint32_t)a.sfa_base, sfa_cols = (uint32_t)a.sfa_cols;
             const uint32_t i_step = (uint32_t)a.item_bytes >> 4, bstep9 = 9u * 2u * 3u * 32u * NCH, sfb_step = (uint32_t)(a.nquad * a.gt * 4);
             uint32_t item = 0;
@@ -859,33 +861,39 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     const size_t S = (size_t)D * H * W;
     CUtensorMap ms; memset(&ms, 0, sizeof ms);
     if (!a.gather) {
-        /* samples as a dimension of their own: the second block of a MX-fp4 item past the last one reads the fill, not the next sample's scales (whose NaN would come through the zero weights) */
-        const cuuint64_t gd[5] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)c->nkb, (cuuint64_t)N};
+        /* MX-fp4: samples as a dimension of their own, so that the second block of an item past the last one reads the fill, not the next sample's scales (whose NaN would come through the
+           zero weights); MX-fp8 reads one block at a time, over all samples' blocks in a row */
+        const bool f8 = c->bits == 8;
+        const cuuint64_t gd[5] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)c->nkb * (f8 ? N : 1), (cuuint64_t)N};
         const cuuint64_t gs[4] = {(cuuint64_t)W, (cuuint64_t)W * H, (cuuint64_t)S, (cuuint64_t)S * c->nkb};
-        const cuuint32_t box[5] = {32, 18, 1, (cuuint32_t)(c->bits == 8 ? 1 : 2), 1}, es[5] = {1, 1, 1, 1, 1};
-        const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        const cuuint32_t box[5] = {32, 18, 1, f8 ? 1u : 2u, 1}, es[5] = {1, 1, 1, 1, 1};
+        const CUresult r0 = ((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, f8 ? 4 : 5, (void *)x_sc, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r0 != CUDA_SUCCESS) return 1;                        /* e.g. a scale plane that is not 16-byte aligned: take the general kernel */
     }
-    a.wr = c->wr; a.x_sc = x_sc; a.ref = ref; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
+    a.wr = c->wr; a.x_sc = x_sc; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
     static int attr_set[16];
     if (!attr_set[dev & 15]) {
-#define UMX_R_KS(ST, GA, MU) (const void *)conv_mxr_k<8, 1, ST, GA, MU>, (const void *)conv_mxr_k<8, 2, ST, GA, MU>, (const void *)conv_mxr_k<4, 1, ST, GA, MU>, (const void *)conv_mxr_k<4, 2, ST, GA, MU>
-        const void *ks[16] = {UMX_R_KS(false, false, false), UMX_R_KS(true, false, false), UMX_R_KS(false, true, false), UMX_R_KS(false, false, true)};
+#define UMX_R_KF(ST, GA, MU, REF) (const void *)conv_mxr_k<8, 1, ST, GA, MU, REF>, (const void *)conv_mxr_k<8, 2, ST, GA, MU, REF>
+#define UMX_R_KS(ST, GA, MU) UMX_R_KF(ST, GA, MU, false), UMX_R_KF(ST, GA, MU, true), (const void *)conv_mxr_k<4, 1, ST, GA, MU>, (const void *)conv_mxr_k<4, 2, ST, GA, MU>
+        const void *ks[24] = {UMX_R_KS(false, false, false), UMX_R_KS(true, false, false), UMX_R_KS(false, true, false), UMX_R_KS(false, false, true)};
 #undef UMX_R_KS
-        for (int i = 0; i < 16; i++) {
+#undef UMX_R_KF
+        for (int i = 0; i < 24; i++) {
             const cudaError_t er = cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
         }
         attr_set[dev & 15] = 1;
     }
-    const int variant = (c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+    const int variant = (ref ? 4 : c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
 #define UMX_R_GO(ST, GA, MU) do { switch (variant) { \
         case 0: umx_launch(conv_mxr_k<8, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
         case 1: umx_launch(conv_mxr_k<8, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
         case 2: umx_launch(conv_mxr_k<4, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        default: umx_launch(conv_mxr_k<4, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); } } while (0)
+        case 3: umx_launch(conv_mxr_k<4, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
+        case 4: umx_launch(conv_mxr_k<8, 1, ST, GA, MU, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
+        default: umx_launch(conv_mxr_k<8, 2, ST, GA, MU, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); } } while (0)
     if (coef) UMX_R_GO(true, false, false);
     else if (a.gather) UMX_R_GO(false, true, false);
     else if (a.ips > 1) UMX_R_GO(false, false, true);
