@@ -148,8 +148,8 @@ void umx_conv_free(umx_conv *c);
 /* x: MX tensor (32-wide blocks) of c->ci channels (UMX_DOWN2: the space-to-depth copy, 8 * ci channels at half resolution) on an
    N x D x H x W grid.  y per out_mode; nb_dst / b0: block count of the destination tensor and first block written (0, 0: the
    conv's own co).  part: optional device doubles for InstanceNorm partial sums (umx_stats_doubles), only with UMX_OUT_H16B.
-   UMX_TCONV2 writes the 2D x 2H x 2W grid.  flags: UMX_X_SPLIT / UMX_Y_SPLIT (an fp8 input in the reference layout is re-laid into
-   scratch first); UMX_X_H16: x is planar fp16 and is quantised to the conv's MX format on the way in (the values the quantiser gives;
+   UMX_TCONV2 writes the 2D x 2H x 2W grid.  flags: UMX_X_SPLIT / UMX_Y_SPLIT (the 3^3 convs read an fp8 input in the
+   reference layout as it is; the others re-lay it into scratch first); UMX_X_H16: x is planar fp16 and is quantised to the conv's MX format on the way in (the values the quantiser gives;
    a 3^3 MX-fp8 conv of ONE input channel into at most 32 outputs with a UMX_OUT_H16B output runs as a tap-packed kernel that reads
    the fp16 tensor directly, the role of conv_fwd_f8s_k, src/lp_f8fwd.cuh:153-400; every other case is quantised into scratch first).
    Returns 0, or -1 after latching an error. */

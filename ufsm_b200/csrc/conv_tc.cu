@@ -9,8 +9,8 @@
    Operand staging.  A 3^3 conv loads, per (input block, dz), one halo plane of 18 x 10 voxels with TMA (out-of-range voxels are
    zero-filled: that is the padding) as two 16-byte-wide planes [k half][y][x][16 B].  In that layout the canonical K-major
    no-swizzle UMMA operand (8 rows x 16 B core matrices; stride 160 B between the 16 y groups, 2880 B between the K halves) of
-   every (dy, dx) tap is the same tile at a start address shifted by (dy * 10 + dx) * 16 bytes (the fp8 planes sit 2944 B apart so
-   that each TMA destination is 128-byte aligned), so nine MMAs reuse one load.
+   every (dy, dx) tap is the same tile at a start address shifted by (dy * 10 + dx) * 16 bytes (2944 B where each half is a load of its own, so
+   that its TMA destination is 128-byte aligned), so nine MMAs reuse one load.
    Weights are prepared once into the exact shared-memory image of a stage ([tap][k half][row][16 B] + scale bytes in the
    TMEM scale layout) and arrive with one bulk copy.  1^3 convs (head, the 2^3 stride-2 down conv on a space-to-depth copy, the
    transposed conv as a GEMM to 8 Cout columns) run the same pipeline with one tap and four K items a stage.
