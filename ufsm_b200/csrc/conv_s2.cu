@@ -391,21 +391,20 @@ int umx_conv_fwd_s2(const umx_conv *c, const void *x, int split, const uint8_t *
     }
     a.err = umx_errflag(); if (!a.err) return -1;
     int dev = 0; cudaGetDevice(&dev); dev &= 15;
-    static int attr_set[16];
-    if (!attr_set[dev]) {
-        const void *ks[4] = {(const void *)conv_s2_k<8, 1>, (const void *)conv_s2_k<8, 2>, (const void *)conv_s2_k<4, 1>, (const void *)conv_s2_k<4, 2>};
-        for (int i = 0; i < 4; i++) {
-            const cudaError_t er = cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
-        }
-        attr_set[dev] = 1;
+    typedef void (*kernel_fn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const ConvSArgs);
+    static const kernel_fn ks[4] = {conv_s2_k<8, 1>, conv_s2_k<8, 2>, conv_s2_k<4, 1>, conv_s2_k<4, 2>};
+    const int variant = (c->bits == 8 ? 0 : 2) | (g.nt == 32 ? 0 : 1);
+    static unsigned attr_set[16];                       /* a bit a kernel: the attribute loads it */
+    if (!(attr_set[dev] >> variant & 1)) {
+        const cudaError_t er = cudaFuncSetAttribute((const void *)ks[variant], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
+        __atomic_fetch_or(&attr_set[dev], 1u << variant, __ATOMIC_RELAXED);
     }
     long long slots = s2_sms() / g.ncol;
     if (umx_conv_r_cap() && slots > umx_conv_r_cap()) slots = umx_conv_r_cap();
     a.gcol = (int)(a.units < slots ? a.units : slots);
     const dim3 grid((unsigned)(a.gcol * g.ncol));
     const size_t smem = (size_t)g.off_ring + (size_t)g.ring * g.stage_bytes;
-    if (c->bits == 8) { if (g.nt == 32) umx_launch(conv_s2_k<8, 1>, grid, dim3(kThreadsS), smem, m[0], m[1], m[2], m[3], a); else umx_launch(conv_s2_k<8, 2>, grid, dim3(kThreadsS), smem, m[0], m[1], m[2], m[3], a); }
-    else { if (g.nt == 32) umx_launch(conv_s2_k<4, 1>, grid, dim3(kThreadsS), smem, m[0], m[1], m[2], m[3], a); else umx_launch(conv_s2_k<4, 2>, grid, dim3(kThreadsS), smem, m[0], m[1], m[2], m[3], a); }
+    umx_launch(ks[variant], grid, dim3(kThreadsS), smem, m[0], m[1], m[2], m[3], a);
     return 0;
 }

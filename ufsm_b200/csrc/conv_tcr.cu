@@ -873,31 +873,19 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     a.wr = c->wr; a.x_sc = x_sc; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
-    static int attr_set[16];
-    if (!attr_set[dev & 15]) {
-#define UMX_R_KF(ST, GA, MU, REF) (const void *)conv_mxr_k<8, 1, ST, GA, MU, REF>, (const void *)conv_mxr_k<8, 2, ST, GA, MU, REF>
-#define UMX_R_KS(ST, GA, MU) UMX_R_KF(ST, GA, MU, false), UMX_R_KF(ST, GA, MU, true), (const void *)conv_mxr_k<4, 1, ST, GA, MU>, (const void *)conv_mxr_k<4, 2, ST, GA, MU>
-        const void *ks[24] = {UMX_R_KS(false, false, false), UMX_R_KS(true, false, false), UMX_R_KS(false, true, false), UMX_R_KS(false, false, true)};
+    typedef void (*kernel_fn)(const CUtensorMap, const CUtensorMap, const ConvRArgs);
+#define UMX_R_KS(ST, GA, MU) {conv_mxr_k<8, 1, ST, GA, MU>, conv_mxr_k<8, 2, ST, GA, MU>, conv_mxr_k<4, 1, ST, GA, MU>, conv_mxr_k<4, 2, ST, GA, MU>, conv_mxr_k<8, 1, ST, GA, MU, true>, conv_mxr_k<8, 2, ST, GA, MU, true>}
+    static const kernel_fn ks[4][6] = {UMX_R_KS(false, false, false), UMX_R_KS(true, false, false), UMX_R_KS(false, true, false), UMX_R_KS(false, false, true)};
 #undef UMX_R_KS
-#undef UMX_R_KF
-        for (int i = 0; i < 24; i++) {
-            const cudaError_t er = cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
-        }
-        attr_set[dev & 15] = 1;
+    const int form = coef ? 1 : a.gather ? 2 : a.ips > 1 ? 3 : 0, variant = (ref ? 4 : c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+    /* the attribute loads a kernel (a millisecond): only of the one that is launched */
+    static unsigned attr_set[16];
+    const unsigned bit = 1u << (6 * form + variant);
+    if (!(attr_set[dev & 15] & bit)) {
+        const cudaError_t er = cudaFuncSetAttribute((const void *)ks[form][variant], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (er != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", er); return -1; }
+        __atomic_fetch_or(&attr_set[dev & 15], bit, __ATOMIC_RELAXED);
     }
-    const int variant = (ref ? 4 : c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
-#define UMX_R_GO(ST, GA, MU) do { switch (variant) { \
-        case 0: umx_launch(conv_mxr_k<8, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        case 1: umx_launch(conv_mxr_k<8, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        case 2: umx_launch(conv_mxr_k<4, 1, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        case 3: umx_launch(conv_mxr_k<4, 2, ST, GA, MU>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        case 4: umx_launch(conv_mxr_k<8, 1, ST, GA, MU, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); break; \
-        default: umx_launch(conv_mxr_k<8, 2, ST, GA, MU, true>, dim3(grid), dim3(kThreadsR), smem, *m0, ms, a); } } while (0)
-    if (coef) UMX_R_GO(true, false, false);
-    else if (a.gather) UMX_R_GO(false, true, false);
-    else if (a.ips > 1) UMX_R_GO(false, false, true);
-    else UMX_R_GO(false, false, false);
-#undef UMX_R_GO
+    umx_launch(ks[form][variant], dim3(grid), dim3(kThreadsR), smem, *m0, ms, a);
     return 0;
 }
