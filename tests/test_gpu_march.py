@@ -189,7 +189,7 @@ def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
     assert np.array_equal(q, orc.blocked_to_mx(orc.pm_to_blocked(got, N, Co, S), 8, N, Co, S))
 
 
-@pytest.mark.parametrize("kind,want_kernel,W", [("conv3", 1, 16), ("conv3", 1, 13), ("conv3s2", 4, 16)])
+@pytest.mark.parametrize("kind,want_kernel,W", [("conv3", 1, 16), ("conv3", 1, 13), ("conv3s2", 4, 16), ("conv1", 2, 16), ("tconv2", 2, 16)])
 def test_nan_scales_stay_in_their_sample(dev, kind, want_kernel, W):
     """MX-fp4 with an odd number of blocks: the last item's second block has zero weights, and its scales are not those of the next sample (0xff, of a block with a NaN, would make NaN
     of zero codes times zero weights)."""
@@ -198,7 +198,7 @@ def test_nan_scales_stay_in_their_sample(dev, kind, want_kernel, W):
     x = synth.rng(351).standard_normal(N * Ci * S).astype(np.float32)
     xn = x.copy()
     xn[Ci * S:] = np.nan
-    w, b = synth.kaiming(352, Co, Ci, 27), synth.bias(353, Co, 0.1)
+    w, b = synth.kaiming(352, Co, Ci, {"conv1": 1, "tconv2": 8}.get(kind, 27), transposed=kind == "tconv2"), synth.bias(353, Co, 0.1)
     mx, want = orc.conv_case(kind, x, w, b, N, Ci, D, H, W, Co, 4)
     mxn, _ = orc.conv_case(kind, xn, w, b, N, Ci, D, H, W, Co, 4)
     dev.umx_conv_r_block_cap(1)

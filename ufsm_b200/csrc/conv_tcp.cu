@@ -98,14 +98,14 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
         /* job = (row tile, column tile), column tile fastest; the indices advance incrementally (no division per job) */
         int ntile = (int)(j0 % a.ntiles), n = (int)((j0 / a.ntiles) / a.rtiles_per_n), tin = (int)((j0 / a.ntiles) % a.rtiles_per_n);
         for (long long job = j0; job < j1 && ok; job++) {
-            const int cx = tin * 256, pl0 = BITS == 8 ? n * a.nkb * 2 : n * a.nkb, cs = tin * 128, pls = n * a.nkb;
+            const int cx = tin * 256, pl0 = BITS == 8 ? n * a.nkb * 2 : n * a.nkb, cs = tin * 128;
             for (int g = 0; g < a.ngroups; g++) {
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, kWaitLimitP))) { if (lane == 0) raise_p(a, abort_flag, 1, it); ok = false; break; }
                 const int items = min(4, a.nki - 4 * g);
                 const uint32_t sb = smem_u32(stages + (size_t)s * a.stage_bytes), bar = bar_tma + 8 * s;
                 if (lead) mbar_expect_tx(bar, (uint32_t)(items * 4096 + a.sw_rows * 128));
                 for (int j = 0; j < items; j++) tma_load_2d(sb + j * 4096, &map0, bar, cx, pl0 + 2 * (4 * g + j), lead);
-                tma_load_2d(sb + a.offSW, &maps, bar, cs, pls + a.sw_rows * g, lead);
+                tma_load_3d(sb + a.offSW, &maps, bar, cs, a.sw_rows * g, n, lead);
                 it++; if (++s == R) { s = 0; ph ^= 1; }
             }
             if (++ntile == a.ntiles) { ntile = 0; if (++tin == (int)a.rtiles_per_n) { tin = 0; n++; } }
@@ -402,9 +402,10 @@ int umx_conv_fwd_p(const umx_conv *c, const void *x, const uint8_t *x_sc, void *
         const cuuint64_t gd[2] = {(cuuint64_t)S * 2, (cuuint64_t)planes}, gs[1] = {(cuuint64_t)S * 16};
         const cuuint32_t box[2] = {256, 2}, es[2] = {1, 1};
         if (((encode_fn)enc_v)(&m0, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void *)x, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
-        const cuuint64_t gd2[2] = {(cuuint64_t)S, (cuuint64_t)N * c->nkb}, gs2[1] = {(cuuint64_t)S};
-        const cuuint32_t box2[2] = {128, (cuuint32_t)a.sw_rows};
-        if (((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)x_sc, gd2, gs2, box2, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
+        /* samples as a dimension of their own: an MX-fp4 item's second block past the last one reads the fill, not the next sample's scales (whose NaN would come through the zero weights) */
+        const cuuint64_t gd2[3] = {(cuuint64_t)S, (cuuint64_t)c->nkb, (cuuint64_t)N}, gs2[2] = {(cuuint64_t)S, (cuuint64_t)S * c->nkb};
+        const cuuint32_t box2[3] = {128, (cuuint32_t)a.sw_rows, 1}, es2[3] = {1, 1, 1};
+        if (((encode_fn)enc_v)(&ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void *)x_sc, gd2, gs2, box2, es2, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
     }
     a.wp = c->wp; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;

@@ -59,6 +59,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
                  "@pl cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(lead) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, uint32_t lead = 1u) {
+    asm volatile("{\n\t.reg .pred pl;\n\tsetp.ne.b32 pl, %6, 0;\n\t"
+                 "@pl cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(lead) : "memory");
+}
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3, int c4, uint32_t lead = 1u) {
     asm volatile("{\n\t.reg .pred pl;\n\tsetp.ne.b32 pl, %8, 0;\n\t"
                  "@pl cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}"
