@@ -87,6 +87,24 @@ def test_conv3_reads_the_reference_layout(dev, N, Ci, Co, D, H, W):
     assert np.isfinite(got).all() and np.array_equal(got, run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8))
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N,Ci,Co,D", [
+    (114, 256, 128, 72),               # 8208 output tiles in the batch, 72 alone
+    (1100, 512, 256, 8),               # two column tiles
+    (33000, 256, 32, 1),               # more blocks than a grid holds along z
+])
+def test_a_sample_splits_k_alone_and_in_any_batch(dev, N, Ci, Co, D, bits):
+    """The K split of a small deep layer follows from one sample's shape: a sample of a batch of any size has the bits it has alone."""
+    one = orc.pm_to_mx(synth.rng(61).standard_normal(Ci * D).astype(np.float32) * np.exp2(synth.rng(62).integers(-6, 7, Ci * D)).astype(np.float32), 0, 1, Ci, D, bits)
+    codes = Ci // 32 * D * 4 * bits
+    mx = np.concatenate([np.tile(one[:codes], N), np.tile(one[codes:], N)])
+    w, b = synth.kaiming(63, Co, Ci, 27), synth.bias(64, Co, 0.1)
+    got = run_pm32("conv3", mx, w, b, N, Ci, D, 1, 1, Co, bits)
+    assert dev.umx_conv_last_kernel() == 0
+    alone = run_pm32("conv3", one, w, b, 1, Ci, D, 1, 1, Co, bits)
+    assert np.isfinite(alone).all() and (got.reshape(N, -1) == alone.reshape(1, -1)).all()
+
+
 @pytest.mark.parametrize("Ci,Co,ybf", [(32, 32, 3), (64, 40, 4), (96, 64, 3), (8, 16, 4), (16, 32, 3)])
 def test_lp_conv_fwd_s2_mxfp4_input(dev, Ci, Co, ybf):
     """lp_conv_fwd_s2_f8 on an MX-fp4 tensor computes in MX-fp4 and says so (returns 3: src/lp_s2.cu:652-716), also for inputs and outputs of

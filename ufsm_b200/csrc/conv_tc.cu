@@ -52,6 +52,7 @@ struct ConvArgs {
     /* K split: the ksplit blocks of an output tile are a cluster; each takes a contiguous range of the stages and keeps its fp32 accumulators in shared
        memory, where the blocks add them up chunk by chunk in split order */
     int ksplit;
+    int first_n;                        /* first sample of this launch */
     /* 3^3 stride-2 pad-1 conv: K item = (tap, input block), each item's A tile is its own strided TMA load from the input grid Di x Hi x Wi */
     int s2, nbi, nit, Di, Hi, Wi;       /* stride-2 conv: blocks of the input tensor, K items per tap, input grid */
     int ref, half;                      /* 3^3 on MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load; bytes between the halves of a stage's A */
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
     const int txy = blockIdx.x, tx = txy % a.tiles_x, ty = txy / a.tiles_x;
     const int z = blockIdx.y;
     const int sp = (int)blockIdx.z % a.ksplit, bz = (int)blockIdx.z / a.ksplit;
-    const int n = bz / a.ntiles_n, ntile = bz % a.ntiles_n;
+    const int n = a.first_n + bz / a.ntiles_n, ntile = bz % a.ntiles_n;
     const int x0 = tx * 8, y0 = ty * 16;
     const int n0 = ntile * a.nt, n_cur = min(a.nt, a.cop - n0);
     /* this block's stages: all of them, or its share (whole input items of a 3^3 conv, so that every share has a live stage) */
@@ -535,8 +536,8 @@ static int stage_layout(const umx_conv *c, int *offA, int *offSFA) {
     *offSFA = *offA + up128(c->taps == 27 ? 2944 + 2880 : 4 * 4096);
     return (*offSFA + c->nquad * 512 + 1023) & ~1023;
 }
-/* K split of the general kernel for the layers with fewer tiles than multiprocessors (the deep levels); chosen from one sample's geometry (the grid of GEMM rows) so that a sample's
-   result does not depend on the batch it is in */
+/* K split of the general kernel for the layers with fewer tiles than multiprocessors (the deep levels); chosen from one sample's geometry (the grid of GEMM rows) and nothing else, so that
+   a sample's result does not depend on the batch it is in */
 int umx_conv_ksplit(const umx_conv *c, int D, int H, int W, int sms) {
     static int no_split = -1;
     if (no_split < 0) { const char *ev = getenv("UMX_KSPLIT"); no_split = ev && *ev == '0'; }
@@ -723,15 +724,21 @@ static int conv_fwd_impl(const umx_conv *c, const void *x, int N, int D, int H, 
         if (e != cudaSuccess) { umx_latch("umx_conv_fwd: shared memory attribute", e); return -1; }
         smem_set[dev] = 227 * 1024;
     }
-    a.ksplit = (long long)N * a.tiles_x * a.tiles_y * D * a.ntiles_n <= 8192 ? umx_conv_ksplit(c, D, H, W, sms) : 1;
-    const dim3 grid(a.tiles_x * a.tiles_y, D, N * a.ntiles_n * a.ksplit);
+    a.ksplit = umx_conv_ksplit(c, D, H, W, sms);
+    const int per_n = a.ntiles_n * a.ksplit, n_max = per_n < 65535 ? 65535 / per_n : 1;      /* a grid has at most 65535 blocks along z: a larger batch goes in several launches */
     const int pid = umx_prof_open(flops);
     /* the parts need 16 KB a 32-column chunk of the ring */
-    auto go = [&](auto k) { if (a.ksplit > 1) umx_launch_cluster(k, grid, dim3(1, 1, (unsigned)a.ksplit), dim3(kThreads), smem, m0, a); else umx_launch(k, grid, dim3(kThreads), smem, m0, a); };
+    auto go = [&](auto k) {
+        for (a.first_n = 0; a.first_n < N; a.first_n += n_max) {
+            const dim3 grid(a.tiles_x * a.tiles_y, D, (unsigned)((N - a.first_n < n_max ? N - a.first_n : n_max) * per_n));
+            if (a.ksplit > 1) umx_launch_cluster(k, grid, dim3(1, 1, (unsigned)a.ksplit), dim3(kThreads), smem, m0, a); else umx_launch(k, grid, dim3(kThreads), smem, m0, a);
+            g_umx_launches++;
+        }
+    };
     if (c->w_src) { if (c->bits == 8) go(conv_mx_k<8, true>); else go(conv_mx_k<4, true>); }
     else if (c->bits == 8) go(conv_mx_k<8, false>); else go(conv_mx_k<4, false>);
     umx_prof_close(pid);
-    g_umx_launches++; g_last_kernel = 0;
+    g_last_kernel = 0;
     UMX_CK("umx_conv_fwd");
     if (nrm) umx_in_stats_coef(y, N, c->co, D, H, W, nrm->gamma, nrm->beta, nrm->eps, part, nrm->coef);
     else if (part) umx_in_part(y, N, c->co, D, H, W, part);
