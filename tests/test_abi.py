@@ -29,6 +29,20 @@ def test_every_declared_symbol_is_exported_and_bound():
         assert n in names, "bound but not declared in the header: " + n
 
 
+def test_kernels_hold_their_tensor_memory_before_a_successor_may_start():
+    """A kernel that lets its successor start early does so behind the barrier after its tcgen05.alloc, which waits without a limit: a successor's block that took the columns first would
+    wait for this kernel, and this kernel for it."""
+    csrc, seen = os.path.join(ROOT, "ufsm_b200", "csrc"), 0
+    for f in sorted(os.listdir(csrc)):
+        src = re.sub(r"/\*.*?\*/", "", open(os.path.join(csrc, f)).read(), flags=re.S)
+        for body in re.split(r"\b__global__\b", src)[1:]:
+            if "tmem_alloc(" in body and "pdl_trigger()" in body:
+                at = body.index("__syncthreads()", body.index("tmem_alloc("))
+                assert body.index("pdl_trigger()") > at, "%s: %s" % (f, body[:120])
+                seen += 1
+    assert seen == 5
+
+
 def test_struct_sizes_match_the_reference():
     assert C.sizeof(ufsm_b200.Shape5) == 20
     assert C.sizeof(ufsm_b200.Split) <= 128 and C.sizeof(ufsm_b200.Split) == 128   # static_assert of src/nn_lp.h:38-41

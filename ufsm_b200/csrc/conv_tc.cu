@@ -100,11 +100,11 @@ __global__ void __launch_bounds__(kThreads, 2) conv_mx_k(const __grid_constant__
         fence_barrier_init();
         fence_proxy_async();
     }
-    pdl_trigger();
     if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), kTmemCols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();                               /* the next kernel cannot take this block's tensor memory any more */
     const uint32_t tmem = uni(*tmem_slot);
     /* The order of a 3^3 block's stages (each the nine (dy, dx) of an input item and a dz): in MX-fp4 dz outermost, which is the z-marching kernel's order, so that the two give the same bits
        and the choice between them may follow the batch; in MX-fp8 the items outermost.  A conv of one item has the two orders in one.  (MX-fp4 sums are exact in fp32 over many octaves of

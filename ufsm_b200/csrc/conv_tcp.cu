@@ -75,7 +75,6 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
         fence_barrier_init();
         fence_proxy_async();
     }
-    pdl_trigger();
     if (threadIdx.x == 0) {
         /* the weight image is a constant of the layer: it may load while the previous kernel of the stream is still running */
         mbar_expect_tx(bar_w, (uint32_t)a.w_bytes);
@@ -85,6 +84,7 @@ __global__ void __launch_bounds__(kThreadsP, 2) conv_mxp_k(const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();                               /* the next kernel cannot take this block's tensor memory any more */
     const uint32_t tmem = uni(*tmem_slot);
     const long long j0 = a.jobs * (long long)blockIdx.x / (long long)gridDim.x, j1 = a.jobs * ((long long)blockIdx.x + 1) / (long long)gridDim.x;
 

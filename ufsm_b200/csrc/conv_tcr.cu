@@ -194,17 +194,16 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
     }
     const int ctile = (int)blockIdx.x / a.gcol;
     if (!a.w_dep && (int)threadIdx.x < a.nt) bias_s[threadIdx.x] = a.e.bias[ctile * a.nt + threadIdx.x];
-    pdl_trigger();
-    if (threadIdx.x == 0) {
-        /* the weight image of a prepared layer is a constant: it may load while the previous kernel of the stream is still running */
-        if (a.w_dep) pdl_wait();
+    auto load_weights = [&]() {
         mbar_expect_tx(bar_w, (uint32_t)a.w_bytes);
         for (int o = 0; o < a.w_bytes; o += 32768) bulk_g2s(smem_u32(wsm + o), a.wr + (size_t)ctile * a.w_bytes + o, (uint32_t)min(32768, a.w_bytes - o), bar_w);
-    }
+    };
+    if (!a.w_dep && threadIdx.x == 0) load_weights();      /* the weight image of a prepared layer is a constant: it may load while the previous kernel of the stream is still running */
     if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), (uint32_t)a.tmem_cols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();                               /* the next kernel cannot take this block's tensor memory any more */
     const uint32_t tmem = uni(*tmem_slot);
     Piece piece = piece_of_block(a);
 
@@ -215,6 +214,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             if (lead) { tma_prefetch_desc(&map0); tma_prefetch_desc(&maps); }
             pdl_wait();      /* the only role that reads activations from global memory; every other role's data comes through this thread's loads,
                                 so the weight load, the B scale copies and the zeroing of the accumulators overlap the previous kernel */
+            if (a.w_dep && lead) load_weights();
             const uint32_t nt = (uint32_t)a.nt, bstep9 = 9u * 2u * 3u * nt;            /* B descriptor step of one input block: nine taps of two halves of 3 nt rows */
             const uint32_t b_lo0 = desc_lo(smem_u32(wsm), 3u * nt * 16u);
             const uint32_t idesc_b = (BITS == 8 ? idesc_mxf8(0, 0, 0) : idesc_mxf4(0, 0, 0)), ntn = (nt >> 3) << 17;
