@@ -29,6 +29,7 @@
    relay, warps 4-7 epilogue.  All waits are bounded as in conv_mx_k. */
 #include "conv_epi.cuh"
 #include "tc_ptx.cuh"
+#include "gather_win.cuh"
 #include <stdlib.h>
 #include <string.h>
 
@@ -389,13 +390,14 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     for (int ki = 0; ki < a.nki && ok; ki += ips) lay(off, MULTI ? min(ips, a.nki - ki) : 1, nullptr);
             }
         } else {
-            /* The window is 18 rows of 10 bytes (two of them for fp4): of each the three words that begin at its first byte, every one put together from the two aligned words
-               it lies in, and bytes outside the row cleared (scale byte 0, under zero codes).  A lane has GN words and asks for them two stages ahead of their use.  Byte by byte
+            /* The window (gather_win.cuh): every word is put together from the two aligned words it lies in, and bytes outside the volume are cleared (scale byte 0, under zero
+               codes).  A lane has GN words and asks for them two stages ahead of their use.  Byte by byte
                this warp was the slowest role in the 64-channel MX-fp4 tiles. */
             pdl_wait();
             Run rn; int zi = 1, zhi = 0, ki = 0; bool live = false; const uint8_t *base = nullptr;
-            unsigned keep[GN];                   /* the bytes of word k that lie in the volume */
+            unsigned keep[GN];                   /* the bytes of word k that are wanted */
             int offs[GN];
+            const uint8_t *end = a.x_sc + (size_t)a.N * a.nkb * a.D * a.H * a.W;
             const size_t S = (size_t)a.D * a.H * a.W;
 #pragma unroll
             for (int k = 0; k < GN; k++) { const int i = (32 * k + lane) % 54; offs[k] = (i / 3) * a.W + i % 3 * 4; }
@@ -407,13 +409,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int x0 = (rn.txy % a.tiles_x) * 8 - 1, y0 = (rn.txy / a.tiles_x) * 16 - 1;
                 base = a.x_sc + (ptrdiff_t)y0 * a.W + x0;
 #pragma unroll
-                for (int k = 0; k < GN; k++) {
-                    const int i = (32 * k + lane) % 54, y = y0 + i / 3, x = x0 + i % 3 * 4;
-                    keep[k] = 0u;
-#pragma unroll
-                    for (int t = 0; t < 4; t++) if (x + t >= 0 && x + t < a.W && i % 3 * 4 + t < 10) keep[k] |= 0xffu << (8 * t);
-                    if (32 * k + lane >= GB || y < 0 || y >= a.H) keep[k] = 0u;
-                }
+                for (int k = 0; k < GN; k++) keep[k] = 32 * k + lane < GB ? gather_keep((32 * k + lane) % 54, x0, y0, a.W, a.H) : 0u;
             };
             auto fetch = [&](unsigned *g) {
                 if (!live) return;
@@ -422,12 +418,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
 #pragma unroll
                 for (int k = 0; k < GN; k++) {
                     const bool second = 32 * k + lane >= 54;                     /* fp4: the window of the item's second block, which may not be there (zero weights) */
-                    const uint8_t *q = p + (second ? S : 0) + offs[k];
-                    const unsigned sh = (unsigned)(size_t)q & 3u, m = !second || two ? keep[k] : 0u;
-                    const unsigned *w = (const unsigned *)(q - sh);
-                    /* an aligned word is read only where it has a byte that is kept; put together in lay, when they have come */
-                    g[4 * k] = m << (8 * sh) ? ld_dep(w) : 0u; g[4 * k + 1] = sh && m >> (32 - 8 * sh) ? ld_dep(w + 1) : 0u;
-                    g[4 * k + 2] = 8 * sh; g[4 * k + 3] = m;
+                    gather_word(p + (second ? S : 0) + offs[k], !second || two ? keep[k] : 0u, end, g + 4 * k, [](auto *q) { return ld_dep(q); });      /* put together in lay, when they have come */
                 }
                 if (++ki == a.nki) { ki = 0; if (++zi > zhi) open(); }
             };
