@@ -24,8 +24,9 @@ struct EpiArgs {
 
 /* v: the 32 fp32 accumulators of GEMM row (n, z, oy, ox), 32-column block cb_g.  Adds the bias, rounds as the output mode asks (v keeps
    the values as stored, which is what the statistics are taken from) and writes the row if it lies inside the volume.  OWN: the block's 32 biases are
-   read from `own` instead, coherently (a bias that a kernel just ahead may have written does not go through the non-coherent path, which otherwise is the faster one: its
-   loads move ahead of the wait for the accumulators; 96 -> 96 in MX-fp4 on 40 x 44 x 45 29.2 us, 36.5 with coherent ones). */
+   read from `own` instead: the kernel's copy in shared memory (conv_mxr_k, conv_s2_k), or the layer's in memory by coherent loads (conv_mx_k, where a kernel just ahead may have written
+   them).  Without it they come through the non-coherent path, whose loads move ahead of the wait for the accumulators (96 -> 96 in MX-fp4 on 40 x 44 x 45 29.2 us, 36.5 with coherent
+   ones from memory). */
 template <bool OWN = false>
 __device__ __forceinline__ void epi_chunk(const EpiArgs &a, int n, int z, int oy, int ox, bool row_ok, int cb_g, float *v, const float *own = nullptr) {
     const size_t S = (size_t)a.D * a.H * a.W;

@@ -13,7 +13,7 @@
    consecutive, so the tile is re-read from L2, not from HBM.  Accumulators alternate between TMEM slots; the epilogue is the
    generic one (bias, fp16 / MX / plane-major output, the transposed conv's scatter).
 
-   Roles (384 threads): warp 0 lane 0 producer, warp 1 MMA issue (the warp runs the loop, an elected lane issues; it also allocates TMEM), warp 2 scale
+   Roles (384 threads): warp 0 producer and warp 1 MMA issue (the warp runs the loop, an elected lane issues; warp 1 also allocates TMEM), warp 2 scale
    layout, warp 3 idle, warps 4-11 epilogue (two groups, jobs in turn).  All waits are bounded as in conv_mx_k. */
 #include "conv_epi.cuh"
 #include "tc_ptx.cuh"

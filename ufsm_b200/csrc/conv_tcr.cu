@@ -18,8 +18,8 @@
    precomputed: TMEM addresses, the N field of the instruction descriptor, B descriptor and B scale addresses, the barriers to wait
    for; (2) the MMA warp's stage is three PTX blocks of three MMAs whose operands are a record field plus an immediate; (3)
    accumulators are never "fresh": the epilogue zeroes a slot after reading it, so every MMA accumulates; (4) the A scale factors are
-   gathered from a TMA-staged window in shared memory with no bounds logic (voxels outside the volume arrive as zero codes with scale
-   byte 0), as far ahead of the MMAs as the ring is deep, and copied to TMEM by the MMA warp (copies and MMAs of one thread run in issue order,
+   laid out from a window in shared memory (voxels outside the volume are zero codes with scale byte 0 in it): staged by TMA, or, where TMA does not take the
+   scale plane's rows, fetched by the scale warp itself with the bytes outside the volume masked (GATHER), as far ahead of the MMAs as the ring is deep, and copied to TMEM by the MMA warp (copies and MMAs of one thread run in issue order,
    so nothing guards the two buffers; copied by the gathering warps, which had to wait for the MMAs of two stages back, 64 -> 64 on 64^3 took
    26.8 us, 25.8 this way); (5) the MMA warp's single commit per stage lands on the stage's `empty` barrier; a relay passes the completion of
    output planes on to the epilogue's accumulator-full barriers; (6) two blocks share a multiprocessor when the weights are small enough: one
@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
         {
             const uint32_t lead = elect_one();
             if (lead) { tma_prefetch_desc(&map0); tma_prefetch_desc(&maps); }
-            pdl_wait();      /* the only role that reads activations from global memory; every other role's data comes through this thread's loads,
-                                so the weight load, the B scale copies and the zeroing of the accumulators overlap the previous kernel */
+            pdl_wait();      /* a prepared layer: the only role that reads what an earlier kernel wrote (GATHER: the scale warp reads the scale plane, behind a wait of its own); every
+                                other role's data comes through this warp's loads, so the weight load, the B scale copies and the zeroing of the accumulators overlap the previous
+                                kernel.  Weights that a kernel just ahead wrote (w_dep) load behind this wait, and the epilogue reads their bias behind its own */
             if (a.w_dep && lead) load_weights();
             const uint32_t nt = (uint32_t)a.nt, bstep9 = 9u * 2u * 3u * nt;            /* B descriptor step of one input block: nine taps of two halves of 3 nt rows */
             const uint32_t b_lo0 = desc_lo(smem_u32(wsm), 3u * nt * 16u);
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
         const size_t plane_b = (size_t)a.H * a.W * 64, row_b = (size_t)a.W * 64;
         /* sample being accumulated and the first sample this block has planes of.  Nothing is written to `part` before the block has taken a plane
            out of TMEM: this kernel may have been started while its predecessor in the stream, which can be a conv that shares `part`, was still
-           running, and only the producer waits for the predecessor; a plane in TMEM means that wait is over.  So the zero entries of the
+           running, and of a prepared layer only the producer waits for the predecessor; a plane in TMEM means that wait is over.  So the zero entries of the
            samples this block has no planes of are written at the end. */
         int n_cur = -1, n_first = -1;
         while (piece.u < piece.u1 && !dead) {
@@ -727,8 +728,8 @@ extern "C" int umx_wait_selftest(long long limit_clocks) {
     return 0;
 }
 
-/* geometry of the weight image; 0 when the z-marching kernel cannot run this conv (3^3 only, one column tile of at most 64 channels,
-   codes + scales resident in shared memory, B scales resident in TMEM beside at least four accumulator slots) */
+/* geometry of the weight image; 0 when the z-marching kernel cannot run this conv (3^3 only; a column tile's codes + scales resident in shared memory,
+   its B scales resident in TMEM beside at least four accumulator slots) */
 struct RGeo { int nt, ncol, w_codes, w_bytes, gt, goff1, goff2, tmem_cols, nslot, sfa_base, sfa_cols, sfb_base; };
 static int r_geometry_nt(const umx_conv *c, int nt, RGeo *g) {
     if (c->cop % nt) return 0;

@@ -7,7 +7,7 @@
    that turns the 2^3 stride-2 down conv into a 1^3 GEMM; the transposed conv is a GEMM to 8 Cout columns whose epilogue scatters
    and requantises straight into the other half of the concat tensor (xtconv_cat_q, src/nn_xnet.cu:1775-1789).  Every tensor's MX
    format is that of the conv that reads it; MX-fp8 tensors are kept in the split layout (two 16-byte planes per block).  All buffers are allocated once at
-   creation. */
+   creation, those of the queued host entry (two slots of patches and results, streams, events) at its first call. */
 #include "../../include/ufsm_mx.h"
 #include <math.h>
 #include <stdio.h>
