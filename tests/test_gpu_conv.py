@@ -71,20 +71,58 @@ def test_conv3_stride2_parity(dev, N, Ci, Co, D, H, W, bits):
     assert np.array_equal(got, run_pm32("conv3s2", mx, w, b, N, Ci, D, H, W, Co, bits, split=False))    # reference-layout input
 
 
-@pytest.mark.parametrize("N,Ci,Co,D,H,W", [
-    (1, 32, 32, 3, 19, 11),            # general kernel, ragged tiles
-    (2, 256, 128, 3, 16, 16),          # K split over a cluster
-    (2, 64, 96, 5, 18, 16),            # batch, three column tiles
-    (1, 32, 32, 40, 40, 45),           # z-marching kernel, gathered scale window
-    (1, 64, 64, 24, 48, 32),           # z-marching kernel, scale window by TMA
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,cap,kernel", [
+    (1, 32, 32, 3, 19, 11, 0, 0),      # general kernel, ragged tiles
+    (2, 256, 128, 3, 16, 16, 0, 0),    # K split over a cluster
+    (2, 64, 96, 5, 18, 16, 0, 1),      # batch, three column tiles, a plane a block
+    (1, 32, 32, 40, 40, 45, 0, 1),     # z-marching kernel, gathered scale window
+    (1, 64, 64, 24, 48, 32, 0, 1),     # z-marching kernel, scale window by TMA
+    (1, 64, 64, 12, 32, 32, 3, 1),     # two input items a stage
+    (2, 96, 32, 9, 24, 32, 2, 1),      # three
+    (1, 128, 64, 7, 20, 16, 1, 1),     # four, two column tiles
+    (1, 64, 64, 20, 30, 33, 2, 1),     # gathered scale window, 64-channel column tile
 ])
-def test_conv3_reads_the_reference_layout(dev, N, Ci, Co, D, H, W):
-    """MX-fp8 codes in 32-byte rows and in the split layout: the same products in the same order, the same bits."""
-    x = synth.rng(51).standard_normal(N * Ci * D * H * W).astype(np.float32)
+def test_conv3_reads_the_reference_layout(dev, N, Ci, Co, D, H, W, cap, kernel):
+    """MX-fp8 codes in 32-byte rows and in the split layout: the same products in the same order, the same bits; on exact operands the oracle's."""
+    S = D * H * W
     w, b = synth.kaiming(52, Co, Ci, 27), synth.bias(53, Co, 0.1)
-    mx = orc.pm_to_mx(x, 0, N, Ci, D * H * W, 8)
-    got = run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8, split=False)
-    assert np.isfinite(got).all() and np.array_equal(got, run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8))
+    mx = orc.pm_to_mx(synth.rng(51).standard_normal(N * Ci * S).astype(np.float32), 0, N, Ci, S, 8)
+    we = exact_operands(55, (Co, Ci, 27), 1)
+    mxe, want = orc.conv_case("conv3", exact_operands(54, (N, Ci, D, H, W), 1).reshape(-1), we, None, N, Ci, D, H, W, Co, 8)
+    dev.umx_conv_r_block_cap(cap)
+    try:
+        got = run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8, split=False)
+        assert dev.umx_conv_last_kernel() == kernel
+        split = run_pm32("conv3", mx, w, b, N, Ci, D, H, W, Co, 8)
+        assert dev.umx_conv_last_kernel() == kernel
+        gote = run_pm32("conv3", mxe, we, None, N, Ci, D, H, W, Co, 8, split=False)
+    finally:
+        dev.umx_conv_r_block_cap(0)
+    assert np.isfinite(got).all() and np.array_equal(got, split)
+    assert np.array_equal(gote, want), "%d of %d differ" % (np.count_nonzero(gote != want), want.size)
+
+
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,cap", [(1, 32, 32, 9, 19, 16, 3), (2, 64, 64, 5, 16, 32, 2), (1, 32, 64, 6, 16, 16, 0)])
+def test_epilogue_statistics_on_the_reference_layout(dev, N, Ci, Co, D, H, W, cap):
+    """umx_conv_fwd_norm with the sums in the epilogue, on MX-fp8 codes in 32-byte rows: halves and coefficients of the split layout's, and the oracle's coefficients."""
+    import ctypes as C
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S = D * H * W
+    mx = orc.pm_to_mx(synth.rng(56).standard_normal(N * Ci * S).astype(np.float32), 0, N, Ci, S, 8)
+    c = G.Conv("conv3", synth.kaiming(57, Co, Ci, 27), synth.bias(58, Co, 0.1), Co, Ci, 8)
+    xd, yd, pd, cd = DevBuf(data=mx), DevBuf(N * Co * S * 2).fill(0xEE), DevBuf(dev.umx_stats_doubles(N, Co, D, H, W) * 8).fill(0xEE), DevBuf(N * Co * 8).fill(0xEE)
+    dev.umx_conv_r_block_cap(cap)
+    try:
+        want, coef = c.fwd_norm(mx, N, D, H, W, epilogue_stats=True)
+        assert dev.umx_conv_fwd_norm(c.h, xd.ptr, N, D, H, W, yd.ptr, pd.ptr, None, None, C.c_float(1e-5), cd.ptr, 4) == 0
+        assert dev.umx_conv_last_kernel() == 1
+        ufsm_b200.check()
+    finally:
+        dev.umx_conv_r_block_cap(0)
+    c.free()
+    assert np.array_equal(yd.download(np.uint16), want.view(np.uint16)) and np.array_equal(cd.download(np.float32), coef)
+    assert np.array_equal(coef, orc.in_coef(orc.in_sums(want.astype(np.float32), N, Co, S), N, Co, S))
 
 
 @pytest.mark.parametrize("bits", [8, 4])
@@ -606,33 +644,48 @@ def test_weights_without_a_key_may_change_between_calls(dev):
         assert np.array_equal(g.download(), wnt)
 
 
-@pytest.mark.parametrize("bits,Ci,Co", [(8, 32, 32), (4, 64, 96), (8, 96, 160)])
-def test_weights_written_by_the_kernel_before(dev, bits, Ci, Co):
+@pytest.mark.parametrize("kind,bits,Ci,Co,D,H,W,cap,kernel", [
+    ("conv3", 8, 32, 32, 2, 8, 16, 0, 1), ("conv3", 4, 64, 96, 2, 8, 16, 0, 1), ("conv3", 8, 96, 160, 2, 8, 16, 0, 1),
+    ("conv3", 8, 256, 128, 2, 8, 16, 0, 0), ("conv3", 4, 256, 256, 3, 8, 8, 0, 0),        # general kernel, K split
+    ("conv3", 8, 32, 32, 9, 18, 13, 2, 1), ("conv3", 4, 64, 64, 9, 18, 13, 2, 1),         # gathered scale window
+    ("conv3s2", 8, 32, 64, 5, 17, 16, 0, 4), ("conv3s2", 4, 64, 96, 6, 16, 18, 0, 4)])
+def test_weights_written_by_the_kernel_before(dev, kind, bits, Ci, Co, D, H, W, cap, kernel):
     """a conv without split_t.wkey whose weights and bias another kernel of the library (lp_mx8_to_f32, which lets its successor start early) has just
     written: eight sets in one buffer, queued without a wait, against handles made from the same values"""
     import ufsm_b200
     from ufsm_b200 import DevBuf, Shape5, Gnp, Split
-    D, H, W, n, r = 2, 8, 16, Ci * 27, synth.rng(701)
-    S = D * H * W
+    n, r = Ci * 27, synth.rng(701)
+    S, So, s2 = D * H * W, D * H * W, kind == "conv3s2"
+    if s2:
+        So = ((D + 1) // 2) * ((H + 1) // 2) * ((W + 1) // 2)
     codes = r.integers(0, 256, (8, Co * n), dtype=np.uint8)
     codes[(codes & 0x7f) == 0x7f] = 0                        # no NaN codes
     sets = [DevBuf(data=np.concatenate([c, r.integers(122, 126, Co // 32 * n, dtype=np.uint8)])) for c in codes]
     bcodes = [DevBuf(data=np.concatenate([r.integers(0, 120, Co, dtype=np.uint8), np.full(Co // 32, 120, np.uint8)])) for _ in codes]
     mx = orc.pm_to_mx(synth.act_h16(702, Ci * S), 2, 1, Ci, S, bits, 32)
     xd, wd, bd = DevBuf(data=mx), DevBuf(Co * n * 4).fill(0), DevBuf(Co * 4).fill(0)
-    ys = [DevBuf(Co * S * 2).fill(0xEE) for _ in codes]
+    ys = [DevBuf(Co * So * 2).fill(0xEE) for _ in codes]
     fn = dev.lp_conv_fwd_f8 if bits == 8 else dev.lp_conv_fwd_f4
+    xdt = 3 if bits == 8 else 4
     ufsm_b200.check()
-    for s, t, y in zip(sets, bcodes, ys):
-        dev.lp_mx8_to_f32(t.ptr, 1, Co, 1, bd.ptr)
-        dev.lp_mx8_to_f32(s.ptr, 1, Co, n, wd.ptr)
-        fn(xd.ptr, 3 if bits == 8 else 4, Shape5(1, Ci, D, H, W), wd.ptr, bd.ptr, Co, y.ptr, 2, Gnp(), None, 0, Split())
-    ufsm_b200.check()
+    dev.umx_conv_r_block_cap(cap)
+    try:
+        for s, t, y in zip(sets, bcodes, ys):
+            dev.lp_mx8_to_f32(t.ptr, 1, Co, 1, bd.ptr)
+            dev.lp_mx8_to_f32(s.ptr, 1, Co, n, wd.ptr)
+            if s2:
+                dev.lp_conv_fwd_s2_f8(xd.ptr, xdt, Shape5(1, Ci, D, H, W), wd.ptr, bd.ptr, Co, y.ptr, 2, Shape5(1, Co, (D + 1) // 2, (H + 1) // 2, (W + 1) // 2), Gnp())
+            else:
+                fn(xd.ptr, xdt, Shape5(1, Ci, D, H, W), wd.ptr, bd.ptr, Co, y.ptr, 2, Gnp(), None, 0, Split())
+            assert dev.umx_conv_last_kernel() == kernel
+        ufsm_b200.check()
+    finally:
+        dev.umx_conv_r_block_cap(0)
     for s, t, y in zip(sets, bcodes, ys):
         dev.lp_mx8_to_f32(t.ptr, 1, Co, 1, bd.ptr)
         dev.lp_mx8_to_f32(s.ptr, 1, Co, n, wd.ptr)
         ufsm_b200.check()
-        c = G.Conv("conv3", wd.download(np.float32), bd.download(np.float32), Co, Ci, bits)
+        c = G.Conv(kind, wd.download(np.float32), bd.download(np.float32), Co, Ci, bits)
         assert np.array_equal(y.download(), c.fwd(mx, 1, D, H, W, G.OUT_PM16)[0])
         c.free()
 

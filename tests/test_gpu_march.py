@@ -111,8 +111,9 @@ def test_small_grids_in_few_blocks(dev, N, Ci, Co, D, H, W, cap, bits):
         assert np.array_equal(y_free.view(np.uint16), y.view(np.uint16)) and np.array_equal(coef, coef_free)
 
 
-@pytest.mark.parametrize("N,Ci,Co,D,H,W,bits", [(1, 32, 32, 3, 16, 16, 8), (2, 32, 24, 4, 19, 16, 8), (1, 64, 64, 3, 9, 48, 8), (1, 32, 96, 5, 16, 32, 4), (1, 64, 33, 12, 5, 16, 8), (1, 32, 1, 2, 16, 16, 8)])
-def test_plane_major_halves(dev, N, Ci, Co, D, H, W, bits):
+@pytest.mark.parametrize("N,Ci,Co,D,H,W,bits,cap", [(1, 32, 32, 3, 16, 16, 8, 0), (2, 32, 24, 4, 19, 16, 8, 0), (1, 64, 64, 3, 9, 48, 8, 0), (1, 32, 96, 5, 16, 32, 4, 0), (1, 64, 33, 12, 5, 16, 8, 0), (1, 32, 1, 2, 16, 16, 8, 0),
+                                                    (1, 128, 64, 6, 20, 16, 8, 1)])       # a stage of three of the four input items, then one of the fourth (blocked halves leave room for all four)
+def test_plane_major_halves(dev, N, Ci, Co, D, H, W, bits, cap):
     """the plane-major fp16 epilogue: the values of the blocked fp16 one, at partial tiles, channel counts that end inside a block or a pair, one and several
     column tiles; an output that is not on a 16-byte boundary takes the general epilogue"""
     import ufsm_b200
@@ -123,7 +124,12 @@ def test_plane_major_halves(dev, N, Ci, Co, D, H, W, bits):
 
     def run(nbytes, shift, mode):
         y = DevBuf(data=np.full(nbytes + shift, 0x5a, np.uint8))
-        assert dev.umx_conv_fwd(c.h, x.ptr, N, D, H, W, y.ptr + shift, mode, 0, 0, 0, None, 1) == 0
+        dev.umx_conv_r_block_cap(cap)
+        try:
+            assert dev.umx_conv_fwd(c.h, x.ptr, N, D, H, W, y.ptr + shift, mode, 0, 0, 0, None, 1) == 0
+        finally:
+            dev.umx_conv_r_block_cap(0)
+        assert dev.umx_conv_last_kernel() == 1
         ufsm_b200.check()
         return y.download()[shift:].copy().view(np.uint16)
     want = run(N * nbo * S * 64, 0, 0).reshape(N, nbo, S, 32).transpose(0, 1, 3, 2).reshape(N, nbo * 32, S)[:, :Co]
@@ -160,11 +166,16 @@ def test_stride2_runs_and_wraps(dev, N, Ci, Co, D, H, W, cap, bits):
     (1, 96, 32, 9, 18, 35, 2),         # three input blocks: in MX-fp4 the second item's second block is not there
     (2, 32, 64, 40, 5, 3, 1),          # a grid narrower than a tile
     (1, 1, 32, 20, 16, 30, 1),         # even width, one channel
+    (1, 64, 64, 11, 19, 24, 2),        # whole tile rows: the plane-major epilogue's wide stores behind a gathered window
+    (1, 32, 33, 7, 16, 40, 1),
 ])
 def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
     """Scale planes whose rows are not multiples of 16 bytes: the scale warp gathers its window.  Random operands within 1e-3 of the oracle (the order of the fp32 sums is the only
-    freedom), exact operands the oracle's bits; fp16 plane-major and MX outputs equal to those of the fp32 output."""
-    S = D * H * W
+    freedom), exact operands the oracle's bits; fp16 plane-major, blocked fp16 and MX outputs equal to those of the fp32 output, with nothing written behind the tensor (blocked halves
+    of several MX-fp8 items are the general kernel's, on exact operands the same)."""
+    import ufsm_b200
+    from ufsm_b200 import DevBuf
+    S, nbo = D * H * W, (Co + 31) // 32
     x = synth.rng(341).standard_normal(N * Ci * S).astype(np.float32) * np.exp2(synth.rng(344).integers(-6, 7, N * Ci * S)).astype(np.float32)
     w, b = synth.kaiming(342, Co, Ci, 27), synth.bias(343, Co, 0.1)
     mx, want = orc.conv_case("conv3", x, w, b, N, Ci, D, H, W, Co, bits)
@@ -180,8 +191,22 @@ def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
         q, _ = c.fwd(mx, N, D, H, W, G.OUT_MXRAW, 8)
         assert dev.umx_conv_last_kernel() == 1
         c.free()
+        blocked = []
+        for w_, b_, m_ in ((w, b, mx), (we, None, mxe)):
+            c = G.Conv("conv3", w_, b_, Co, Ci, bits)
+            xd, yd = DevBuf(data=G.to_split(m_, N, (Ci + 31) // 32 * 32, S, bits)), DevBuf(N * nbo * S * 64 + 256).fill(0x5a)
+            assert dev.umx_conv_fwd(c.h, xd.ptr, N, D, H, W, yd.ptr, G.OUT_H16B, 0, 0, 0, None, 3) == 0
+            ufsm_b200.check()
+            assert dev.umx_conv_last_kernel() == (0 if bits == 8 and Ci > 32 else 1)
+            c.free()
+            raw = yd.download()
+            assert (raw[N * nbo * S * 64:] == 0x5a).all()
+            blocked.append(raw[:N * nbo * S * 64].view(np.float16))
     finally:
         dev.umx_conv_r_block_cap(0)
+    if not (bits == 8 and Ci > 32):
+        assert np.array_equal(blocked[0], orc.pm_to_blocked(got, N, Co, S).astype(np.float16))
+    assert np.array_equal(blocked[1], orc.pm_to_blocked(wante, N, Co, S).astype(np.float16))
     e = orc.rel_l2(got, want)
     assert np.isfinite(got).all() and e < TOL, "relative L2 %.3g" % e
     assert np.array_equal(gote, wante), "%d of %d differ" % (np.count_nonzero(gote != wante), wante.size)
@@ -236,11 +261,20 @@ def test_a_batch_may_take_the_other_kernel(dev, N, Ci, Co, D, H, W, bits, kernel
 
 @pytest.mark.parametrize("Ci,bits,kernel", [(64, 8, 0), (32, 8, 1), (64, 4, 1)])
 def test_network_layers_keep_their_order_of_sums(dev, Ci, bits, kernel):
-    """Rows that TMA does not take, blocked halves out (a network's layer): several MX-fp8 input items are added item by item, by the general kernel, at every size."""
-    N, Co, D, H, W = 1, 32, 40, 64, 40
-    S = D * H * W
-    x = synth.rng(371).standard_normal(N * Ci * S).astype(np.float32)
-    c = G.Conv("conv3", synth.kaiming(372, Co, Ci, 27), synth.bias(373, Co, 0.1), Co, Ci, bits)
-    y, _ = c.fwd(orc.pm_to_mx(x, 0, N, Ci, S, bits, 32), N, D, H, W, G.OUT_H16B)
-    assert dev.umx_conv_last_kernel() == kernel and np.isfinite(y.view(np.float16)).all()
+    """Rows that TMA does not take, blocked halves out (a network's layer): several MX-fp8 input items are added item by item, by the general kernel, at every size.  The planes that a
+    volume of the first six has in common with the whole one have its bits, although the general kernel takes the small one in every case; and the halves are the oracle's."""
+    N, Co, D, H, W, d = 1, 32, 40, 64, 40, 6
+    S, s = D * H * W, d * H * W
+    x = synth.rng(371).standard_normal(N * Ci * S).astype(np.float32) * np.exp2(synth.rng(374).integers(-6, 7, N * Ci * S)).astype(np.float32)
+    w, b = synth.kaiming(372, Co, Ci, 27), synth.bias(373, Co, 0.1)
+    c = G.Conv("conv3", w, b, Co, Ci, bits)
+    mx, want = orc.conv_case("conv3", x, w, b, N, Ci, D, H, W, Co, bits)
+    y, _ = c.fwd(mx, N, D, H, W, G.OUT_H16B)
+    assert dev.umx_conv_last_kernel() == kernel
+    z, _ = c.fwd(orc.pm_to_mx(np.ascontiguousarray(x.reshape(Ci, S)[:, :s]).reshape(-1), 0, N, Ci, s, bits, 32), N, d, H, W, G.OUT_H16B)
+    assert dev.umx_conv_last_kernel() == 0
     c.free()
+    y, z, same = y.view(np.float16), z.view(np.float16), (d - 1) * H * W * 32
+    assert np.array_equal(y[:same], z[:same])
+    e = orc.rel_l2(y.astype(np.float32), orc.pm_to_blocked(want, N, Co, S))
+    assert np.isfinite(y).all() and e < TOL, "relative L2 %.3g" % e
