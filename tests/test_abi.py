@@ -3,8 +3,11 @@ reference's sizes, the host-only scheduler logic is right, and compute entries f
 import ctypes as C
 import os
 import re
+import shutil
+import subprocess
 
 import numpy as np
+import pytest
 
 import ufsm_b200
 from ufsm_b200 import _lib
@@ -41,6 +44,15 @@ def test_kernels_hold_their_tensor_memory_before_a_successor_may_start():
                 assert body.index("pdl_trigger()") > at, "%s: %s" % (f, body[:120])
                 seen += 1
     assert seen == 5
+
+
+def test_no_object_holds_more_than_a_form_of_the_z_marching_conv():
+    """A process loads an object's kernels as a whole when it first launches one of them: all 24 instances in one made its first 3^3 conv take 10.6 ms."""
+    objs = [os.path.join(ROOT, "build", f) for f in os.listdir(os.path.join(ROOT, "build")) if f.endswith(".cu.o")] if os.path.isdir(os.path.join(ROOT, "build")) else []
+    if not objs or shutil.which("nm") is None:
+        pytest.skip("the objects of the build are not here")
+    counts = [len(re.findall(r"\bconv_mxr_k<", subprocess.run(["nm", "-C", o], stdout=subprocess.PIPE, text=True).stdout)) for o in objs]
+    assert max(counts) <= 6 and sum(counts) >= 24
 
 
 def test_struct_sizes_match_the_reference():
