@@ -170,6 +170,7 @@ def test_stride2_runs_and_wraps(dev, N, Ci, Co, D, H, W, cap, bits):
     (1, 32, 33, 7, 16, 40, 1),
     (1, 64, 32, 7, 17, 13, 2),         # scale bytes that end inside a word, in MX-fp4 of an item with both blocks
     (1, 64, 32, 24, 1, 5, 2),          # planes of a few voxels
+    (1, 64, 32, 25, 1, 2, 2),
 ])
 def test_widths_that_tma_does_not_take(dev, N, Ci, Co, D, H, W, cap, bits):
     """Scale planes whose rows are not multiples of 16 bytes: the scale warp gathers its window.  Random operands within 1e-3 of the oracle (the order of the fp32 sums is the only

@@ -73,7 +73,6 @@ static int r_plan(const umx_conv *c, const uint8_t *x_sc, int N, int D, int H, i
     RGeo g;
     if (!r_geometry(c, &g)) return 0;
     a.gather = (W & 15) || ((size_t)x_sc & 15);      /* TMA takes the scale plane only in rows that are multiples of 16 bytes */
-    if (a.gather && (long long)H * W < 4) return 0;  /* a word of the gathered window holds voxels of two planes at most */
     a.w_codes = g.w_codes; a.w_bytes = g.w_bytes; a.gt = g.gt; a.goff1 = g.goff1 * 4; a.goff2 = g.goff2 * 4;   /* TMEM column offsets of the dz >= 1, 2 images */
     a.tmem_cols = g.tmem_cols; a.nslot = g.nslot; a.sfa_base = g.sfa_base; a.sfa_cols = g.sfa_cols; a.sfb_base = g.sfb_base;
     a.N = N; a.D = D; a.H = H; a.W = W; a.nkb = c->nkb; a.nki = c->nki; a.bits = c->bits; a.nt = g.nt; a.ncol = g.ncol;
@@ -159,8 +158,8 @@ int umx_conv_fwd_r(const umx_conv *c, const uint8_t *x_sc, const CUtensorMap *m0
     a.wr = c->wr; a.x_sc = x_sc; a.w_dep = c->w_src != nullptr; a.e = e; a.err = umx_errflag();
     if (!a.err) return -1;
     const size_t smem = (size_t)a.off_ring + (size_t)a.ring * a.stage_bytes;
-    static const conv_r_fn *const ks[4] = {umx_conv_r_one, umx_conv_r_stats, umx_conv_r_gather, umx_conv_r_multi};
-    const int form = coef ? 1 : a.gather ? 2 : a.ips > 1 ? 3 : 0, variant = (ref ? 4 : c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
+    static const conv_r_fn *const ks[5] = {umx_conv_r_one, umx_conv_r_stats, umx_conv_r_gather, umx_conv_r_multi, umx_conv_r_ends};
+    const int form = coef ? 1 : a.gather ? (gather_ends(N, c->nkb, D, H, W) ? 4 : 2) : a.ips > 1 ? 3 : 0, variant = (ref ? 4 : c->bits == 8 ? 0 : 2) | (a.nt == 32 ? 0 : 1);
     /* the attribute loads the form's kernels (1.3 ms) the first time: only when one is launched */
     static unsigned attr_set[16];
     const unsigned bit = 1u << (6 * form + variant);

@@ -33,6 +33,7 @@
 #include "gather_win.cuh"
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 
 
 #define UMX_STR_(x) #x
@@ -76,11 +77,11 @@ struct ConvRArgs {
     EpiArgs e;
     int *err;
 };
-/* The instances come in four forms, each in a source file of its own with a table of six: MX-fp8 and MX-fp4 with 32- and 64-channel column tiles, MX-fp8 in the reference's layout with
-   either.  A process loads a source file's kernels as a whole, unpacked, when it first launches one of them, and should not pay for forms it does not use: with all 24 in one
+/* The instances come in five forms, each in a source file of its own with a table of six: MX-fp8 and MX-fp4 with 32- and 64-channel column tiles, MX-fp8 in the reference's layout with
+   either.  A process loads a source file's kernels as a whole, unpacked, when it first launches one of them, and should not pay for forms it does not use: with all (24 then) in one
    the first 3^3 conv of a process took 10.6 ms and the first forward of the network on 128^3 17 ms; 1.5 (and 1.3 where it meets a second form) and 8.9 this way. */
 typedef void (*conv_r_fn)(const CUtensorMap, const CUtensorMap, const ConvRArgs);
-extern const conv_r_fn umx_conv_r_one[6], umx_conv_r_stats[6], umx_conv_r_gather[6], umx_conv_r_multi[6];
+extern const conv_r_fn umx_conv_r_one[6], umx_conv_r_stats[6], umx_conv_r_gather[6], umx_conv_r_ends[6], umx_conv_r_multi[6];
 #define UMX_R_FORM(ST, GA, MU) {conv_mxr_k<8, 1, ST, GA, MU>, conv_mxr_k<8, 2, ST, GA, MU>, conv_mxr_k<4, 1, ST, GA, MU>, conv_mxr_k<4, 2, ST, GA, MU>, conv_mxr_k<8, 1, ST, GA, MU, true>, conv_mxr_k<8, 2, ST, GA, MU, true>}
 
 namespace {
@@ -171,10 +172,10 @@ __device__ unsigned g_conv_tickets[64];      /* one per column tile; the block t
 
 /* NCH: 32-channel chunks of the column tile (1: two blocks per multiprocessor and at most 128 registers; 2: one block, more registers);
    STATS: the epilogue also takes the InstanceNorm sums; GATHER: the scale warp fetches its window of scale bytes itself, for scale planes whose rows TMA does not
-   take (W not a multiple of 16); MULTI: a stage holds up to a.ips input items of its plane (see r_plan), else one; REF:
+   take (W not a multiple of 16), 2: of a tensor that ends inside a word (gather_win.cuh); MULTI: a stage holds up to a.ips input items of its plane (see r_plan), else one; REF:
    MX-fp8 codes in the reference's layout (32-byte rows): a half of a row a load, the halves 2944 bytes apart in a stage (as a branch on an argument it cost the split layout 1.3 % on
    32 -> 32, 64^3) */
-template <int BITS, int NCH, bool STATS, bool GATHER, bool MULTI, bool REF = false>
+template <int BITS, int NCH, bool STATS, int GATHER, bool MULTI, bool REF = false>
 __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap maps, const ConvRArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint64_t *bars = (uint64_t *)smem_raw;
@@ -345,8 +346,8 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
            dx of a row are neighbours, so two words and a funnel shift fetch them.  The warp lays the nine shifted scale sets out in shared
            memory in the tcgen05.cp layout, as far ahead of the MMAs as the ring is deep. */
         int it = 0, s = 0, ph = 0; bool ok = true;
-        /* one stage: window -> scale sets; off: this lane's first byte of the window, gw: the window's bytes (GATHER), last: those of one word that came apart */
-        auto lay = [&](int off, int nit, const unsigned *gw, uint2 last) {
+        /* one stage: window -> scale sets; off: this lane's first byte of the window, gw: the window's bytes (GATHER) */
+        auto lay = [&](int off, int nit, const unsigned *gw) {
             if (!__all_sync(0xffffffffu, mbar_wait(bar_tma + 8 * s, ph, abort_flag, kWaitLimitR))) { if (lane == 0) raise_r(a, abort_flag, 4, it, 8 * s, ph); ok = false; return; }
             uint8_t *stg = stages + (size_t)s * a.stage_bytes;
             for (int i = 0; i < (MULTI ? nit : 1); i++, stg += a.item_bytes) {
@@ -356,7 +357,6 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                     const int i = 32 * k + lane;
                     if (i < GB) *(unsigned *)(stg + a.offSW + win_at(i)) = __funnelshift_r(gw[4 * k], gw[4 * k + 1], gw[4 * k + 2]) & gw[4 * k + 3];
                 }
-                if (last.x) *(unsigned *)(stg + a.offSW + win_at((int)(last.x & 3u) * 32 + lane)) |= last.y;
                 __syncwarp();
             }
             const int sh = (off & 3) * 8;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 const int zlo = max(0, rn.zb - 1), zhi = min(a.D - 1, rn.ze);
                 const int off = off0 + (x0 - 1) - (((x0 - 1) >> 4) << 4);
                 for (int zi = zlo; zi <= zhi && ok; zi++)
-                    for (int ki = 0; ki < a.nki && ok; ki += ips) lay(off, MULTI ? min(ips, a.nki - ki) : 1, nullptr, make_uint2(0u, 0u));
+                    for (int ki = 0; ki < a.nki && ok; ki += ips) lay(off, MULTI ? min(ips, a.nki - ki) : 1, nullptr);
             }
         } else {
             /* The window (gather_win.cuh): every word is put together from the two aligned words it lies in, and bytes outside the volume are cleared (scale byte 0, under zero
@@ -406,16 +406,9 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
             Run rn; int zi = 1, zhi = 0, ki = 0; bool live = false; const uint8_t *base = nullptr;
             unsigned keep[GN];                   /* the bytes of word k that are wanted */
             int offs[GN];
-            int x0 = 0, y0 = 0, last_z = -1;     /* the run's window; the last sample: its last plane, when bytes come apart */
-            unsigned apart = 0u;                 /* those of the coming stage that this lane puts in: the word's number k in bits 0 and 1, bit 2, the bytes in `apart_w` */
-            unsigned apart_w = 0u;
+            const uint8_t *end = a.x_sc + (size_t)a.N * a.nkb * a.D * a.H * a.W;
+            int tail_z = 0;
             const size_t S = (size_t)a.D * a.H * a.W;
-            const int rest = gather_rest(a.N, a.nkb, a.D, a.H, a.W);
-            /* not put together before they are used: where this warp waited for them, at the start or in their stage, a launch took 1 to 3 us longer */
-            uint32_t rest_b[3];
-#pragma unroll
-            for (int t = 0; t < 3; t++) rest_b[t] = t < rest ? ld_dep(a.x_sc + (size_t)a.N * a.nkb * S - rest + t) : 0u;
-            const int w_last = BITS == 4 && !(a.nkb & 1) ? 54 : 0;               /* first word of the last block's window */
 #pragma unroll
             for (int k = 0; k < GN; k++) { const int i = (32 * k + lane) % 54; offs[k] = (i / 3) * a.W + i % 3 * 4; }
             auto open = [&]() {
@@ -423,49 +416,35 @@ __global__ void __launch_bounds__(kThreadsR, NCH == 1 ? 2 : 1) conv_mxr_k(const 
                 if (!live) return;
                 rn = next_run(a, piece);
                 zi = max(0, rn.zb - 1); zhi = min(a.D - 1, rn.ze); ki = 0;
-                x0 = (rn.txy % a.tiles_x) * 8 - 1; y0 = (rn.txy / a.tiles_x) * 16 - 1;
+                const int x0 = (rn.txy % a.tiles_x) * 8 - 1, y0 = (rn.txy / a.tiles_x) * 16 - 1;
                 base = a.x_sc + (ptrdiff_t)y0 * a.W + x0;
-                last_z = rest && rn.n == a.N - 1 ? a.D - 1 : -1;
-            };
-            auto masks = [&](bool last) {
-                apart = 0u;
+                if (GATHER == 2) tail_z = gather_tail(rn.n, a.N, a.D, a.H, a.W);
 #pragma unroll
-                for (int k = 0; k < GN; k++) {
-                    const int i = 32 * k + lane;
-                    const bool l = last && i / 54 * 54 == w_last;
-                    keep[k] = i < GB ? gather_keep(i % 54, x0, y0, a.W, a.H, l ? a.H * a.W - rest : a.H * a.W) : 0u;
-                    if (l && i < GB) { bool has; const uint32_t w = gather_last(i % 54, x0, y0, a.W, a.H, rest, rest_b[0] | rest_b[1] << 8 | rest_b[2] << 16, &has); if (has) { apart = 4u | (unsigned)k; apart_w = w; } }
-                }
+                for (int k = 0; k < GN; k++) keep[k] = 32 * k + lane < GB ? gather_keep((32 * k + lane) % 54, x0, y0, a.W, a.H) : 0u;
             };
-            auto fetch = [&](unsigned *g, uint2 &last) {
-                last = make_uint2(apart, apart_w);
+            auto fetch = [&](unsigned *g) {
                 if (!live) return;
                 const uint8_t *p = base + ((size_t)rn.n * a.nkb + (BITS == 8 ? ki : 2 * ki)) * S + (size_t)zi * a.H * a.W;
                 const bool two = BITS == 4 && 2 * ki + 1 < a.nkb;
+                /* fp4: words of the item's second block, which may not be there (zero weights); put together in lay, when they have come */
+                auto words = [&](auto tail) {
 #pragma unroll
-                for (int k = 0; k < GN; k++) {
-                    const bool second = 32 * k + lane >= 54;                     /* fp4: the window of the item's second block, which may not be there (zero weights) */
-                    gather_word(p + (second ? S : 0) + offs[k], !second || two ? keep[k] : 0u, g + 4 * k, [](auto *q) { return ld_dep(q); });      /* put together in lay, when they have come */
-                }
-                bool fresh = false;
-                if (++ki == a.nki) { ki = 0; if (++zi > zhi) { open(); fresh = live; } }
-                const bool at_last = zi == last_z && ki == a.nki - 1;
-                if (fresh || at_last) masks(at_last);
+                    for (int k = 0; k < GN; k++) {
+                        const bool second = 32 * k + lane >= 54;
+                        gather_word<decltype(tail)::value>(p + (second ? S : 0) + offs[k], !second || two ? keep[k] : 0u, end, g + 4 * k, [](auto *q) { return ld_dep(q); });
+                    }
+                };
+                if (GATHER == 1 || zi < tail_z) words(std::false_type()); else words(std::true_type());
+                if (++ki == a.nki) { ki = 0; if (++zi > zhi) open(); }
             };
             unsigned g0[4 * GN], g1[4 * GN];
-            uint2 a0, a1;
             open();
-            if (live) masks(zi == last_z && a.nki == 1);
-            bool l0 = live, l1; fetch(g0, a0);
-            for (;;) {
-                l1 = live; fetch(g1, a1);
-                if (!l0) break;
-                lay(off0, 1, g0, a0);
-                if (!ok) break;
-                l0 = live; fetch(g0, a0);
-                if (!l1) break;
-                lay(off0, 1, g1, a1);
-                if (!ok) break;
+            bool l0 = live; fetch(g0);
+            bool l1 = live; fetch(g1);
+            while (ok && l0) {
+                lay(off0, 1, g0); l0 = live; fetch(g0);
+                if (!ok || !l1) break;
+                lay(off0, 1, g1); l1 = live; fetch(g1);
             }
         }
     } else if (warp == 3) {
